@@ -45,7 +45,10 @@ struct DevBuf {
             return e;
         }
         cap = want;
-        if (zero) e = cudaMemset(p, 0, want * sizeof(T));
+        if (zero) {  // complete before a context's own (non-blocking) stream uses it
+            e = cudaMemset(p, 0, want * sizeof(T));
+            if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+        }
         return e;
     }
     void release() {
@@ -80,26 +83,25 @@ struct orb_ctx {
     DevBuf<uint32_t> idx;
     DevBuf<orb_cell_t> heap;
     DevBuf<uint2> ranges;
-    DevBuf<uint32_t> tile_off, hist_off, below, inb, part_s, part_i, part_le, out_counts;
+    DevBuf<uint32_t> tile_off, hist_off, hdone, below, inb, part_done, out_counts;
+    DevBuf<CellPart> part;
+    DevBuf<uint2> swap_list;
     DevBuf<uint32_t> htile_cell, ptile_cell;
-    // test hooks (orb_test_set_scan_wait): polls of a look-back wait, and the value the
-    // tile scan's block ticket starts from (0 normally; 1 leaves the first block's status
-    // unpublished, so its successor's wait runs out)
-    uint32_t spin_limit = kLookbackSpinLimit;
-    uint32_t scan_ticket_start = 0;
+    // test hook (orb_test_set_scan_wait): what the arrivals of a cell's partition tiles start
+    // from below zero (0 normally; otherwise the last arrival never comes)
+    uint32_t done_offset = 0;
     // launch tuning (orb_set_tuning / orb_autotune_batch); cta_min_cells = 0 means never
     orb_tuning tune = {(uint32_t)kHistBlocksPerSm, 8u, (uint32_t)kTileBlocksPerSm, 64u, 0u, 4u, 0u};
-    DevBuf<uint8_t> hist_k, state, iters, listed, cmp_bad;
-    DevBuf<uint32_t> cmp_off, cmp_cnt, pred;
+    DevBuf<uint8_t> state, iters;
+    DevBuf<uint32_t> cmp_off, cmp_cnt, cmp_pos, pred;
     DevBuf<float> cmp_keys;
     DevBuf<uint32_t> hist;
     DevBuf<uint32_t> ptile_off, ge_bits, le_bits, pt_ge, pt_le, pt_ge_pre, pt_le_pre;
-    DevBuf<unsigned long long> pt_status;
     DevBuf<int> slots;
     DevBuf<BuildCounters> counters;
     DevBuf<orb_cell_t> staging;
     DevBuf<BatchRoot> batch_roots;
-    DevBuf<int> batch_slots;
+    DevBuf<int> batch_slots, batch_child;
     DevBuf<float> tune_src[3], tune_work[3];  // autotuner: input copy, build arrays
     DevBuf<float2> hint;      // warm builds: starting bracket per heap slot
     DevBuf<int> hint_axis;
@@ -178,7 +180,10 @@ bool is_device_ptr(const void *p) {
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
-orb_status ensure_ptile_buffers(orb_ctx *ctx, uint64_t ptiles) {
+// Levels of at most this many cells per SM send every cell through the count passes.
+constexpr int kCountCells = 1;
+
+orb_status ensure_ptile_buffers(orb_ctx *ctx, uint64_t ptiles, uint64_t cells) {
     ORB_CUDA(ctx->ptile_cell.ensure(ptiles));
     ORB_CUDA(ctx->ge_bits.ensure(ptiles * kPWords));
     ORB_CUDA(ctx->le_bits.ensure(ptiles * kPWords));
@@ -186,40 +191,42 @@ orb_status ensure_ptile_buffers(orb_ctx *ctx, uint64_t ptiles) {
     ORB_CUDA(ctx->pt_le.ensure(ptiles));
     ORB_CUDA(ctx->pt_ge_pre.ensure(ptiles + 1));
     ORB_CUDA(ctx->pt_le_pre.ensure(ptiles + 1));
-    ORB_CUDA(ctx->pt_status.ensure(ptiles + 1));
+    ORB_CUDA(ctx->swap_list.ensure(ptiles + cells));  // left tiles, or one empty item a cell
     return ORB_OK;
 }
 
 // Level buffers for up to `max_cells` cells per level over n particles.
 orb_status ensure_level_buffers(orb_ctx *ctx, uint64_t n, uint32_t max_cells, uint32_t heap_cells) {
     const uint64_t max_ptiles = n / kPTile + max_cells + 2;
-    const uint64_t max_bins = n / 2 + 16ull * max_cells + 16;
+    // histogram cells of a level: cells of more than kTile particles, or every cell on levels of
+    // few or large cells (small_cells)
+    const uint64_t max_hist = n / kTile + (uint64_t)(kCountCells * ctx->num_sms) + 2;
+    const uint64_t max_bins = max_hist << kMaxBinsLog2;
     ORB_CUDA(ctx->heap.ensure(heap_cells));
     ORB_CUDA(ctx->ranges.ensure(heap_cells));
-    ORB_CUDA(ctx->tile_off.ensure(max_cells + 1));
+    ORB_CUDA(ctx->tile_off.ensure(max_cells));
     ORB_CUDA(ctx->htile_cell.ensure(n / kTile + max_cells + 2));
-    ORB_CUDA(ctx->hist_off.ensure(max_cells + 1));
+    ORB_CUDA(ctx->hist_off.ensure(max_cells));
+    ORB_CUDA(ctx->hdone.ensure(max_cells));
     ORB_CUDA(ctx->below.ensure(max_cells));
     ORB_CUDA(ctx->inb.ensure(max_cells));
-    ORB_CUDA(ctx->part_s.ensure(max_cells));
-    ORB_CUDA(ctx->part_i.ensure(max_cells));
-    ORB_CUDA(ctx->part_le.ensure(max_cells));
+    ORB_CUDA(ctx->part.ensure(max_cells));
+    ORB_CUDA(ctx->part_done.ensure(max_cells));
     ORB_CUDA(ctx->out_counts.ensure(max_cells));
-    ORB_CUDA(ctx->hist_k.ensure(max_cells));
     ORB_CUDA(ctx->state.ensure(max_cells));
     ORB_CUDA(ctx->iters.ensure(max_cells));
-    ORB_CUDA(ctx->listed.ensure(max_cells));
-    ORB_CUDA(ctx->cmp_bad.ensure(max_cells));
-    ORB_CUDA(ctx->cmp_off.ensure(max_cells + 1));
+    ORB_CUDA(ctx->cmp_off.ensure(max_cells));
     ORB_CUDA(ctx->cmp_cnt.ensure(max_cells));
     ORB_CUDA(ctx->pred.ensure(max_cells));
-    // compaction lists: n/8 per cell of more than one tile, at least 2048 (list_capacity)
-    ORB_CUDA(ctx->cmp_keys.ensure(n / 8 + 2048ull * (n / kTile + 1) + 16));
+    // lists of bracket keys: at most max(2048, n/64) per histogram cell (list_capacity)
+    const uint64_t max_list = n / 64 + 2048ull * max_hist;
+    ORB_CUDA(ctx->cmp_keys.ensure(max_list));
+    ORB_CUDA(ctx->cmp_pos.ensure(max_list));
     ORB_CUDA(ctx->slots.ensure(max_cells));
     ORB_CUDA(ctx->hist.ensure(max_bins, true));
-    ORB_CUDA(ctx->ptile_off.ensure(max_cells + 1));
+    ORB_CUDA(ctx->ptile_off.ensure(max_cells));
     ORB_CUDA(ctx->counters.ensure(1, true));
-    return ensure_ptile_buffers(ctx, max_ptiles);
+    return ensure_ptile_buffers(ctx, max_ptiles, max_cells);
 }
 
 Level make_level(orb_ctx *ctx, float *x, float *y, float *z) {
@@ -232,21 +239,22 @@ Level make_level(orb_ctx *ctx, float *x, float *y, float *z) {
     v.heap = ctx->heap.p;
     v.ranges = ctx->ranges.p;
     v.slots = nullptr;
+    v.plan_bins = 1;
+    v.tot = &ctx->counters.p->plan[0];
     v.tile_off = ctx->tile_off.p;
     v.htile_cell = ctx->htile_cell.p;
     v.ptile_cell = ctx->ptile_cell.p;
     v.hist_off = ctx->hist_off.p;
-    v.hist_k = ctx->hist_k.p;
     v.state = ctx->state.p;
     v.iters = ctx->iters.p;
-    v.listed = ctx->listed.p;
-    v.cmp_bad = ctx->cmp_bad.p;
     v.cmp_off = ctx->cmp_off.p;
     v.cmp_cnt = ctx->cmp_cnt.p;
     v.cmp_keys = ctx->cmp_keys.p;
+    v.cmp_pos = ctx->cmp_pos.p;
     v.pred = ctx->pred.p;
     v.pred_sigmas = (float)ctx->tune.predict_sigmas;
     v.hist = ctx->hist.p;
+    v.hdone = ctx->hdone.p;
     v.below = ctx->below.p;
     v.inb = ctx->inb.p;
     v.ptile_off = ctx->ptile_off.p;
@@ -256,14 +264,12 @@ Level make_level(orb_ctx *ctx, float *x, float *y, float *z) {
     v.pt_le = ctx->pt_le.p;
     v.pt_ge_pre = ctx->pt_ge_pre.p;
     v.pt_le_pre = ctx->pt_le_pre.p;
-    v.pt_status = ctx->pt_status.p;
-    v.ticket = &ctx->counters.p->ticket;
-    v.part_s = ctx->part_s.p;
-    v.part_i = ctx->part_i.p;
-    v.part_le = ctx->part_le.p;
+    v.part = ctx->part.p;
+    v.swap_list = ctx->swap_list.p;
+    v.part_done = ctx->part_done.p;
+    v.done_start = 0u - ctx->done_offset;
     v.out_counts = ctx->out_counts.p;
     v.sparse_per_tile = ctx->tune.sparse_keys_per_tile;
-    v.spin_limit = ctx->spin_limit;
     v.pdl = ctx->use_pdl ? 1 : 0;
     v.counters = ctx->counters.p;
     return v;
@@ -432,21 +438,20 @@ std::vector<uint64_t> level_key(orb_ctx *ctx, const Level &v) {
     std::vector<uint64_t> key;
     for (const void *p : {(const void *)v.x, (const void *)v.y, (const void *)v.z, (const void *)v.idx,
                           (const void *)v.heap, (const void *)v.ranges, (const void *)v.tile_off,
-                          (const void *)v.hist_off, (const void *)v.hist_k, (const void *)v.state,
+                          (const void *)v.hist_off, (const void *)v.hdone, (const void *)v.state,
                           (const void *)v.iters, (const void *)v.hist, (const void *)v.below,
-                          (const void *)v.listed, (const void *)v.cmp_keys, (const void *)v.cmp_off,
-                          (const void *)v.inb, (const void *)v.htile_cell,
+                          (const void *)v.cmp_keys, (const void *)v.cmp_pos, (const void *)v.cmp_off,
+                          (const void *)v.cmp_cnt, (const void *)v.inb, (const void *)v.htile_cell,
                           (const void *)v.ptile_cell, (const void *)v.ptile_off, (const void *)v.ge_bits,
                           (const void *)v.le_bits, (const void *)v.pt_ge, (const void *)v.pt_le,
-                          (const void *)v.pt_ge_pre, (const void *)v.pt_le_pre, (const void *)v.pt_status,
-                          (const void *)v.part_s, (const void *)v.part_i, (const void *)v.part_le,
-                          (const void *)v.pred, (const void *)v.counters, (const void *)v.wt,
-                          (const void *)v.whist, (const void *)v.wbelow, (const void *)v.wtot})
+                          (const void *)v.pt_ge_pre, (const void *)v.pt_le_pre, (const void *)v.part,
+                          (const void *)v.swap_list, (const void *)v.part_done, (const void *)v.pred,
+                          (const void *)v.counters, (const void *)v.wt, (const void *)v.whist,
+                          (const void *)v.wbelow, (const void *)v.wtot})
         key_add(key, p);
-    key.push_back((uint64_t)ctx->pt_status.cap);
     key_add(key, ctx->sub_flag.p);
     key.push_back(ctx->prof_mask);
-    key.push_back(((uint64_t)ctx->spin_limit << 8) | ctx->scan_ticket_start);
+    key.push_back(ctx->done_offset);
     key.push_back(ctx->use_pdl ? 1u : 0u);
     for (uint32_t t : {ctx->tune.hist_blocks_per_sm, ctx->tune.part_blocks_per_sm, ctx->tune.tile_blocks_per_sm,
                        ctx->tune.sparse_keys_per_tile, ctx->tune.cta_min_cells, ctx->tune.subtree_levels,
@@ -455,54 +460,64 @@ std::vector<uint64_t> level_key(orb_ctx *ctx, const Level &v) {
     return key;
 }
 
-void partition_level(orb_ctx *ctx, const Level &v, bool do_split) {
-    const int g = pass_grid(ctx);
-    // look-back state of the tile scan: status words cleared, ticket at zero
-    cudaMemsetAsync(ctx->pt_status.p, 0, ctx->pt_status.cap * sizeof(unsigned long long), ctx->stream);
-    cudaMemsetAsync(&ctx->counters.p->ticket, 0, sizeof(uint32_t), ctx->stream);
-    if (ctx->scan_ticket_start)  // test hook: the low byte (little-endian) of the ticket
-        cudaMemsetAsync(&ctx->counters.p->ticket, (int)ctx->scan_ticket_start, 1, ctx->stream);
-    run_kernel(ctx, kKPartClassify, v, g);
-    run_kernel(ctx, kKPartScan, v, g, (int)(ctx->pt_ge_pre.cap / 1024 + 1));
-    run_kernel(ctx, kKPartCells, v, g);
+// Most partition tiles of a level of v.C cells over n particles.
+uint64_t ptiles_of(const Level &v, uint64_t n) { return n / kPTile + (uint64_t)v.C; }
+
+void partition_level(orb_ctx *ctx, Level v, uint64_t n, bool do_split) {
+    const uint64_t tiles = ptiles_of(v, n), swap_ctas = (uint64_t)ctx->num_sms * swap_blocks_per_sm();
+    // at most one swap tile a CTA (about half of the tiles hold left elements): the swap also
+    // finishes the cells
+    v.fuse = tiles <= 2 * swap_ctas ? 1 : 0;
+    run_kernel(ctx, kKPartClassify, v, (int)std::min<uint64_t>(pass_grid(ctx), tiles / (kThreads / 32) + 1));
+    run_kernel(ctx, kKPartCells, v, ctx->num_sms);
     if (ctx->yz_pending) {  // the first kernel that reads y and z
         cudaStreamWaitEvent(ctx->stream, ctx->yz_ready, ctx->capturing ? cudaEventWaitExternal : 0);
         ctx->yz_pending = false;
     }
-    run_kernel(ctx, kKPartSwap, v, ctx->num_sms * swap_blocks_per_sm());
-    run_kernel(ctx, kKPartFinish, v, g, do_split ? 1 : 0);
+    run_kernel(ctx, kKPartSwap, v, (int)std::min<uint64_t>(swap_ctas, tiles), do_split ? 1 : 0);
+    if (!v.fuse) run_kernel(ctx, kKPartFinish, v, ctx->num_sms, do_split ? 1 : 0);
 }
 
-// Bisection of every cell of the level to completion (found or capped): a fixed number of
-// histogram/resolve passes, with no host round trip (a pass after the level is done exits
-// at once on the device).
+// Bisection of every cell of the level with count tiles until it is found, capped or ready
+// for its list: a fixed number of histogram passes, with no host round trip (a pass after the
+// level is done exits at once on the device).
 // first: the count pass the first pass uses: 1 every cell dense (a cold level without
 // sampled brackets), 2 a sampled level, 0 the general one (warm builds).
-orb_status run_bisection(orb_ctx *ctx, Level v, uint32_t *passes, int first) {
+orb_status run_bisection(orb_ctx *ctx, Level v, uint64_t n, uint32_t *passes, int first) {
     // a cold first pass over every key is never discarded: 3 passes reach the cap
     const int npasses = first == 1 ? kColdHistPasses : kHistPasses;
+    const uint64_t tiles = n / kTile + (uint64_t)v.C;
     v.last_pass = npasses - 1;
     for (int pass = 0; pass < npasses; ++pass) {
         v.pass = pass;
-        run_kernel(ctx, kKHist, v, ctx->num_sms * (int)ctx->tune.hist_blocks_per_sm,
+        run_kernel(ctx, kKHist, v,
+                   (int)std::min<uint64_t>(ctx->num_sms * (uint64_t)ctx->tune.hist_blocks_per_sm, tiles),
                    pass == 0 ? first : 0);
-        run_kernel(ctx, kKResolve, v, pass_grid(ctx));
         ++*passes;
     }
     ORB_CUDA(cudaGetLastError());
     return ORB_OK;
 }
 
-// One level of the tree: heap slots [base, base + C) or the explicit slot list `slots`.
+// One level of the tree: heap slots [base, base + C) or the explicit slot list `slots`;
+// child_map: where the cells' children stand in the next level (null: 2c and 2c + 1).
 struct LevelDesc {
     int base;
     const int *slots;
     int C;
+    const int *child_map;
 };
 
-// The reference's level loop (src/orbit.cpp:102-275) over every cell of every level: plan,
-// bisection (one warp for small cells, one CTA per cell or the multi-CTA histogram passes
-// for the rest), partition and split.
+// Cells of at most this many particles take the one-tile bisection (a warp a cell) on a level
+// of C cells; larger ones the count passes. A level of large cells (one instance, more than
+// 4 tiles expected a cell) or of few cells sends every cell through the count passes: a warp
+// takes 36-42 us for a cell of 2^14 particles where the passes' CTAs take 10, so the
+// one-tile bisection pays only where its warps fill the GPU.
+uint32_t small_cells(const orb_ctx *ctx, const Level &v, uint64_t max_n, size_t li, int C) {
+    if (v.wt || C <= kCountCells * ctx->num_sms) return 0;
+    return !v.slots && (max_n >> li) > 4ull * kTile ? 0u : (uint32_t)kTile;
+}
+
 // The level from which subtree CTAs finish the tree (-1: none): the first level whose cells
 // (at most max_n >> l particles plus a few per split: each split leaves a cell within 3 of
 // half) all fit one CTA, that has enough cells to fill the GPU, and that is at most
@@ -519,24 +534,33 @@ int subtree_from(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, uint64_t 
     return -1;
 }
 
+// The reference's level loop (src/orbit.cpp:102-275) over every cell of every level: the
+// bisection (one warp for cells of at most one tile, the histogram passes for the rest, or one
+// CTA per cell), then the partition, which also splits the cells and plans the next level.
+// The first level's cells are planned by the init kernel.
 // sub_from >= 0: from level lv[sub_from] down, one CTA per cell finishes the tree when every
-// cell of that level fits one (k_subtree_check decides on the device); the level kernels of
-// those levels then return at once.
-// max_n: the largest instance's particles (cells of level l hold about max_n >> l); levels
-// whose cells can be large enough get a sampled first count pass (k_sample_bin, k_sample_pick).
+// cell of that level fits one (k_subtree_check decides on the device).
+// n: all particles; max_n: the largest instance's (cells of level l hold about max_n >> l;
+// levels whose cells can be large enough get a sampled first count pass (k_sample_bin,
+// k_sample_pick)).
 // rest = false: the levels above sub_from, then (sub_from >= 0) the subtree check and the
 // subtree kernel for the levels from sub_from down; rest = true: the levels from sub_from
 // down one by one, for builds whose subtree path the device refused.
 // [from, to): only those levels (staged builds run the levels in pieces).
 orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, uint32_t *passes,
-                      int sub_from, uint64_t max_n, bool rest = false, size_t from = 0,
+                      int sub_from, uint64_t n, uint64_t max_n, bool rest = false, size_t from = 0,
                       size_t to = SIZE_MAX) {
     to = std::min(to, lv.size());
+    v.plan_bins = v.wt ? 0u : 1u;
     for (size_t li = rest ? (size_t)sub_from : from; li < to; ++li) {
         const LevelDesc &d = lv[li];
         v.base = d.base;
         v.slots = d.slots;
         v.C = d.C;
+        v.depth = (uint32_t)li;
+        v.prev_C = li ? (uint32_t)lv[li - 1].C : 0u;
+        v.tot = &ctx->counters.p->plan[li & 1];
+        v.tot_next = &ctx->counters.p->plan[(li + 1) & 1];
         if (!rest && (int)li == sub_from) {
             if (v.C == 0) break;
             v.skip = ctx->sub_flag.p;
@@ -548,16 +572,24 @@ orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, u
             break;
         }
         if (v.C == 0) continue;
-        run_kernel(ctx, kKPlan, v, 1);
-        run_kernel(ctx, kKTileMap, v, pass_grid(ctx));
-        if (v.hint) run_kernel(ctx, kKWarmStart, v, 1);  // warm build: hinted brackets
+        v.small = small_cells(ctx, v, max_n, li, d.C);
+        v.next_C = 0;  // nothing to plan below the last level or at the subtree level
+        if (li + 1 < lv.size() && (rest || (int)li + 1 != sub_from)) {
+            v.next_C = lv[li + 1].C;
+            v.child_map = d.child_map;
+            v.small_next = small_cells(ctx, v, max_n, li + 1, lv[li + 1].C);
+        }
+        if (rest && (int)li == sub_from) {
+            // this level was not planned by the one above
+            ORB_CUDA(cudaMemsetAsync(&ctx->counters.p->plan[0], 0, 2 * sizeof(PlanTotals), ctx->stream));
+            run_kernel(ctx, kKPlan, v, 1);
+        }
         if (v.wt) {
             // weighted build: every cell through the weighted passes (kWPasses reach the cap)
-            run_kernel(ctx, kKWStart, v, pass_grid(ctx));
+            const uint64_t tiles = n / kTile + (uint64_t)v.C;
             for (int pass = 0; pass < kWPasses; ++pass) {
                 v.pass = pass;
-                run_kernel(ctx, kKWHist, v, pass_grid(ctx));
-                run_kernel(ctx, kKWResolve, v, 0);
+                run_kernel(ctx, kKWHist, v, (int)std::min<uint64_t>(pass_grid(ctx), tiles));
                 ++*passes;
             }
         } else if (ctx->tune.cta_min_cells && !v.hint && (uint32_t)v.C >= ctx->tune.cta_min_cells) {
@@ -572,14 +604,26 @@ orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, u
                 run_kernel(ctx, kKSample, v, 0);
                 run_kernel(ctx, kKSamplePick, v, 0);
             }
-            run_kernel(ctx, kKBisectTile, v, std::min(v.C, ctx->num_sms * (int)ctx->tune.tile_blocks_per_sm));
-            orb_status st = run_bisection(ctx, v, passes, v.hint ? 0 : (sampled ? 2 : 1));
+            if (v.small)
+                run_kernel(ctx, kKBisectTile, v, std::min(v.C, ctx->num_sms * (int)ctx->tune.tile_blocks_per_sm));
+            orb_status st = run_bisection(ctx, v, n, passes, v.hint ? 0 : (sampled ? 2 : 1));
             if (st != ORB_OK) return st;
         }
-        partition_level(ctx, v, true);
+        partition_level(ctx, v, n, true);
         ORB_CUDA(cudaGetLastError());
     }
     return ORB_OK;
+}
+
+constexpr const char *kUnfinished = "a cell's tiles did not all report or a bisection did not finish";
+
+// After a build (its counters read back): no step flagged an error and every cell of the first
+// `levels` levels, the ones the level kernels ran, was finished.
+bool build_finished(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, size_t levels) {
+    if (ctx->h_counters->error) return false;
+    for (size_t li = 0; li < levels; ++li)
+        if (ctx->h_counters->done[li] != (uint32_t)lv[li].C) return false;
+    return true;
 }
 
 // After the main graph of a build that planned subtrees (sub_from >= 0): waits for it and
@@ -588,7 +632,7 @@ orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, u
 // build's end event is recorded again after it.
 orb_status finish_subtree_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv,
                                  std::vector<uint64_t> key, uint32_t *passes, int sub_from,
-                                 uint64_t max_n, bool *taken) {
+                                 uint64_t n, uint64_t max_n, bool *taken) {
     *taken = false;
     if (sub_from < 0) return ORB_OK;
     ORB_CUDA(cudaMemcpyAsync(ctx->h_sub_flag, ctx->sub_flag.p, sizeof(uint32_t), cudaMemcpyDeviceToHost,
@@ -600,7 +644,7 @@ orb_status finish_subtree_levels(orb_ctx *ctx, Level v, const std::vector<LevelD
     key.push_back(0x5E57u);  // the levels from sub_from down
     v.skip = nullptr;
     orb_status st = run_graphed(ctx, key, passes, [&](uint32_t *pp) -> orb_status {
-        return run_levels(ctx, v, lv, pp, sub_from, max_n, true);
+        return run_levels(ctx, v, lv, pp, sub_from, n, max_n, true);
     });
     if (st != ORB_OK) return st;
     ORB_CUDA(cudaEventRecord(ctx->ev[1], ctx->stream));
@@ -713,14 +757,14 @@ orb_status orb_ctx_destroy(orb_ctx *ctx) {
     ctx->yraw.release(); ctx->zraw.release();
     ctx->idx.release();
     ctx->heap.release(); ctx->ranges.release();
-    ctx->tile_off.release(); ctx->hist_off.release(); ctx->below.release(); ctx->inb.release();
-    ctx->part_s.release(); ctx->part_i.release(); ctx->part_le.release(); ctx->out_counts.release();
-    ctx->hist_k.release(); ctx->state.release(); ctx->iters.release(); ctx->hist.release();
+    ctx->tile_off.release(); ctx->hist_off.release(); ctx->hdone.release(); ctx->below.release();
+    ctx->inb.release(); ctx->part.release(); ctx->part_done.release(); ctx->swap_list.release();
+    ctx->out_counts.release(); ctx->state.release(); ctx->iters.release(); ctx->hist.release();
     ctx->ptile_off.release(); ctx->ge_bits.release(); ctx->le_bits.release(); ctx->pt_ge.release();
-    ctx->pt_le.release(); ctx->pt_ge_pre.release(); ctx->pt_le_pre.release(); ctx->pt_status.release();
+    ctx->pt_le.release(); ctx->pt_ge_pre.release(); ctx->pt_le_pre.release(); ctx->pred.release();
     ctx->slots.release(); ctx->counters.release(); ctx->staging.release();
     ctx->htile_cell.release(); ctx->ptile_cell.release();
-    ctx->batch_roots.release(); ctx->batch_slots.release();
+    ctx->batch_roots.release(); ctx->batch_slots.release(); ctx->batch_child.release();
     for (int a = 0; a < 3; ++a) {
         ctx->tune_src[a].release();
         ctx->tune_work[a].release();
@@ -728,8 +772,7 @@ orb_status orb_ctx_destroy(orb_ctx *ctx) {
     ctx->hint.release(); ctx->hint_axis.release(); ctx->warm.release(); ctx->sub_flag.release();
     ctx->w.release(); ctx->whist.release(); ctx->wbelow.release(); ctx->wtot.release();
     ctx->gen_starts.release();
-    ctx->listed.release(); ctx->cmp_bad.release(); ctx->cmp_off.release(); ctx->cmp_cnt.release();
-    ctx->cmp_keys.release();
+    ctx->cmp_off.release(); ctx->cmp_cnt.release(); ctx->cmp_keys.release(); ctx->cmp_pos.release();
     if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
     if (ctx->h_sub_flag) cudaFreeHost(ctx->h_sub_flag);
     if (ctx->h_win) cudaFreeHost(ctx->h_win);
@@ -816,7 +859,7 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     if (st != ORB_OK) return st;
     ORB_CUDA(ctx->idx.ensure(n + 1));
     if (weighted) {
-        ORB_CUDA(ctx->whist.ensure((size_t)max_cells * kWBins));
+        ORB_CUDA(ctx->whist.ensure((size_t)max_cells * kWBins, true));  // all-zero between passes
         ORB_CUDA(ctx->wbelow.ensure(max_cells));
         ORB_CUDA(ctx->wtot.ensure(max_cells));
         if (!dev) ORB_CUDA(ctx->w.ensure(n + 1));
@@ -828,7 +871,7 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     ctx->yz_pending = false;
     std::vector<LevelDesc> lv;
     for (uint32_t l = 1; l <= levels; ++l)
-        lv.push_back({sl.first(l), nullptr, sl.count(l)});  // src/orbit.cpp:104-107
+        lv.push_back({sl.first(l), nullptr, sl.count(l), nullptr});  // src/orbit.cpp:104-107
     // subtrees finish complete unweighted trees only: d a power of two, built to its leaves
     const int sub_from = subtree_from(ctx, lv, n, !weighted && sl.pow2 && levels == sl.depth);
     if (sub_from >= 0) ORB_CUDA(ctx->sub_flag.ensure(1));
@@ -895,6 +938,9 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
         v.wbelow = ctx->wbelow.p;
         v.wtot = ctx->wtot.p;
     }
+    v.C = lv.empty() ? 0 : lv[0].C;  // the init kernel plans the root
+    v.small = small_cells(ctx, v, n, 0, v.C);
+    v.plan_bins = weighted ? 0u : 1u;
     std::vector<uint64_t> key = level_key(ctx, v);
     key.push_back(0xB111D);  // single build
     key.push_back(n);
@@ -934,7 +980,7 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
         if (!staged) {
             launch_init(v, n, lower, upper, d, (int)heap_cells, s);
             ORB_CUDA(cudaGetLastError());
-            return run_levels(ctx, v, lv, pp, sub_from, n);
+            return run_levels(ctx, v, lv, pp, sub_from, n, n);
         }
         const unsigned wf = ctx->capturing ? cudaEventWaitExternal : 0;
         Level v1 = v;  // level 1: x and the permutation
@@ -942,17 +988,17 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
         v1.idx = ctx->idx.p;
         launch_init(v1, n, lower, upper, d, (int)heap_cells, s);
         ORB_CUDA(cudaGetLastError());
-        orb_status ls = run_levels(ctx, v1, lv, pp, sub_from, n, false, 0, 1);
+        orb_status ls = run_levels(ctx, v1, lv, pp, sub_from, n, n, false, 0, 1);
         if (ls != ORB_OK) return ls;
         ORB_CUDA(cudaStreamWaitEvent(s, ctx->y_ready, wf));
         run_stage_gather(ctx, dy, ctx->yraw.p, n);
         Level v2 = v1;  // level 2: x, y and the permutation
         v2.y = dy;
-        if ((ls = run_levels(ctx, v2, lv, pp, sub_from, n, false, 1, 2)) != ORB_OK) return ls;
+        if ((ls = run_levels(ctx, v2, lv, pp, sub_from, n, n, false, 1, 2)) != ORB_OK) return ls;
         ORB_CUDA(cudaStreamWaitEvent(s, ctx->yz_ready, wf));
         run_stage_gather(ctx, dz, ctx->zraw.p, n);
         ORB_CUDA(cudaGetLastError());
-        return run_levels(ctx, v, lv, pp, sub_from, n, false, 2);  // the rest
+        return run_levels(ctx, v, lv, pp, sub_from, n, n, false, 2);  // the rest
     });
     if (st != ORB_OK) return st;
     if (ctx->yz_pending || (!dev && n)) {
@@ -1009,7 +1055,7 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     bool streamed = false;
     if (windows && (st = stream_windows(&streamed)) != ORB_OK) return st;
     bool taken = false;  // the subtree kernel finished the tree
-    st = finish_subtree_levels(ctx, v, lv, key, &passes, sub_from, n, &taken);
+    st = finish_subtree_levels(ctx, v, lv, key, &passes, sub_from, n, n, &taken);
     if (st != ORB_OK) return st;
     bool written = false;  // the particles are in the host arrays (or on their way there)
     if (!dev) {
@@ -1039,8 +1085,8 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     if (!dev) ORB_CUDA(cudaEventRecord(ctx->ev[3], on_cs ? ctx->copy_stream : s));
     ORB_CUDA(cudaStreamSynchronize(s));
     if (on_cs) ORB_CUDA(cudaStreamSynchronize(ctx->copy_stream));
-    if (ctx->h_counters->error)
-        return fail(ctx, ORB_ERR_TIMEOUT, "a bounded device wait gave up or a bisection did not finish");
+    if (!build_finished(ctx, lv, taken ? (size_t)sub_from : lv.size()))
+        return fail(ctx, ORB_ERR_TIMEOUT, kUnfinished);
     float dev_ms = 0.f;
     ORB_CUDA(cudaEventElapsedTime(&dev_ms, ctx->ev[0], ctx->ev[1]));
     collect_profile(ctx);
@@ -1290,7 +1336,7 @@ static orb_status service_prepare(orb_ctx *ctx, const orb_cell_t *cells, uint32_
         if (spans[i].first < spans[i - 1].second)
             return fail(ctx, ORB_ERR_INVALID_ARGUMENT, "cells with overlapping particle ranges");
     {
-        orb_status pst = ensure_ptile_buffers(ctx, tiles + 2);
+        orb_status pst = ensure_ptile_buffers(ctx, tiles + 2, n_cells);
         if (pst != ORB_OK) return pst;
     }
     // Each cell is placed at heap slot == id, so child slots are 2id+1 and 2id+2.
@@ -1303,6 +1349,7 @@ static orb_status service_prepare(orb_ctx *ctx, const orb_cell_t *cells, uint32_
     v.slots = ctx->slots.p;
     v.base = 0;
     v.C = (int)n_cells;
+    v.plan_bins = 0;
     *out = v;
     return ORB_OK;
 }
@@ -1335,9 +1382,10 @@ orb_status orb_count_left(orb_ctx *ctx, const orb_cell_t *cells, uint32_t n_cell
     if (st != ORB_OK || n_cells == 0) return st;
     cudaStream_t s = ctx->stream;
     ORB_CUDA(cudaMemsetAsync(ctx->out_counts.p, 0, n_cells * sizeof(uint32_t), s));
+    ORB_CUDA(cudaMemsetAsync(&ctx->counters.p->plan[0], 0, sizeof(PlanTotals), s));
     run_kernel(ctx, kKPlan, v, 1);
-    run_kernel(ctx, kKTileMap, v, pass_grid(ctx));
-    run_kernel(ctx, kKCountLeft, v, pass_grid(ctx));
+    run_kernel(ctx, kKCountLeft, v,
+               (int)std::min<uint64_t>(pass_grid(ctx), ctx->loaded_n / kTile + (uint64_t)v.C));
     ORB_CUDA(cudaGetLastError());
     std::vector<uint32_t> res(n_cells);
     collect_profile(ctx);
@@ -1357,16 +1405,19 @@ orb_status orb_partition(orb_ctx *ctx, const orb_cell_t *cells, uint32_t n_cells
     if (st != ORB_OK || n_cells == 0) return st;
     cudaStream_t s = ctx->stream;
     ORB_CUDA(cudaMemsetAsync(&ctx->counters.p->error, 0, sizeof(uint32_t), s));
+    ORB_CUDA(cudaMemsetAsync(&ctx->counters.p->plan[0], 0, sizeof(PlanTotals), s));
+    ORB_CUDA(cudaMemsetAsync(&ctx->counters.p->done[0], 0, sizeof(uint32_t), s));
     run_kernel(ctx, kKPlan, v, 1);
-    run_kernel(ctx, kKTileMap, v, pass_grid(ctx));
-    partition_level(ctx, v, false);
+    partition_level(ctx, v, ctx->loaded_n, false);
     ORB_CUDA(cudaGetLastError());
     ORB_CUDA(cudaMemcpyAsync(&ctx->h_counters->error, &ctx->counters.p->error, sizeof(uint32_t),
                              cudaMemcpyDeviceToHost, s));
+    ORB_CUDA(cudaMemcpyAsync(&ctx->h_counters->done[0], &ctx->counters.p->done[0], sizeof(uint32_t),
+                             cudaMemcpyDeviceToHost, s));
     ORB_CUDA(cudaStreamSynchronize(s));
     collect_profile(ctx);
-    if (ctx->h_counters->error)
-        return fail(ctx, ORB_ERR_TIMEOUT, "a bounded device wait gave up or a bisection did not finish");
+    if (ctx->h_counters->error || ctx->h_counters->done[0] != n_cells)
+        return fail(ctx, ORB_ERR_TIMEOUT, kUnfinished);
     return ORB_OK;
 }
 
@@ -1423,6 +1474,7 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
     uint32_t max_levels = 0;
     std::vector<std::pair<uint64_t, uint64_t>> spans;
     for (uint32_t i = 0; i < k; ++i) {
+        roots[i].cell = -1;
         const orb_batch_instance &b = inst[i];
         if (b.d == 0 || b.d > (1u << 30))
             return fail(ctx, ORB_ERR_INVALID_ARGUMENT, "instance d must be in [1, 2^30]");
@@ -1451,17 +1503,25 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
     for (size_t i = 1; i < spans.size(); ++i)
         if (spans[i].first < spans[i - 1].second)
             return fail(ctx, ORB_ERR_INVALID_ARGUMENT, "instances overlap");
-    std::vector<int> slots;
+    std::vector<int> slots, child;  // per level: the cells' heap slots, their children's map
     std::vector<LevelDesc> lv;
     std::vector<size_t> lv_off;
     uint32_t max_cells = 1;
     for (uint32_t l = 1; l <= max_levels; ++l) {
         lv_off.push_back(slots.size());
+        int next = 0;  // index in level l + 1 of the instance's first cell there
         for (uint32_t i = 0; i < k; ++i) {
             if (lev[i] < l) continue;
             const Slices sl(inst[i].d);
             const int first = (int)roots[i].heap_base + sl.first(l);
-            for (int j = 0; j < sl.count(l); ++j) slots.push_back(first + j);
+            const int below = lev[i] > l ? sl.count(l + 1) : 0;
+            if (l == 1) roots[i].cell = (int)slots.size();
+            for (int j = 0; j < sl.count(l); ++j) {
+                slots.push_back(first + j);
+                const int c0 = 2 * j, has = (c0 < below ? 1 : 0) | (c0 + 1 < below ? 2 : 0);
+                child.push_back(4 * (next + c0) | has);
+            }
+            next += below;
         }
         max_cells = std::max<uint32_t>(max_cells, (uint32_t)(slots.size() - lv_off.back()));
     }
@@ -1471,6 +1531,7 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
     ORB_CUDA(ctx->idx.ensure(n_total + 1));
     ORB_CUDA(ctx->batch_roots.ensure(k + 1));
     ORB_CUDA(ctx->batch_slots.ensure(slots.size() + 1));
+    ORB_CUDA(ctx->batch_child.ensure(slots.size() + 1));
     cudaStream_t s = ctx->stream;
     float *dx = x, *dy = y, *dz = z;
     float h2d_ms = 0.f, d2h_ms = 0.f;
@@ -1522,7 +1583,10 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
     }
     if (k) ORB_CUDA(cudaMemcpyAsync(ctx->batch_roots.p, roots.data(), k * sizeof(BatchRoot), cudaMemcpyHostToDevice, s));
     if (!slots.empty())
+    {
         ORB_CUDA(cudaMemcpyAsync(ctx->batch_slots.p, slots.data(), slots.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+        ORB_CUDA(cudaMemcpyAsync(ctx->batch_child.p, child.data(), child.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+    }
     ORB_CUDA(cudaEventRecord(ctx->ev[0], s));
     Level v = make_level(ctx, dx, dy, dz);
     if (!perm) v.idx = nullptr;  // no permutation asked for: only x, y, z move
@@ -1533,7 +1597,7 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
     }
     for (uint32_t l = 1; l <= max_levels; ++l) {
         const size_t a = lv_off[l - 1], b = l < max_levels ? lv_off[l] : slots.size();
-        lv.push_back({0, ctx->batch_slots.p + a, (int)(b - a)});
+        lv.push_back({0, ctx->batch_slots.p + a, (int)(b - a), ctx->batch_child.p + a});
     }
     std::vector<uint64_t> key = level_key(ctx, v);
     key.push_back(warm ? 0xBA7C4A : 0xBA7C4);  // batched build (warm)
@@ -1542,6 +1606,7 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
     key.push_back(n_total);
     key_add(key, ctx->batch_roots.p);
     key_add(key, ctx->batch_slots.p);
+    key_add(key, ctx->batch_child.p);
     for (uint32_t i = 0; i < k; ++i) {
         key.push_back(inst[i].offset);
         key.push_back(inst[i].n);
@@ -1569,14 +1634,20 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
         ORB_CUDA(cudaMemsetAsync(ctx->ranges.p, 0, heap_cells * sizeof(uint2), s));
         ORB_CUDA(cudaMemsetAsync(ctx->counters.p, 0, sizeof(BuildCounters), s));
         ctx->launches[kKInit] += 1;
-        launch_init_batch(v, ctx->batch_roots.p, (int)k, n_total, s);
+        Level v0 = v;  // the init kernel plans the roots
+        if (!lv.empty()) {
+            v0.slots = lv[0].slots;
+            v0.C = lv[0].C;
+        }
+        v0.small = small_cells(ctx, v0, max_n, 0, v0.C);
+        launch_init_batch(v0, ctx->batch_roots.p, (int)k, n_total, s);
         ORB_CUDA(cudaGetLastError());
-        return run_levels(ctx, v, lv, pp, sub_from, max_n);
+        return run_levels(ctx, v, lv, pp, sub_from, n_total, max_n);
     });
     if (st != ORB_OK) return st;
     ORB_CUDA(cudaEventRecord(ctx->ev[1], s));
     bool taken = false;
-    st = finish_subtree_levels(ctx, v, lv, key, &passes, sub_from, max_n, &taken);
+    st = finish_subtree_levels(ctx, v, lv, key, &passes, sub_from, n_total, max_n, &taken);
     if (st != ORB_OK) return st;
     if (!dev) {
         ORB_CUDA(cudaStreamSynchronize(s));
@@ -1603,8 +1674,8 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
     ORB_CUDA(cudaMemcpyAsync(ctx->h_counters, ctx->counters.p, sizeof(BuildCounters), cudaMemcpyDeviceToHost, s));
     if (!dev) ORB_CUDA(cudaEventRecord(ctx->ev[3], s));
     ORB_CUDA(cudaStreamSynchronize(s));
-    if (ctx->h_counters->error)
-        return fail(ctx, ORB_ERR_TIMEOUT, "a bounded device wait gave up or a bisection did not finish");
+    if (!build_finished(ctx, lv, taken ? (size_t)sub_from : lv.size()))
+        return fail(ctx, ORB_ERR_TIMEOUT, kUnfinished);
     // ranges relative to each instance (cells the build filled)
     for (uint32_t i = 0; i < k; ++i) {
         const uint64_t filled = Slices(inst[i].d).filled(lev[i]);
@@ -1688,8 +1759,8 @@ orb_status orb_test_set_scan_wait(orb_ctx *ctx, uint32_t spin_limit, uint32_t ti
     if (!ctx) return ORB_ERR_INVALID_ARGUMENT;
     ctx->err.clear();
     if (ticket_start > 255) return fail(ctx, ORB_ERR_INVALID_ARGUMENT, "ticket_start above 255");
-    ctx->spin_limit = spin_limit ? spin_limit : kLookbackSpinLimit;
-    ctx->scan_ticket_start = ticket_start;
+    (void)spin_limit;  // no device wait polls (see orb.h)
+    ctx->done_offset = ticket_start;
     return ORB_OK;
 }
 

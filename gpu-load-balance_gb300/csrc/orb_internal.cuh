@@ -25,6 +25,7 @@ constexpr int kMaxBinsLog2 = 11;     // deepest midpoint tree one histogram pass
 // cut) costs one more, hence 4 for levels that may have one.
 constexpr int kHistPasses = 4;
 constexpr int kColdHistPasses = 3;
+static_assert(kHistPasses <= 4, "BuildCounters::any_active holds the passes");
 constexpr int kThreads = 256;
 // resident CTAs of the count-left pass (its launch bound: 65536 / (256 x 6) = 40 registers)
 #ifndef ORB_HIST_BLOCKS_PER_SM
@@ -47,41 +48,53 @@ constexpr int kWPasses = 4;
 static_assert(kWPasses * kWBinsLog2 >= 32, "the weighted passes reach the iteration cap");
 
 // kSmall: at most kWarpKeys keys (one warp bisects it); kOneTile: at most kTile keys (one CTA)
-enum CellState : uint8_t { kActive = 0, kFound = 1, kCapped = 2, kSmall = 3, kOneTile = 4 };
+// kReady: its bracket holds few enough keys for a list: the classify pass lists them and
+// k_part_cells finishes the bisection on the list
+enum CellState : uint8_t { kActive = 0, kFound = 1, kCapped = 2, kSmall = 3, kOneTile = 4, kReady = 5 };
 constexpr int kWarpKeys = 1024;      // cells up to this size bisect in one warp's registers
-// Polls of a decoupled look-back wait (64 ns apart) before it gives up: about 0.3 s, far
-// beyond any real wait; the kernel then flags the error and finishes its work.
-constexpr uint32_t kLookbackSpinLimit = 1u << 22;
+constexpr int kMaxLevels = 30;       // d is at most 2^30
 
 // Kernel kinds, for launch counting, event timing and algorithmic-byte accounting.
 enum Kernel : int {
     kKInit = 0,
     kKPlan,
     kKHist,
-    kKResolve,
     kKPartClassify,
-    kKPartScan,
     kKPartCells,
     kKPartSwap,
     kKPartFinish,
     kKCountLeft,
     kKGenerate,
     kKBisectCta,
-    kKTileMap,
     kKBisectTile,
-    kKWarmStart,
     kKSubtreeCheck,
     kKSubtree,
     kKSample,
     kKSamplePick,
-    kKWStart,
     kKWHist,
-    kKWResolve,
     kKStageGather,
     kNumKernels
 };
 static_assert(kNumKernels <= 32, "BuildCounters::bytes holds 32 kernel kinds");
 extern const char *const kKernelNames[kNumKernels];
+
+// Totals of one level's plan. A level's cells take their tiles, histogram bins and list slots
+// from these counters (one allocation per cell, in the order the cells become known).
+struct PlanTotals {
+    unsigned long long tiles;  // count tiles << 32 | partition tiles
+    unsigned long long pools;  // histogram cells << 32 | list slots
+    uint32_t swaps;            // partition tiles with pairs to swap (the swap's work list)
+    uint32_t pad_;
+};
+
+// What the partition found for one cell (32 bytes, read at once by the swap).
+struct CellPart {
+    uint32_t b, n;   // first particle, particles
+    uint32_t s, i;   // Hoare swaps, split index (cell-relative; n when clamped)
+    uint32_t le;     // keys <= cut
+    uint32_t t0, T;  // first partition tile, tiles
+    uint32_t left;   // tiles that can hold left elements of pairs
+};
 
 // Device-side counters of one build (read back at the end).
 struct BuildCounters {
@@ -89,9 +102,10 @@ struct BuildCounters {
     uint32_t zero_volume;
     uint32_t unfound;
     uint32_t max_iters;
-    uint32_t any_active[2];  // pass p: cleared by hist p, set by resolve p if a cell goes on
+    uint32_t any_active[4];  // histogram pass p left a cell active
     uint32_t error;       // set when a bounded device wait gave up
-    uint32_t ticket;      // block ticket of the tile scan (reset before each launch)
+    uint32_t done[kMaxLevels + 1];  // cells whose children (or leaves) are final, per level
+    PlanTotals plan[2];   // levels 1, 3, ... and 2, 4, ...
     uint32_t warm_cells;  // warm builds: cells that started from a hinted bracket
     uint32_t warm_resets; // ... whose hinted bracket missed the target (restarted cold)
     uint32_t pred_cells;  // cells whose first count pass used a sampled bracket
@@ -112,7 +126,9 @@ struct HostWindows {
 };
 
 // Everything a level's kernels need. Cells of the level are heap slots [base, base + C)
-// unless `slots` is non-null (service calls over an arbitrary cell list).
+// unless `slots` is non-null (batched builds, service calls over an arbitrary cell list).
+// The partition of a level plans the next one: whoever finishes a cell allocates its
+// children's tiles and writes their tile maps and state.
 struct Level {
     float *x, *y, *z;
     uint32_t *idx;          // original particle index (perm), may be null
@@ -123,53 +139,62 @@ struct Level {
     int C;
     int pass;               // histogram pass index within the level
     int last_pass;          // index of the level's last histogram pass
+    uint32_t depth;         // index of the level within the build (0: the root's)
+    // the next level: its cells (0: none is planned), where a cell's children stand among
+    // them (child_map[c] = 4 x index of the first child | bit per child in the level; null:
+    // 2c and 2c+1) and the cells the one-tile bisection takes there (up to small_next
+    // particles; larger ones get count tiles)
+    int next_C;
+    const int *child_map;
+    const int *next_slots;  // heap slots of the next level's cells (null: implied)
+    uint32_t small_next;
+    uint32_t small;         // ... on this level (k_plan, k_init)
+    uint32_t plan_bins;     // 1: cells with count tiles get histogram bins and a list
     // plan
-    uint32_t *tile_off;     // [C+1] first tile of each cell
-    uint32_t *htile_cell;   // [tiles] cell of each count-left tile (null: binary search)
-    uint32_t *ptile_cell;   // [ptiles] cell of each partition tile (null: binary search)
-    uint32_t *hist_off;     // [C+1] first bin of each cell in the histogram pool
-    uint8_t *hist_k;        // [C]   tree depth of each cell's histogram
-    uint8_t *state;         // [C]   CellState
-    uint8_t *iters;         // [C]   bisection iterations done
+    PlanTotals *tot, *tot_next;
+    uint32_t *tile_off;     // [C] first count tile of each cell
+    uint32_t *htile_cell;   // [tiles] cell of each count-left tile
+    uint32_t *ptile_off;    // [C] first partition tile of each cell
+    uint32_t *ptile_cell;   // [ptiles] cell of each partition tile
+    uint32_t *hist_off;     // [C] first bin of each cell in the histogram pool
+    uint8_t *state;         // [C] CellState
+    uint8_t *iters;         // [C] bisection iterations done
     uint32_t *hist;         // histogram pool (kept all-zero between passes)
-    uint32_t *below;        // [C]   keys below the left margin in the current pass
-    uint32_t *inb;          // [C]   keys inside the current bracket (n before the first pass)
-    // in-bracket compaction: a sparse pass also writes its bracket keys to the cell's list;
-    // every later pass of the cell reads the list only (count below L carried by resolve)
-    uint32_t *cmp_off;      // [C+1] first list slot of each cell (capacity = difference)
-    uint32_t *cmp_cnt;      // [C]   keys written to the list
+    uint32_t *hdone;        // [C] count tiles finished in the current pass
+    uint32_t *below;        // [C] keys below the left margin
+    uint32_t *inb;          // [C] keys inside the current bracket (n before the first pass)
+    // bracket keys the classify pass lists for a kReady cell (their keys and positions)
+    uint32_t *cmp_off;      // [C] first list slot of each cell
+    uint32_t *cmp_cnt;      // [C] keys written to the list
     float *cmp_keys;        // the lists
-    uint8_t *listed;        // [C]   1: this pass reads the cell's list instead of its keys
-    uint8_t *cmp_bad;       // [C]   1: a tile's bracket keys overflowed (no list)
+    uint32_t *cmp_pos;
     // sampled first pass: leaves [lo, hi) of the first pass's midpoint tree predicted to hold
     // the cut (k_sample_bin, k_sample_pick); that pass counts the keys below leaf lo and bins
-    // only the keys of [lo, hi). Packed (lo | hi << 12 | flags); 0: no prediction (dense)
+    // only the keys of [lo, hi). Packed (lo | hi << 12 | flag); 0: no prediction (dense)
     uint32_t *pred;         // [C]
     float pred_sigmas;      // half-width of the sampled bracket in standard errors (0: off)
     // partition
-    uint32_t *ptile_off;    // [C+1] first partition tile of each cell
     uint32_t *ge_bits;      // [ptiles * kPWords] bit p: key >= cut
     uint32_t *le_bits;      // [ptiles * kPWords] bit p: key <= cut
     uint32_t *pt_ge;        // [ptiles] set bits per tile
     uint32_t *pt_le;
-    uint32_t *pt_ge_pre;    // [ptiles+1] exclusive prefix over all tiles of the level
+    uint32_t *pt_ge_pre;    // [ptiles] exclusive prefix within the cell
     uint32_t *pt_le_pre;
-    unsigned long long *pt_status;  // look-back status word per scan block (zeroed per level)
-    uint32_t *ticket;       // block ticket counter of the tile scan
-    uint32_t *part_s;       // [C] number of Hoare swaps
-    uint32_t *part_i;       // [C] split index (cell-relative); n when clamped
-    uint32_t *part_le;      // [C] keys <= cut in the cell
+    CellPart *part;         // [C]
+    uint2 *swap_list;       // [ptiles] (cell, tile within the cell) of the swap's tiles
+    uint32_t *part_done;    // [C] tiles swapped
+    int fuse;               // 1: the swap kernel finishes the cells (else k_part_finish)
+    uint32_t done_start;    // what part_done starts from (0; the test hook's offset otherwise)
     uint32_t *out_counts;   // service calls: per-cell result
-    uint32_t sparse_per_tile;  // count pass: sparse once the bracket holds <= this x tiles keys
-    uint32_t spin_limit;    // polls of one look-back wait before it gives up (error flag)
+    uint32_t sparse_per_tile;  // a bracket of at most this many keys a count tile is listed
     int pdl;                // level kernels launched with programmatic dependent launch
     // warm builds (null otherwise): per heap slot the previous tree's cut and w x its extent
     // (x NaN: no hint) and that tree's cut axis
     const float2 *hint;     // (cut, w x extent) from the previous tree
     const int *hint_axis;
     uint8_t *warm;          // [C] 1 while a hinted bracket is not yet checked
-    // subtrees: 1 when one CTA per cell finishes the tree from this level down (then the
-    // level kernels of the levels below return at once); null when not attempted
+    // subtrees: 1 when one CTA per cell finishes the tree from this level down; null when
+    // not attempted
     uint32_t *skip;
     // window reports (null otherwise): the host-mapped reports, a finished-cell counter per
     // window, root cells per window
@@ -177,12 +202,13 @@ struct Level {
     uint32_t *win_cnt;
     uint32_t win_cells;
     // weighted builds (null otherwise): an integer weight per particle, moved with it, and
-    // per cell of the level its weight bins (kWBins), the weight below its bracket and its
-    // total weight
+    // per cell of the level its weight bins (kWBins, kept all-zero between passes), the
+    // weight below its bracket and its total weight
     uint32_t *wt;
     unsigned long long *whist;
     unsigned long long *wbelow;
     unsigned long long *wtot;
+    uint32_t prev_C;        // cells of the level above (checked against counters->done)
     BuildCounters *counters;
 };
 
@@ -271,6 +297,7 @@ struct BatchRoot {
     uint32_t n;          // particles
     uint32_t d;          // leaf cells
     uint32_t heap_base;  // heap slot of the root
+    int32_t cell;        // its index among level 1's cells (-1: no split level)
     float lower[3], upper[3];
 };
 

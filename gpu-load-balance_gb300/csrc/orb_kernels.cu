@@ -1,19 +1,22 @@
 // ORB engine kernels for sm_103a.
 //
 // Per level of the tree (all cells of the level in every launch):
-//   plan       per-cell tile and histogram offsets (one CTA scan)
 //   hist       count-left: every key of an active cell is binned into a midpoint tree of
-//              depth K over the cell's bracket [cutMarginLeft, cutMarginRight); keys below
-//              the bracket are counted. One pass resolves up to K bisection iterations.
-//   resolve    replays the reference's bisection (src/orbit.cpp:146-232) on the histogram:
-//              the same cuts, the same integer counts, the same float32 test.
-//   partition  the Hoare partition of src/services/partition.cpp:30-52 computed in
-//              parallel: with L_k the k-th key >= cut from the left and R_k the k-th key
-//              <= cut from the right, Hoare swaps exactly (L_k, R_k) for k <= s where
+//              depth 11 over the cell's bracket [cutMarginLeft, cutMarginRight); keys below
+//              the bracket are counted. The CTA that finishes a cell's last tile replays up
+//              to 11 iterations of the reference's bisection (src/orbit.cpp:146-232) on the
+//              histogram: the same cuts, the same integer counts, the same float32 test.
+//   classify   masks of the keys >= cut and <= cut; a cell whose bracket holds few keys is
+//              classified against the bracket, and the bracket's keys are listed
+//   cells      the rest of the bisection on the cell's list, the listed keys' mask bits, and
+//              the Hoare partition of src/services/partition.cpp:30-52 characterised: with
+//              L_k the k-th key >= cut from the left and R_k the k-th key <= cut from the
+//              right, Hoare swaps exactly (L_k, R_k) for k <= s where
 //              s = max_x min(#{>= cut in [0,x)}, #{<= cut in [x,n)}), stops at
-//              i = min(L_{s+1}, R_s) and swaps (i, n-1). Counts, a per-cell scan, rank
-//              tables and a swap pass reproduce the permutation exactly.
-//   split      src/cell.h:78-126 and src/orbit.cpp:235-250 on the device.
+//              i = min(L_{s+1}, R_s) and swaps (i, n-1).
+//   swap       the pairs; whoever finishes a cell's last tile does the final swap and the split
+//              (src/cell.h:78-126, src/orbit.cpp:235-250) and plans the children for the
+//              next level.
 // Beside them: the bisection of cells of at most one tile in one launch (a warp per cell),
 // the subtree kernel (one CTA finishes a cell's last levels with its particles in L2), the
 // optional sampled first pass, the service count-left, seeded generators and the batched
@@ -26,11 +29,10 @@
 namespace orb {
 
 const char *const kKernelNames[kNumKernels] = {
-    "init", "plan", "count_left_hist", "bisect_resolve", "part_classify", "part_scan",
-    "part_cells", "part_swap", "part_finish", "count_left", "generate", "bisect_cta",
-    "tile_map", "bisect_tile", "warm_start", "subtree_check", "subtree",
-    "count_left_sample", "count_left_sample_pick", "weighted_start", "count_left_weighted",
-    "bisect_resolve_weighted", "stage_gather"};
+    "init", "plan", "count_left_hist", "part_classify", "part_cells", "part_swap", "part_finish",
+    "count_left",
+    "generate", "bisect_cta", "bisect_tile", "subtree_check", "subtree", "count_left_sample",
+    "count_left_sample_pick", "count_left_weighted", "stage_gather"};
 
 namespace {
 
@@ -48,6 +50,31 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;" :::);
 }
 
+// A level may not start when a cell of the level above was never finished (its arrivals
+// never completed) or an earlier step flagged an error: the build is flagged and its
+// remaining kernels do nothing (ORB_ERR_TIMEOUT).
+__device__ __forceinline__ bool level_failed(const Level &v) {
+    const volatile BuildCounters *ctr = v.counters;
+    if (ctr->error) return true;
+    if (v.prev_C && ctr->done[v.depth - 1] != v.prev_C) {
+        if (threadIdx.x == 0) atomicExch(&v.counters->error, 1u);
+        return true;
+    }
+    return false;
+}
+
+// Arrival at a counter, by one thread after a barrier of its CTA: the CTA's writes before the
+// barrier are visible to whoever sees the count. Returns the count before. Release only: a
+// __threadfence() also drops the SM's L1 lines, and one of those per tile (and thread) made
+// the swap 30% slower. Whoever finds itself last calls acquire() before it reads the others'
+// writes.
+__device__ __forceinline__ uint32_t arrive_release(uint32_t *counter, uint32_t k) {
+    uint32_t old;
+    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(counter), "r"(k) : "memory");
+    return old;
+}
+__device__ __forceinline__ void acquire() { __threadfence(); }
+
 // ------------------------------------------------------------------------------------
 // Block helpers
 // ------------------------------------------------------------------------------------
@@ -60,12 +87,6 @@ __device__ __forceinline__ uint32_t warp_sum(uint32_t v) {
 __device__ __forceinline__ uint32_t warp_max(uint32_t v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
-__device__ __forceinline__ uint32_t warp_min(uint32_t v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
 }
 
@@ -150,19 +171,6 @@ __device__ __forceinline__ uint2 block_excl_scan2(uint32_t a, uint32_t b, uint32
     return r;
 }
 
-// Largest c in [0, C] with off[c] <= t (off non-decreasing, off[0] = 0).
-__device__ __forceinline__ int find_cell(const uint32_t *off, int C, uint32_t t) {
-    int lo = 0, hi = C;  // invariant: off[lo] <= t, answer in [lo, hi]
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (off[mid] <= t)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    return lo;
-}
-
 // Visits every key of [e0, e1) once, float4 loads over the 16-byte aligned body.
 template <class F>
 __device__ __forceinline__ void for_keys(const float *__restrict__ keys, uint32_t e0, uint32_t e1,
@@ -195,7 +203,7 @@ struct TileRef {
 
 __device__ __forceinline__ TileRef tile_ref(const Level &v, uint32_t t) {
     TileRef r;
-    r.c = v.htile_cell ? (int)v.htile_cell[t] : find_cell(v.tile_off, v.C, t);
+    r.c = (int)v.htile_cell[t];
     r.slot = level_slot(v, r.c);
     r.local = t - v.tile_off[r.c];
     const uint2 rg = v.ranges[r.slot];
@@ -204,27 +212,133 @@ __device__ __forceinline__ TileRef tile_ref(const Level &v, uint32_t t) {
     return r;
 }
 
-// Capacity of a cell's compaction list: cells the histogram passes bisect (more than one
-// tile) get n/8 keys, at least 2048 (16x the sparse threshold's bracket): room for the
-// sampled bracket of a first pass (at most kPredCompactShare of the keys) and for the
-// bracket of a sparse pass.
-__host__ __device__ __forceinline__ uint32_t list_capacity(uint32_t n) {
-    return n > (uint32_t)kTile ? (n / 8 > 2048u ? n / 8 : 2048u) : 0u;
+// Slots of a cell's list: a cell whose bracket holds at most that many keys is finished on
+// the list (sparse_per_tile a count tile; the lists of a level fit n/8 + n/64 slots and 2048
+// a cell).
+__device__ __forceinline__ uint32_t list_capacity(const Level &v, uint32_t n) {
+    const unsigned long long want =
+        (unsigned long long)v.sparse_per_tile * ((n + (uint32_t)kTile - 1) / (uint32_t)kTile);
+    return (uint32_t)min(want, (unsigned long long)max(2048u, n / 64));
 }
 
-// Cells of more than kTile keys (the count passes' cells) get the deepest tree, so the cold
-// passes reach the iteration cap.
-static_assert(kTile >= (2 << kMaxBinsLog2), "cells of more than kTile keys get trees of depth 11");
 static_assert(kColdHistPasses * kMaxBinsLog2 >= kMaxIterations, "3 cold passes reach the cap");
-__device__ __forceinline__ int tree_depth(uint32_t n) {
-    int lg = 31 - __clz(max(n, 1u));  // floor(log2 n)
-    return max(4, min(kMaxBinsLog2, lg - 1));
+
+// ------------------------------------------------------------------------------------
+// Plan: a cell's tiles, histogram bins, list and state, set when the cell becomes known
+// (the root by init, a child when its parent is finished, service cells by k_plan). Tiles
+// and pool slots are taken from the level's totals with one or two atomics a cell, so no
+// scan over the level's cells and no launch of its own is needed; the order of the
+// allocations changes where scratch lies, never a result.
+// ------------------------------------------------------------------------------------
+struct PlanCell {
+    int c;           // the cell's index in its level (-1: not planned)
+    uint32_t t0, T;  // partition tiles
+    uint32_t h0, H;  // count tiles
+};
+
+// Warm builds: a cell whose previous tree cut on the same axis starts from the hinted bracket
+// (clipped to its extent) when that narrows it.
+__device__ __forceinline__ void warm_start_cell(const Level &v, int c, int slot, uint32_t n) {
+    orb_cell_t &cell = v.heap[slot];
+    const float2 h = v.hint[slot];
+    uint8_t w = 0;
+    if (n > 1 && !isnan(h.x) && v.hint_axis[slot] == cell.cutAxis && cell.cutAxis >= 0) {
+        // half-width w x extent / sqrt(n): about w sqrt(n) keys each side if evenly spread,
+        // the scale by which a median drifts when the particles move a little
+        const float L = cell.cutMarginLeft, R = cell.cutMarginRight;
+        const float half = __fdiv_rn(h.y, sqrtf((float)n));
+        const float Lw = fmaxf(L, __fsub_rn(h.x, half)), Rw = fminf(R, __fadd_rn(h.x, half));
+        if (Lw < Rw && (Lw > L || Rw < R)) {
+            cell.cutMarginLeft = Lw;
+            cell.cutMarginRight = Rw;
+            w = 1;
+            v.inb[c] = n - 1;  // the first pass counts the keys below the bracket
+            atomicAdd(&v.counters->warm_cells, 1u);
+        }
+    }
+    v.warm[c] = w;
+}
+
+// One thread: plans cell c (heap slot `slot`, particles [rg.x, rg.y)) with the totals `tot`;
+// cells of at most `small` particles get no count tiles.
+__device__ PlanCell plan_cell(const Level &v, PlanTotals *tot, uint32_t small, int c, int slot, uint2 rg) {
+    PlanCell p;
+    const uint32_t n = rg.y - rg.x;
+    p.c = c;
+    p.T = (n + (uint32_t)kPTile - 1) / (uint32_t)kPTile;
+    p.H = n > small ? (n + (uint32_t)kTile - 1) / (uint32_t)kTile : 0u;
+    p.t0 = p.h0 = 0;
+    if (p.T) {
+        const unsigned long long a =
+            atomicAdd(&tot->tiles, ((unsigned long long)p.H << 32) | (unsigned long long)p.T);
+        p.t0 = (uint32_t)a;
+        p.h0 = (uint32_t)(a >> 32);
+    }
+    v.ptile_off[c] = p.t0;
+    v.tile_off[c] = p.h0;
+    if (p.H && v.plan_bins) {
+        const unsigned long long a =
+            atomicAdd(&tot->pools, (1ull << 32) | (unsigned long long)list_capacity(v, n));
+        v.hist_off[c] = (uint32_t)(a >> 32) << kMaxBinsLog2;
+        v.cmp_off[c] = (uint32_t)a;
+    }
+    uint8_t st = kActive;
+    uint32_t it = 0;
+    if (n <= small && small) {
+        st = n <= (uint32_t)kWarpKeys ? kSmall : kOneTile;
+    } else if (n == 0) {
+        // no key: the first cut is found (src/orbit.cpp:204-213 with count 0)
+        st = kFound;
+        it = 1;
+        v.heap[slot].foundCut = 1;
+        atomicMax(&v.counters->max_iters, 1u);
+    }
+    v.state[c] = st;
+    v.iters[c] = (uint8_t)it;
+    v.hdone[c] = 0;
+    v.below[c] = 0;
+    v.inb[c] = n;
+    v.cmp_cnt[c] = 0;
+    v.pred[c] = 0u;  // no sampled bracket unless k_sample_pick sets one
+    if (v.wt) {
+        v.wbelow[c] = 0ull;
+        v.wtot[c] = 0ull;
+    }
+    if (v.hint) warm_start_cell(v, c, slot, n);
+    return p;
+}
+
+// The tile maps of a planned cell, by nt threads.
+__device__ __forceinline__ void plan_fill(const Level &v, const PlanCell &p, uint32_t ti, uint32_t nt) {
+    if (p.c < 0) return;
+    for (uint32_t t = ti; t < p.T; t += nt) v.ptile_cell[p.t0 + t] = (uint32_t)p.c;
+    for (uint32_t t = ti; t < p.H; t += nt) v.htile_cell[p.h0 + t] = (uint32_t)p.c;
+}
+
+// Plans every cell of the level, a warp per cell (service calls, and the levels a refused
+// subtree path leaves). The totals are zero.
+__global__ void __launch_bounds__(kThreads) k_plan(const __grid_constant__ Level v) {
+    pdl_enter();
+    const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    const uint32_t lane = threadIdx.x & 31;
+    if (c >= v.C) return;
+    PlanCell p = {};
+    if (lane == 0) {
+        const int slot = level_slot(v, c);
+        p = plan_cell(v, v.tot, v.small, c, slot, v.ranges[slot]);
+    }
+    p.c = c;
+    p.t0 = __shfl_sync(0xffffffffu, p.t0, 0);
+    p.T = __shfl_sync(0xffffffffu, p.T, 0);
+    p.h0 = __shfl_sync(0xffffffffu, p.h0, 0);
+    p.H = __shfl_sync(0xffffffffu, p.H, 0);
+    plan_fill(v, p, lane, 32);
 }
 
 // ------------------------------------------------------------------------------------
 // Init: identity permutation, zeroed heap/ranges, root cell (src/orbit.cpp:74-81)
 // ------------------------------------------------------------------------------------
-__global__ void k_init(Level v, uint32_t n, float lo0, float lo1, float lo2, float hi0,
+__global__ void k_init(const __grid_constant__ Level v, uint32_t n, float lo0, float lo1, float lo2, float hi0,
                        float hi1, float hi2, uint32_t d, int heap_cells) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -234,6 +348,9 @@ __global__ void k_init(Level v, uint32_t n, float lo0, float lo1, float lo2, flo
     const uint64_t words = (uint64_t)heap_cells * 13;
     for (uint64_t i = g + 13; i < words; i += stride) hw[i] = 0u;
     for (uint64_t i = g + 1; i < (uint64_t)heap_cells; i += stride) v.ranges[i] = make_uint2(0u, 0u);
+    // the root's tile maps (its index in level 1 is 0)
+    for (uint64_t i = g; i * kPTile < n; i += stride) v.ptile_cell[i] = 0u;
+    for (uint64_t i = g; i * kTile < n; i += stride) v.htile_cell[i] = 0u;
     if (g == 0) {
         orb_cell_t r;
         r.id = 0;
@@ -254,13 +371,15 @@ __global__ void k_init(Level v, uint32_t n, float lo0, float lo1, float lo2, flo
         v.ranges[0] = make_uint2(0u, n);
         BuildCounters z = {};
         *v.counters = z;
+        if (v.C) plan_cell(v, v.tot, v.small, 0, 0, make_uint2(0u, n));
     }
 }
 
 // Batched init: every instance's root cell and root range (heap and ranges are zeroed by
 // the host before) and idx = position relative to the instance. blockIdx.y walks the
 // instances, blockIdx.x their particles.
-__global__ void k_init_batch(Level v, const BatchRoot *roots, int k) {
+__global__ void k_init_batch(const __grid_constant__ Level v, const BatchRoot *roots, int k) {
+    __shared__ PlanCell s_plan;
     for (int i = blockIdx.y; i < k; i += gridDim.y) {
         const BatchRoot r = roots[i];
         if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -278,7 +397,15 @@ __global__ void k_init_batch(Level v, const BatchRoot *roots, int k) {
             c.cutMarginLeft = r.lower[0];  // setCutMargin, orbit.cpp:76
             c.cutMarginRight = r.upper[0];
             v.heap[r.heap_base] = c;
-            v.ranges[r.heap_base] = make_uint2(r.offset, r.offset + r.n);
+            const uint2 rg = make_uint2(r.offset, r.offset + r.n);
+            v.ranges[r.heap_base] = rg;
+            s_plan.c = -1;
+            if (r.cell >= 0) s_plan = plan_cell(v, v.tot, v.small, r.cell, (int)r.heap_base, rg);
+        }
+        if (blockIdx.x == 0) {
+            __syncthreads();
+            plan_fill(v, s_plan, threadIdx.x, blockDim.x);
+            __syncthreads();
         }
         if (v.idx)
             for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < r.n; p += gridDim.x * blockDim.x)
@@ -303,87 +430,6 @@ __device__ __forceinline__ void warm_reset(orb_cell_t &cell, float &L, float &R,
     cell.cutMarginLeft = L;
     cell.cutMarginRight = R;
     atomicAdd(&ctr->warm_resets, 1u);
-}
-
-// ------------------------------------------------------------------------------------
-// Plan: per-cell tile and histogram offsets (single CTA, any C).
-// ------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) k_plan(Level v) {
-    pdl_enter();
-    if (v.skip && *(volatile const uint32_t *)v.skip) return;  // subtrees took this level
-    __shared__ uint32_t sh[96];
-    const int C = v.C, tid = threadIdx.x, nt = blockDim.x;
-    const int per = (C + nt - 1) / nt;
-    const int c0 = min(C, tid * per), c1 = min(C, c0 + per);
-    uint32_t ta = 0, tb = 0, tp = 0, tc = 0;
-    for (int c = c0; c < c1; ++c) {
-        const uint2 rg = v.ranges[level_slot(v, c)];
-        const uint32_t n = rg.y - rg.x;
-        ta += (n + kTile - 1) / kTile;
-        tb += 1u << tree_depth(n);
-        tp += (n + kPTile - 1) / kPTile;
-        tc += list_capacity(n);
-    }
-    uint32_t tot_a, tot_b, tot_p, tot_c;
-    uint2 p = block_excl_scan2(ta, tb, sh, &tot_a, &tot_b);
-    const uint2 pc = block_excl_scan2(tp, tc, sh, &tot_p, &tot_c);
-    uint32_t pp = pc.x, cc = pc.y;
-    for (int c = c0; c < c1; ++c) {
-        const uint2 rg = v.ranges[level_slot(v, c)];
-        const uint32_t n = rg.y - rg.x;
-        v.tile_off[c] = p.x;
-        v.hist_off[c] = p.y;
-        v.ptile_off[c] = pp;
-        v.cmp_off[c] = cc;
-        pp += (n + kPTile - 1) / kPTile;
-        cc += list_capacity(n);
-        p.x += (n + kTile - 1) / kTile;
-        p.y += 1u << tree_depth(n);
-    }
-    if (tid == 0) {
-        v.tile_off[C] = tot_a;
-        v.hist_off[C] = tot_b;
-        v.ptile_off[C] = tot_p;
-        v.cmp_off[C] = tot_c;
-    }
-}
-
-// Warm builds, after the plan: a cell whose previous tree cut on the same axis starts from
-// the hinted bracket (clipped to its extent) when that narrows it. Its first count pass is
-// then sparse: most keys lie outside. One thread per cell.
-__global__ void k_warm_start(Level v) {
-    pdl_enter();
-    if (v.skip && *(volatile const uint32_t *)v.skip) return;  // subtrees took this level
-    const int c = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    uint32_t nwarm = 0;
-    if (c < v.C) {
-        const int slot = level_slot(v, c);
-        orb_cell_t &cell = v.heap[slot];
-        const uint2 rg = v.ranges[slot];
-        const uint32_t n = rg.y - rg.x;
-        const float2 h = v.hint[slot];
-        uint8_t w = 0;
-        if (n > 1 && !isnan(h.x) && v.hint_axis[slot] == cell.cutAxis && cell.cutAxis >= 0) {
-            // half-width w x extent / sqrt(n): about w sqrt(n) keys each side if evenly spread,
-            // the scale by which a median drifts when the particles move a little
-            const float L = cell.cutMarginLeft, R = cell.cutMarginRight;
-            const float half = __fdiv_rn(h.y, sqrtf((float)n));
-            const float Lw = fmaxf(L, __fsub_rn(h.x, half)), Rw = fminf(R, __fadd_rn(h.x, half));
-            if (Lw < Rw && (Lw > L || Rw < R)) {
-                cell.cutMarginLeft = Lw;
-                cell.cutMarginRight = Rw;
-                w = 1;
-                // keys in the bracket if spread evenly, capped so the first pass is sparse
-                const float share = __fdiv_rn(__fsub_rn(Rw, Lw), __fsub_rn(R, L));
-                const uint32_t tiles = (n + kTile - 1) / kTile;
-                v.inb[c] = min((uint32_t)fminf((float)n, ceilf(share * (float)n)), v.sparse_per_tile * tiles);
-                nwarm = 1;
-            }
-        }
-        v.warm[c] = w;
-    }
-    nwarm = warp_sum(nwarm);
-    if ((threadIdx.x & 31) == 0 && nwarm) atomicAdd(&v.counters->warm_cells, nwarm);
 }
 
 // ------------------------------------------------------------------------------------
@@ -578,97 +624,26 @@ __device__ __forceinline__ int fast_bin(float k, const Guess &g, int top, const 
 
 
 
-// A sparse pass sends its bracket keys to the cell's global bins, or to shared bins first
-// when its bracket holds more than kSparseGlobalKeys keys a tile.
-constexpr uint32_t kSparseGlobalKeys = 8;
-constexpr int kCmpTile = 2048;  // bracket keys a CTA compacts for one cell's run of tiles, or
-                                // for one tile of a sampled pass (more: the cell keeps no list)
-
 // The cell a count pass's CTA is working on, in shared memory (thread 0 fills it when the
 // CTA's tiles move to a new cell): the rare paths read it there, so the streaming loop keeps
 // only what it needs in registers.
-constexpr uint32_t kHDense = 1, kHLocal = 2, kHCompact = 4, kHListed = 8, kHPred = 16;
+constexpr uint32_t kHDense = 1, kHBracket = 2, kHPred = 4;
 struct HistCell {
     const float *keys;  // the cut axis
     uint32_t *gh;       // the cell's global bins
-    float L, R, scale;
-    int K;
-    uint32_t mode;      // kHDense, kHPred (sampled bracket; kHCompact: its keys to the
-                        // list), else sparse (kHLocal: bracket keys to shared bins first;
-                        // kHCompact: and to the list), or kHListed
+    float L, R;
+    uint32_t mode;      // kHDense (first pass over the extent: nearly every key inside
+                        // [L, R)), kHBracket (many keys outside) or kHPred (sampled bracket)
     uint32_t base, end; // the cell's key range [base, end)
     uint32_t t0;        // its first tile
     uint32_t below;     // dense: keys below L met by the exact path
     float pa, pb;       // kHPred: the sampled bracket [e(lo), e(hi)) of the tree over [L, R)
-    Guess gs;           // dense and kHPred: the scaled guess
+    Guess gs;           // the scaled guess
+    uint32_t whole;     // the CTA read every tile of the cell: its bins and count are complete
+    uint32_t last;      // the CTA finished the cell's last tile
 };
-
-// Count pass over a cell whose bracket keys an earlier pass compacted: tile j of the cell's
-// t tiles takes the j-th of t equal runs of the list and bins its keys inside [L, R) (the
-// keys below L are already counted: resolve carried them). Returns the keys read.
-__device__ __noinline__ uint32_t listed_tile(const Level &v, int c, uint32_t local, const HistCell *hc) {
-    const float L = hc->L, R = hc->R;
-    const int K = hc->K;
-    uint32_t *gh = hc->gh;
-    const uint32_t cnt = v.cmp_cnt[c];
-    // the list split evenly over the cell's tiles, so the CTAs of all of them share it
-    const uint32_t tiles = v.tile_off[c + 1] - v.tile_off[c];
-    const uint32_t chunk = (cnt + tiles - 1) / tiles;
-    const uint32_t lo = local * chunk, hi = min(cnt, lo + chunk);
-    const float *list = v.cmp_keys + v.cmp_off[c];
-    for (uint32_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-        const float k = list[i];
-        if (k >= L && k < R) atomicAdd(&gh[tree_bin(k, L, R, K)], 1u);
-    }
-    return hi > lo ? hi - lo : 0u;
-}
-
-// Appends the bracket keys a CTA compacted for cell c (*s_ncmp of them in s_cmp) to the cell's
-// list and clears the count: one reservation per run of the cell's tiles; an overflow (of the
-// buffer or the list) marks the cell as having no list. Returns the keys written. Every
-// thread of the CTA calls it once its scans are done.
-__device__ __noinline__ uint32_t append_list(const Level &v, int c, const float *s_cmp, uint32_t *s_ncmp,
-                                             uint32_t *s_base) {
-    __syncthreads();  // every key of the tile kept
-    const uint32_t nk = *s_ncmp;
-    if (threadIdx.x == 0) {
-        const uint32_t cap = v.cmp_off[c + 1] - v.cmp_off[c];
-        *s_base = 0xffffffffu;
-        if (nk > (uint32_t)kCmpTile) {
-            v.cmp_bad[c] = 1;
-        } else if (nk) {
-            const uint32_t b = atomicAdd(&v.cmp_cnt[c], nk);
-            if (b + nk > cap)
-                v.cmp_bad[c] = 1;
-            else
-                *s_base = b;
-        }
-    }
-    __syncthreads();
-    const uint32_t b = *s_base;
-    if (threadIdx.x == 0) *s_ncmp = 0;
-    uint32_t wrote = 0;
-    if (b != 0xffffffffu) {
-        float *list = v.cmp_keys + v.cmp_off[c] + b;
-        for (uint32_t i = threadIdx.x; i < nk; i += blockDim.x) list[i] = s_cmp[i];
-        wrote = nk;
-    }
-    __syncthreads();  // s_cmp and the count are reused by the next tile
-    return wrote;
-}
-
-// A sparse pass's bracket key (L <= k < R): into the cell's bins (shared when kHLocal) and,
-// with kHCompact, into the tile's list buffer.
-__device__ __forceinline__ void sparse_key(float k, const HistCell *hc, uint32_t *s_hist, float *s_cmp,
-                                        uint32_t *s_ncmp) {
-    const uint32_t mode = hc->mode;
-    const uint32_t b = (uint32_t)tree_bin(k, hc->L, hc->R, hc->K);
-    atomicAdd(mode & kHLocal ? &s_hist[b] : &hc->gh[b], 1u);
-    if (mode & kHCompact) {
-        const uint32_t i = atomicAdd(s_ncmp, 1u);
-        if (i < (uint32_t)kCmpTile) s_cmp[i] = k;
-    }
-}
+constexpr int kHistK = kMaxBinsLog2;  // depth of the count passes' midpoint trees
+constexpr uint32_t kHistBins = 1u << kHistK;
 
 // A dense pass's key the scaled guess did not settle: below L counted, inside [L, R) binned
 // by the edge table (near_bin), at or past R (or NaN) ignored.
@@ -677,28 +652,15 @@ __device__ __forceinline__ void dense_exact(float k, HistCell *hc, uint32_t *s_h
     if (k < L)
         atomicAdd(&hc->below, 1u);
     else if (k < R)
-        atomicAdd(&s_hist[near_bin(k, hc->gs, s_edge, (1u << hc->K) - 1u)], 1u);
+        atomicAdd(&s_hist[near_bin(k, hc->gs, s_edge, kHistBins - 1u)], 1u);
 }
 
 // A sampled pass's bracket key (e(lo) <= k < e(hi), inside [L, R)): its bin by the scaled
-// guess (the edge table when the guess is not proven) into the shared bins and,
-// when the pass compacts, into the tile's list buffer (one shared reservation for the
-// threads that arrive together).
-__device__ __noinline__ void pred_key(float k, const HistCell *hc, uint32_t *s_hist, float *s_cmp,
-                                      uint32_t *s_ncmp, const float *s_edge) {
+// guess (the edge table when the guess is not proven) into the shared bins.
+__device__ __noinline__ void pred_key(float k, const HistCell *hc, uint32_t *s_hist, const float *s_edge) {
     uint32_t g;
-    if (!guess_bin(hc->gs, k, &g)) g = near_bin(k, hc->gs, s_edge, (1u << hc->K) - 1u);
+    if (!guess_bin(hc->gs, k, &g)) g = near_bin(k, hc->gs, s_edge, kHistBins - 1u);
     atomicAdd(&s_hist[g], 1u);
-    if (hc->mode & kHCompact) {
-        const uint32_t m = __activemask();
-        const uint32_t lane = threadIdx.x & 31u;
-        const uint32_t leader = (uint32_t)__ffs(m) - 1u;
-        uint32_t base = 0;
-        if (lane == leader) base = atomicAdd(s_ncmp, (uint32_t)__popc(m));
-        base = __shfl_sync(m, base, (int)leader);
-        const uint32_t i = base + (uint32_t)__popc(m & ((1u << lane) - 1u));
-        if (i < (uint32_t)kCmpTile) s_cmp[i] = k;
-    }
 }
 
 // A compile-time flag passed to a generic lambda.
@@ -860,18 +822,22 @@ __device__ __forceinline__ void dense_tile(const float *keys, uint32_t e0, uint3
     for (uint32_t i = a0 + (n4 << 2) + ti; i < e1; i += kThreads) one(__ldg(keys + i));
 }
 
-// A sparse pass's tile [e0, e1): keys below L counted in `below`, keys inside [L, R) (a few a
-// tile) handed to key(k) right after their round, keys at or above R and NaN ignored. Same
-// rounds as dense_tile.
-template <class Key>
-__device__ __forceinline__ void sparse_tile(const float *keys, uint32_t e0, uint32_t e1, float L, float R,
-                                            uint32_t &below, Key key) {
+// A later pass's tile [e0, e1): keys below L counted in `below`, keys inside [L, R) binned by
+// the scaled guess (a key the guess does not settle exactly right after its round), keys at
+// or above R and NaN ignored. Same rounds as dense_tile; a key outside the bracket costs its
+// comparisons only (the dense loop would send each one through the exact path: clustered
+// cells' second passes ran at 1.7 TB/s that way).
+__device__ __forceinline__ void bracket_tile(const float *keys, uint32_t e0, uint32_t e1, const Guess gs, float L,
+                                             float R, uint32_t &below, uint32_t *s_hist, const float *s_edge) {
     const uint32_t ti = threadIdx.x;
     auto one = [&](float k) {
-        if (k < L)
+        if (k < L) {
             ++below;
-        else if (k < R)
-            key(k);
+        } else if (k < R) {
+            uint32_t g;
+            if (!guess_bin(gs, k, &g)) g = near_bin(k, gs, s_edge, kHistBins - 1u);
+            atomicAdd(&s_hist[g], 1u);
+        }
     };
     const uintptr_t addr = reinterpret_cast<uintptr_t>(keys + e0);
     const uint32_t a0 = min(e1, e0 + (uint32_t)(((16u - (addr & 15u)) & 15u) >> 2));
@@ -892,13 +858,17 @@ __device__ __forceinline__ void sparse_tile(const float *keys, uint32_t e0, uint
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 if (kk[c] < L) ++below;
-                if (kk[c] >= L && kk[c] < R) miss |= 1u << (4 * u + c);
+                uint32_t g;
+                const bool ok = guess_bin(gs, kk[c], &g);
+                if (ok) atomicAdd(&s_hist[g], 1u);
+                if (!ok && kk[c] >= L && kk[c] < R) miss |= 1u << (4 * u + c);
             }
         }
         while (miss) {
             const uint32_t b = (uint32_t)__ffs(miss) - 1u;
             miss &= miss - 1u;
-            key(__ldg(kb + 4 * (j0 + (b >> 2) * kThreads + ti) + (b & 3u)));
+            const float k = __ldg(kb + 4 * (j0 + (b >> 2) * kThreads + ti) + (b & 3u));
+            atomicAdd(&s_hist[near_bin(k, gs, s_edge, kHistBins - 1u)], 1u);
         }
     }
     for (uint32_t j = j0 + ti; j < n4; j += kThreads) {
@@ -911,13 +881,6 @@ __device__ __forceinline__ void sparse_tile(const float *keys, uint32_t e0, uint
     for (uint32_t i = a0 + (n4 << 2) + ti; i < e1; i += kThreads) one(__ldg(keys + i));
 }
 
-// Whether pass v.pass over cell c (`tiles` tiles) is sparse: only the bracket's keys are
-// binned, the keys below it counted. The first pass of a cold level is dense for every cell;
-// later passes are sparse once the bracket holds at most sparse_per_tile keys a tile.
-__device__ __forceinline__ bool sparse_pass(const Level &v, int c, uint32_t tiles) {
-    return !(v.pass == 0 && v.warm == nullptr) && v.inb[c] <= v.sparse_per_tile * tiles;
-}
-
 // ------------------------------------------------------------------------------------
 // Sampled first pass. The first count pass of a cold level bins every key of a cell into
 // the 2^K leaves of its midpoint tree. k_sample_bin and k_sample_pick predict from a strided
@@ -925,15 +888,15 @@ __device__ __forceinline__ bool sparse_pass(const Level &v, int c, uint32_t tile
 // (one key per 2^kSampleShift) a run of leaves [lo, hi) holding the cut: the sample's
 // median +- pred_sigmas standard errors (sqrt(s)/2 sample keys), widened to leaf edges
 // a = e(lo), b = e(hi). That pass then counts the keys below a and bins only the keys of
-// [a, b). Its replay in k_resolve is the reference loop unchanged once the exact counts
+// [a, b). Its replay in resolve_cell is the reference loop unchanged once the exact counts
 // show count(< a) with difference <= -3 and count(< b) with difference >= 3: every tested
 // cut below a then has a count <= count(< a) and moves L, every cut above b has one
 // >= count(< b) and moves R (the float test is monotone in the count), and cuts inside
 // [a, b] get their exact counts from the bins. Otherwise the pass is discarded and the
 // next one bins every key. Same cuts, same integer counts, same iterations either way.
-// (k_resolve checks the counts; sample sizes and widths only change the speed.)
+// (resolve_cell checks the counts; sample sizes and widths only change the speed.)
 // ------------------------------------------------------------------------------------
-constexpr uint32_t kPredValid = 1u << 25, kPredCompact = 1u << 24;
+constexpr uint32_t kPredValid = 1u << 25;
 __device__ __forceinline__ uint32_t pred_lo(uint32_t p) { return p & 0xfffu; }
 __device__ __forceinline__ uint32_t pred_hi(uint32_t p) { return (p >> 12) & 0xfffu; }
 constexpr int kSampleThreads = 256;
@@ -941,10 +904,6 @@ constexpr int kSampleShift = 8;              // one sample key per 256 keys of t
 constexpr uint32_t kSampleMax = 16384;       // sample keys per cell at most
 constexpr uint32_t kSampleMin = 1024;        // fewer: no prediction (a dense first pass)
 constexpr uint32_t kSamplePerCta = 4 * kSampleThreads;
-constexpr float kPredCompactShare = 0.09f;   // compact the bracket keys when the sample puts
-                                             // at most this share of the cell inside it
-static_assert(kPredCompactShare * kTile * 1.25f < kCmpTile, "a tile's bracket keys fit the buffer");
-
 __device__ __forceinline__ uint32_t sample_count(uint32_t n) {
     const uint32_t ns = min(n >> kSampleShift, kSampleMax);
     return ns >= kSampleMin ? ns : 0u;
@@ -955,9 +914,9 @@ __device__ __forceinline__ uint32_t sample_count(uint32_t n) {
 // ((2j+1) n / (2 ns)) (fixed point), binned into the cell's histogram bins (all zero
 // between passes) by the scaled guess or the descent; samples below L are counted in
 // pred[c], which k_sample_pick then replaces by the prediction.
-__global__ void __launch_bounds__(kSampleThreads) k_sample_bin(Level v) {
+__global__ void __launch_bounds__(kSampleThreads) k_sample_bin(const __grid_constant__ Level v) {
     pdl_enter();
-    if (v.skip && *(volatile const uint32_t *)v.skip) return;  // subtrees took this level
+    if (level_failed(v)) return;
     const uint32_t ti = threadIdx.x;
     for (int c = blockIdx.y; c < v.C; c += gridDim.y) {
         if (v.state[c] != kActive) continue;
@@ -969,8 +928,8 @@ __global__ void __launch_bounds__(kSampleThreads) k_sample_bin(Level v) {
         if (j0 >= ns) continue;
         const orb_cell_t &cell = v.heap[slot];
         const float L = cell.cutMarginLeft, R = cell.cutMarginRight;
-        const int K = v.hist_k[c];
-        const uint32_t nb = 1u << K;
+        constexpr int K = kHistK;
+        constexpr uint32_t nb = kHistBins;
         const float *keys = axis_keys(v, eff_axis(cell.cutAxis)) + rg.x;
         uint32_t *gh = v.hist + v.hist_off[c];
         // (2j+1) step >> 17 < n for j < ns: step = floor(n 2^16 / ns) < 2^37, products < 2^52
@@ -1005,9 +964,9 @@ __global__ void __launch_bounds__(kSampleThreads) k_sample_bin(Level v) {
 // again. Each thread holds 8 consecutive bins in registers.
 constexpr int kPickThreads = 256;
 static_assert((1 << kMaxBinsLog2) == 8 * kPickThreads, "8 bins a thread");
-__global__ void __launch_bounds__(kPickThreads) k_sample_pick(Level v) {
+__global__ void __launch_bounds__(kPickThreads) k_sample_pick(const __grid_constant__ Level v) {
     pdl_enter();
-    if (v.skip && *(volatile const uint32_t *)v.skip) return;  // subtrees took this level
+    if (level_failed(v)) return;
     __shared__ uint32_t s_red[72];
     const uint32_t ti = threadIdx.x;
     for (int c = blockIdx.x; c < v.C; c += gridDim.x) {
@@ -1015,7 +974,7 @@ __global__ void __launch_bounds__(kPickThreads) k_sample_pick(Level v) {
         const uint2 rg = v.ranges[level_slot(v, c)];
         const uint32_t ns = sample_count(rg.y - rg.x);
         if (!ns) continue;
-        const uint32_t nb = 1u << v.hist_k[c];
+        constexpr uint32_t nb = kHistBins;
         uint4 *gh4 = reinterpret_cast<uint4 *>(v.hist + v.hist_off[c]);
         const uint32_t below = v.pred[c];  // samples below L
         // thread t owns leaves [8t, 8t + 8) (none past nb)
@@ -1055,21 +1014,10 @@ __global__ void __launch_bounds__(kPickThreads) k_sample_pick(Level v) {
         n_lt = block_sum(n_lt, s_red);
         // lo: the last edge with at most r_lo samples below it; hi: the first with at least r_hi
         const uint32_t lo = n_le ? n_le - 1u : 0u, hi = min(n_lt, nb);
-        uint32_t ca = 0, cb = 0;
-        cum = below + pre;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            if (8 * ti + i == lo) ca = cum;
-            if (8 * ti + i == hi) cb = cum;
-            cum += h[i];
-        }
-        ca = block_sum(ca, s_red);
-        cb = hi == nb ? below + total : block_sum(cb, s_red);
         if (ti == 0) {
             uint32_t p = 0u;
             if (n_le > 0 && lo < hi && (lo > 0 || hi < nb)) {
-                const float share = (float)(cb - ca) / (float)ns;
-                p = lo | (hi << 12) | kPredValid | (share <= kPredCompactShare ? kPredCompact : 0u);
+                p = lo | (hi << 12) | kPredValid;
                 atomicAdd(&v.counters->pred_cells, 1u);
             }
             v.pred[c] = p;
@@ -1078,75 +1026,183 @@ __global__ void __launch_bounds__(kPickThreads) k_sample_pick(Level v) {
     }
 }
 
-// One count-left pass over the tiles of the level's active cells (cells of more than one
-// tile), a tile loop over all CTAs. Dense cells are binned into a shared-memory histogram
-// added to the cell's global bins; sparse cells (few keys in the bracket, known from the
-// previous pass) count the keys below the bracket and send the bracket's keys to the global
-// bins (to shared bins first when there are more than a few a tile). Each CTA takes a run of
-// consecutive tiles (runs of equal length to one tile); a cell's shared bins, count below
-// and compacted keys stay with the CTA while its tiles follow one another and are added to
-// the global ones once per run.
+// Replay of up to 11 iterations of the reference loop (src/orbit.cpp:146-232) on the finished
+// histogram of cell c, by the CTA that finished its last tile (every thread; hc describes the
+// cell). The bins are read, cleared and turned into prefix counts in shared memory, so a step
+// is one shared load and the float test. The cell then is found, capped, ready (its bracket's
+// keys fit a list: the classify pass lists them, k_part_cells goes on) or active for the next
+// pass. Fused here: as a kernel of its own behind every pass it took 9-10 us a launch, three
+// times a level, most of it launch and load latency.
+__device__ __noinline__ void resolve_cell(const Level &v, int c, const HistCell *hc, uint32_t *s_hist, uint32_t *s_red) {
+    static_assert(kHistBins == 8 * kThreads, "8 bins a thread");
+    const uint32_t tid = threadIdx.x;
+    uint4 a, b;
+    if (hc->whole) {
+        a = reinterpret_cast<const uint4 *>(s_hist)[2 * tid];
+        b = reinterpret_cast<const uint4 *>(s_hist)[2 * tid + 1];
+    } else {
+        uint4 *g4 = reinterpret_cast<uint4 *>(hc->gh) + 2 * tid;
+        a = __ldcg(g4);  // other CTAs' atomics: from L2
+        b = __ldcg(g4 + 1);
+        g4[0] = make_uint4(0u, 0u, 0u, 0u);
+        g4[1] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    const uint32_t h[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t loc = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) loc += h[j];
+    uint32_t tot, unused;
+    uint32_t run = block_excl_scan2(loc, 0u, s_red, &tot, &unused).x;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        s_hist[8 * tid + j] = run;
+        run += h[j];
+    }
+    __syncthreads();
+    if (tid >= 32) return;  // one warp replays (identically in every lane)
+    const int slot = level_slot(v, c);
+    orb_cell_t &cell = v.heap[slot];
+    const uint32_t n = hc->end - hc->base;
+    const float ratio = leaf_ratio(cell.nLeafCells);  // src/orbit.cpp:204
+    float L = hc->L, R = hc->R;
+    uint32_t it = v.iters[c];
+    const uint32_t below = hc->whole ? hc->below : __ldcg(&v.below[c]);
+    const uint32_t pr = v.pass == 0 ? v.pred[c] : 0u;
+    const bool warm = v.warm && v.warm[c];
+    // a sampled or hinted bracket must hold the cut (see k_sample_bin, warm_bracket_holds);
+    // else the pass is discarded and the next one bins the whole extent
+    const bool pred_miss = (pr & kPredValid) && !(convergence(below, n, ratio) < 0 && convergence(below + tot, n, ratio) > 0);
+    const bool warm_miss = warm && !warm_bracket_holds(below, below + tot, n, ratio);
+    __syncwarp();
+    if (pred_miss || warm_miss) {
+        if (tid == 0) {
+            if (pred_miss) atomicAdd(&v.counters->pred_misses, 1u);
+            if (warm_miss) {
+                warm_reset(cell, L, R, v.counters);
+                v.warm[c] = 0;
+            }
+            v.inb[c] = n;
+            v.below[c] = 0;
+            v.hdone[c] = 0;
+            v.counters->any_active[v.pass] = 1u;
+        }
+        return;
+    }
+    uint32_t pos = 0, width = kHistBins;
+    uint8_t st = kActive;
+    for (int step = 0; step < kHistK; ++step) {
+        if (it >= (uint32_t)kMaxIterations) break;
+        const uint32_t half = width >> 1;
+        const uint32_t cl = below + s_hist[pos + half];
+        ++it;
+        const int dir = convergence(cl, n, ratio);
+        if (dir == 0) {
+            st = kFound;
+            break;
+        }
+        const float cut = mid_cut(L, R);
+        if (dir > 0) {
+            R = cut;
+        } else {
+            L = cut;
+            pos += half;
+        }
+        width = half;
+    }
+    if (st == kActive && it >= (uint32_t)kMaxIterations) st = kCapped;
+    if (tid != 0) return;
+    cell.cutMarginLeft = L;
+    cell.cutMarginRight = R;
+    cell.foundCut = st == kFound ? 1 : 0;
+    v.iters[c] = (uint8_t)it;
+    v.hdone[c] = 0;
+    if (warm) v.warm[c] = 0;
+    if (st == kActive) {
+        // keys in the bracket the next step looks at, and keys below it
+        const uint32_t inb = (pos + 1 < kHistBins ? s_hist[pos + 1] : tot) - s_hist[pos];
+        v.inb[c] = inb;
+        if (inb <= list_capacity(v, n)) {
+            st = kReady;
+            v.below[c] = below + s_hist[pos];
+        } else {
+            v.below[c] = 0;
+            v.counters->any_active[v.pass] = 1u;
+            // the last pass leaves no cell active (tree depth 11): flag it if one does
+            if (v.pass == v.last_pass) atomicExch(&v.counters->error, 1u);
+        }
+    } else {
+        atomicMax(&v.counters->max_iters, it);
+        if (st == kCapped) atomicAdd(&v.counters->unfound, 1u);
+    }
+    v.state[c] = st;
+}
+
+// One count-left pass over the tiles of the level's active cells, a tile loop over all CTAs.
+// A cell's keys are binned into a shared-memory histogram added to the cell's global bins.
+// Each CTA takes a run of consecutive tiles (runs of equal length to one tile); a cell's
+// shared bins and count below stay with the CTA while its tiles follow one another and are
+// added to the global ones once per run; the CTA that brings a cell's last tile resolves it.
 // Allowed: the modes this instance handles (the other paths are compiled out, which keeps
 // each instance's streaming loop within its registers): kHFirstDense, the first pass of a
 // cold level without sampled brackets (every cell dense); kHFirstSampled, the first pass of
 // a sampled level (sampled or dense cells); kHRest, every other pass.
-constexpr uint32_t kHSparse = 32;  // (allowed only) the sparse modes
 constexpr uint32_t kHFirstDense = kHDense;
-constexpr uint32_t kHFirstSampled = kHDense | kHPred | kHCompact;
-constexpr uint32_t kHRest = kHDense | kHLocal | kHCompact | kHListed | kHSparse;
+constexpr uint32_t kHFirstSampled = kHDense | kHPred;
+constexpr uint32_t kHRest = kHDense | kHBracket;
 template <uint32_t Allowed>
-__global__ void __launch_bounds__(kThreads, kHistBlocksPerSm) k_hist(Level v) {
+__global__ void __launch_bounds__(kThreads, kHistBlocksPerSm) k_hist(const __grid_constant__ Level v) {
     pdl_enter();
-    if (v.skip && *(volatile const uint32_t *)v.skip) return;  // subtrees took this level
-    constexpr bool kAny = Allowed != kHDense;
-    __shared__ uint32_t s_hist[(1 << kMaxBinsLog2) + 32];  // + the dense loop's spare bins
-    __shared__ float s_edge[(1 << kMaxBinsLog2) + 1];      // dense and sampled: the tree's edges
-    __shared__ uint32_t s_red[32];
-    __shared__ float s_cmp[(Allowed & kHCompact) ? kCmpTile : 1];  // bracket keys on their way to the list
-    __shared__ uint32_t s_ncmp, s_base;
+    __shared__ __align__(16) uint32_t s_hist[kHistBins + 32];  // + the dense loop's spare bins
+    __shared__ float s_edge[kHistBins + 1];                    // the tree's edges
+    __shared__ uint32_t s_red[72];
     __shared__ HistCell s_hc;
     __shared__ uint32_t s_run[2];           // the CTA's tiles [first, end)
     __shared__ unsigned long long s_bytes;  // thread 0's count of bytes read
-    if (blockIdx.x == 0 && threadIdx.x == 0) v.counters->any_active[v.pass & 1] = 0u;
+    if (v.pass == 0 && level_failed(v)) return;
     // every cell of the level finished in an earlier pass: nothing to bin
-    if (v.pass > 0 && *(volatile uint32_t *)&v.counters->any_active[(v.pass - 1) & 1] == 0u) return;
+    if (v.pass > 0 && *(volatile uint32_t *)&v.counters->any_active[v.pass - 1] == 0u) return;
     if (threadIdx.x == 0) {
-        const uint64_t total = v.tile_off[v.C];
+        const uint64_t total = v.tot->tiles >> 32;
         s_run[0] = (uint32_t)(total * blockIdx.x / gridDim.x);
         s_run[1] = (uint32_t)(total * (blockIdx.x + 1) / gridDim.x);
         s_bytes = 0;
-        s_ncmp = 0;
     }
     __syncthreads();
-    int cur = -1;        // the cell s_hc describes (every thread follows it)
-    uint32_t below = 0;  // sparse: this thread's keys below L in the cell's tiles so far
-    // the current cell's count below L and its shared bins to the global ones
+    int cur = -1;         // the cell s_hc describes (every thread follows it)
+    uint32_t ntiles = 0;  // the CTA's tiles of it so far
+    uint32_t below = 0;   // this thread's keys below L in them
+    // the current cell's count below L and its shared bins to the global ones; then, with the
+    // cell's last tile, its replay
     auto end_cell = [&]() {
         below = block_sum(below, s_red);
-        const uint32_t mode = s_hc.mode;
+        const uint32_t tiles = (s_hc.end - s_hc.base + (uint32_t)kTile - 1) / (uint32_t)kTile;
+        const bool whole = ntiles == tiles;  // CTA-uniform: nothing to add up with other CTAs
         if (threadIdx.x == 0) {
             const uint32_t tot = below + s_hc.below;
-            if (tot) atomicAdd(&v.below[cur], tot);
+            s_hc.whole = s_hc.last = whole ? 1u : 0u;
+            s_hc.below = tot;
+            if (tot && !whole) atomicAdd(&v.below[cur], tot);
         }
-        if (mode & (kHDense | kHLocal | kHPred)) {
-            const uint32_t nb = 1u << s_hc.K;
+        if (!whole) {
             uint32_t *gh = s_hc.gh;
-            for (uint32_t b = threadIdx.x; b < nb; b += kThreads) {
+            for (uint32_t b = threadIdx.x; b < kHistBins; b += kThreads) {
                 const uint32_t h = s_hist[b];
                 if (h) atomicAdd(&gh[b], h);
             }
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                s_hc.last = arrive_release(&v.hdone[cur], ntiles) + ntiles == tiles;
+                if (s_hc.last) acquire();
+            }
         }
-        if ((Allowed & kHCompact) && (mode & kHCompact)) {
-            const uint32_t wrote = append_list(v, cur, s_cmp, &s_ncmp, &s_base);
-            if (threadIdx.x == 0) s_bytes += 4ull * wrote;
-        }
+        __syncthreads();
+        if (s_hc.last) resolve_cell(v, cur, &s_hc, s_hist, s_red);
         __syncthreads();  // s_hc and s_hist free for the next cell
         below = 0;
+        ntiles = 0;
     };
     const uint32_t t_end = s_run[1];
-    auto tile_cell = [&](uint32_t t) {
-        return t < t_end ? (v.htile_cell ? (int)v.htile_cell[t] : find_cell(v.tile_off, v.C, t)) : -1;
-    };
+    auto tile_cell = [&](uint32_t t) { return t < t_end ? (int)v.htile_cell[t] : -1; };
     int c_next = tile_cell(s_run[0]);
     int skip_c = -1;  // an inactive cell whose tiles are being passed over
     for (uint32_t t = s_run[0]; t < t_end; ++t) {
@@ -1154,6 +1210,8 @@ __global__ void __launch_bounds__(kThreads, kHistBlocksPerSm) k_hist(Level v) {
         c_next = tile_cell(t + 1);  // the next tile's cell, loaded while this tile is read
         if (c == skip_c) continue;
         if (c != cur) {
+            // a cell with a tile still to come is not resolved in this pass, so its state
+            // stands while this CTA reads it
             if (v.state[c] != kActive) {  // the run's tiles of a cell are consecutive
                 skip_c = c;
                 continue;
@@ -1164,65 +1222,41 @@ __global__ void __launch_bounds__(kThreads, kHistBlocksPerSm) k_hist(Level v) {
                 const int slot = level_slot(v, c);
                 const orb_cell_t &cell = v.heap[slot];
                 const uint2 rg = v.ranges[slot];
-                const uint32_t t0 = v.tile_off[c], tiles = v.tile_off[c + 1] - t0;
                 const float L = cell.cutMarginLeft, R = cell.cutMarginRight;
-                const int K = v.hist_k[c];
-                const uint32_t nb = 1u << K;
-                const float scale = __fdiv_rn((float)nb, __fsub_rn(R, L));
-                uint32_t mode;
-                const uint32_t pr = (Allowed & kHPred) && v.pass == 0 && v.pred ? v.pred[c] : 0u;
-                if (!kAny)
-                    mode = kHDense;  // a cold first pass without sampled brackets
-                else if ((Allowed & kHListed) && v.listed[c])
-                    mode = kHListed;
-                else if (pr & kPredValid)
-                    mode = kHPred | (pr & kPredCompact ? kHCompact : 0u);
-                else if (!sparse_pass(v, c, tiles))
-                    mode = kHDense;
-                else
-                    // more than a few bracket keys a tile: shared bins first; more than a few a
-                    // bin after this pass (a further pass follows): compacted into the list
-                    mode = (v.inb[c] > kSparseGlobalKeys * tiles ? kHLocal : 0u) |
-                           (v.inb[c] > (8u << K) ? kHCompact : 0u);
+                const uint32_t pr = (Allowed & kHPred) ? v.pred[c] : 0u;
+                uint32_t mode = kHDense;
+                if (pr & kPredValid)
+                    mode = kHPred;
+                else if ((Allowed & kHBracket) && v.inb[c] != rg.y - rg.x)
+                    mode = kHBracket;
                 s_hc.keys = axis_keys(v, eff_axis(cell.cutAxis));
                 s_hc.gh = v.hist + v.hist_off[c];
                 s_hc.L = L;
                 s_hc.R = R;
-                s_hc.scale = scale;
-                s_hc.K = K;
                 s_hc.mode = mode;
                 s_hc.base = rg.x;
                 s_hc.end = rg.y;
-                s_hc.t0 = t0;
+                s_hc.t0 = v.tile_off[c];
                 s_hc.below = 0;
-                s_hc.pa = pr & kPredValid ? tree_edge(L, R, K, pred_lo(pr)) : L;
-                s_hc.pb = pr & kPredValid ? tree_edge(L, R, K, pred_hi(pr)) : R;
-                s_hc.gs = make_guess(L, R, scale, nb);
+                s_hc.pa = pr & kPredValid ? tree_edge(L, R, kHistK, pred_lo(pr)) : L;
+                s_hc.pb = pr & kPredValid ? tree_edge(L, R, kHistK, pred_hi(pr)) : R;
+                s_hc.gs = make_guess(L, R, __fdiv_rn((float)kHistBins, __fsub_rn(R, L)), kHistBins);
             }
             __syncthreads();
-            if (s_hc.mode & (kHDense | kHLocal | kHPred)) {
-                for (uint32_t j = threadIdx.x; j < (1u << s_hc.K); j += kThreads) s_hist[j] = 0u;
-                if (s_hc.mode & (kHDense | kHPred))
-                    fill_edges(s_edge, s_hc.L, s_hc.R, s_hc.K, threadIdx.x, kThreads);
-                __syncthreads();
-            }
+            for (uint32_t j = threadIdx.x; j < kHistBins; j += kThreads) s_hist[j] = 0u;
+            fill_edges(s_edge, s_hc.L, s_hc.R, kHistK, threadIdx.x, kThreads);
+            __syncthreads();
         }
-        const uint32_t local = t - s_hc.t0;
+        ++ntiles;
         const uint32_t mode = s_hc.mode;
-        if ((Allowed & kHListed) && (mode & kHListed)) {
-            const uint32_t nread = listed_tile(v, c, local, &s_hc);
-            if (threadIdx.x == 0) s_bytes += 4ull * nread;
-            continue;
-        }
-        const uint32_t e0 = s_hc.base + local * (uint32_t)kTile;
+        const uint32_t e0 = s_hc.base + (t - s_hc.t0) * (uint32_t)kTile;
         const uint32_t e1 = min(s_hc.end, e0 + (uint32_t)kTile);
         const float *keys = s_hc.keys;
         if ((Allowed & kHPred) && (mode & kHPred)) {
             // sampled bracket [pa, pb): keys below it counted, keys inside it (a few percent)
-            // binned afterwards (and compacted, the list flushed after every tile so the
-            // buffer holds one tile's keys), keys above it and NaN ignored
+            // binned afterwards, keys above it and NaN ignored
             const float pa = s_hc.pa, pb = s_hc.pb;
-            auto key = [&](float k) { pred_key(k, &s_hc, s_hist, s_cmp, &s_ncmp, s_edge); };
+            auto key = [&](float k) { pred_key(k, &s_hc, s_hist, s_edge); };
             scan_tile<kThreads>(
                 keys, e0, e1, s_hc.R,
                 [&](float k) {
@@ -1236,18 +1270,12 @@ __global__ void __launch_bounds__(kThreads, kHistBlocksPerSm) k_hist(Level v) {
                     else if (k < pb)
                         key(k);
                 });
-            if (mode & kHCompact) {
-                const uint32_t wrote = append_list(v, c, s_cmp, &s_ncmp, &s_base);
-                if (threadIdx.x == 0) s_bytes += 4ull * wrote;
-            }
-        } else if (!kAny || (mode & kHDense)) {
+        } else if ((Allowed & kHBracket) && (mode & kHBracket)) {
+            bracket_tile(keys, e0, e1, s_hc.gs, s_hc.L, s_hc.R, below, s_hist, s_edge);
+        } else {
             // every key by the scaled guess (no range test: guess_bin fails keys outside
             // [L, R) and NaN, which dense_exact then counts or ignores)
             dense_tile(keys, e0, e1, s_hc.gs, s_hist, &s_hc, s_edge);
-        } else if (Allowed & kHSparse) {
-            // keys below L counted, keys in [L, R) (few) binned after their round
-            sparse_tile(keys, e0, e1, s_hc.L, s_hc.R, below,
-                        [&](float k) { sparse_key(k, &s_hc, s_hist, s_cmp, &s_ncmp); });
         }
         if (threadIdx.x == 0) s_bytes += 4ull * (e1 - e0);
     }
@@ -1337,9 +1365,9 @@ constexpr int kTileBins = 1 << kTileBinsLog2;
 constexpr int kListPerLane = 8;     // bracket keys a lane can hold
 constexpr uint32_t kListKeys = 64;  // bracket size that switches to the register list
 
-__global__ void __launch_bounds__(kThreads, kTileBlocksPerSm) k_bisect_tile(Level v) {
+__global__ void __launch_bounds__(kThreads, kTileBlocksPerSm) k_bisect_tile(const __grid_constant__ Level v) {
     pdl_enter();
-    if (v.skip && *(volatile const uint32_t *)v.skip) return;  // subtrees took this level
+    if (level_failed(v)) return;
     __shared__ uint32_t s_bins[kThreads / 32][kTileBins];
     __shared__ float s_edges[kThreads / 32][kTileBins + 1];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1496,168 +1524,6 @@ __global__ void __launch_bounds__(kThreads, kTileBlocksPerSm) k_bisect_tile(Leve
 }
 
 // ------------------------------------------------------------------------------------
-// Resolve: replay up to K bisection iterations per cell on its histogram (warp per cell).
-// ------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads) k_resolve(Level v) {
-    pdl_enter();
-    if (v.skip && *(volatile const uint32_t *)v.skip) return;  // subtrees took this level
-    const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (c >= v.C) return;
-    if (v.state[c] != kActive) return;
-    const int slot = level_slot(v, c);
-    orb_cell_t &cell = v.heap[slot];
-    const uint2 rg = v.ranges[slot];
-    const uint32_t n = rg.y - rg.x;
-    const float ratio = leaf_ratio(cell.nLeafCells);  // src/orbit.cpp:204
-    const int K = v.hist_k[c];
-    uint32_t *g = v.hist + v.hist_off[c];
-    float L = cell.cutMarginLeft, R = cell.cutMarginRight;
-    uint32_t it = v.iters[c];
-    uint32_t prefix = v.below[c];
-    uint32_t pos = 0, width = 1u << K;
-    uint8_t st = kActive;
-    // The replay reads the bins through two loads: lane l first sums its run of 2^K/32 bins
-    // (the steps whose halves span whole runs add up lanes), then, once a half lies inside
-    // one run, the lanes hold that run's bins two each. No other step waits on memory.
-    const uint32_t RUN = max((1u << K) >> 5, 1u);  // bins a lane's run covers (K = 4: lanes
-                                                    // 16.. hold none)
-    uint32_t run_sum = 0;
-    if (RUN >= 4) {
-        const uint4 *g4 = reinterpret_cast<const uint4 *>(g + lane * RUN);
-#pragma unroll 4
-        for (uint32_t j = 0; j < RUN / 4; ++j) {
-            const uint4 w = g4[j];
-            run_sum += w.x + w.y + w.z + w.w;
-        }
-    } else {
-        for (uint32_t j = 0; j < RUN; ++j)
-            if (lane * RUN + j < (1u << K)) run_sum += g[lane * RUN + j];
-    }
-    uint32_t q = 0xffffffffu;  // the run whose bins the lanes hold
-    uint2 pair = make_uint2(0u, 0u);
-    // bins [a, a + w) summed over the warp (a multiple of w, w a power of two)
-    auto sum_bins = [&](uint32_t a, uint32_t w) -> uint32_t {
-        if (w >= RUN) {
-            const uint32_t l0 = a / RUN, l1 = (a + w) / RUN;
-            return warp_sum(lane >= l0 && lane < l1 ? run_sum : 0u);
-        }
-        const uint32_t r = a / RUN;
-        if (r != q) {
-            q = r;
-            const uint32_t b0 = r * RUN + 2 * lane;
-            pair.x = 2 * lane < RUN ? g[b0] : 0u;
-            pair.y = 2 * lane + 1 < RUN ? g[b0 + 1] : 0u;
-        }
-        const uint32_t b0 = q * RUN + 2 * lane;
-        return warp_sum((b0 >= a && b0 < a + w ? pair.x : 0u) + (b0 + 1 >= a && b0 + 1 < a + w ? pair.y : 0u));
-    };
-    uint32_t first_half = 0xffffffffu;  // bins below the first cut, when already summed
-    const uint32_t pr = v.pass == 0 && v.pred ? v.pred[c] : 0u;
-    if (pr & kPredValid) {
-        // sampled pass: prefix = keys below e(lo), the bins hold the keys of [e(lo), e(hi));
-        // the replay below is exact when the cut lies between them (see k_sample_bin)
-        const uint32_t tot = sum_bins(0, 1u << K);
-        const bool holds = convergence(prefix, n, ratio) < 0 && convergence(prefix + tot, n, ratio) > 0;
-        __syncwarp();
-        if (!holds) {
-            for (uint32_t b = lane; b < (1u << K); b += 32) g[b] = 0u;
-            if (lane == 0) {
-                v.inb[c] = n;  // the next pass bins every key (dense)
-                v.below[c] = 0;
-                v.listed[c] = 0;
-                v.cmp_cnt[c] = 0;
-                v.cmp_bad[c] = 0;
-                v.counters->any_active[v.pass & 1] = 1u;
-                atomicAdd(&v.counters->pred_misses, 1u);
-                add_bytes(v, kKResolve, 8ull << K);
-            }
-            return;
-        }
-    }
-    if (v.warm && v.warm[c]) {
-        // first pass of a hinted bracket: check it holds the target before replaying (the
-        // total and the first step's count)
-        const uint32_t h0 = 1u << (K - 1);
-        const uint32_t lo = sum_bins(0, h0), hi = sum_bins(h0, h0);
-        first_half = lo;
-        const bool holds = warm_bracket_holds(prefix, prefix + lo + hi, n, ratio);
-        __syncwarp();
-        if (!holds) {
-            for (uint32_t b = lane; b < (1u << K); b += 32) g[b] = 0u;
-            if (lane == 0) {
-                warm_reset(cell, L, R, v.counters);
-                v.warm[c] = 0;
-                v.inb[c] = n;
-                v.below[c] = 0;
-                v.listed[c] = 0;
-                v.cmp_cnt[c] = 0;
-                v.cmp_bad[c] = 0;
-                v.counters->any_active[v.pass & 1] = 1u;
-            }
-            return;  // the next pass bins the whole extent
-        }
-        if (lane == 0) v.warm[c] = 0;
-    }
-    for (int step = 0; step < K; ++step) {
-        if (it >= (uint32_t)kMaxIterations) {
-            st = kCapped;
-            break;
-        }
-        const uint32_t half = width >> 1;
-        const uint32_t sum = step == 0 && first_half != 0xffffffffu ? first_half : sum_bins(pos, half);
-        const uint32_t cl = prefix + sum;
-        ++it;
-        const int dir = convergence(cl, n, ratio);
-        if (dir == 0) {
-            st = kFound;
-            break;
-        }
-        const float cut = mid_cut(L, R);
-        if (dir > 0) {
-            R = cut;
-        } else {
-            L = cut;
-            prefix += sum;
-            pos += half;
-        }
-        width = half;
-    }
-    if (st == kActive && it >= (uint32_t)kMaxIterations) st = kCapped;
-    const uint32_t next_inb = sum_bins(pos, 1);  // keys in the bracket the next pass would bin
-    // the next pass reads the cell's list when this pass read one or wrote a complete one
-    // (a sparse pass compacts its bracket keys); then the keys below the new L are known
-    const uint32_t tiles = v.tile_off[c + 1] - v.tile_off[c];
-    const bool compacted = pr & kPredValid ? (pr & kPredCompact) != 0
-                                           : sparse_pass(v, c, tiles) && v.inb[c] > (8u << K);
-    const bool list_next = v.listed[c] || (compacted && !v.cmp_bad[c]);
-    __syncwarp();
-    for (uint32_t b = lane; b < (1u << K); b += 32) g[b] = 0u;
-    if (st == kActive && lane == 0) {
-        v.inb[c] = next_inb;
-        v.listed[c] = list_next ? 1 : 0;
-    }
-    if (lane == 0) {
-        add_bytes(v, kKResolve, 8ull << K);  // bins read and cleared
-        cell.cutMarginLeft = L;
-        cell.cutMarginRight = R;
-        cell.foundCut = st == kFound ? 1 : 0;
-        v.iters[c] = (uint8_t)it;
-        v.state[c] = st;
-        v.below[c] = st == kActive && list_next ? prefix : 0u;
-        atomicMax(&v.counters->max_iters, it);
-        if (st == kCapped) atomicAdd(&v.counters->unfound, 1u);
-        if (st == kActive) {
-            v.counters->any_active[v.pass & 1] = 1u;
-            // the last pass leaves no cell active (tree depth 11): flag it if one does
-            if (v.pass == v.last_pass) atomicExch(&v.counters->error, 1u);
-        }
-    }
-}
-
-
-
-// ------------------------------------------------------------------------------------
 // Bisection with one CTA per cell, for levels with many cells (no multi-CTA passes, no
 // global histograms, no host round trip). Every round bins the candidate keys of the cell
 // into a shared-memory midpoint tree and replays up to K iterations of the reference loop
@@ -1674,9 +1540,9 @@ constexpr size_t kCtaSmemBytes = kListCap * sizeof(float) +
                                  (1u << kMaxBinsLog2) * sizeof(uint32_t) +
                                  ((1u << kMaxBinsLog2) + 1) * sizeof(float);
 
-__global__ void __launch_bounds__(kCtaThreads) k_bisect_cta(Level v) {
+__global__ void __launch_bounds__(kCtaThreads) k_bisect_cta(const __grid_constant__ Level v) {
     pdl_enter();
-    if (v.skip && *(volatile const uint32_t *)v.skip) return;  // subtrees took this level
+    if (level_failed(v)) return;
     extern __shared__ __align__(16) unsigned char cta_smem[];
     float *list = reinterpret_cast<float *>(cta_smem);
     uint32_t *s_hist = reinterpret_cast<uint32_t *>(list + kListCap);
@@ -1828,104 +1694,147 @@ __global__ void __launch_bounds__(kCtaThreads) k_bisect_cta(Level v) {
     }
 }
 
-// Tile -> cell maps of the level (one binary search per tile, once per level).
-// ... and the per-cell state of the level, in parallel (the plan only computes the offsets).
-__global__ void k_tile_map(Level v) {
-    pdl_enter();
-    if (v.skip && *(volatile const uint32_t *)v.skip) return;  // subtrees took this level
-    const uint32_t ht = v.tile_off[v.C], pt = v.ptile_off[v.C], C = (uint32_t)v.C;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < max(max(ht, pt), C);
-         t += gridDim.x * blockDim.x) {
-        if (t < ht) v.htile_cell[t] = find_cell(v.tile_off, v.C, t);
-        if (t < pt) v.ptile_cell[t] = find_cell(v.ptile_off, v.C, t);
-        if (t < C) {
-            const uint2 rg = v.ranges[level_slot(v, (int)t)];
-            const uint32_t n = rg.y - rg.x;
-            v.hist_k[t] = (uint8_t)tree_depth(n);
-            v.state[t] = n <= (uint32_t)kWarpKeys ? kSmall : (n <= (uint32_t)kTile ? kOneTile : kActive);
-            v.iters[t] = 0;
-            v.below[t] = 0;
-            v.inb[t] = n;
-            v.cmp_cnt[t] = 0;
-            v.listed[t] = 0;
-            v.cmp_bad[t] = 0;
-            if (v.pred) v.pred[t] = 0u;  // no sampled bracket unless k_sample_pick sets one
-        }
-    }
-}
-
 // ------------------------------------------------------------------------------------
 // Partition
 //
 // Partition tiles are kPTile consecutive positions of one cell. Per tile, the classify
-// pass stores two bitmasks (key >= cut, key <= cut) and their counts; one scan over all
-// tiles of the level gives every tile its exclusive prefix (in-cell prefix = difference
-// with the cell's first tile). A warp per cell then finds s and the split index i, and a
-// CTA per tile performs the swaps of the pairs whose left element lies in that tile.
+// pass stores two bitmasks (key >= cut, key <= cut) and their counts; k_part_cells turns the
+// counts into prefixes within the cell and finds s and the split index i, and a CTA per tile
+// performs the swaps of the pairs whose left element lies in that tile.
 // ------------------------------------------------------------------------------------
 __device__ __forceinline__ float cell_cut(const orb_cell_t &c) {
     return mid_cut(c.cutMarginLeft, c.cutMarginRight);
 }
 
-
-// Status word of one scan block in the look-back: flag (bits 62-63), count of keys
-// >= cut (bits 31-61) and keys <= cut (bits 0-30). Level totals stay below 2^31.
-constexpr unsigned long long kStAggregate = 1ull << 62;
-constexpr unsigned long long kStInclusive = 2ull << 62;
-constexpr unsigned long long kStFlags = 3ull << 62;
-
-__device__ __forceinline__ unsigned long long pack_status(unsigned long long flag, uint32_t g,
-                                                          uint32_t l) {
-    return flag | ((unsigned long long)g << 31) | (unsigned long long)l;
+// The next float above c (NaN for NaN and +inf, above which no key lies): k >= next_above(c)
+// exactly when k > c.
+__device__ __forceinline__ float next_above(float c) {
+    const int32_t b = __float_as_int(c);
+    if (!(c < __int_as_float(0x7f800000))) return __int_as_float(0x7fc00000);
+    if (c == 0.0f) return __int_as_float(1);
+    return __int_as_float(b > 0 ? b + 1 : b - 1);
 }
 
 // P1: bitmasks of keys >= cut and keys <= cut per partition tile, and their counts.
 // One warp per tile: the metadata chains (tile -> cell -> range, cut) of the CTA's warps
 // overlap, and each lane keeps kClassifyLoads loads in flight. The mask words are staged in
 // shared memory and stored coalesced.
+// A cell with a final cut is classified against it. A kReady cell's cut lies in its bracket
+// [L, R): keys below L are <= cut, keys at or above R are >= cut (and not <=, unless the cut
+// comes out as R itself: k_part_cells then classifies the cell again), NaN is both, and the
+// keys in between (a few in a thousand) go to the cell's list. So the pass that would only
+// count the bracket's keys and the pass over the final cut are one read of the keys. With
+// a = k >= lo and b = k < hi, both kinds are le = !a, ge = !b, listed = a and b: a final cut
+// takes hi = cut and lo = the next float above it, which leaves no listed key.
 constexpr int kClassifyLoads = 16;
+constexpr uint32_t kListStage = 128;  // listed keys a warp stages before it appends them
 
-__global__ void __launch_bounds__(kThreads) k_part_classify(Level v) {
+__global__ void __launch_bounds__(kThreads) k_part_classify(const __grid_constant__ Level v) {
     pdl_enter();
-    if (v.skip && *(volatile const uint32_t *)v.skip) return;  // subtrees took this level
+    if (blockIdx.x == 0 && threadIdx.x < 4) {
+        // the next level's plan and count passes start from zero (neither is in use now)
+        v.counters->any_active[threadIdx.x] = 0u;
+        if (threadIdx.x == 0 && v.tot_next) {
+            v.tot_next->tiles = 0ull;
+            v.tot_next->pools = 0ull;
+            v.tot_next->swaps = 0u;
+        }
+    }
+    if (level_failed(v)) return;
     __shared__ uint32_t s_words[kThreads / 32][2][kPWords];
-    const uint32_t total = v.ptile_off[v.C];
+    __shared__ float s_lkey[kThreads / 32][kListStage];
+    __shared__ uint32_t s_lpos[kThreads / 32][kListStage];
+    const uint64_t total = (uint32_t)v.tot->tiles;
     const int lane = threadIdx.x & 31;
     uint32_t(*sw)[kPWords] = s_words[threadIdx.x >> 5];
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    float *lkey = s_lkey[threadIdx.x >> 5];
+    uint32_t *lpos = s_lpos[threadIdx.x >> 5];
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     unsigned long long bytes = 0;
-    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < total; t += nwarps) {
-        const int c = v.ptile_cell ? (int)v.ptile_cell[t] : find_cell(v.ptile_off, v.C, t);
-        const uint32_t t0 = v.ptile_off[c];
-        const int slot = level_slot(v, c);
-        const orb_cell_t &cell = v.heap[slot];
-        const float cut = cell_cut(cell);
-        const float *keys = axis_keys(v, eff_axis(cell.cutAxis));
-        const uint2 rg = v.ranges[slot];
+    // a run of consecutive tiles a warp: a cell's bracket and its staged keys stay with it
+    const uint32_t t_end = (uint32_t)(total * (warp + 1) / nwarps);
+    int c = -1;
+    uint32_t t0 = 0, nl = 0;  // nl: staged listed keys of cell c
+    float lo = 0.f, hi = 0.f;
+    const float *keys = nullptr;
+    uint2 rg = make_uint2(0u, 0u);
+    auto flush = [&]() {
+        __syncwarp();
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(&v.cmp_cnt[c], nl);
+        base = v.cmp_off[c] + __shfl_sync(0xffffffffu, base, 0);
+        for (uint32_t j = lane; j < nl; j += 32) {
+            v.cmp_keys[base + j] = lkey[j];
+            v.cmp_pos[base + j] = lpos[j];
+        }
+        __syncwarp();
+        nl = 0;
+    };
+    for (uint32_t t = (uint32_t)(total * warp / nwarps); t < t_end; ++t) {
+        const int ct = (int)v.ptile_cell[t];
+        if (ct != c) {
+            if (nl) flush();
+            c = ct;
+            t0 = v.ptile_off[c];
+            const int slot = level_slot(v, c);
+            const orb_cell_t &cell = v.heap[slot];
+            const bool ready = v.state[c] == kReady;
+            const float cut = cell_cut(cell);
+            lo = ready ? cell.cutMarginLeft : next_above(cut);
+            hi = ready ? cell.cutMarginRight : cut;
+            keys = axis_keys(v, eff_axis(cell.cutAxis));
+            rg = v.ranges[slot];
+        }
         const uint32_t p0 = rg.x + (t - t0) * (uint32_t)kPTile;
         const uint32_t m = min((uint32_t)kPTile, rg.y - p0);
         uint32_t cg = 0, cl = 0;
-#pragma unroll 1
-        for (int r = 0; r < kPWords; r += kClassifyLoads) {
+        // the words of kClassifyLoads loads a lane; a full tile needs no bounds
+        auto round = [&](int r, auto full) {
+            constexpr bool kFull = decltype(full)::value;
             float k[kClassifyLoads];
 #pragma unroll
             for (int u = 0; u < kClassifyLoads; ++u) {
                 const uint32_t i = (uint32_t)(r + u) * 32u + lane;
-                k[u] = i < m ? __ldg(keys + p0 + i) : 0.0f;
+                k[u] = kFull || i < m ? __ldg(keys + p0 + i) : 0.0f;
             }
+            uint32_t listed = 0;  // words of this round with listed keys
 #pragma unroll
             for (int u = 0; u < kClassifyLoads; ++u) {
-                const int w = r + u;
-                const bool valid = (uint32_t)w * 32u + lane < m;
-                const uint32_t gb = __ballot_sync(0xffffffffu, valid && !(k[u] < cut));
-                const uint32_t lb = __ballot_sync(0xffffffffu, valid && !(k[u] > cut));
+                const uint32_t w0 = (uint32_t)(r + u) * 32u;  // the word's first position
+                uint32_t vm = 0xffffffffu;
+                if (!kFull) vm = w0 + 32u <= m ? vm : (w0 < m ? (1u << (m - w0)) - 1u : 0u);
+                const uint32_t gb = __ballot_sync(0xffffffffu, !(k[u] < hi)) & vm;
+                const uint32_t lb = __ballot_sync(0xffffffffu, !(k[u] >= lo)) & vm;
                 if (lane == u) {
-                    sw[0][w] = gb;
-                    sw[1][w] = lb;
+                    sw[0][r + u] = gb;
+                    sw[1][r + u] = lb;
                 }
                 cg += __popc(gb);
                 cl += __popc(lb);
+                if ((gb | lb) != vm) listed |= 1u << u;
             }
+            while (listed) {  // warp-uniform
+                const int u = __ffs(listed) - 1;
+                listed &= listed - 1;
+                const uint32_t i = (uint32_t)(r + u) * 32u + lane;
+                const float kk = i < m ? __ldg(keys + p0 + i) : hi;
+                const bool in = kk >= lo && kk < hi;
+                const uint32_t ib = __ballot_sync(0xffffffffu, in);
+                if (nl + 32 > kListStage) flush();
+                if (in) {
+                    const uint32_t q = nl + __popc(ib & ((1u << lane) - 1u));
+                    lkey[q] = kk;
+                    lpos[q] = p0 + i;
+                }
+                nl += __popc(ib);
+            }
+        };
+        if (m == (uint32_t)kPTile) {
+#pragma unroll 1
+            for (int r = 0; r < kPWords; r += kClassifyLoads) round(r, Flag<true>());
+        } else {
+#pragma unroll 1
+            for (int r = 0; r < kPWords; r += kClassifyLoads) round(r, Flag<false>());
         }
         uint32_t *gw = v.ge_bits + (size_t)t * kPWords;
         uint32_t *lw = v.le_bits + (size_t)t * kPWords;
@@ -1942,103 +1851,56 @@ __global__ void __launch_bounds__(kThreads) k_part_classify(Level v) {
             bytes += 4ull * m + 8ull * kPWords + 8ull;
         }
     }
+    if (nl) flush();
     if (lane == 0 && bytes) add_bytes(v, kKPartClassify, bytes);
 }
 
-// P2: global exclusive prefix of the per-tile counts over every tile of the level:
-// pt_*_pre[t] = sum over tiles before t, entry [total] = grand total. Blocks of 1024 tiles
-// take logical indices by ticket and chain their prefixes with a decoupled look-back (a
-// block only waits on blocks that started before it; the wait is bounded all the same).
-// In-cell prefixes are differences with the cell's first tile.
-constexpr int kScanBlock = 1024;
+// Position of the bit of rank r (0-based) in w (r < popc(w)).
+__device__ __forceinline__ uint32_t select_in_word(uint32_t w, uint32_t r) {
+    uint32_t pos = 0;
+#pragma unroll
+    for (int step = 16; step >= 1; step >>= 1) {
+        const uint32_t c = (uint32_t)__popc(w & ((1u << step) - 1u));
+        if (r >= c) {
+            r -= c;
+            w >>= step;
+            pos += (uint32_t)step;
+        }
+    }
+    return pos;
+}
 
-__global__ void __launch_bounds__(kScanBlock) k_tile_scan(Level v) {
-    pdl_enter();
-    if (v.skip && *(volatile const uint32_t *)v.skip) return;  // subtrees took this level
-    __shared__ uint32_t sh[96];
-    __shared__ uint32_t s_b;
-    __shared__ uint32_t s_pre[2];
-    const uint32_t total = v.ptile_off[v.C];
-    const uint32_t nblk = total / kScanBlock + 1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    volatile unsigned long long *status = v.pt_status;
-    if (threadIdx.x == 0) s_b = atomicAdd(v.ticket, 1u);
-    __syncthreads();
-    const uint32_t b = s_b;
-    if (b >= nblk) return;
-    const uint32_t t = b * kScanBlock + threadIdx.x;
-    const uint32_t g = t < total ? v.pt_ge[t] : 0u;
-    const uint32_t l = t < total ? v.pt_le[t] : 0u;
-    uint32_t ag, al;
-    const uint2 ex = block_excl_scan2(g, l, sh, &ag, &al);
-    if (warp == 0) {
-        uint32_t pg = 0, pl = 0;
-        if (b == 0) {
-            if (lane == 0) status[0] = pack_status(kStInclusive, ag, al);
-        } else {
-            if (lane == 0) status[b] = pack_status(kStAggregate, ag, al);
-            long long j = (long long)b - 1;
-            for (;;) {  // 32 predecessors at a time; blocks before 0 count as inclusive zero
-                const long long jj = j - lane;
-                unsigned long long st = kStInclusive;
-                if (jj >= 0) {
-                    uint32_t spins = 0;
-                    while (((st = status[jj]) & kStFlags) == 0ull) {
-                        if (++spins > v.spin_limit) {
-                            atomicExch(&v.counters->error, 1u);
-                            st = kStInclusive;
-                            break;
-                        }
-                        __nanosleep(64);
-                    }
-                }
-                const uint32_t incl = __ballot_sync(0xffffffffu, (st & kStFlags) == kStInclusive);
-                const int first = incl ? __ffs(incl) - 1 : 32;
-                const bool take = lane <= first;
-                pg += warp_sum(take ? (uint32_t)((st >> 31) & 0x7fffffffull) : 0u);
-                pl += warp_sum(take ? (uint32_t)(st & 0x7fffffffull) : 0u);
-                if (incl) break;
-                j -= 32;
-            }
-            if (lane == 0) status[b] = pack_status(kStInclusive, pg + ag, pl + al);
-        }
-        if (lane == 0) {
-            s_pre[0] = pg;
-            s_pre[1] = pl;
-        }
+// Largest u in [lo, hi] with pre[u] <= r, for a nondecreasing pre with pre[lo] <= r: a 32-way
+// search (every lane probes one point per round, the passing probes are a prefix of the
+// lanes), three rounds for 2^15 candidates. Warp-uniform result.
+__device__ __forceinline__ uint32_t warp_last_at_most(const uint32_t *pre, uint32_t lo, uint32_t hi,
+                                                      uint32_t r) {
+    const uint32_t lane = threadIdx.x & 31;
+    while (lo < hi) {
+        const uint32_t step = (hi - lo + 31) / 32;
+        const uint32_t u = lo + (lane + 1) * step;
+        const bool ok = u <= hi && pre[u] <= r;
+        const uint32_t cnt = (uint32_t)__popc(__ballot_sync(0xffffffffu, ok));
+        lo += cnt * step;
+        hi = min(hi, lo + step - 1);
     }
-    __syncthreads();
-    if (t <= total) {
-        v.pt_ge_pre[t] = s_pre[0] + ex.x;
-        v.pt_le_pre[t] = s_pre[1] + ex.y;
-    }
-    if (threadIdx.x == 0) add_bytes(v, kKPartScan, 16ull * min((uint32_t)kScanBlock, total + 1 - b * kScanBlock));
+    return lo;
 }
 
 // Position (cell-relative) of the set bit with in-cell rank `rank` among the bitmasks of
-// tiles [t0, t1), `pre` the level's global exclusive tile prefix (warp-cooperative; every
-// lane returns the answer).
+// tiles [t0, t1), `pre` the cell's exclusive tile prefix (warp-cooperative; every lane
+// returns the answer). The masks are read from L2 (atomics may have set bits).
 __device__ uint32_t warp_select(const uint32_t *bits, const uint32_t *pre, uint32_t t0, uint32_t t1,
                                 uint32_t rank) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t base0 = pre[t0];
-    uint32_t lo = t0, hi = t1 - 1;  // largest t with pre[t] - base0 <= rank
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (pre[mid] - base0 <= rank)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    const uint32_t r = rank - (pre[lo] - base0);
-    const uint32_t *w = bits + (size_t)lo * kPWords + lane * (kPWords / 32);
-    uint32_t words[kPWords / 32];
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t lo = warp_last_at_most(pre, t0, t1 - 1, rank);
+    const uint32_t r = rank - pre[lo];
+    static_assert(kPWords == 128, "four mask words a lane");
+    const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(bits + (size_t)lo * kPWords) + lane);
+    const uint32_t words[4] = {q.x, q.y, q.z, q.w};
     uint32_t cnt = 0;
 #pragma unroll
-    for (int j = 0; j < kPWords / 32; ++j) {
-        words[j] = w[j];
-        cnt += __popc(words[j]);
-    }
+    for (int j = 0; j < 4; ++j) cnt += __popc(words[j]);
     uint32_t tot;
     const uint32_t ex = warp_excl_scan(cnt, &tot);
     const bool mine = r >= ex && r < ex + cnt;
@@ -2046,14 +1908,11 @@ __device__ uint32_t warp_select(const uint32_t *bits, const uint32_t *pre, uint3
     if (mine) {
         uint32_t rr = r - ex;
 #pragma unroll
-        for (int j = 0; j < kPWords / 32; ++j) {
+        for (int j = 0; j < 4; ++j) {
             const uint32_t pc = __popc(words[j]);
             if (rr < pc) {
-                uint32_t word = words[j];
-                for (uint32_t q = 0; q < rr; ++q) word &= word - 1;  // drop rr lowest set bits
-                pos = (lo - t0) * (uint32_t)kPTile + (uint32_t)(lane * (kPWords / 32) + j) * 32u +
-                      (uint32_t)(__ffs(word) - 1);
-                rr = 0xffffffffu;
+                pos = (lo - t0) * (uint32_t)kPTile + (lane * 4 + (uint32_t)j) * 32u +
+                      select_in_word(words[j], rr);
                 break;
             }
             rr -= pc;
@@ -2063,263 +1922,33 @@ __device__ uint32_t warp_select(const uint32_t *bits, const uint32_t *pre, uint3
     return __shfl_sync(0xffffffffu, pos, __ffs(who) - 1);
 }
 
-// A look-back wait of the tile scan (or a bisection) gave up and flagged the build: the tile
-// prefixes may be incomplete, so the kernels that read them do nothing and the build
-// returns ORB_ERR_TIMEOUT.
-__device__ __forceinline__ bool scan_failed(const Level &v) {
-    return *(volatile const uint32_t *)&v.counters->error != 0u;
-}
-
-// P3: per cell (one warp): totals, the swap count s and the split index i.
-//   s = max_x min(f(x), g(x)), f(x) = #{>= cut in [0,x)}, g(x) = #{<= cut in [x,n)}
-//   i = min(L_{s+1}, R_s); i == n marks the clamped case (every key below the cut).
-__global__ void __launch_bounds__(kThreads) k_part_cells(Level v) {
-    pdl_enter();
-    if (v.skip && *(volatile const uint32_t *)v.skip) return;  // subtrees took this level
-    if (scan_failed(v)) return;  // a look-back wait gave up: the prefixes are not valid
-    const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (c >= v.C) return;
-    const int slot = level_slot(v, c);
-    const uint2 rg = v.ranges[slot];
-    const uint32_t n = rg.y - rg.x;
-    const uint32_t t0 = v.ptile_off[c], t1 = v.ptile_off[c + 1];
-    const uint32_t G0 = v.pt_ge_pre[t0], L0 = v.pt_le_pre[t0];
-    const uint32_t ge_tot = v.pt_ge_pre[t1] - G0, le_tot = v.pt_le_pre[t1] - L0;
-    uint32_t s = 0, i = n;
-    if (t1 > t0) {
-        // crossing tile: first tile whose end has f >= g (the last tile always does)
-        uint32_t lo = t0, hi = t1 - 1;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            const uint32_t f_end = v.pt_ge_pre[mid + 1] - G0;
-            const uint32_t g_end = le_tot - (v.pt_le_pre[mid + 1] - L0);
-            if (f_end >= g_end)
-                hi = mid;
-            else
-                lo = mid + 1;
-        }
-        const uint32_t *gw = v.ge_bits + (size_t)lo * kPWords + lane * (kPWords / 32);
-        const uint32_t *lw = v.le_bits + (size_t)lo * kPWords + lane * (kPWords / 32);
-        uint32_t gwd[kPWords / 32], lwd[kPWords / 32];
-        uint32_t cg = 0, cl = 0;
-#pragma unroll
-        for (int j = 0; j < kPWords / 32; ++j) {
-            gwd[j] = gw[j];
-            lwd[j] = lw[j];
-            cg += __popc(gwd[j]);
-            cl += __popc(lwd[j]);
-        }
-        uint32_t tg, tl;
-        const uint32_t eg = warp_excl_scan(cg, &tg);
-        const uint32_t el = warp_excl_scan(cl, &tl);
-        uint32_t f = (v.pt_ge_pre[lo] - G0) + eg;
-        uint32_t g = le_tot - (v.pt_le_pre[lo] - L0) - el;
-        uint32_t best = min(f, g);
-#pragma unroll
-        for (int j = 0; j < kPWords / 32; ++j) {
-            uint32_t a = gwd[j], b = lwd[j];
-            for (int q = 0; q < 32; ++q) {
-                f += a & 1u;
-                g -= b & 1u;
-                a >>= 1;
-                b >>= 1;
-                best = max(best, min(f, g));
-            }
-        }
-        s = warp_max(best);
-        if (ge_tot > s) i = min(i, warp_select(v.ge_bits, v.pt_ge_pre, t0, t1, s));
-        if (s >= 1) i = min(i, warp_select(v.le_bits, v.pt_le_pre, t0, t1, le_tot - s));
-    }
-    if (lane == 0) {
-        v.part_s[c] = s;
-        v.part_i[c] = i;
-        v.part_le[c] = le_tot;
-        add_bytes(v, kKPartCells, 16ull * 3 + (t1 > t0 ? 3ull * 2 * 4 * kPWords : 0ull));
-    }
-}
-
-// Writes the cell-relative positions of the set bits of one tile's mask whose in-cell rank
-// lies in [lo, hi) to out[f(rank)], f(rank) = rank - lo (forward) or (top - rank) (reverse).
-// Block-cooperative; `sh` holds >= 96 words.
-__device__ __forceinline__ void emit_positions(const uint32_t *words, uint32_t rank_base,
-                                               uint32_t lo, uint32_t hi, uint32_t rel_base,
-                                               bool reverse, uint32_t top, uint32_t *out,
-                                               uint32_t *sh) {
-    const uint32_t tid = threadIdx.x;
-    const uint32_t w = tid < (uint32_t)kPWords ? words[tid] : 0u;
-    uint32_t ta, tb;
-    const uint2 ex = block_excl_scan2(__popc(w), 0u, sh, &ta, &tb);
-    uint32_t r = rank_base + ex.x;
-    uint32_t word = w;
-    while (word) {
-        const uint32_t b = (uint32_t)(__ffs(word) - 1);
-        word &= word - 1;
-        if (r >= lo && r < hi) out[reverse ? top - r : r - lo] = rel_base + tid * 32u + b;
-        ++r;
-    }
-}
-
 // (y or z null: that array is not moved at this level; builds from host memory reorder it
-// later through the permutation, see orb_build)
+// later through the permutation, see orb_build.) Read from L2: in the swap kernel other CTAs
+// wrote these particles.
 __device__ __forceinline__ void swap_particles(const Level &v, uint32_t a, uint32_t b) {
-    const float xa = v.x[a], xb = v.x[b];
+    const float xa = __ldcg(v.x + a), xb = __ldcg(v.x + b);
     v.x[a] = xb;
     v.x[b] = xa;
     if (v.y) {
-        const float ya = v.y[a], yb = v.y[b];
+        const float ya = __ldcg(v.y + a), yb = __ldcg(v.y + b);
         v.y[a] = yb;
         v.y[b] = ya;
     }
     if (v.z) {
-        const float za = v.z[a], zb = v.z[b];
+        const float za = __ldcg(v.z + a), zb = __ldcg(v.z + b);
         v.z[a] = zb;
         v.z[b] = za;
     }
     if (v.idx) {
-        const uint32_t ia = v.idx[a], ib = v.idx[b];
+        const uint32_t ia = __ldcg(v.idx + a), ib = __ldcg(v.idx + b);
         v.idx[a] = ib;
         v.idx[b] = ia;
     }
     if (v.wt) {
-        const uint32_t wa = v.wt[a], wb = v.wt[b];
+        const uint32_t wa = __ldcg(v.wt + a), wb = __ldcg(v.wt + b);
         v.wt[a] = wb;
         v.wt[b] = wa;
     }
-}
-
-// Largest u in [lo, hi] with pre[u] - base <= r, for a nondecreasing pre with
-// pre[lo] - base <= r: a 32-way search (every lane probes one point per round, the passing
-// probes are a prefix of the lanes), three rounds for 2^15 candidates. Warp-uniform result.
-__device__ __forceinline__ uint32_t warp_last_at_most(const uint32_t *pre, uint32_t base,
-                                                      uint32_t lo, uint32_t hi, uint32_t r) {
-    const uint32_t lane = threadIdx.x & 31;
-    while (lo < hi) {
-        const uint32_t step = (hi - lo + 31) / 32;
-        const uint32_t u = lo + (lane + 1) * step;
-        const bool ok = u <= hi && pre[u] - base <= r;
-        const uint32_t cnt = (uint32_t)__popc(__ballot_sync(0xffffffffu, ok));
-        lo += cnt * step;
-        hi = min(hi, lo + step - 1);
-    }
-    return lo;
-}
-
-// P4: the Hoare swaps. The CTA of tile t takes the pairs (L_k, R_k) whose left element
-// L_k lies in t (k < s); their right partners are the keys <= cut of left-to-right rank
-// le_tot-1-k, found in the right tiles' masks. Positions of each side are disjoint
-// (L_k < i <= R_k), so the CTAs never touch the same particle.
-// Tuning (compile time): pairs per thread per round, and the CTAs per SM the register
-// budget is sized for (4 x 256 threads: 64 registers a thread).
-#ifndef ORB_SWAP_BATCH
-#define ORB_SWAP_BATCH 4
-#endif
-#ifndef ORB_SWAP_MIN_BLOCKS
-#define ORB_SWAP_MIN_BLOCKS 4
-#endif
-#ifndef ORB_SWAP_THREADS
-#define ORB_SWAP_THREADS 256  // threads of a swap CTA (at least kPWords: one mask word each)
-#endif
-constexpr int kSwapThreads = ORB_SWAP_THREADS;
-static_assert(kSwapThreads >= kPWords && kSwapThreads % 32 == 0, "a swap CTA scans a tile's mask words");
-// kWt: weighted builds, whose weights move with their particles. kYZ: bit 0 y moves, bit 1 z
-// moves (3 normally; the first levels of a build from host memory move x before y and z have
-// arrived, see orb_build).
-template <bool kWt, int kYZ>
-__global__ void __launch_bounds__(kSwapThreads, ORB_SWAP_MIN_BLOCKS) k_part_swap(Level v) {
-    pdl_enter();
-    if (v.skip && *(volatile const uint32_t *)v.skip) return;  // subtrees took this level
-    if (scan_failed(v)) return;  // a look-back wait gave up: the prefixes are not valid
-    __shared__ uint32_t posL[kPTile];
-    __shared__ uint32_t posR[kPTile];
-    __shared__ uint32_t sh[96];
-    const uint32_t total = v.ptile_off[v.C];
-    unsigned long long bytes = 0;  // pairs swapped by this CTA
-    for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
-        const int c = v.ptile_cell ? (int)v.ptile_cell[t] : find_cell(v.ptile_off, v.C, t);
-        const uint32_t t0 = v.ptile_off[c], t1 = v.ptile_off[c + 1];
-        const uint32_t s = v.part_s[c];
-        const uint32_t G0 = v.pt_ge_pre[t0], L0 = v.pt_le_pre[t0];
-        const uint32_t ka = v.pt_ge_pre[t] - G0;
-        const uint32_t kb = min(s, v.pt_ge_pre[t + 1] - G0);
-        if (ka >= kb) continue;
-        const uint32_t cnt = kb - ka;
-        const uint32_t le_tot = v.part_le[c];
-        const uint32_t b = v.ranges[level_slot(v, c)].x;
-        // left elements: ranks [ka, kb) of this tile's >= mask, in order
-        emit_positions(v.ge_bits + (size_t)t * kPWords, ka, ka, kb, (t - t0) * (uint32_t)kPTile,
-                       false, 0u, posL, sh);
-        // right partners: left-to-right <= ranks [le_tot-kb, le_tot-ka); rank r pairs with
-        // k = le_tot-1-r, stored at posR[k - ka] = posR[(le_tot-1-ka) - r]
-        const uint32_t ra = le_tot - kb, rb = le_tot - ka;
-        const uint32_t u0 = warp_last_at_most(v.pt_le_pre, L0, t0, t1 - 1, ra);
-        for (uint32_t u = u0; u < t1 && v.pt_le_pre[u] - L0 < rb; ++u)
-            emit_positions(v.le_bits + (size_t)u * kPWords, v.pt_le_pre[u] - L0, ra, rb,
-                           (u - t0) * (uint32_t)kPTile, true, le_tot - 1 - ka, posR, sh);
-        __syncthreads();
-        // kB pairs per thread per round: every load is issued before any store
-        constexpr int kB = ORB_SWAP_BATCH;
-        for (uint32_t j0 = 0; j0 < cnt; j0 += kB * blockDim.x) {
-            uint32_t pa[kB], pb[kB];
-            float xa[kB], xb[kB], ya[kB], yb[kB], za[kB], zb[kB];
-            uint32_t ia[kB], ib[kB], wa[kB], wb[kB];
-#pragma unroll
-            for (int q = 0; q < kB; ++q) {
-                const uint32_t j = j0 + q * blockDim.x + threadIdx.x;
-                const bool ok = j < cnt;
-                pa[q] = ok ? b + posL[j] : 0xffffffffu;
-                pb[q] = ok ? b + posR[j] : 0xffffffffu;
-                if (ok) {
-                    xa[q] = v.x[pa[q]];
-                    xb[q] = v.x[pb[q]];
-                    if constexpr ((kYZ & 1) != 0) {
-                        ya[q] = v.y[pa[q]];
-                        yb[q] = v.y[pb[q]];
-                    }
-                    if constexpr ((kYZ & 2) != 0) {
-                        za[q] = v.z[pa[q]];
-                        zb[q] = v.z[pb[q]];
-                    }
-                    if (v.idx) {
-                        ia[q] = v.idx[pa[q]];
-                        ib[q] = v.idx[pb[q]];
-                    }
-                    if constexpr (kWt) {
-                        wa[q] = v.wt[pa[q]];
-                        wb[q] = v.wt[pb[q]];
-                    }
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < kB; ++q) {
-                if (pa[q] == 0xffffffffu) continue;
-                v.x[pa[q]] = xb[q];
-                v.x[pb[q]] = xa[q];
-                if constexpr ((kYZ & 1) != 0) {
-                    v.y[pa[q]] = yb[q];
-                    v.y[pb[q]] = ya[q];
-                }
-                if constexpr ((kYZ & 2) != 0) {
-                    v.z[pa[q]] = zb[q];
-                    v.z[pb[q]] = za[q];
-                }
-                if (v.idx) {
-                    v.idx[pa[q]] = ib[q];
-                    v.idx[pb[q]] = ia[q];
-                }
-                if constexpr (kWt) {
-                    v.wt[pa[q]] = wb[q];
-                    v.wt[pb[q]] = wa[q];
-                }
-            }
-        }
-        bytes += cnt;
-        __syncthreads();
-    }
-    // per pair: both elements of x, y, z (and idx, weights) read and written
-    if (threadIdx.x == 0 && bytes)
-        add_bytes(v, kKPartSwap, (16ull * (1 + (kYZ & 1) + ((kYZ >> 1) & 1)) + (v.idx ? 16ull : 0ull) +
-                                  (kWt ? 16ull : 0ull)) * bytes);
 }
 
 __device__ void set_axis_and_margin(orb_cell_t &c, BuildCounters *ctr) {
@@ -2381,14 +2010,625 @@ __device__ void finish_cell(const Level &v, int slot, uint32_t i, bool do_split)
     v.heap[rslot] = rc;
 }
 
-// P5: finish_cell for every cell of the level.
-__global__ void __launch_bounds__(kThreads) k_part_finish(Level v, int do_split) {
+// One thread: finish_cell for cell c of the level, its children planned for the next one.
+struct Kids {
+    PlanCell p[2];
+};
+__device__ __noinline__ Kids finish_and_plan(const Level &v, int c, uint32_t i, bool do_split) {
+    const int slot = level_slot(v, c);
+    const uint2 rg = v.ranges[slot];
+    const int id = v.heap[slot].id;
+    finish_cell(v, slot, i, do_split);
+    Kids k;
+    k.p[0].c = k.p[1].c = -1;
+    if (v.next_C) {
+        const int m = v.child_map ? v.child_map[c]
+                                  : 8 * c + (2 * c < v.next_C ? 1 : 0) + (2 * c + 1 < v.next_C ? 2 : 0);
+        const int first = m >> 2, lslot = slot + id + 1;
+        if (m & 1) k.p[0] = plan_cell(v, v.tot_next, v.small_next, first, lslot, make_uint2(rg.x, rg.x + i));
+        if (m & 2) k.p[1] = plan_cell(v, v.tot_next, v.small_next, first + 1, lslot + 1, make_uint2(rg.x + i, rg.y));
+    }
+    atomicAdd(&v.counters->done[v.depth], 1u);
+    return k;
+}
+
+// P2: per cell: the bisection of a kReady cell finished on its list, the tile prefixes, the
+// swap count s and the split index i.
+//   s = max_x min(f(x), g(x)), f(x) = #{>= cut in [0,x)}, g(x) = #{<= cut in [x,n)}
+//   i = min(L_{s+1}, R_s); i == n marks the clamped case (every key below the cut).
+// The cell's left tiles go on the swap's work list (one empty item for a cell without pairs:
+// the swap kernel finishes every cell). A warp takes a cell of few tiles and listed keys, a
+// CTA a larger one, several CTAs one of a level with few cells: each of those bisects the
+// whole list, sets the mask bits of its share of the listed keys, and the last one goes on
+// (one CTA alone took 270 us for the 65536 listed keys of a root of 2^27 particles, nearly
+// all of it the 4 atomics a key).
+// One launch where a look-back scan over the level's tiles, its clearing and a kernel per
+// cell took three (the scan's 7-9 us and most of the other's 10-15 us a level were latency:
+// a binary search over the tiles and a serial walk of 128 positions a lane).
+constexpr uint32_t kWarpTiles = 160;  // tiles of a cell a warp takes (5 a lane)
+constexpr uint32_t kWarpList = 512;   // listed keys a warp takes (16 a lane)
+
+struct CellsSmem {
+    uint32_t bins[kHistBins];
+    float edges[kHistBins + 1];
+    float list[kWarpList];
+    uint32_t red[72];
+    uint32_t count;
+    float L, R;
+    uint32_t it, st;
+    uint32_t cross;      // the tile where f crosses g
+    uint32_t last;       // the cell's other CTAs have arrived
+};
+
+// The rest of the reference loop on at most kWarpList bracket keys, 16 a lane (lanes past m
+// hold R, which no cut in [L, R] exceeds); `below` keys lie below all of them. Every lane.
+__device__ __forceinline__ int bisect_list(const float (&kl)[kWarpList / 32], uint32_t below, uint32_t n, float ratio,
+                                           float &L, float &R, uint32_t &it) {
+    for (;;) {
+        if (it >= (uint32_t)kMaxIterations) return kCapped;
+        const float cut = mid_cut(L, R);
+        uint32_t c = 0;
+#pragma unroll
+        for (int q = 0; q < (int)kWarpList / 32; ++q) c += kl[q] < cut;
+        ++it;
+        const int dir = convergence(below + __reduce_add_sync(0xffffffffu, c), n, ratio);
+        if (dir == 0) return kFound;
+        if (dir > 0)
+            R = cut;
+        else
+            L = cut;
+    }
+}
+
+__device__ __forceinline__ void store_bisection(const Level &v, int c, orb_cell_t &cell, float L, float R,
+                                                uint32_t it, int st) {
+    cell.cutMarginLeft = L;
+    cell.cutMarginRight = R;
+    cell.foundCut = st == kFound ? 1 : 0;
+    v.iters[c] = (uint8_t)it;
+    v.state[c] = (uint8_t)st;
+    atomicMax(&v.counters->max_iters, it);
+    if (st == kCapped) atomicAdd(&v.counters->unfound, 1u);
+}
+
+// Mask bits of one listed key (position `pos`) against the final cut.
+__device__ __forceinline__ void patch_key(const Level &v, uint32_t t0, uint32_t rel, float k, float cut) {
+    const uint32_t t = t0 + rel / (uint32_t)kPTile, in = rel % (uint32_t)kPTile;
+    const uint32_t bit = 1u << (in & 31u);
+    const size_t w = (size_t)t * kPWords + (in >> 5);
+    if (!(k < cut)) {
+        atomicOr(&v.ge_bits[w], bit);
+        atomicAdd(&v.pt_ge[t], 1u);
+    }
+    if (!(k > cut)) {
+        atomicOr(&v.le_bits[w], bit);
+        atomicAdd(&v.pt_le[t], 1u);
+    }
+}
+
+// The final cut is the classify pass's upper bracket end: keys equal to it are <= cut too.
+// (Only a bracket a few floats wide ends there.) Sets their bits; threads ti of nt.
+__device__ __noinline__ void patch_upper(const Level &v, const orb_cell_t &cell, uint2 rg, uint32_t t0, float cut,
+                                         uint32_t ti, uint32_t nt) {
+    const float *keys = axis_keys(v, eff_axis(cell.cutAxis));
+    for (uint32_t p = rg.x + ti; p < rg.y; p += nt)
+        if (keys[p] == cut) {
+            const uint32_t rel = p - rg.x, t = t0 + rel / (uint32_t)kPTile, in = rel % (uint32_t)kPTile;
+            atomicOr(&v.le_bits[(size_t)t * kPWords + (in >> 5)], 1u << (in & 31u));
+            atomicAdd(&v.pt_le[t], 1u);
+        }
+}
+
+// One warp: s and i of a cell from its tile prefixes and the crossing tile (see P2), its
+// record, and its tiles on the swap's list.
+__device__ void cell_split_point(const Level &v, int c, uint2 rg, uint32_t t0, uint32_t T, uint32_t cross,
+                                 uint32_t ge_tot, uint32_t le_tot) {
+    const uint32_t lane = threadIdx.x & 31, n = rg.y - rg.x;
+    uint32_t s = 0, i = n;
+    if (T) {
+        const size_t w0 = (size_t)cross * kPWords;
+        const uint4 qg = __ldcg(reinterpret_cast<const uint4 *>(v.ge_bits + w0) + lane);
+        const uint4 ql = __ldcg(reinterpret_cast<const uint4 *>(v.le_bits + w0) + lane);
+        const uint32_t gw[4] = {qg.x, qg.y, qg.z, qg.w}, lw[4] = {ql.x, ql.y, ql.z, ql.w};
+        uint32_t tg, tl;
+        uint32_t f = v.pt_ge_pre[cross] + warp_excl_scan(__popc(gw[0]) + __popc(gw[1]) + __popc(gw[2]) + __popc(gw[3]), &tg);
+        uint32_t g = le_tot - v.pt_le_pre[cross] -
+                     warp_excl_scan(__popc(lw[0]) + __popc(lw[1]) + __popc(lw[2]) + __popc(lw[3]), &tl);
+        // min(f, g) rises while f < g and falls after: its maximum lies in the first word at
+        // whose end f >= g (the tile's last word at the latest)
+        uint32_t wa = gw[3], wb = lw[3], wf = 0, wg = 0;
+        bool hit = false;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t fe = f + __popc(gw[j]), ge = g - __popc(lw[j]);
+            if (!hit && (fe >= ge || j == 3)) {
+                wa = gw[j];
+                wb = lw[j];
+                wf = f;
+                wg = g;
+                hit = fe >= ge;
+            }
+            f = fe;
+            g = ge;
+        }
+        const uint32_t hb = __ballot_sync(0xffffffffu, hit);
+        const int src = hb ? __ffs(hb) - 1 : 31;
+        wa = __shfl_sync(0xffffffffu, wa, src);
+        wb = __shfl_sync(0xffffffffu, wb, src);
+        wf = __shfl_sync(0xffffffffu, wf, src);
+        wg = __shfl_sync(0xffffffffu, wg, src);
+        const uint32_t upto = 0xffffffffu >> (31u - lane);
+        s = max(min(wf, wg), min(wf + __popc(wa & upto), wg - __popc(wb & upto)));
+        s = __reduce_max_sync(0xffffffffu, s);
+        if (ge_tot > s) i = min(i, warp_select(v.ge_bits, v.pt_ge_pre, t0, t0 + T, s));
+        if (s >= 1) i = min(i, warp_select(v.le_bits, v.pt_le_pre, t0, t0 + T, le_tot - s));
+    }
+    const uint32_t left = s ? min(T, (i + (uint32_t)kPTile - 1) / (uint32_t)kPTile) : 1u;
+    uint32_t at = 0;
+    if (lane == 0) {
+        CellPart p;
+        p.b = rg.x;
+        p.n = n;
+        p.s = s;
+        p.i = i;
+        p.le = le_tot;
+        p.t0 = t0;
+        p.T = T;
+        p.left = left;
+        v.part[c] = p;
+        v.part_done[c] = v.done_start;
+        at = atomicAdd(&v.tot->swaps, left);
+    }
+    at = __shfl_sync(0xffffffffu, at, 0);
+    for (uint32_t j = lane; j < left; j += 32) v.swap_list[at + j] = make_uint2((uint32_t)c, j);
+}
+
+// A cell of at most kWarpTiles tiles and kWarpList listed keys, by one warp.
+__device__ void cells_warp(const Level &v, int c) {
+    const uint32_t lane = threadIdx.x & 31;
+    const int slot = level_slot(v, c);
+    orb_cell_t &cell = v.heap[slot];
+    const uint2 rg = v.ranges[slot];
+    const uint32_t n = rg.y - rg.x, t0 = v.ptile_off[c], T = (n + (uint32_t)kPTile - 1) / (uint32_t)kPTile;
+    if (v.state[c] == kReady) {
+        const uint32_t m = v.cmp_cnt[c], off = v.cmp_off[c];
+        const float ratio = leaf_ratio(cell.nLeafCells);  // src/orbit.cpp:204
+        float L = cell.cutMarginLeft, R = cell.cutMarginRight;
+        const float hi = R;  // the classify pass's bracket end
+        uint32_t it = v.iters[c];
+        float kl[kWarpList / 32];
+#pragma unroll
+        for (int q = 0; q < (int)kWarpList / 32; ++q) {
+            const uint32_t j = (uint32_t)q * 32u + lane;
+            kl[q] = j < m ? v.cmp_keys[off + j] : R;
+        }
+        const int st = bisect_list(kl, v.below[c], n, ratio, L, R, it);
+        __syncwarp();
+        if (lane == 0) store_bisection(v, c, cell, L, R, it, st);
+        const float cut = mid_cut(L, R);
+#pragma unroll
+        for (int q = 0; q < (int)kWarpList / 32; ++q) {
+            const uint32_t j = (uint32_t)q * 32u + lane;
+            if (j < m) patch_key(v, t0, v.cmp_pos[off + j] - rg.x, kl[q], cut);
+        }
+        if (cut == hi) patch_upper(v, cell, rg, t0, cut, lane, 32);
+        __threadfence();
+        __syncwarp();
+    }
+    // prefixes within the cell, tiles lane, 32 + lane, ... in a lane
+    constexpr int kPer = (int)kWarpTiles / 32;
+    uint32_t g[kPer], l[kPer], pg[kPer], pl[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const uint32_t u = (uint32_t)q * 32u + lane;
+        g[q] = u < T ? __ldcg(&v.pt_ge[t0 + u]) : 0u;
+        l[q] = u < T ? __ldcg(&v.pt_le[t0 + u]) : 0u;
+    }
+    uint32_t ge_tot = 0, le_tot = 0;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const uint32_t u = (uint32_t)q * 32u + lane;
+        uint32_t tg, tl;
+        pg[q] = ge_tot + warp_excl_scan(g[q], &tg);
+        pl[q] = le_tot + warp_excl_scan(l[q], &tl);
+        ge_tot += tg;
+        le_tot += tl;
+        if (u < T) {
+            v.pt_ge_pre[t0 + u] = pg[q];
+            v.pt_le_pre[t0 + u] = pl[q];
+        }
+    }
+    __syncwarp();
+    // crossing tile: the first whose end has f >= g (the last always does)
+    uint32_t cross = 0;
+#pragma unroll
+    for (int q = kPer - 1; q >= 0; --q) {
+        const uint32_t u = (uint32_t)q * 32u + lane;
+        const uint32_t b = __ballot_sync(0xffffffffu, u < T && pg[q] + g[q] >= le_tot - pl[q] - l[q]);
+        if (b) cross = (uint32_t)q * 32u + (uint32_t)__ffs(b) - 1u;
+    }
+    cell_split_point(v, c, rg, t0, T, t0 + cross, ge_tot, le_tot);
+}
+
+// A larger cell, by the CTA, or by nchunks CTAs of which this is number `chunk`.
+template <int NT>
+__device__ void cells_cta(const Level &v, int c, uint32_t chunk, uint32_t nchunks, CellsSmem &sm) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    const int slot = level_slot(v, c);
+    orb_cell_t &cell = v.heap[slot];
+    const uint2 rg = v.ranges[slot];
+    const uint32_t n = rg.y - rg.x, t0 = v.ptile_off[c], T = (n + (uint32_t)kPTile - 1) / (uint32_t)kPTile;
+    if (v.state[c] == kReady) {
+        const uint32_t m = v.cmp_cnt[c];
+        const float *keys = v.cmp_keys + v.cmp_off[c];
+        const uint32_t *pos = v.cmp_pos + v.cmp_off[c];
+        const float ratio = leaf_ratio(cell.nLeafCells);  // src/orbit.cpp:204
+        float L = cell.cutMarginLeft, R = cell.cutMarginRight;
+        const float hi = R;
+        uint32_t it = v.iters[c], cand = m, below = v.below[c];  // keys below L
+        int st = kActive;
+        // histogram rounds over the bracket's midpoint tree, until the bracket fits a warp
+        while (st == kActive && cand > kWarpList) {
+            const int K = min(kMaxBinsLog2, 32 - __clz(cand));
+            const uint32_t nb = 1u << K;
+            for (uint32_t j = tid; j < kHistBins; j += NT) sm.bins[j] = 0u;
+            fill_edges(sm.edges, L, R, K, tid, NT);
+            __syncthreads();
+            const Guess gs = make_guess(L, R, __fdiv_rn((float)nb, __fsub_rn(R, L)), nb);
+#pragma unroll 4
+            for (uint32_t j = tid; j < m; j += NT) {
+                const float k = keys[j];
+                if (k >= L && k < R) {
+                    uint32_t g;
+                    if (!guess_bin(gs, k, &g)) g = near_bin(k, gs, sm.edges, nb - 1u);
+                    atomicAdd(&sm.bins[g], 1u);
+                }
+            }
+            __syncthreads();
+            constexpr uint32_t kPer = kHistBins / NT;  // bins a thread
+            uint32_t h[kPer], loc = 0;
+#pragma unroll
+            for (uint32_t j = 0; j < kPer; ++j) {
+                h[j] = sm.bins[tid * kPer + j];
+                loc += h[j];
+            }
+            uint32_t tot, unused;
+            uint32_t run = block_excl_scan2(loc, 0u, sm.red, &tot, &unused).x;
+#pragma unroll
+            for (uint32_t j = 0; j < kPer; ++j) {
+                sm.bins[tid * kPer + j] = run;
+                run += h[j];
+            }
+            __syncthreads();
+            uint32_t p = 0, width = nb;
+            for (int step = 0; step < K; ++step) {
+                if (it >= (uint32_t)kMaxIterations) {
+                    st = kCapped;
+                    break;
+                }
+                const uint32_t half = width >> 1;
+                ++it;
+                const int dir = convergence(below + sm.bins[p + half], n, ratio);
+                if (dir == 0) {
+                    st = kFound;
+                    break;
+                }
+                const float cut = mid_cut(L, R);
+                if (dir > 0) {
+                    R = cut;
+                } else {
+                    L = cut;
+                    p += half;
+                }
+                width = half;
+            }
+            if (st == kActive && it >= (uint32_t)kMaxIterations) st = kCapped;
+            if (st == kActive) {
+                cand = (p + 1 < nb ? sm.bins[p + 1] : tot) - sm.bins[p];
+                below += sm.bins[p];
+            }
+            __syncthreads();
+        }
+        if (st == kActive) {
+            // the bracket's keys gathered; warp 0 finishes
+            if (tid == 0) sm.count = 0;
+            __syncthreads();
+#pragma unroll 4
+            for (uint32_t j = tid; j < m; j += NT) {
+                const float k = keys[j];
+                if (k >= L && k < R) sm.list[atomicAdd(&sm.count, 1u)] = k;
+            }
+            __syncthreads();
+            if (tid < 32) {
+                float kl[kWarpList / 32];
+#pragma unroll
+                for (int q = 0; q < (int)kWarpList / 32; ++q) {
+                    const uint32_t j = (uint32_t)q * 32u + lane;
+                    kl[q] = j < cand ? sm.list[j] : R;
+                }
+                st = bisect_list(kl, below, n, ratio, L, R, it);
+            }
+        }
+        if (tid == 0) {
+            sm.L = L;
+            sm.R = R;
+            sm.it = it;
+            sm.st = (uint32_t)st;
+        }
+        __syncthreads();
+        const float cut = mid_cut(sm.L, sm.R);
+        for (uint32_t j = chunk * NT + tid; j < m; j += nchunks * NT) patch_key(v, t0, pos[j] - rg.x, keys[j], cut);
+        if (cut == hi) patch_upper(v, cell, rg, t0, cut, chunk * NT + tid, nchunks * NT);
+        __threadfence();
+        __syncthreads();
+    }
+    if (nchunks > 1) {
+        if (tid == 0) {
+            sm.last = arrive_release(&v.hdone[c], 1u) + 1u == nchunks;
+            if (sm.last) acquire();
+        }
+        __syncthreads();
+        if (!sm.last) return;
+    }
+    // (the cell and its state are the other CTAs' inputs: written once all have arrived)
+    if (tid == 0 && v.state[c] == kReady) store_bisection(v, c, cell, sm.L, sm.R, sm.it, (int)sm.st);
+    // prefixes within the cell: a run of consecutive tiles a warp, 32 at a time
+    const uint32_t warp = tid >> 5;
+    constexpr uint32_t kWarps = NT / 32;
+    const uint32_t per = (T + kWarps * 32 - 1) / (kWarps * 32) * 32;
+    const uint32_t u0 = min(T, warp * per), u1 = min(T, u0 + per);
+    uint32_t cg = 0, cl = 0;
+#pragma unroll 8
+    for (uint32_t u = u0 + lane; u < u1; u += 32) {
+        cg += __ldcg(&v.pt_ge[t0 + u]);
+        cl += __ldcg(&v.pt_le[t0 + u]);
+    }
+    // (block_excl_scan2 runs over threads in order: a warp's tiles precede the next warp's)
+    uint32_t ge_tot, le_tot;
+    const uint2 ex = block_excl_scan2(cg, cl, sm.red, &ge_tot, &le_tot);
+    uint32_t f = __shfl_sync(0xffffffffu, ex.x, 0), l = __shfl_sync(0xffffffffu, ex.y, 0);
+    if (tid == 0) sm.cross = 0xffffffffu;
+    __syncthreads();
+    for (uint32_t b = u0; b < u1; b += 32) {
+        const uint32_t u = b + lane;
+        const uint32_t g1 = u < u1 ? __ldcg(&v.pt_ge[t0 + u]) : 0u, l1 = u < u1 ? __ldcg(&v.pt_le[t0 + u]) : 0u;
+        uint32_t tg, tl;
+        const uint32_t pf = f + warp_excl_scan(g1, &tg), pl = l + warp_excl_scan(l1, &tl);
+        if (u < u1) {
+            v.pt_ge_pre[t0 + u] = pf;
+            v.pt_le_pre[t0 + u] = pl;
+        }
+        // crossing tile: the first whose end has f >= g (the last always does)
+        const uint32_t x = __ballot_sync(0xffffffffu, u < u1 && pf + g1 >= le_tot - pl - l1);
+        if (lane == 0 && x) atomicMin(&sm.cross, t0 + b + (uint32_t)__ffs(x) - 1u);
+        f += tg;
+        l += tl;
+    }
+    __syncthreads();
+    if (tid < 32) cell_split_point(v, c, rg, t0, T, sm.cross, ge_tot, le_tot);
+    __syncthreads();  // sm reused by the next cell
+}
+
+// kPerCell: gridDim.x CTAs a cell (levels of few cells); else a warp a cell, the larger ones
+// by the CTA.
+template <int NT, bool kPerCell>
+__global__ void __launch_bounds__(NT) k_part_cells(const __grid_constant__ Level v) {
     pdl_enter();
-    if (v.skip && *(volatile const uint32_t *)v.skip) return;  // subtrees took this level
-    if (scan_failed(v)) return;  // a look-back wait gave up: the prefixes are not valid
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ CellsSmem sm;
+    if (level_failed(v)) return;
+    auto fits_warp = [&](int c) {
+        const uint2 rg = v.ranges[level_slot(v, c)];
+        return rg.y - rg.x <= kWarpTiles * (uint32_t)kPTile && !(v.state[c] == kReady && v.cmp_cnt[c] > kWarpList);
+    };
+    const int warp = (int)threadIdx.x >> 5;
+    if (kPerCell) {
+        const int c = (int)blockIdx.y;
+        const bool fits = fits_warp(c);
+        __syncthreads();  // every thread has looked before the state changes
+        if (!fits)
+            cells_cta<NT>(v, c, blockIdx.x, gridDim.x, sm);
+        else if (warp == 0 && (gridDim.x == 1 || blockIdx.x == 0))
+            cells_warp(v, c);
+        if (threadIdx.x == 0 && blockIdx.x == 0) add_bytes(v, kKPartCells, 512ull);
+        return;
+    }
+    constexpr int kW = NT / 32;
+    const int c0 = (int)blockIdx.x * kW;
+    __shared__ uint32_t s_big;  // the CTA's cells a warp cannot take
+    if (threadIdx.x == 0) s_big = 0;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0 && c0 + warp < v.C && !fits_warp(c0 + warp)) atomicOr(&s_big, 1u << warp);
+    __syncthreads();
+    uint32_t big = s_big;
+    if (c0 + warp < v.C && !((big >> warp) & 1u)) cells_warp(v, c0 + warp);
+    for (; big; big &= big - 1u) cells_cta<NT>(v, c0 + __ffs(big) - 1, 0u, 1u, sm);
+    if (threadIdx.x == 0 && c0 < v.C) add_bytes(v, kKPartCells, 512ull * (unsigned)min(kW, v.C - c0));
+}
+
+// Writes the cell-relative positions of the set bits of one tile's mask whose in-cell rank
+// lies in [lo, hi) to out[f(rank)], f(rank) = rank - lo (forward) or (top - rank) (reverse).
+// Block-cooperative; `sh` holds >= 96 words.
+__device__ __forceinline__ void emit_positions(const uint32_t *words, uint32_t rank_base,
+                                               uint32_t lo, uint32_t hi, uint32_t rel_base,
+                                               bool reverse, uint32_t top, uint32_t *out,
+                                               uint32_t *sh) {
+    const uint32_t tid = threadIdx.x;
+    const uint32_t w = tid < (uint32_t)kPWords ? words[tid] : 0u;
+    uint32_t ta, tb;
+    const uint2 ex = block_excl_scan2(__popc(w), 0u, sh, &ta, &tb);
+    uint32_t r = rank_base + ex.x;
+    uint32_t word = w;
+    while (word) {
+        const uint32_t b = (uint32_t)(__ffs(word) - 1);
+        word &= word - 1;
+        if (r >= lo && r < hi) out[reverse ? top - r : r - lo] = rel_base + tid * 32u + b;
+        ++r;
+    }
+}
+
+// P4: the Hoare swaps. The CTA of tile t takes the pairs (L_k, R_k) whose left element
+// L_k lies in t (k < s); their right partners are the keys <= cut of left-to-right rank
+// le_tot-1-k, found in the right tiles' masks. Positions of each side are disjoint
+// (L_k < i <= R_k), so the CTAs never touch the same particle.
+// Tuning (compile time): pairs per thread per round, and the CTAs per SM the register
+// budget is sized for (4 x 256 threads: 64 registers a thread).
+#ifndef ORB_SWAP_BATCH
+#define ORB_SWAP_BATCH 4
+#endif
+#ifndef ORB_SWAP_MIN_BLOCKS
+#define ORB_SWAP_MIN_BLOCKS 4
+#endif
+#ifndef ORB_SWAP_THREADS
+#define ORB_SWAP_THREADS 256  // threads of a swap CTA (at least kPWords: one mask word each)
+#endif
+constexpr int kSwapThreads = ORB_SWAP_THREADS;
+static_assert(kSwapThreads >= kPWords && kSwapThreads % 32 == 0, "a swap CTA scans a tile's mask words");
+// kWt: weighted builds, whose weights move with their particles. kYZ: bit 0 y moves, bit 1 z
+// moves (3 normally; the first levels of a build from host memory move x before y and z have
+// arrived, see orb_build).
+// kFuse: the CTA that brings a cell's last tile also finishes the cell (levels of at most one
+// tile a CTA, where a launch less counts); else k_part_finish does. Arrivals between a CTA's
+// tiles made the swap of the headline's deep levels 40% slower (570 -> 850 us a level: each
+// waits for the SM's stores), so larger levels take the separate launch.
+template <bool kWt, int kYZ, bool kFuse>
+__global__ void __launch_bounds__(kSwapThreads, ORB_SWAP_MIN_BLOCKS) k_part_swap(const __grid_constant__ Level v, int do_split) {
+    pdl_enter();
+    if (level_failed(v)) return;
+    __shared__ uint32_t posL[kPTile];
+    __shared__ uint32_t posR[kPTile];
+    __shared__ uint32_t sh[96];
+    const uint32_t total = v.tot->swaps;
+    unsigned long long bytes = 0;  // pairs swapped by this CTA
+    for (uint32_t w = blockIdx.x; w < total; w += gridDim.x) {
+        const uint2 item = v.swap_list[w];
+        const int c = (int)item.x;
+        const CellPart P = v.part[c];
+        const uint32_t t0 = P.t0, t1 = t0 + P.T, t = t0 + item.y;
+        const uint32_t s = P.s, le_tot = P.le, b = P.b;
+        const uint32_t ka = s ? v.pt_ge_pre[t] : 0u;  // (a cell without pairs has one empty item)
+        const uint32_t kb = s ? max(ka, min(s, ka + v.pt_ge[t])) : 0u;
+        const uint32_t cnt = kb - ka;
+        if (cnt) {
+            // left elements: ranks [ka, kb) of this tile's >= mask, in order
+            emit_positions(v.ge_bits + (size_t)t * kPWords, ka, ka, kb, item.y * (uint32_t)kPTile, false, 0u,
+                           posL, sh);
+            // right partners: left-to-right <= ranks [le_tot-kb, le_tot-ka); rank r pairs with
+            // k = le_tot-1-r, stored at posR[k - ka] = posR[(le_tot-1-ka) - r]
+            const uint32_t ra = le_tot - kb, rb = le_tot - ka;
+            const uint32_t u0 = warp_last_at_most(v.pt_le_pre, t0, t1 - 1, ra);
+            for (uint32_t u = u0; u < t1 && v.pt_le_pre[u] < rb; ++u)
+                emit_positions(v.le_bits + (size_t)u * kPWords, v.pt_le_pre[u], ra, rb,
+                               (u - t0) * (uint32_t)kPTile, true, le_tot - 1 - ka, posR, sh);
+        }
+        __syncthreads();
+        // kB pairs per thread per round: every load is issued before any store
+        constexpr int kB = ORB_SWAP_BATCH;
+        for (uint32_t j0 = 0; j0 < cnt; j0 += kB * blockDim.x) {
+            uint32_t pa[kB], pb[kB];
+            float xa[kB], xb[kB], ya[kB], yb[kB], za[kB], zb[kB];
+            uint32_t ia[kB], ib[kB], wa[kB], wb[kB];
+#pragma unroll
+            for (int q = 0; q < kB; ++q) {
+                const uint32_t j = j0 + q * blockDim.x + threadIdx.x;
+                const bool ok = j < cnt;
+                pa[q] = ok ? b + posL[j] : 0xffffffffu;
+                pb[q] = ok ? b + posR[j] : 0xffffffffu;
+                if (ok) {
+                    xa[q] = v.x[pa[q]];
+                    xb[q] = v.x[pb[q]];
+                    if constexpr ((kYZ & 1) != 0) {
+                        ya[q] = v.y[pa[q]];
+                        yb[q] = v.y[pb[q]];
+                    }
+                    if constexpr ((kYZ & 2) != 0) {
+                        za[q] = v.z[pa[q]];
+                        zb[q] = v.z[pb[q]];
+                    }
+                    if (v.idx) {
+                        ia[q] = v.idx[pa[q]];
+                        ib[q] = v.idx[pb[q]];
+                    }
+                    if constexpr (kWt) {
+                        wa[q] = v.wt[pa[q]];
+                        wb[q] = v.wt[pb[q]];
+                    }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < kB; ++q) {
+                if (pa[q] == 0xffffffffu) continue;
+                v.x[pa[q]] = xb[q];
+                v.x[pb[q]] = xa[q];
+                if constexpr ((kYZ & 1) != 0) {
+                    v.y[pa[q]] = yb[q];
+                    v.y[pb[q]] = ya[q];
+                }
+                if constexpr ((kYZ & 2) != 0) {
+                    v.z[pa[q]] = zb[q];
+                    v.z[pb[q]] = za[q];
+                }
+                if (v.idx) {
+                    v.idx[pa[q]] = ib[q];
+                    v.idx[pb[q]] = ia[q];
+                }
+                if constexpr (kWt) {
+                    v.wt[pa[q]] = wb[q];
+                    v.wt[pb[q]] = wa[q];
+                }
+            }
+        }
+        bytes += cnt;
+        __syncthreads();
+        if constexpr (kFuse) {
+            __shared__ Kids s_kids;
+            __shared__ bool s_last;
+            if (threadIdx.x == 0) {
+                s_last = arrive_release(&v.part_done[c], 1u) + 1u == P.left;
+                if (s_last) {
+                    acquire();
+                    s_kids = finish_and_plan(v, c, P.i, do_split != 0);
+                }
+            }
+            __syncthreads();
+            if (s_last) {
+                plan_fill(v, s_kids.p[0], threadIdx.x, kSwapThreads);
+                plan_fill(v, s_kids.p[1], threadIdx.x, kSwapThreads);
+                __syncthreads();
+            }
+        } else if (threadIdx.x == 0) {
+            atomicAdd(&v.part_done[c], 1u);
+        }
+    }
+    // per pair: both elements of x, y, z (and idx, weights) read and written
+    if (threadIdx.x == 0 && bytes)
+        add_bytes(v, kKPartSwap, (16ull * (1 + (kYZ & 1) + ((kYZ >> 1) & 1)) + (v.idx ? 16ull : 0ull) +
+                                  (kWt ? 16ull : 0ull)) * bytes);
+}
+
+// P5: the final swap, the split and the children's plan of every cell, a CTA a cell on levels of
+// few cells (large maps to fill), else a warp. A cell whose tiles did not all report is left
+// alone: its missing count stops the build.
+template <bool kPerCell>
+__global__ void __launch_bounds__(kThreads) k_part_finish(const __grid_constant__ Level v, int do_split) {
+    pdl_enter();
+    if (level_failed(v)) return;
+    __shared__ Kids s_kids[kThreads / 32];
+    const uint32_t warp = threadIdx.x >> 5, nt = kPerCell ? kThreads : 32u;
+    const uint32_t ti = kPerCell ? threadIdx.x : threadIdx.x & 31u;
+    const int c = kPerCell ? (int)blockIdx.x : (int)(blockIdx.x * (kThreads / 32) + warp);
+    Kids &k = s_kids[kPerCell ? 0 : warp];
+    if (c < v.C && ti == 0) {
+        const CellPart P = v.part[c];
+        k.p[0].c = k.p[1].c = -1;
+        if (v.part_done[c] == P.left) k = finish_and_plan(v, c, P.i, do_split != 0);
+    }
+    if (kPerCell)
+        __syncthreads();
+    else
+        __syncwarp();
     if (c >= v.C) return;
-    finish_cell(v, level_slot(v, c), v.part_i[c], do_split != 0);
+    plan_fill(v, k.p[0], ti, nt);
+    plan_fill(v, k.p[1], ti, nt);
 }
 
 // ------------------------------------------------------------------------------------
@@ -2419,21 +2659,6 @@ struct SubSmem {
     uint32_t word, count;                            // broadcast values
     int root;                                        // the CTA's current root cell
 };
-
-// Position of the bit of rank r (0-based) in w (r < popc(w)).
-__device__ __forceinline__ uint32_t select_in_word(uint32_t w, uint32_t r) {
-    uint32_t pos = 0;
-#pragma unroll
-    for (int step = 16; step >= 1; step >>= 1) {
-        const uint32_t c = (uint32_t)__popc(w & ((1u << step) - 1u));
-        if (r >= c) {
-            r -= c;
-            w >>= step;
-            pos += (uint32_t)step;
-        }
-    }
-    return pos;
-}
 
 // sub_select() through the rank table t (t[b] = the word holding rank 64 b): a few steps
 // from the table's word instead of a search.
@@ -2919,7 +3144,7 @@ __device__ __forceinline__ int levels_below(const orb_cell_t &c) {
 // (<= kSubLevels, the descendant queue) levels below it. One CTA.
 constexpr int kSubLevels = kSubMaxLevels;
 static_assert((2 << (kSubLevels - 1)) <= kSubQueue, "the last level's children fit the queue");
-__global__ void __launch_bounds__(1024) k_subtree_check(Level v, int max_levels) {
+__global__ void __launch_bounds__(1024) k_subtree_check(const __grid_constant__ Level v, int max_levels) {
     pdl_enter();
     __shared__ uint32_t sh[96];
     uint32_t mx = 0, ml = 0;
@@ -2931,10 +3156,11 @@ __global__ void __launch_bounds__(1024) k_subtree_check(Level v, int max_levels)
     }
     mx = block_max(mx, sh);
     ml = block_max(ml, sh);
+    const bool failed = level_failed(v);
     if (v.win_cnt)
         for (int w = threadIdx.x; w < kMaxWindows; w += blockDim.x) v.win_cnt[w] = 0u;
     if (threadIdx.x == 0) {
-        const uint32_t take = mx <= kSubMax && (int)ml <= min(max_levels, kSubLevels) ? 1u : 0u;
+        const uint32_t take = !failed && mx <= kSubMax && (int)ml <= min(max_levels, kSubLevels) ? 1u : 0u;
         *v.skip = take;
         v.counters->sub_next = 0u;  // the subtree kernel's work queue starts at the level's first cell
         if (v.hwin) {
@@ -2950,7 +3176,7 @@ __global__ void __launch_bounds__(1024) k_subtree_check(Level v, int max_levels)
 // by side); without it every cell is the whole CTA's (the instance for trees whose cells
 // never get that small keeps its registers for the CTA path). Same results either way.
 template <bool kWarpSmall>
-__global__ void __launch_bounds__(kSubThreads, 4) k_subtree(Level v) {
+__global__ void __launch_bounds__(kSubThreads, 4) k_subtree(const __grid_constant__ Level v) {
     pdl_enter();
     __shared__ SubSmem sm;
     if (*(volatile const uint32_t *)v.skip == 0u) return;  // the level kernels run instead
@@ -3037,25 +3263,10 @@ __global__ void __launch_bounds__(kSubThreads, 4) k_subtree(Level v) {
 // (the thesis's weighted ORB, documentation/notes.tex:259-271; never implemented by the
 // reference). Per level: every cell starts active; kWPasses passes each bin the weights of
 // every active cell's bracket into its midpoint tree of depth kWBinsLog2 (the exact
-// descent: the reference's own cuts) and sum the weights below the bracket; a resolve per
-// cell replays up to kWBinsLog2 iterations of the loop on the prefix sums with the weighted
-// test. Integer sums: the same results in any order.
+// descent: the reference's own cuts) and sum the weights below the bracket; the CTA that
+// brings a cell's last tile replays up to kWBinsLog2 iterations of the loop on the prefix
+// sums with the weighted test. Integer sums: the same results in any order.
 // ------------------------------------------------------------------------------------
-__global__ void k_wstart(Level v) {
-    pdl_enter();
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < (uint32_t)v.C;
-         c += gridDim.x * blockDim.x) {
-        v.state[c] = kActive;
-        v.iters[c] = 0;
-        v.wbelow[c] = 0ull;
-        v.wtot[c] = 0ull;
-    }
-    const uint64_t nb = (uint64_t)v.C * kWBins;
-    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nb;
-         j += (uint64_t)gridDim.x * blockDim.x)
-        v.whist[j] = 0ull;
-}
-
 __device__ __forceinline__ unsigned long long block_sum_u64(unsigned long long x,
                                                             unsigned long long *sh) {
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
@@ -3068,11 +3279,74 @@ __device__ __forceinline__ unsigned long long block_sum_u64(unsigned long long x
     return t;
 }
 
-__global__ void __launch_bounds__(kThreads) k_whist(Level v) {
+// The replay of up to kWBinsLog2 iterations of src/orbit.cpp:146-232 on cell c's finished
+// weight bins, with the weighted test, by the CTA that brought its last tile; the bins are
+// cleared for the next pass. (As a kernel of its own it took 9-10 us a pass.)
+__device__ __noinline__ void wresolve_cell(const Level &v, int c, bool whole, unsigned long long *s_pre,
+                                           unsigned long long *s_red) {
+    static_assert(kWBins == kThreads, "one bin a thread");
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned long long *g = v.whist + (size_t)c * kWBins;
+    const unsigned long long x = whole ? s_pre[tid] : __ldcg(g + tid);
+    if (!whole) g[tid] = 0ull;
+    unsigned long long inc = x;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o) inc += t;
+    }
+    if (lane == 31) s_red[warp] = inc;
+    __syncthreads();
+    for (uint32_t w = 0; w < warp; ++w) inc += s_red[w];
+    s_pre[tid] = inc - x;
+    __syncthreads();
+    if (tid != 0) return;
+    const int slot = level_slot(v, c);
+    orb_cell_t &cell = v.heap[slot];
+    const uint2 rg = v.ranges[slot];
+    const uint32_t n = rg.y - rg.x;
+    const unsigned long long W = __ldcg(&v.wtot[c]), below = __ldcg(&v.wbelow[c]);
+    float L = cell.cutMarginLeft, R = cell.cutMarginRight;
+    uint32_t it = v.iters[c], pos = 0, width = kWBins;
+    uint8_t st = kActive;
+    for (int step = 0; step < kWBinsLog2; ++step) {
+        if (it >= (uint32_t)kMaxIterations) break;
+        const uint32_t half = width >> 1;
+        const unsigned long long wl = below + s_pre[pos + half];
+        ++it;
+        const int dir = convergence_weighted(wl, W, n, cell.nLeafCells);
+        if (dir == 0) {
+            st = kFound;
+            break;
+        }
+        const float cut = mid_cut(L, R);
+        if (dir > 0) {
+            R = cut;
+        } else {
+            L = cut;
+            pos += half;
+        }
+        width = half;
+    }
+    if (st == kActive && it >= (uint32_t)kMaxIterations) st = kCapped;
+    cell.cutMarginLeft = L;
+    cell.cutMarginRight = R;
+    cell.foundCut = st == kFound ? 1 : 0;
+    v.iters[c] = (uint8_t)it;
+    v.state[c] = st;
+    v.hdone[c] = 0;
+    // the weight below the new bracket [L, R): below the old one plus the bins left of it
+    v.wbelow[c] = below + s_pre[pos];
+    if (st != kActive) atomicMax(&v.counters->max_iters, it);
+    if (st == kCapped) atomicAdd(&v.counters->unfound, 1u);
+}
+
+__global__ void __launch_bounds__(kThreads) k_whist(const __grid_constant__ Level v) {
     pdl_enter();
+    if (level_failed(v)) return;
     __shared__ unsigned long long s_bins[kWBins];
     __shared__ unsigned long long s_red[kThreads / 32];
-    const uint32_t total = v.tile_off[v.C];
+    __shared__ uint32_t s_last;
+    const uint32_t total = (uint32_t)(v.tot->tiles >> 32);
     unsigned long long bytes = 0, wkeys = 0;  // this thread's bracket weight reads; the CTA's keys
     for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
         const TileRef tr = tile_ref(v, t);
@@ -3118,14 +3392,28 @@ __global__ void __launch_bounds__(kThreads) k_whist(Level v) {
             tot = block_sum_u64(tot, s_red);
         }
         __syncthreads();
-        unsigned long long *g = v.whist + (size_t)tr.c * kWBins;
-        for (uint32_t j = threadIdx.x; j < (uint32_t)kWBins; j += blockDim.x)
-            if (s_bins[j]) atomicAdd(&g[j], s_bins[j]);
-        if (threadIdx.x == 0 && first) {
-            if (below) atomicAdd(&v.wbelow[tr.c], below);
-            if (tot) atomicAdd(&v.wtot[tr.c], tot);
+        const uint2 rg = v.ranges[tr.slot];
+        const uint32_t tiles = (rg.y - rg.x + (uint32_t)kTile - 1) / (uint32_t)kTile;
+        if (threadIdx.x == 0) {
+            wkeys += tr.e1 - tr.e0;
+            s_last = tiles == 1 ? 1u : 0u;
+            if (first) {
+                if (below) atomicAdd(&v.wbelow[tr.c], below);
+                if (tot) atomicAdd(&v.wtot[tr.c], tot);
+            }
         }
-        if (threadIdx.x == 0) wkeys += tr.e1 - tr.e0;
+        if (tiles > 1) {
+            unsigned long long *g = v.whist + (size_t)tr.c * kWBins;
+            for (uint32_t j = threadIdx.x; j < (uint32_t)kWBins; j += blockDim.x)
+                if (s_bins[j]) atomicAdd(&g[j], s_bins[j]);
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                s_last = arrive_release(&v.hdone[tr.c], 1u) + 1u == tiles;
+                if (s_last) acquire();
+            }
+        }
+        __syncthreads();
+        if (s_last) wresolve_cell(v, tr.c, tiles == 1, s_bins, s_red);
         __syncthreads();  // s_bins reused by the next tile
     }
     // 4 B per key read (every pass), 4 B per weight read (every key in the first pass, the
@@ -3137,91 +3425,13 @@ __global__ void __launch_bounds__(kThreads) k_whist(Level v) {
     }
 }
 
-// A warp per cell: the replay of up to kWBinsLog2 iterations of src/orbit.cpp:146-232 on the
-// pass's weight bins, with the weighted test; the bins and the weight below are cleared for
-// the next pass.
-__global__ void __launch_bounds__(kThreads) k_wresolve(Level v) {
-    pdl_enter();
-    __shared__ unsigned long long s_pre[kThreads / 32][kWBins];
-    const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (c >= v.C) return;
-    if (v.state[c] != kActive) return;  // warp-uniform
-    unsigned long long *pre = s_pre[threadIdx.x >> 5];
-    unsigned long long *g = v.whist + (size_t)c * kWBins;
-    constexpr int kPer = kWBins / 32;
-    unsigned long long loc[kPer], run = 0;
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-        loc[j] = g[lane * kPer + j];
-        g[lane * kPer + j] = 0ull;
-        run += loc[j];
-    }
-    // exclusive prefix of the lanes' runs
-    unsigned long long inc = run;
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
-    }
-    unsigned long long acc = inc - run;
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-        pre[lane * kPer + j] = acc;
-        acc += loc[j];
-    }
-    __syncwarp();
-    const int slot = level_slot(v, c);
-    orb_cell_t &cell = v.heap[slot];
-    const uint2 rg = v.ranges[slot];
-    const uint32_t n = rg.y - rg.x;
-    const unsigned long long W = v.wtot[c], below = v.wbelow[c];
-    float L = cell.cutMarginLeft, R = cell.cutMarginRight;
-    uint32_t it = v.iters[c], pos = 0, width = kWBins;
-    uint8_t st = kActive;
-    for (int step = 0; step < kWBinsLog2; ++step) {
-        if (it >= (uint32_t)kMaxIterations) {
-            st = kCapped;
-            break;
-        }
-        const uint32_t half = width >> 1;
-        const unsigned long long wl = below + pre[pos + half];
-        ++it;
-        const int dir = convergence_weighted(wl, W, n, cell.nLeafCells);
-        if (dir == 0) {
-            st = kFound;
-            break;
-        }
-        const float cut = mid_cut(L, R);
-        if (dir > 0) {
-            R = cut;
-        } else {
-            L = cut;
-            pos += half;
-        }
-        width = half;
-    }
-    if (st == kActive && it >= (uint32_t)kMaxIterations) st = kCapped;
-    __syncwarp();
-    if (lane == 0) {
-        cell.cutMarginLeft = L;
-        cell.cutMarginRight = R;
-        cell.foundCut = st == kFound ? 1 : 0;
-        v.iters[c] = (uint8_t)it;
-        v.state[c] = st;
-        // the weight below the new bracket [L, R): below the old one plus the bins left of it
-        v.wbelow[c] = below + pre[pos];
-        if (st != kActive) atomicMax(&v.counters->max_iters, it);
-        if (st == kCapped) atomicAdd(&v.counters->unfound, 1u);
-    }
-}
-
 // ------------------------------------------------------------------------------------
 // Service count-left: one plain pass at getCut() per cell, found cells skipped.
 // ------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads) k_count_left(Level v) {
+__global__ void __launch_bounds__(kThreads) k_count_left(const __grid_constant__ Level v) {
     pdl_enter();
     __shared__ uint32_t s_red[32];
-    const uint32_t total = v.tile_off[v.C];
+    const uint32_t total = (uint32_t)(v.tot->tiles >> 32);
     for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
         const TileRef tr = tile_ref(v, t);
         const orb_cell_t &cell = v.heap[tr.slot];
@@ -3468,12 +3678,25 @@ void launch_kernel(bool pdl, void (*kern)(P...), dim3 grid, dim3 block, size_t s
     cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+template <bool kFuse>
+void launch_swap(bool p, const Level &v, int grid, int arg, cudaStream_t st) {
+    const dim3 T(kSwapThreads);
+    if (v.wt)
+        launch_kernel(p, k_part_swap<true, 3, kFuse>, dim3(grid), T, 0, st, v, arg);
+    else if (!v.y)
+        launch_kernel(p, k_part_swap<false, 0, kFuse>, dim3(grid), T, 0, st, v, arg);
+    else if (!v.z)
+        launch_kernel(p, k_part_swap<false, 1, kFuse>, dim3(grid), T, 0, st, v, arg);
+    else
+        launch_kernel(p, k_part_swap<false, 3, kFuse>, dim3(grid), T, 0, st, v, arg);
+}
+
 void launch_level_kernel(Kernel k, const Level &v, int grid, int arg, cudaStream_t st) {
     const bool p = v.pdl != 0;
     const dim3 T(kThreads);
     const unsigned per_cell_warps = (unsigned)grid_for((uint64_t)v.C * 32, kThreads, 1 << 30);
     switch (k) {
-        case kKPlan: launch_kernel(p, k_plan, dim3(1), dim3(1024), 0, st, v); break;
+        case kKPlan: launch_kernel(p, k_plan, dim3(per_cell_warps), T, 0, st, v); break;
         case kKHist:  // arg: 1 first pass, all cells dense; 2 first pass of a sampled level
             if (arg == 1)
                 launch_kernel(p, k_hist<kHFirstDense>, dim3(grid), T, 0, st, v);
@@ -3483,9 +3706,6 @@ void launch_level_kernel(Kernel k, const Level &v, int grid, int arg, cudaStream
                 launch_kernel(p, k_hist<kHRest>, dim3(grid), T, 0, st, v);
             break;
         case kKBisectTile: launch_kernel(p, k_bisect_tile, dim3(grid), T, 0, st, v); break;
-        case kKWarmStart:
-            launch_kernel(p, k_warm_start, dim3(grid_for((uint64_t)v.C, kThreads, 1 << 30)), T, 0, st, v);
-            break;
         case kKSubtreeCheck: launch_kernel(p, k_subtree_check, dim3(1), dim3(1024), 0, st, v, arg); break;
         case kKSubtree:  // arg: 1 when cells of at most kWarpKeys particles can occur
             if (arg)
@@ -3496,27 +3716,28 @@ void launch_level_kernel(Kernel k, const Level &v, int grid, int arg, cudaStream
         case kKBisectCta:
             launch_kernel(p, k_bisect_cta, dim3(grid), dim3(kCtaThreads), kCtaSmemBytes, st, v);
             break;
-        case kKTileMap: launch_kernel(p, k_tile_map, dim3(grid), T, 0, st, v); break;
-        case kKResolve: launch_kernel(p, k_resolve, dim3(per_cell_warps), T, 0, st, v); break;
         case kKPartClassify: launch_kernel(p, k_part_classify, dim3(grid), T, 0, st, v); break;
-        case kKPartScan: launch_kernel(p, k_tile_scan, dim3(arg), dim3(kScanBlock), 0, st, v); break;
-        case kKPartCells: launch_kernel(p, k_part_cells, dim3(per_cell_warps), T, 0, st, v); break;
-        case kKPartSwap:
-            if (v.wt)
-                launch_kernel(p, k_part_swap<true, 3>, dim3(grid), dim3(kSwapThreads), 0, st, v);
-            else if (!v.y)
-                launch_kernel(p, k_part_swap<false, 0>, dim3(grid), dim3(kSwapThreads), 0, st, v);
-            else if (!v.z)
-                launch_kernel(p, k_part_swap<false, 1>, dim3(grid), dim3(kSwapThreads), 0, st, v);
+        case kKPartCells:
+            // grid = the SM count: levels of few cells take large CTAs, several a cell
+            if (v.C <= grid)
+                launch_kernel(p, k_part_cells<1024, true>, dim3((unsigned)std::max(1, std::min(64, grid / v.C)), v.C),
+                              dim3(1024), 0, st, v);
             else
-                launch_kernel(p, k_part_swap<false, 3>, dim3(grid), dim3(kSwapThreads), 0, st, v);
+                launch_kernel(p, k_part_cells<kThreads, false>, dim3(per_cell_warps), T, 0, st, v);
             break;
-        case kKWStart: launch_kernel(p, k_wstart, dim3(grid), T, 0, st, v); break;
+        case kKPartSwap:
+            if (v.fuse)
+                launch_swap<true>(p, v, grid, arg, st);
+            else
+                launch_swap<false>(p, v, grid, arg, st);
+            break;
+        case kKPartFinish:  // grid = the SM count
+            if (v.C <= grid)
+                launch_kernel(p, k_part_finish<true>, dim3(v.C), T, 0, st, v, arg);
+            else
+                launch_kernel(p, k_part_finish<false>, dim3(per_cell_warps), T, 0, st, v, arg);
+            break;
         case kKWHist: launch_kernel(p, k_whist, dim3(grid), T, 0, st, v); break;
-        case kKWResolve: launch_kernel(p, k_wresolve, dim3(per_cell_warps), T, 0, st, v); break;
-        case kKPartFinish:
-            launch_kernel(p, k_part_finish, dim3(grid_for(v.C, kThreads, 1 << 30)), T, 0, st, v, arg);
-            break;
         case kKCountLeft: launch_kernel(p, k_count_left, dim3(grid), T, 0, st, v); break;
         case kKSample:
             launch_kernel(p, k_sample_bin, dim3(kSampleMax / kSamplePerCta, (unsigned)min(v.C, 65535)),
@@ -3538,7 +3759,7 @@ int swap_blocks_per_sm() {
     // the swap's CTAs walk the tiles grid-stride: one resident wave, none waiting behind it
     static const int blocks = [] {
         int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_part_swap<false, 3>, kSwapThreads, 0) != cudaSuccess ||
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_part_swap<false, 3, false>, kSwapThreads, 0) != cudaSuccess ||
             b < 1) {
             cudaGetLastError();
             b = ORB_SWAP_MIN_BLOCKS;

@@ -406,14 +406,14 @@ orb_status orb_count_left_static(const float *x, const float *y, const float *z,
                                  void *stream);
 
 /*
- * Test hook of the bounded device waits (no counterpart in the reference, whose errors end
- * the process, src/constants.h:19-23). The partition's tile scan chains its blocks with a
- * decoupled look-back; each wait polls a predecessor's status at most spin_limit times
- * (0 = the default, about 2^22 polls), then flags the build and gives up: the kernels that
- * would read the scan's prefixes do nothing and the build returns ORB_ERR_TIMEOUT. The
- * context stays usable. ticket_start (0..255, normally 0) is the value the scan's block
- * ticket starts from: 1 means no block takes the first status slot, so its successor's
- * wait runs out, a wait that can never end made into one that ends in a bounded time.
+ * Test hook of the device's failure detection (no counterpart in the reference, whose errors
+ * end the process, src/constants.h:19-23). No kernel of the engine waits for another CTA: the
+ * partition's tiles count their arrivals per cell and whoever brings a cell's last one
+ * finishes the cell. A cell whose last arrival never comes is found by the next level's
+ * kernels, which then do nothing, and by the host at the build's end: the build returns
+ * ORB_ERR_TIMEOUT and the context stays usable. ticket_start (0..255, normally 0) makes every
+ * cell's arrivals start that far below zero, so that with 1 the last one is never counted.
+ * spin_limit: accepted for callers of earlier versions, which polled with that bound.
  * Settings stay until changed; (0, 0) restores the defaults.
  */
 orb_status orb_test_set_scan_wait(orb_ctx *ctx, uint32_t spin_limit, uint32_t ticket_start);

@@ -1,0 +1,51 @@
+"""The level kernels at the sizes and keys where their steps change: partition and count tile
+edges (4096 and 16384 positions), cells a warp or a CTA finishes, brackets a few floats wide
+(whose cut can come out as the bracket's upper end), keys at the box ends, NaN, and lists of
+bracket keys from almost none to every key. Bit for bit against the oracle."""
+import numpy as np
+import pytest
+
+from test_gpu_parity import run_both
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture()
+def tuned(ctx):
+    saved = ctx.get_tuning()
+    yield ctx
+    ctx.set_tuning(**saved)
+
+
+def keys(kind, n, seed):
+    rng = np.random.default_rng(seed)
+    u = rng.random((3, n), dtype=np.float32) - np.float32(0.5)
+    if kind == "narrow":  # a few neighbouring floats: every bracket ends a few ulps wide
+        base = np.float32(0.25).view(np.int32)
+        u = (base + rng.integers(0, 5, (3, n)).astype(np.int32)).view(np.float32)
+    elif kind == "ends":  # many keys on the box ends and on the first cuts, some NaN
+        pick = rng.integers(0, 6, (3, n))
+        u[pick == 0] = -0.5
+        u[pick == 1] = 0.5
+        u[pick == 2] = 0.0
+        u[(pick == 3) & (rng.random((3, n)) < 0.05)] = np.nan
+    return tuple(np.ascontiguousarray(a) for a in u)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "narrow", "ends"])
+@pytest.mark.parametrize("n", [1023, 4095, 4097, 16384, 16385, 65537, (1 << 18) + 1, (1 << 20) + 4097])
+def test_level_kernels_match_oracle(tuned, oracle, kind, n):
+    x, y, z = keys(kind, n, n)
+    for sparse in (64, 1, 16384):
+        tuned.set_tuning(sparse_keys_per_tile=sparse, subtree_levels=4 if sparse == 64 else 0)
+        run_both(tuned, oracle, x, y, z, 16)
+        run_both(tuned, oracle, x, y, z, 11)
+
+
+def test_many_listed_keys_in_one_cell(tuned, oracle):
+    """A root whose bracket holds tens of thousands of keys for the list (several CTAs on one
+    cell) and one whose list a single warp takes."""
+    tuned.set_tuning(sparse_keys_per_tile=16384)
+    for n in ((1 << 22) + 3, 300001):
+        x, y, z = keys("uniform", n, n)
+        run_both(tuned, oracle, x, y, z, 8)
