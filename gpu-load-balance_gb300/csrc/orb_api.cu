@@ -91,7 +91,7 @@ struct orb_ctx {
     // from below zero (0 normally; otherwise the last arrival never comes)
     uint32_t done_offset = 0;
     // launch tuning (orb_set_tuning / orb_autotune_batch); cta_min_cells = 0 means never
-    orb_tuning tune = {(uint32_t)kHistBlocksPerSm, 8u, (uint32_t)kTileBlocksPerSm, 64u, 0u, 4u, 0u};
+    orb_tuning tune = {(uint32_t)kHistBlocksPerSm, 8u, (uint32_t)kTileBlocksPerSm, 64u, 0u, kSubDefaultLevels, 0u};
     DevBuf<uint8_t> state, iters;
     DevBuf<uint32_t> cmp_off, cmp_cnt, cmp_pos, pred;
     DevBuf<float> cmp_keys;
@@ -107,6 +107,7 @@ struct orb_ctx {
     DevBuf<int> hint_axis;
     DevBuf<uint8_t> warm;
     DevBuf<uint32_t> sub_flag;  // subtree path taken (one word)
+    DevBuf<int> sub_list;       // the subtree kernel's cells by class
     DevBuf<uint32_t> w;         // weighted builds from host memory: the weights
     DevBuf<unsigned long long> gen_starts;  // xorshf96 generator: chunk start states
     DevBuf<unsigned long long> whist, wbelow, wtot;  // weighted builds: per-cell weight sums
@@ -450,6 +451,7 @@ std::vector<uint64_t> level_key(orb_ctx *ctx, const Level &v) {
                           (const void *)v.wbelow, (const void *)v.wtot})
         key_add(key, p);
     key_add(key, ctx->sub_flag.p);
+    key_add(key, ctx->sub_list.p);
     key.push_back(ctx->prof_mask);
     key.push_back(ctx->done_offset);
     key.push_back(ctx->use_pdl ? 1u : 0u);
@@ -520,18 +522,29 @@ uint32_t small_cells(const orb_ctx *ctx, const Level &v, uint64_t max_n, size_t 
 
 // The level from which subtree CTAs finish the tree (-1: none): the first level whose cells
 // (at most max_n >> l particles plus a few per split: each split leaves a cell within 3 of
-// half) all fit one CTA, that has enough cells to fill the GPU, and that is at most
-// tune.subtree_levels levels above the leaves. full: every tree is built to its leaves.
-int subtree_from(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, uint64_t max_n, bool full) {
-    const uint32_t want = std::min<uint32_t>(ctx->tune.subtree_levels, (uint32_t)kSubMaxLevels);
+// half) all fit one CTA and that is at most kSubMaxLevels above the leaves
+// (tune.subtree_levels below its default: at most that many). As many levels as fit: a level
+// there takes 5-10 ps a particle where the level kernels take 7-12 (2^27 uniform, 2^26
+// clustered), and 20-30 us instead of 45 where the cells are few. full: every tree is built to
+// its leaves. from: the levels before it are level kernels' (staged builds).
+int subtree_from(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, uint64_t max_n, bool full, size_t from) {
+    const uint32_t tuned = ctx->tune.subtree_levels;
+    const uint32_t want = tuned < kSubDefaultLevels ? tuned : (uint32_t)kSubMaxLevels;
     if (!full || want == 0) return -1;
-    for (size_t li = 0; li < lv.size(); ++li) {
-        const uint64_t expect = (max_n >> li) + 1 + 8ull * li;
-        if (expect <= kSubMaxParticles && (uint64_t)lv[li].C >= 2ull * (uint64_t)ctx->num_sms &&
-            lv.size() - li <= want)
-            return (int)li;
+    for (size_t li = from; li < lv.size(); ++li) {
+        if ((max_n >> li) + 1 + 8ull * li <= kSubMaxParticles && lv.size() - li <= want) return (int)li;
     }
     return -1;
+}
+
+// Warm builds: the first level that starts from the cells' extents (SIZE_MAX: none; see
+// kHintSubMax).
+size_t hint_levels(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, uint64_t max_n, bool full) {
+    for (size_t li = 0; full && li < lv.size(); ++li)
+        if ((max_n >> li) + 1 + 8ull * li <= kHintSubMax && lv[li].C >= 2 * ctx->num_sms &&
+            lv.size() - li <= std::min<uint32_t>(ctx->tune.subtree_levels, (uint32_t)kSubMaxLevels))
+            return li;
+    return SIZE_MAX;
 }
 
 // The reference's level loop (src/orbit.cpp:102-275) over every cell of every level: the
@@ -547,9 +560,10 @@ int subtree_from(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, uint64_t 
 // subtree kernel for the levels from sub_from down; rest = true: the levels from sub_from
 // down one by one, for builds whose subtree path the device refused.
 // [from, to): only those levels (staged builds run the levels in pieces).
+// v.hint set: levels below hint_to start from their hints (warm builds).
 orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, uint32_t *passes,
                       int sub_from, uint64_t n, uint64_t max_n, bool rest = false, size_t from = 0,
-                      size_t to = SIZE_MAX) {
+                      size_t to = SIZE_MAX, size_t hint_to = 0) {
     to = std::min(to, lv.size());
     v.plan_bins = v.wt ? 0u : 1u;
     for (size_t li = rest ? (size_t)sub_from : from; li < to; ++li) {
@@ -564,15 +578,15 @@ orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, u
         if (!rest && (int)li == sub_from) {
             if (v.C == 0) break;
             v.skip = ctx->sub_flag.p;
+            v.sub_list = ctx->sub_list.p;
+            v.sub_wide = v.C <= ctx->num_sms ? 1 : 0;
             run_kernel(ctx, kKSubtreeCheck, v, 1, (int)(lv.size() - li));
-            // the warp path for small cells when the deepest split cells can be that small
-            // (about max_n >> (levels - 1) particles, twice kWarpKeys allowing for uneven cells)
-            const bool small = (max_n >> (lv.size() - 1)) <= 2ull * kWarpKeys;
-            run_kernel(ctx, kKSubtree, v, std::min(v.C, ctx->num_sms * kSubtreeBlocksPerSm), small ? 1 : 0);
+            run_kernel(ctx, kKSubtree, v, std::min(v.C, ctx->num_sms));
             break;
         }
         if (v.C == 0) continue;
         v.small = small_cells(ctx, v, max_n, li, d.C);
+        const bool hinted = v.hint && li < hint_to;
         v.next_C = 0;  // nothing to plan below the last level or at the subtree level
         if (li + 1 < lv.size() && (rest || (int)li + 1 != sub_from)) {
             v.next_C = lv[li + 1].C;
@@ -582,8 +596,10 @@ orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, u
         if (rest && (int)li == sub_from) {
             // this level was not planned by the one above
             ORB_CUDA(cudaMemsetAsync(&ctx->counters.p->plan[0], 0, 2 * sizeof(PlanTotals), ctx->stream));
+            v.plan_hint = hinted ? 1 : 0;
             run_kernel(ctx, kKPlan, v, 1);
         }
+        v.plan_hint = v.hint && li + 1 < hint_to ? 1 : 0;
         if (v.wt) {
             // weighted build: every cell through the weighted passes (kWPasses reach the cap)
             const uint64_t tiles = n / kTile + (uint64_t)v.C;
@@ -592,21 +608,21 @@ orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, u
                 run_kernel(ctx, kKWHist, v, (int)std::min<uint64_t>(pass_grid(ctx), tiles));
                 ++*passes;
             }
-        } else if (ctx->tune.cta_min_cells && !v.hint && (uint32_t)v.C >= ctx->tune.cta_min_cells) {
+        } else if (ctx->tune.cta_min_cells && !hinted && (uint32_t)v.C >= ctx->tune.cta_min_cells) {
             // many cells: one CTA bisects one cell, no host round trip
             run_kernel(ctx, kKBisectCta, v, std::min(v.C, ctx->num_sms * 4));
         } else {
             // cold levels with cells of at least 2^18 particles: sampled brackets for the
             // first count pass (decided per cell on the device; result-invariant)
             const bool sampled =
-                !v.hint && ctx->tune.predict_sigmas && (max_n >> li) + 8ull * li >= (1ull << 18);
+                !hinted && ctx->tune.predict_sigmas && (max_n >> li) + 8ull * li >= (1ull << 18);
             if (sampled) {
                 run_kernel(ctx, kKSample, v, 0);
                 run_kernel(ctx, kKSamplePick, v, 0);
             }
             if (v.small)
                 run_kernel(ctx, kKBisectTile, v, std::min(v.C, ctx->num_sms * (int)ctx->tune.tile_blocks_per_sm));
-            orb_status st = run_bisection(ctx, v, n, passes, v.hint ? 0 : (sampled ? 2 : 1));
+            orb_status st = run_bisection(ctx, v, n, passes, hinted ? 0 : (sampled ? 2 : 1));
             if (st != ORB_OK) return st;
         }
         partition_level(ctx, v, n, true);
@@ -632,19 +648,23 @@ bool build_finished(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, size_t
 // build's end event is recorded again after it.
 orb_status finish_subtree_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv,
                                  std::vector<uint64_t> key, uint32_t *passes, int sub_from,
-                                 uint64_t n, uint64_t max_n, bool *taken) {
+                                 uint64_t n, uint64_t max_n, size_t hint_to, bool *taken) {
     *taken = false;
     if (sub_from < 0) return ORB_OK;
     ORB_CUDA(cudaMemcpyAsync(ctx->h_sub_flag, ctx->sub_flag.p, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                              ctx->stream));
     ORB_CUDA(cudaStreamSynchronize(ctx->stream));
-    *taken = *ctx->h_sub_flag != 0;
+    *taken = *ctx->h_sub_flag == 1u;
     if (*taken) return ORB_OK;
     if (ctx->use_graphs) collect_graph_profile(ctx);  // the main graph's kernel events
     key.push_back(0x5E57u);  // the levels from sub_from down
     v.skip = nullptr;
+    // warm builds: a refusal for another reason than the subtree kernel's shared memory leaves
+    // the levels to their hints
+    if (v.hint && *ctx->h_sub_flag == 0u) hint_to = SIZE_MAX;
+    key.push_back(hint_to == SIZE_MAX ? 1u : 0u);
     orb_status st = run_graphed(ctx, key, passes, [&](uint32_t *pp) -> orb_status {
-        return run_levels(ctx, v, lv, pp, sub_from, n, max_n, true);
+        return run_levels(ctx, v, lv, pp, sub_from, n, max_n, true, 0, SIZE_MAX, hint_to);
     });
     if (st != ORB_OK) return st;
     ORB_CUDA(cudaEventRecord(ctx->ev[1], ctx->stream));
@@ -770,6 +790,7 @@ orb_status orb_ctx_destroy(orb_ctx *ctx) {
         ctx->tune_work[a].release();
     }
     ctx->hint.release(); ctx->hint_axis.release(); ctx->warm.release(); ctx->sub_flag.release();
+    ctx->sub_list.release();
     ctx->w.release(); ctx->whist.release(); ctx->wbelow.release(); ctx->wtot.release();
     ctx->gen_starts.release();
     ctx->cmp_off.release(); ctx->cmp_cnt.release(); ctx->cmp_keys.release(); ctx->cmp_pos.release();
@@ -872,9 +893,6 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     std::vector<LevelDesc> lv;
     for (uint32_t l = 1; l <= levels; ++l)
         lv.push_back({sl.first(l), nullptr, sl.count(l), nullptr});  // src/orbit.cpp:104-107
-    // subtrees finish complete unweighted trees only: d a power of two, built to its leaves
-    const int sub_from = subtree_from(ctx, lv, n, !weighted && sl.pow2 && levels == sl.depth);
-    if (sub_from >= 0) ORB_CUDA(ctx->sub_flag.ensure(1));
     // Staged build from host memory: the copies of x, y and z follow one another, and the
     // levels start as soon as the coordinates they read are on the device. Level 1 cuts along
     // x (src/orbit.cpp:75), so it runs on x alone while y arrives; its swaps move x and the
@@ -884,8 +902,13 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     // first-longest rule of setCutAxis (src/cell.h:102-121) picks x or y there, so level 2
     // runs on x and y while z arrives. Same cuts, same swaps: the result is the unstaged one.
     const float y_ext = upper[1] - lower[1], z_ext = upper[2] - lower[2];
-    const bool staged = !dev && n && !weighted && ctx->use_stage && levels >= 2 &&
-                        (sub_from < 0 || sub_from >= 2) && y_ext > 0.f && y_ext >= z_ext;
+    const bool staged = !dev && n && !weighted && ctx->use_stage && levels >= 2 && y_ext > 0.f && y_ext >= z_ext;
+    // subtrees finish complete unweighted trees only: d a power of two, built to its leaves
+    const int sub_from = subtree_from(ctx, lv, n, !weighted && sl.pow2 && levels == sl.depth, staged ? 2 : 0);
+    if (sub_from >= 0) {
+        ORB_CUDA(ctx->sub_flag.ensure(1));
+        ORB_CUDA(ctx->sub_list.ensure(4 * (size_t)lv[sub_from].C));
+    }
     if (!dev) {
         ORB_CUDA(ctx->x.ensure(n + 1));
         ORB_CUDA(ctx->y.ensure(n + 1));
@@ -1055,7 +1078,7 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     bool streamed = false;
     if (windows && (st = stream_windows(&streamed)) != ORB_OK) return st;
     bool taken = false;  // the subtree kernel finished the tree
-    st = finish_subtree_levels(ctx, v, lv, key, &passes, sub_from, n, n, &taken);
+    st = finish_subtree_levels(ctx, v, lv, key, &passes, sub_from, n, n, 0, &taken);
     if (st != ORB_OK) return st;
     bool written = false;  // the particles are in the host arrays (or on their way there)
     if (!dev) {
@@ -1625,8 +1648,14 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
         full = full && sl.pow2 && lev[i] == sl.depth;
         max_n = std::max<uint64_t>(max_n, inst[i].n);
     }
-    const int sub_from = subtree_from(ctx, lv, max_n, full);
-    if (sub_from >= 0) ORB_CUDA(ctx->sub_flag.ensure(1));
+    // warm: the subtree kernel only on levels that take no hints
+    const size_t hint_to = warm ? hint_levels(ctx, lv, max_n, full) : 0;
+    const int sub_from = hint_to == SIZE_MAX ? -1 : subtree_from(ctx, lv, max_n, full, hint_to);
+    key.push_back((uint64_t)hint_to);
+    if (sub_from >= 0) {
+        ORB_CUDA(ctx->sub_flag.ensure(1));
+        ORB_CUDA(ctx->sub_list.ensure(4 * (size_t)lv[sub_from].C));
+    }
     key.push_back((uint64_t)(int64_t)sub_from);
     uint32_t passes = 0;
     st = run_graphed(ctx, key, &passes, [&](uint32_t *pp) -> orb_status {
@@ -1640,14 +1669,15 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
             v0.C = lv[0].C;
         }
         v0.small = small_cells(ctx, v0, max_n, 0, v0.C);
+        v0.plan_hint = warm && hint_to > 0 ? 1 : 0;
         launch_init_batch(v0, ctx->batch_roots.p, (int)k, n_total, s);
         ORB_CUDA(cudaGetLastError());
-        return run_levels(ctx, v, lv, pp, sub_from, n_total, max_n);
+        return run_levels(ctx, v, lv, pp, sub_from, n_total, max_n, false, 0, SIZE_MAX, hint_to);
     });
     if (st != ORB_OK) return st;
     ORB_CUDA(cudaEventRecord(ctx->ev[1], s));
     bool taken = false;
-    st = finish_subtree_levels(ctx, v, lv, key, &passes, sub_from, n_total, max_n, &taken);
+    st = finish_subtree_levels(ctx, v, lv, key, &passes, sub_from, n_total, max_n, hint_to, &taken);
     if (st != ORB_OK) return st;
     if (!dev) {
         ORB_CUDA(cudaStreamSynchronize(s));

@@ -33,11 +33,13 @@ constexpr int kThreads = 256;
 #endif
 constexpr int kHistBlocksPerSm = ORB_HIST_BLOCKS_PER_SM;
 constexpr int kTileBlocksPerSm = 4;  // resident CTAs of the one-tile cell bisection
-constexpr int kSubtreeBlocksPerSm = 4;  // CTAs of the subtree kernel per SM (its grid)
-#ifndef ORB_SUB_MAX
-#define ORB_SUB_MAX 34816  // 2^15 + 2048: a 2^27-particle tree takes its last 4 levels
-#endif
-constexpr uint32_t kSubMaxParticles = ORB_SUB_MAX;  // largest cell one subtree CTA takes
+constexpr uint32_t kSubMaxParticles = 33024;  // largest cell one subtree CTA takes (2^15 + 256)
+// Warm builds: hints apply to the levels above the first one of at least two cells per SM whose
+// cells have at most this many particles and that is at most tune.subtree_levels above the
+// leaves (which levels start from hints decides the trees, so the line stays where it was
+// whatever the subtree kernel takes).
+constexpr uint32_t kHintSubMax = 34816;
+constexpr uint32_t kSubDefaultLevels = 4;     // default of tune.subtree_levels
 constexpr int kSubMaxLevels = 6;              // deepest tree one subtree CTA finishes
 
 // Weighted builds: every active cell's bracket is binned into a midpoint tree of this depth
@@ -110,7 +112,8 @@ struct BuildCounters {
     uint32_t warm_resets; // ... whose hinted bracket missed the target (restarted cold)
     uint32_t pred_cells;  // cells whose first count pass used a sampled bracket
     uint32_t pred_misses; // ... whose sampled bracket did not hold the cut (binned again)
-    uint32_t sub_next;    // next root cell of the subtree kernel's work queue
+    uint32_t sub_cells[4];  // the subtree kernel's cells by class, and its work queues
+    uint32_t sub_next[4];
     unsigned long long bytes[32];  // algorithmic bytes per Kernel kind
 };
 
@@ -193,9 +196,12 @@ struct Level {
     const float2 *hint;     // (cut, w x extent) from the previous tree
     const int *hint_axis;
     uint8_t *warm;          // [C] 1 while a hinted bracket is not yet checked
+    int plan_hint;          // 1: the cells being planned start from their hints
     // subtrees: 1 when one CTA per cell finishes the tree from this level down; null when
     // not attempted
     uint32_t *skip;
+    int *sub_list;          // [4 C] the subtree kernel's cells by class
+    int sub_wide;           // 1: all of a CTA's warps on every cell (levels of few cells)
     // window reports (null otherwise): the host-mapped reports, a finished-cell counter per
     // window, root cells per window
     HostWindows *hwin;

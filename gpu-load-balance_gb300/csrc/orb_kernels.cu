@@ -304,7 +304,10 @@ __device__ PlanCell plan_cell(const Level &v, PlanTotals *tot, uint32_t small, i
         v.wbelow[c] = 0ull;
         v.wtot[c] = 0ull;
     }
-    if (v.hint) warm_start_cell(v, c, slot, n);
+    if (v.warm) {
+        v.warm[c] = 0;
+        if (v.plan_hint) warm_start_cell(v, c, slot, n);
+    }
     return p;
 }
 
@@ -1969,6 +1972,29 @@ __device__ void set_axis_and_margin(orb_cell_t &c, BuildCounters *ctr) {
     c.cutMarginRight = c.upper[a];
 }
 
+// The children of a cell at its cut: Cell::cut (src/cell.h:78-100) and src/orbit.cpp:238-246.
+__device__ __forceinline__ void split_cell(const orb_cell_t &cell, orb_cell_t &lc, orb_cell_t &rc,
+                                           BuildCounters *ctr) {
+    const float cut = cell_cut(cell);
+    const int a = eff_axis(cell.cutAxis);
+    const int n_left = (cell.nLeafCells + 1) / 2;
+    lc.id = 2 * cell.id + 1;
+    rc.id = 2 * cell.id + 2;
+    lc.nLeafCells = n_left;
+    rc.nLeafCells = cell.nLeafCells - n_left;
+    lc.prevCutAxis = rc.prevCutAxis = cell.cutAxis;
+    lc.foundCut = rc.foundCut = 0;
+    lc.pad_[0] = lc.pad_[1] = lc.pad_[2] = 0;
+    rc.pad_[0] = rc.pad_[1] = rc.pad_[2] = 0;
+    for (int k = 0; k < 3; ++k) {
+        lc.lower[k] = rc.lower[k] = cell.lower[k];
+        lc.upper[k] = rc.upper[k] = cell.upper[k];
+        if (k == a) lc.upper[k] = rc.lower[k] = cut;
+    }
+    set_axis_and_margin(rc, ctr);
+    set_axis_and_margin(lc, ctr);
+}
+
 // Final swap(i, n-1) of a partitioned cell (src/services/partition.cpp:52), its children's
 // ranges and (optionally) its children's cells.
 __device__ void finish_cell(const Level &v, int slot, uint32_t i, bool do_split) {
@@ -1985,27 +2011,8 @@ __device__ void finish_cell(const Level &v, int slot, uint32_t i, bool do_split)
     v.ranges[lslot] = make_uint2(rg.x, rg.x + i);
     v.ranges[rslot] = make_uint2(rg.x + i, rg.y);
     if (!do_split) return;
-    // Cell::cut (src/cell.h:78-100) and src/orbit.cpp:238-246
-    const float cut = cell_cut(cell);
-    const int a = eff_axis(cell.cutAxis);
-    const int n_left = (cell.nLeafCells + 1) / 2;
     orb_cell_t lc, rc;
-    lc.id = 2 * cell.id + 1;
-    rc.id = 2 * cell.id + 2;
-    lc.nLeafCells = n_left;
-    rc.nLeafCells = cell.nLeafCells - n_left;
-    lc.prevCutAxis = rc.prevCutAxis = cell.cutAxis;
-    lc.foundCut = rc.foundCut = 0;
-    lc.pad_[0] = lc.pad_[1] = lc.pad_[2] = 0;
-    rc.pad_[0] = rc.pad_[1] = rc.pad_[2] = 0;
-    for (int k = 0; k < 3; ++k) {
-        lc.lower[k] = rc.lower[k] = cell.lower[k];
-        lc.upper[k] = rc.upper[k] = cell.upper[k];
-    }
-    lc.upper[a] = cut;
-    rc.lower[a] = cut;
-    set_axis_and_margin(rc, v.counters);
-    set_axis_and_margin(lc, v.counters);
+    split_cell(cell, lc, rc, v.counters);
     v.heap[lslot] = lc;
     v.heap[rslot] = rc;
 }
@@ -2060,16 +2067,17 @@ struct CellsSmem {
     uint32_t last;       // the cell's other CTAs have arrived
 };
 
-// The rest of the reference loop on at most kWarpList bracket keys, 16 a lane (lanes past m
+// The rest of the reference loop on at most 32 N bracket keys, N a lane (slots past them
 // hold R, which no cut in [L, R] exceeds); `below` keys lie below all of them. Every lane.
-__device__ __forceinline__ int bisect_list(const float (&kl)[kWarpList / 32], uint32_t below, uint32_t n, float ratio,
+template <int N>
+__device__ __forceinline__ int bisect_list(const float (&kl)[N], uint32_t below, uint32_t n, float ratio,
                                            float &L, float &R, uint32_t &it) {
     for (;;) {
         if (it >= (uint32_t)kMaxIterations) return kCapped;
         const float cut = mid_cut(L, R);
         uint32_t c = 0;
 #pragma unroll
-        for (int q = 0; q < (int)kWarpList / 32; ++q) c += kl[q] < cut;
+        for (int q = 0; q < N; ++q) c += kl[q] < cut;
         ++it;
         const int dir = convergence(below + __reduce_add_sync(0xffffffffu, c), n, ratio);
         if (dir == 0) return kFound;
@@ -2632,537 +2640,148 @@ __global__ void __launch_bounds__(kThreads) k_part_finish(const __grid_constant_
 }
 
 // ------------------------------------------------------------------------------------
-// Subtrees: once every cell of a level holds at most kSubMax particles, one CTA takes a
-// cell and finishes all the levels below it (bisection, Hoare partition and split of each
-// descendant, breadth first), the same steps as the level kernels at CTA scale. A cell's
-// particles (at most 408 KB) stay in L2 across its levels instead of crossing DRAM once per
-// level, and the level kernels of those levels do not run.
+// Subtrees: once every cell of a level fits one CTA, the rest of each cell's tree (bisection,
+// Hoare partition and split of every descendant, breadth first) is built in shared memory
+// without moving a particle until the end: a group of warps holds one axis of the cell's keys
+// in their original order and the current order as 16-bit positions. A level loads the axis
+// its cells cut along (a coalesced copy of 4 B a particle, mostly from L2), reads the keys
+// through the positions, and its swaps exchange 2-byte positions. At the end each coordinate
+// is loaded once more and written through the positions: in all 4 B a particle and level plus
+// 24 B (32 B with the permutation), every access coalesced. The cells of a level are worked on
+// side by side, the group's warps divided evenly among them, all in step.
+//
+// Measured (GB300): the last four levels of 2^27 uniform particles into 2^16 leaves (cells of
+// 2^15) take 2.68 ms, against 3.88 ms for a CTA of 256 threads that moved the particles in
+// global memory at every level (four such CTAs an SM, its cells re-read from L2); 2^26
+// clustered into 2^18, the last four levels: 2.12 against 3.69 ms.
+//
+// The kernel is bound by instructions and shared memory, so the bisection avoids exact binning: a histogram by
+// the rounded scaled key finds a window [a, b) of floats around the target rank (a few dozen
+// keys); the pass that writes the masks counts the keys below a and above b exactly and lists
+// those inside; then the reference loop (src/orbit.cpp:146-232) is replayed from the cell's own
+// margins: a cut at or below a has a count of at most count(< a), one at or above b at least
+// count(< b), so where the exact counts show the first too low and the second too high the
+// loop moves that margin (the float test is monotone in the count), and a cut inside the
+// window gets its exact count from the list. A cell whose replay meets a cut the window
+// cannot settle (many equal keys, a box far wider than its keys) counts every cut over all
+// its keys instead. Same cuts, same integer counts, same iterations on every path.
+//
+// A group is the CTA's 32 warps, or 16, 8 or 2 of them for smaller cells (by size): small
+// cells are bound by the latency of their steps, so an SM keeps 2, 4 or 16 in flight.
 // ------------------------------------------------------------------------------------
-constexpr uint32_t kSubMax = kSubMaxParticles;  // particles of a cell a CTA can take (masks)
-constexpr int kSubWords = (int)(kSubMax / 32);
-constexpr int kSubThreads = 256;
-constexpr int kSubBinsLog2 = 9;
-constexpr int kSubQueue = 64;                 // descendants of one level held at once
+constexpr int kSubLevels = kSubMaxLevels;
+constexpr int kSubCells = 1 << (kSubLevels - 1);  // cells of the deepest level split
+constexpr int kSubThreads = 1024;                 // of the CTA, one on an SM
+constexpr uint32_t kSubSpins = 1u << 20;           // polls of one copy's wait (each waits in hardware)
+constexpr uint32_t kSubDirect = 256;              // cells up to this size: one warp's registers
+constexpr uint32_t kSubWindowList = 256;          // most listed keys of a cell (8 a lane)
 
-constexpr int kSubList = 256;                 // bracket keys gathered for the last iterations
-constexpr int kSubRankBlocks = (int)(kSubMax / 64) + 2;
-
-struct SubSmem {
-    uint32_t ge[kSubWords], le[kSubWords];           // key >= cut, key <= cut
-    uint32_t pge[kSubWords + 1], ple[kSubWords + 1];  // exclusive prefix popcounts
-    uint16_t tge[kSubRankBlocks], tle[kSubRankBlocks];  // word holding rank 64 b
-    uint32_t bins[1 << kSubBinsLog2];
-    float edges[(1 << kSubBinsLog2) + 1];
-    float list[kSubList];
-    uint32_t red[96];
-    int queue[2][kSubQueue];
-    uint32_t word, count;                            // broadcast values
-    int root;                                        // the CTA's current root cell
+struct SubCell {
+    int id, leaves, axis;
+    float lower[3], upper[3];
+    uint16_t b, m;  // first position within the root cell, particles
 };
 
-// sub_select() through the rank table t (t[b] = the word holding rank 64 b): a few steps
-// from the table's word instead of a search.
-__device__ __forceinline__ uint32_t sub_select_t(const uint32_t *bits, const uint32_t *pre,
-                                                 const uint16_t *t, uint32_t r) {
-    uint32_t w = t[r >> 6];
-    while (pre[w + 1] <= r) ++w;
-    return w * 32u + select_in_word(bits[w], r - pre[w]);
-}
+// Bisection and partition state of one cell of the level.
+enum : uint32_t { kSubOpen = 0, kSubDone = 1, kSubWindow = 2, kSubCount = 3 };
+struct SubState {
+    float L, R;          // the bisection's bracket
+    float a, b;          // the window (kSubOpen: being narrowed; kSubWindow: classified)
+    uint32_t mode;       // kSubOpen, kSubWindow, kSubCount (counts every cut), kSubDone
+    uint16_t it, found;
+    uint32_t cand;       // keys in the window by the last histogram (~0: none yet)
+    uint32_t cnt;        // kSubCount: keys below the cut
+    uint32_t nlist;      // listed keys
+    uint32_t tot;        // keys >= cut | keys <= cut << 16
+    uint32_t cross, s, i;
+};
 
-// Position (cell-relative) of the set bit of rank r (0-based) of the mask `bits`, given
-// its exclusive word prefix `pre` over W words.
-__device__ __forceinline__ uint32_t sub_select(const uint32_t *bits, const uint32_t *pre, int W,
-                                               uint32_t r) {
-    int lo = 0, hi = W - 1;  // last word with pre <= r
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (pre[mid] <= r)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    return (uint32_t)lo * 32u + select_in_word(bits[lo], r - pre[lo]);
-}
+template <int NW>
+struct SubSmem {
+    static constexpr uint32_t kBins = NW >= 16 ? 2048 : (NW == 8 ? 1024 : 256);   // a level's cells together
+    static constexpr uint32_t kLists = NW >= 16 ? 1024 : (NW == 8 ? 512 : 256);
+    SubCell cell[2][kSubCells];
+    SubState state[kSubCells];
+    uint32_t bins[kBins];
+    float lkey[kLists];
+    uint16_t lpos[kLists];
+    uint32_t part[NW];
+    uint32_t axes;    // axes the level's cells cut along
+    uint32_t counted; // ... those of cells too large for one warp's registers
+    uint32_t more, direct;
+    uint32_t max_it, unfound, degenerate;
+    int item, root;
+    alignas(8) unsigned long long arrived;  // mbarrier of the key copies
+};
 
-// The reference's bisection (src/orbit.cpp:146-232) of one cell by the CTA: a warp with the
-// keys in registers for at most kWarpKeys keys, else rounds of a shared-memory histogram over
-// the midpoint tree of the bracket (tree depth from the keys left in it) each replaying up to
-// K iterations, as k_bisect_tile does per warp.
-__device__ void sub_bisect(const Level &v, int slot, SubSmem &sm, unsigned long long &bytes) {
-    orb_cell_t &cell = v.heap[slot];
-    const uint2 rg = v.ranges[slot];
-    const uint32_t n = rg.y - rg.x;
-    // subtrees run for d a power of two only: every cell below has an even leaf count
-    const float ratio = 0.5f;  // leaf_ratio(cell.nLeafCells), src/orbit.cpp:204
-    const float *keys = axis_keys(v, eff_axis(cell.cutAxis));
-    const uint32_t tid = threadIdx.x, lane = tid & 31;
-    float L = cell.cutMarginLeft, R = cell.cutMarginRight;
-    uint32_t it = 0;
-    int st = kActive;
-    if (n <= (uint32_t)kWarpKeys) {
-        if (tid < 32) {
-            float k[kWarpKeysPerLane];
-#pragma unroll
-            for (int j = 0; j < kWarpKeysPerLane; ++j) {
-                const uint32_t i = (uint32_t)(j * 32) + lane;
-                k[j] = i < n ? keys[rg.x + i] : __int_as_float(0x7fc00000);  // coherent: moved here
-            }
-            while (st == kActive) {
-                if (it >= (uint32_t)kMaxIterations) {
-                    st = kCapped;
-                    break;
-                }
-                const float cut = mid_cut(L, R);
-                uint32_t cnt = 0;
-#pragma unroll
-                for (int j = 0; j < kWarpKeysPerLane; ++j) cnt += k[j] < cut;
-                cnt = warp_sum(cnt);
-                ++it;
-                const int dir = convergence(cnt, n, ratio);
-                if (dir == 0)
-                    st = kFound;
-                else if (dir > 0)
-                    R = cut;
-                else
-                    L = cut;
-            }
-        }
-        if (tid == 0) bytes += 4ull * n;
-    } else {
-        uint32_t cand = n;
-        while (st == kActive) {
-            // about one key a bin once the bracket is small: two rounds for most cells
-            const int K = max(1, min(kSubBinsLog2, 32 - __clz(max(cand, 1u))));
-            const uint32_t nb = 1u << K;
-            for (uint32_t j = tid; j < nb; j += blockDim.x) sm.bins[j] = 0u;
-            fill_edges(sm.edges, L, R, K, tid, blockDim.x);
-            __syncthreads();
-            const float scale = __fdiv_rn((float)nb, __fsub_rn(R, L));
-            const Guess gs = make_guess(L, R, scale, nb);
-            const int top = (int)nb - 1;
-            uint32_t below = 0;
-            auto one = [&](float k) {
-                if (k < L)
-                    ++below;
-                else if (k < R)
-                    atomicAdd(&sm.bins[fast_bin(k, gs, top, sm.edges)], 1u);
-            };
-            visit_keys<false>(keys, rg.x, rg.y, R, tid, blockDim.x, one, each(one));
-            if (tid == 0) bytes += 4ull * n;
-            below = block_sum(below, sm.red);
-            // exclusive prefix of the bins in place (each thread its own run)
-            const uint32_t per = max(1u, nb / blockDim.x), j0 = tid * per, j1 = min(nb, j0 + per);
-            uint32_t loc = 0;
-            for (uint32_t j = j0; j < j1; ++j) loc += sm.bins[j];
-            uint32_t tot, unused;
-            uint32_t run = block_excl_scan2(loc, 0u, sm.red, &tot, &unused).x;
-            for (uint32_t j = j0; j < j1; ++j) {
-                const uint32_t h = sm.bins[j];
-                sm.bins[j] = run;
-                run += h;
-            }
-            __syncthreads();
-            uint32_t pos = 0, width = nb;
-            for (int step = 0; step < K; ++step) {
-                if (it >= (uint32_t)kMaxIterations) {
-                    st = kCapped;
-                    break;
-                }
-                const uint32_t half = width >> 1;
-                const uint32_t cl = below + sm.bins[pos + half];
-                ++it;
-                const int dir = convergence(cl, n, ratio);
-                if (dir == 0) {
-                    st = kFound;
-                    break;
-                }
-                const float cut = mid_cut(L, R);
-                if (dir > 0) {
-                    R = cut;
-                } else {
-                    L = cut;
-                    pos += half;
-                }
-                width = half;
-            }
-            if (st == kActive && it >= (uint32_t)kMaxIterations) st = kCapped;
-            if (st == kActive) cand = (pos + 1 < nb ? sm.bins[pos + 1] : tot) - sm.bins[pos];
-            const uint32_t below_L = below + sm.bins[pos];  // keys below the new L
-            __syncthreads();  // the bins are rewritten by the next round
-            if (st == kActive && cand <= (uint32_t)kSubList) {
-                // the bracket's keys into a shared list; warp 0 finishes the bisection on it
-                if (tid == 0) sm.count = 0;
-                __syncthreads();
-                auto gather = [&](float k) {
-                    if (!(k < L) && k < R) sm.list[atomicAdd(&sm.count, 1u)] = k;
-                };
-                visit_keys<false>(keys, rg.x, rg.y, R, tid, blockDim.x, gather, each(gather));
-                if (tid == 0) bytes += 4ull * n;
-                __syncthreads();
-                if (tid < 32) {
-                    const uint32_t m = sm.count;
-                    constexpr int kPer = kSubList / 32;
-                    float kl[kPer];
-#pragma unroll
-                    for (int q = 0; q < kPer; ++q) {
-                        const uint32_t i = (uint32_t)q * 32u + lane;
-                        kl[q] = i < m ? sm.list[i] : R;  // R: never below a cut in [L, R]
-                    }
-                    while (st == kActive) {
-                        if (it >= (uint32_t)kMaxIterations) {
-                            st = kCapped;
-                            break;
-                        }
-                        const float cut = mid_cut(L, R);
-                        uint32_t c = 0;
-#pragma unroll
-                        for (int q = 0; q < kPer; ++q) c += kl[q] < cut;
-                        const uint32_t cl = below_L + warp_sum(c);
-                        ++it;
-                        const int dir = convergence(cl, n, ratio);
-                        if (dir == 0)
-                            st = kFound;
-                        else if (dir > 0)
-                            R = cut;
-                        else
-                            L = cut;
-                    }
-                }
-                break;  // warp 0 holds the result (thread 0 writes it)
-            }
-        }
-    }
-    if (tid == 0) {
-        cell.cutMarginLeft = L;
-        cell.cutMarginRight = R;
-        cell.foundCut = st == kFound ? 1 : 0;
-        atomicMax(&v.counters->max_iters, it);
-        if (st == kCapped) atomicAdd(&v.counters->unfound, 1u);
-    }
-    __syncthreads();
+// Shared memory of a group: SubSmem, keys (up to three words of misalignment), mask words and
+// their prefixes (a partial word a cell), order.
+__host__ __device__ constexpr uint32_t sub_words(uint32_t nmax) { return nmax / 32 + kSubCells + 2; }
+template <int NW>
+__host__ __device__ constexpr uint32_t sub_bytes(uint32_t nmax) {
+    return ((uint32_t)((sizeof(SubSmem<NW>) + 15) / 16 * 16) + (nmax + 4) * 4 + sub_words(nmax) * 12 + nmax * 2 + 15) / 16 * 16;
 }
-
-// Hoare partition of one cell by the CTA (same characterisation as the level kernels: the
-// pairs (L_k, R_k), k < s, swapped, then i = min(L_{s+1}, R_s) and swap(i, n-1)), then the
-// split into its children.
-__device__ void sub_partition(const Level &v, int slot, SubSmem &sm, unsigned long long &bytes) {
-    const orb_cell_t &cell = v.heap[slot];
-    const uint2 rg = v.ranges[slot];
-    const uint32_t n = rg.y - rg.x, b = rg.x;
-    const float *keys = axis_keys(v, eff_axis(cell.cutAxis));
-    const float cut = cell_cut(cell);
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    const int W = (int)((n + 31) / 32);
-    // masks: a warp per word, kSubLoads words of a warp in flight at once
-    constexpr int kSubLoads = 8;
-    for (int w0 = (int)warp; w0 < W; w0 += (int)nwarps * kSubLoads) {
-        float k[kSubLoads];
-#pragma unroll
-        for (int u = 0; u < kSubLoads; ++u) {
-            const int w = w0 + u * (int)nwarps;
-            const uint32_t i = (uint32_t)w * 32u + lane;
-            k[u] = (w < W && i < n) ? keys[b + i] : 0.0f;  // coherent: the CTA moved these keys
-        }
-#pragma unroll
-        for (int u = 0; u < kSubLoads; ++u) {
-            const int w = w0 + u * (int)nwarps;
-            if (w >= W) break;
-            const bool valid = (uint32_t)w * 32u + lane < n;
-            const uint32_t gb = __ballot_sync(0xffffffffu, valid && !(k[u] < cut));
-            const uint32_t lb = __ballot_sync(0xffffffffu, valid && !(k[u] > cut));
-            if (lane == 0) {
-                sm.ge[w] = gb;
-                sm.le[w] = lb;
-            }
-        }
-    }
-    __syncthreads();
-    // exclusive prefix popcounts of both masks
-    const int per = (W + (int)blockDim.x - 1) / (int)blockDim.x;
-    const int w0 = (int)tid * per, w1 = min(W, w0 + per);
-    uint32_t cg = 0, cl = 0;
-    for (int w = w0; w < w1; ++w) {
-        cg += __popc(sm.ge[w]);
-        cl += __popc(sm.le[w]);
-    }
-    uint32_t ge_tot, le_tot;
-    const uint2 ex = block_excl_scan2(cg, cl, sm.red, &ge_tot, &le_tot);
-    uint32_t rg_ = ex.x, rl = ex.y;
-    for (int w = w0; w < w1; ++w) {
-        sm.pge[w] = rg_;
-        sm.ple[w] = rl;
-        rg_ += __popc(sm.ge[w]);
-        rl += __popc(sm.le[w]);
-    }
-    if (tid == 0) {
-        sm.pge[W] = ge_tot;
-        sm.ple[W] = le_tot;
-    }
-    __syncthreads();  // prefixes complete
-    // rank tables: the word holding rank 64 b of each mask
-    for (int w = (int)tid; w < W; w += (int)blockDim.x) {
-        for (uint32_t r = (sm.pge[w] + 63u) & ~63u; r < sm.pge[w + 1]; r += 64u) sm.tge[r >> 6] = (uint16_t)w;
-        for (uint32_t r = (sm.ple[w] + 63u) & ~63u; r < sm.ple[w + 1]; r += 64u) sm.tle[r >> 6] = (uint16_t)w;
-    }
-    // s = max over x of min(#>= in [0,x), #<= in [x,n)): min(f, g) rises while f < g and
-    // falls after, so the maximum lies in the first word at whose end f >= g (one thread)
-    if (tid == 0) {
-        uint32_t s_max = 0;
-        if (W > 0) {
-            int lo = 0, hi = W - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (sm.pge[mid + 1] >= le_tot - sm.ple[mid + 1])
-                    hi = mid;
-                else
-                    lo = mid + 1;
-            }
-            uint32_t f = sm.pge[lo], g = le_tot - sm.ple[lo];
-            uint32_t a = sm.ge[lo], c = sm.le[lo];
-            s_max = min(f, g);
-            for (int q = 0; q < 32; ++q) {
-                f += a & 1u;
-                g -= c & 1u;
-                a >>= 1;
-                c >>= 1;
-                s_max = max(s_max, min(f, g));
-            }
-        }
-        sm.count = s_max;
-    }
-    __syncthreads();
-    const uint32_t s_pairs = sm.count;
-    // split index i = min(L_{s+1}, R_s); n when every key is below the cut
-    if (tid == 0) {
-        uint32_t i = n;
-        if (ge_tot > s_pairs) i = min(i, sub_select(sm.ge, sm.pge, W, s_pairs));
-        if (s_pairs >= 1) i = min(i, sub_select(sm.le, sm.ple, W, le_tot - s_pairs));
-        sm.word = i;
-    }
-    // the swaps: pair k = (rank k of >=, rank le_tot-1-k of <=); sides disjoint; a thread
-    // loads kSubPairs pairs before it stores any
-    constexpr int kSubPairs = 2;
-    for (uint32_t k0 = tid; k0 < s_pairs; k0 += blockDim.x * kSubPairs) {
-        uint32_t pa[kSubPairs], pb[kSubPairs];
-        float xa[kSubPairs], xb[kSubPairs], ya[kSubPairs], yb[kSubPairs], za[kSubPairs], zb[kSubPairs];
-        uint32_t ia[kSubPairs], ib[kSubPairs];
-#pragma unroll
-        for (int q = 0; q < kSubPairs; ++q) {
-            const uint32_t k = k0 + q * blockDim.x;
-            pa[q] = pb[q] = 0xffffffffu;
-            if (k < s_pairs) {
-                pa[q] = b + sub_select_t(sm.ge, sm.pge, sm.tge, k);
-                pb[q] = b + sub_select_t(sm.le, sm.ple, sm.tle, le_tot - 1 - k);
-                xa[q] = v.x[pa[q]];
-                xb[q] = v.x[pb[q]];
-                ya[q] = v.y[pa[q]];
-                yb[q] = v.y[pb[q]];
-                za[q] = v.z[pa[q]];
-                zb[q] = v.z[pb[q]];
-                if (v.idx) {
-                    ia[q] = v.idx[pa[q]];
-                    ib[q] = v.idx[pb[q]];
-                }
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < kSubPairs; ++q) {
-            if (pa[q] == 0xffffffffu) continue;
-            v.x[pa[q]] = xb[q];
-            v.x[pb[q]] = xa[q];
-            v.y[pa[q]] = yb[q];
-            v.y[pb[q]] = ya[q];
-            v.z[pa[q]] = zb[q];
-            v.z[pb[q]] = za[q];
-            if (v.idx) {
-                v.idx[pa[q]] = ib[q];
-                v.idx[pb[q]] = ia[q];
-            }
-        }
-    }
-    if (tid == 0) bytes += (v.idx ? 64ull : 48ull) * s_pairs + 4ull * n;
-    __syncthreads();  // swaps done, sm.word visible
-    if (tid == 0) finish_cell(v, slot, sm.word, true);
-    __syncthreads();
-}
-
-// ---- small cells (at most kWarpKeys particles) by one warp each, inside the subtree kernel:
-// the same bisection and Hoare characterisation as sub_bisect / sub_partition, with the
-// cell's keys in the warp's registers (lane l holds positions 32 j + l) and its masks one
-// word a lane, so the CTA's warps finish eight small cells at once.
-
-// Position of the set bit of rank r in the warp's mask (lane w holds word w, pre = its
-// exclusive prefix popcount, W <= 32 words); r may differ from lane to lane: each lane
-// searches the lanes' prefixes for the last word with pre <= r (5 shuffle steps, every lane
-// taking part in every shuffle).
-__device__ __forceinline__ uint32_t warp_mask_select(uint32_t word, uint32_t pre, uint32_t W,
-                                                     uint32_t r) {
-    int lo = 0, hi = (int)W - 1;
-#pragma unroll
-    for (int step = 0; step < 5; ++step) {
-        const int mid = (lo + hi + 1) >> 1;
-        const uint32_t pm = __shfl_sync(0xffffffffu, pre, mid);
-        if (lo < hi) {
-            if (pm <= r)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
-    }
-    const uint32_t ww = __shfl_sync(0xffffffffu, word, lo);
-    const uint32_t pw = __shfl_sync(0xffffffffu, pre, lo);
-    return (uint32_t)lo * 32u + select_in_word(ww, r - pw);
-}
-
-// The bisection of one small cell by the calling warp (src/orbit.cpp:146-232).
-__device__ __noinline__ void warp_bisect_cell(const Level &v, int slot, uint32_t lane, unsigned long long &bytes) {
-    orb_cell_t &cell = v.heap[slot];
-    const uint2 rg = v.ranges[slot];
-    const uint32_t n = rg.y - rg.x;
-    const float ratio = 0.5f;  // subtrees: powers of two only (leaf_ratio of an even count)
-    const float *keys = axis_keys(v, eff_axis(cell.cutAxis));
-    float k[kWarpKeysPerLane];
-#pragma unroll
-    for (int j = 0; j < kWarpKeysPerLane; ++j) {
-        const uint32_t i = (uint32_t)(j * 32) + lane;
-        k[j] = i < n ? keys[rg.x + i] : __int_as_float(0x7fc00000);  // coherent: moved here
-    }
-    float L = cell.cutMarginLeft, R = cell.cutMarginRight;
-    uint32_t it = 0;
-    int st = kActive;
-    while (st == kActive) {
-        if (it >= (uint32_t)kMaxIterations) {
-            st = kCapped;
-            break;
-        }
-        const float cut = mid_cut(L, R);
-        uint32_t cnt = 0;
-#pragma unroll
-        for (int j = 0; j < kWarpKeysPerLane; ++j) cnt += k[j] < cut;
-        cnt = warp_sum(cnt);
-        ++it;
-        const int dir = convergence(cnt, n, ratio);
-        if (dir == 0)
-            st = kFound;
-        else if (dir > 0)
-            R = cut;
-        else
-            L = cut;
-    }
-    if (lane == 0) {
-        cell.cutMarginLeft = L;
-        cell.cutMarginRight = R;
-        cell.foundCut = st == kFound ? 1 : 0;
-        atomicMax(&v.counters->max_iters, it);
-        if (st == kCapped) atomicAdd(&v.counters->unfound, 1u);
-        bytes += 4ull * n;
-    }
-    __syncwarp();
-}
-
-// The Hoare partition (src/services/partition.cpp:30-52) of one small cell by the calling
-// warp: masks of keys >= cut and <= cut (word w: positions 32 w .. 32 w + 31), the swap count
-// s from the word where the two counts cross, the pairs (L_k, R_k) k < s swapped lane by
-// lane, then i = min(L_{s+1}, R_s) and the final swap and split by lane 0 (finish_cell).
-__device__ __noinline__ void warp_partition_cell(const Level &v, int slot, uint32_t lane, unsigned long long &bytes) {
-    const orb_cell_t &cell = v.heap[slot];
-    const uint2 rg = v.ranges[slot];
-    const uint32_t n = rg.y - rg.x, b = rg.x;
-    const float *keys = axis_keys(v, eff_axis(cell.cutAxis));
-    const float cut = cell_cut(cell);
-    const uint32_t W = (n + 31) / 32;
-    uint32_t gw = 0, lw = 0;  // this lane's words (w = lane)
-    for (uint32_t w = 0; w < W; ++w) {
-        const uint32_t i = w * 32u + lane;
-        const float k = i < n ? keys[b + i] : 0.0f;  // coherent: moved here
-        const uint32_t gb = __ballot_sync(0xffffffffu, i < n && !(k < cut));
-        const uint32_t lb = __ballot_sync(0xffffffffu, i < n && !(k > cut));
-        if (lane == w) {
-            gw = gb;
-            lw = lb;
-        }
-    }
-    uint32_t ge_tot, le_tot;
-    const uint32_t pge = warp_excl_scan((uint32_t)__popc(gw), &ge_tot);
-    const uint32_t ple = warp_excl_scan((uint32_t)__popc(lw), &le_tot);
-    // s = max over x of min(#>= in [0,x), #<= in [x,n)): it lies in the first word at whose end
-    // f >= g (f rises, g falls)
-    uint32_t s = 0;
-    if (W > 0) {
-        const bool cross = lane < W && pge + (uint32_t)__popc(gw) >= le_tot - ple - (uint32_t)__popc(lw);
-        const uint32_t cb = __ballot_sync(0xffffffffu, cross);
-        const int w = cb ? __ffs(cb) - 1 : (int)W - 1;
-        uint32_t f = __shfl_sync(0xffffffffu, pge, w), g = le_tot - __shfl_sync(0xffffffffu, ple, w);
-        uint32_t a = __shfl_sync(0xffffffffu, gw, w), c = __shfl_sync(0xffffffffu, lw, w);
-        s = min(f, g);
-        for (int q = 0; q < 32; ++q) {
-            f += a & 1u;
-            g -= c & 1u;
-            a >>= 1;
-            c >>= 1;
-            s = max(s, min(f, g));
-        }
-    }
-    uint32_t i = n;  // split index, n when every key is below the cut
-    if (ge_tot > s) i = min(i, warp_mask_select(gw, pge, W, s));
-    if (s >= 1) i = min(i, warp_mask_select(lw, ple, W, le_tot - s));
-    for (uint32_t k0 = 0; k0 < s; k0 += 32) {
-        const uint32_t k = k0 + lane;
-        const uint32_t kk = k < s ? k : s - 1;  // every lane runs the selects (shuffles)
-        const uint32_t pa = b + warp_mask_select(gw, pge, W, kk);
-        const uint32_t pb = b + warp_mask_select(lw, ple, W, le_tot - 1 - kk);
-        if (k < s) {
-            const float xa = v.x[pa], xb = v.x[pb], ya = v.y[pa], yb = v.y[pb];
-            const float za = v.z[pa], zb = v.z[pb];
-            v.x[pa] = xb;
-            v.x[pb] = xa;
-            v.y[pa] = yb;
-            v.y[pb] = ya;
-            v.z[pa] = zb;
-            v.z[pb] = za;
-            if (v.idx) {
-                const uint32_t ia = v.idx[pa], ib = v.idx[pb];
-                v.idx[pa] = ib;
-                v.idx[pb] = ia;
-            }
-        }
-    }
-    __syncwarp();  // the swaps are visible to lane 0's final swap
-    if (lane == 0) {
-        bytes += (v.idx ? 64ull : 48ull) * s + 4ull * n;
-        finish_cell(v, slot, i, true);
-    }
-    __syncwarp();
-}
+// particles of a cell a group of 32, 16, 8, 2 warps takes
+constexpr uint32_t kSub32 = kSubMaxParticles, kSub16 = 14848, kSub8 = 6656, kSub2 = 1088;
+constexpr uint32_t kSubBytes = sub_bytes<32>(kSub32);
+static_assert(kSubBytes <= 232448, "a CTA's shared memory");
+static_assert(2 * sub_bytes<16>(kSub16) <= kSubBytes && 4 * sub_bytes<8>(kSub8) <= kSubBytes && 16 * sub_bytes<2>(kSub2) <= kSubBytes,
+              "the smaller groups' slices");
 
 // Levels below a cell in a full build: log2 of its leaf count (d is a power of two).
-__device__ __forceinline__ int levels_below(const orb_cell_t &c) {
-    return c.nLeafCells > 1 ? 31 - __clz((uint32_t)c.nLeafCells) : 0;
-}
+__device__ __forceinline__ int levels_below(int leaves) { return leaves > 1 ? 31 - __clz((uint32_t)leaves) : 0; }
 
 // Flag for k_subtree: every cell of the level fits a CTA and has at most `max_levels`
-// (<= kSubLevels, the descendant queue) levels below it. One CTA.
-constexpr int kSubLevels = kSubMaxLevels;
-static_assert((2 << (kSubLevels - 1)) <= kSubQueue, "the last level's children fit the queue");
+// (<= kSubLevels) levels below it. Then the cells with levels below them, by class (all of
+// the first class on levels of few cells, v.sub_wide), in order. One CTA.
 __global__ void __launch_bounds__(1024) k_subtree_check(const __grid_constant__ Level v, int max_levels) {
     pdl_enter();
     __shared__ uint32_t sh[96];
+    const bool failed = level_failed(v);
     uint32_t mx = 0, ml = 0;
     for (int c = threadIdx.x; c < v.C; c += blockDim.x) {
         const int slot = level_slot(v, c);
         const uint2 rg = v.ranges[slot];
         mx = max(mx, rg.y - rg.x);
-        ml = max(ml, (uint32_t)levels_below(v.heap[slot]));
+        ml = max(ml, (uint32_t)levels_below(v.heap[slot].nLeafCells));
     }
     mx = block_max(mx, sh);
     ml = block_max(ml, sh);
-    const bool failed = level_failed(v);
+    const bool take = !failed && mx <= kSub32 && (int)ml <= min(max_levels, kSubLevels);
+    // v.sub_list: four stretches of v.C cells, one a class
+    uint32_t n0 = 0, n1 = 0, n2 = 0, n3 = 0;
+    for (int base = 0; take && base < v.C; base += (int)blockDim.x) {
+        const int c = base + (int)threadIdx.x;
+        int k = 4;
+        if (c < v.C) {
+            const int slot = level_slot(v, c);
+            const uint2 rg = v.ranges[slot];
+            const uint32_t n = rg.y - rg.x;
+            if (v.heap[slot].nLeafCells > 1)
+                k = v.sub_wide || n > kSub16 ? 0 : (n > kSub8 ? 1 : (n > kSub2 ? 2 : 3));
+        }
+        uint32_t ta, tb;
+        const uint2 ex = block_excl_scan2((k == 0 ? 1u : 0u) | (k == 1 ? 0x10000u : 0u),
+                                          (k == 2 ? 1u : 0u) | (k == 3 ? 0x10000u : 0u), sh, &ta, &tb);
+        if (k == 0) v.sub_list[n0 + (ex.x & 0xffffu)] = c;
+        if (k == 1) v.sub_list[v.C + n1 + (ex.x >> 16)] = c;
+        if (k == 2) v.sub_list[2 * v.C + n2 + (ex.y & 0xffffu)] = c;
+        if (k == 3) v.sub_list[3 * v.C + n3 + (ex.y >> 16)] = c;
+        n0 += ta & 0xffffu;
+        n1 += ta >> 16;
+        n2 += tb & 0xffffu;
+        n3 += tb >> 16;
+    }
     if (v.win_cnt)
         for (int w = threadIdx.x; w < kMaxWindows; w += blockDim.x) v.win_cnt[w] = 0u;
     if (threadIdx.x == 0) {
-        const uint32_t take = !failed && mx <= kSubMax && (int)ml <= min(max_levels, kSubLevels) ? 1u : 0u;
-        *v.skip = take;
-        v.counters->sub_next = 0u;  // the subtree kernel's work queue starts at the level's first cell
+        // 2: refused for this kernel's shared memory alone (see kHintSubMax)
+        *v.skip = take ? 1u : (!failed && mx <= kHintSubMax ? 2u : 0u);
+        v.counters->sub_cells[0] = n0;
+        v.counters->sub_cells[1] = n1;
+        v.counters->sub_cells[2] = n2;
+        v.counters->sub_cells[3] = n3;
+        for (int k = 0; k < 4; ++k) v.counters->sub_next[k] = 0u;
         if (v.hwin) {
             __threadfence_system();
             *(volatile uint32_t *)&v.hwin->decision = take ? 1u : 2u;
@@ -3170,81 +2789,682 @@ __global__ void __launch_bounds__(1024) k_subtree_check(const __grid_constant__ 
     }
 }
 
-// One CTA per cell of the level: every level below it (its leaf count's log2), breadth
-// first; with window reports (v.hwin), the last cell of each window reports it to the host.
-// kWarpSmall: cells of at most kWarpKeys particles go to one warp each (the CTA's warps side
-// by side); without it every cell is the whole CTA's (the instance for trees whose cells
-// never get that small keeps its registers for the CTA path). Same results either way.
-template <bool kWarpSmall>
-__global__ void __launch_bounds__(kSubThreads, 4) k_subtree(const __grid_constant__ Level v) {
-    pdl_enter();
-    __shared__ SubSmem sm;
-    if (*(volatile const uint32_t *)v.skip == 0u) return;  // the level kernels run instead
-    unsigned long long bytes = 0;
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    for (int k = 0;; ++k) {
-        // root cells: from a queue where cells can be small or uneven (CTAs that finish small
-        // cells take more), else one in gridDim.x
-        int c;
-        if constexpr (kWarpSmall) {
-            if (threadIdx.x == 0) sm.root = (int)atomicAdd(&v.counters->sub_next, 1u);
+extern __shared__ __align__(16) unsigned char sub_mem[];
+
+// One group of NW warps: the cells of one class, from its work queue. `slice`: where the
+// group's shared memory starts (named here, not passed as a pointer, so that every access is a
+// shared-memory one); ti: thread of the group; bar: its named barrier.
+template <int NW>
+__device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32_t ti, int bar) {
+    unsigned char *const mem = sub_mem + slice;
+    constexpr int kClass = NW == 32 ? 0 : (NW == 16 ? 1 : (NW == 8 ? 2 : 3));
+    constexpr uint32_t NT = NW * 32, nmax = NW == 32 ? kSub32 : (NW == 16 ? kSub16 : (NW == 8 ? kSub8 : kSub2)), nwords = sub_words(nmax);
+    constexpr uint32_t kBins = SubSmem<NW>::kBins, kLists = SubSmem<NW>::kLists;
+    constexpr int kU = 8;  // words of a warp in flight
+    auto sync = [&]() {
+        if (NW == 32)
             __syncthreads();
-            c = sm.root;
-        } else {
-            c = (int)blockIdx.x + k * (int)gridDim.x;
+        else
+            asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"((int)NT) : "memory");
+    };
+    SubSmem<NW> &sm = *reinterpret_cast<SubSmem<NW> *>(mem);
+    uint32_t *keys = reinterpret_cast<uint32_t *>(mem + (sizeof(SubSmem<NW>) + 15) / 16 * 16);
+    uint2 *mask = reinterpret_cast<uint2 *>(keys + nmax + 4);  // .x: key >= cut, .y: key <= cut
+    uint32_t *pre = reinterpret_cast<uint32_t *>(mask + nwords);
+    uint16_t *order = reinterpret_cast<uint16_t *>(pre + nwords);
+    // the pairs to swap (the keys are done then): a cell's left positions, then its right ones
+    uint16_t *pairs = reinterpret_cast<uint16_t *>(keys);
+    const uint32_t lane = ti & 31, warp = ti >> 5, lt = (1u << lane) - 1u;
+    const uint32_t keys_at = (uint32_t)__cvta_generic_to_shared(keys);
+    const uint32_t ncells = v.counters->sub_cells[kClass];
+    const int *list = v.sub_list + kClass * v.C;
+    unsigned long long bytes = 0;
+    // Copies the n words at src into keys[off ...] (off: src's misalignment in words, so that
+    // 16-byte pieces stay aligned on both sides): one bulk copy for the whole pieces, plain loads
+    // for the rest. begin_load after a barrier that ends the keys' last use; end_load, then a
+    // barrier, before they are read. The wait is bounded; a copy that does not come flags the build.
+    const uint32_t arrived = (uint32_t)__cvta_generic_to_shared(&sm.arrived);
+    uint32_t parity = 0;
+    if (ti == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(arrived) : "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    sync();
+    // each thread's last plain access to the keys, before the barrier ahead of a bulk copy
+    auto done_with_keys = [&]() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); };
+    auto begin_load = [&](const void *from, uint32_t n) -> uint32_t {
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(from);
+        const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(src) >> 2) & 3u;
+        const uint32_t head = min(n, (4u - off) & 3u), body = (n - head) & ~3u;
+        if (ti == 0) {
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(arrived), "r"(4u * body) : "memory");
+            if (body)
+                asm volatile(
+                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                        keys_at + 4 * (off + head)),
+                    "l"(src + head), "r"(4u * body), "r"(arrived)
+                    : "memory");
         }
-        if (c >= v.C) break;
-        int cur = 0, nq = 1;
-        const int root = level_slot(v, c);
-        const int levels = levels_below(v.heap[root]);
-        if (threadIdx.x == 0) sm.queue[0][0] = root;
-        __syncthreads();
-        for (int l = 0; l < levels; ++l) {
-            // children of queue entry q at 2q, 2q+1 of the next level's queue (the warp path:
-            // here, before the cells are processed in any order; else after each cell below)
-            if (kWarpSmall && (int)threadIdx.x < nq && 2 * (int)threadIdx.x + 2 <= kSubQueue) {
-                const int slot = sm.queue[cur][threadIdx.x];
-                const int id = v.heap[slot].id;
-                sm.queue[cur ^ 1][2 * threadIdx.x] = slot + id + 1;
-                sm.queue[cur ^ 1][2 * threadIdx.x + 1] = slot + id + 2;
-            }
-            // cells of more than kWarpKeys particles by the whole CTA, one after the other
-            for (int q = 0; q < nq; ++q) {
-                const int slot = sm.queue[cur][q];
-                const uint2 rg = v.ranges[slot];
-                if (kWarpSmall && rg.y - rg.x <= (uint32_t)kWarpKeys) continue;  // CTA-uniform
-                sub_bisect(v, slot, sm, bytes);
-                sub_partition(v, slot, sm, bytes);
-                if (!kWarpSmall && threadIdx.x == 0 && 2 * q + 2 <= kSubQueue) {
-                    const int id = v.heap[slot].id;
-                    sm.queue[cur ^ 1][2 * q] = slot + id + 1;
-                    sm.queue[cur ^ 1][2 * q + 1] = slot + id + 2;
+        if (ti < head) keys[off + ti] = __ldcg(src + ti);
+        if (ti >= 32 && ti - 32 < n - head - body) keys[off + head + body + ti - 32] = __ldcg(src + head + body + ti - 32);
+        return off;
+    };
+    auto end_load = [&]() {
+        uint32_t ok = 0;
+        for (uint32_t spins = 0; !ok && spins < kSubSpins; ++spins)
+            asm volatile(
+                "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.b32 %0, 1, 0, p;\n}"
+                : "=r"(ok)
+                : "r"(arrived), "r"(parity)
+                : "memory");
+        if (!ok) atomicExch(&v.counters->error, 1u);
+        parity ^= 1u;
+    };
+    auto take = [&]() -> int {
+        const uint32_t k = atomicAdd(&v.counters->sub_next[kClass], 1u);
+        return k < ncells ? list[k] : -1;
+    };
+    auto prefetch = [&](const void *p, uint32_t words) {  // whole 16-byte pieces
+        const uintptr_t a = (reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15;
+        const uintptr_t e = (reinterpret_cast<uintptr_t>(p) + 4ull * words) & ~(uintptr_t)15;
+        if (e > a)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((uint32_t)(e - a)) : "memory");
+    };
+    int next = -1;  // thread 0: the cell after this one
+    bool started = false;
+    for (;;) {
+        if (ti == 0) {
+            // this cell, and the next one, whose particles start their way into L2 meanwhile
+            if (!started) next = take();
+            started = true;
+            sm.item = next;
+            if (next >= 0) {
+                next = take();
+                if (next >= 0) {
+                    const uint2 r = v.ranges[level_slot(v, next)];
+                    prefetch(v.x + r.x, r.y - r.x);
+                    prefetch(v.y + r.x, r.y - r.x);
+                    prefetch(v.z + r.x, r.y - r.x);
+                    if (v.idx) prefetch(v.idx + r.x, r.y - r.x);
                 }
             }
-            // the small ones by one warp each, the CTA's warps side by side
-            for (int q = (int)warp; kWarpSmall && q < nq; q += (int)nwarps) {
-                const int slot = sm.queue[cur][q];
+            sm.max_it = sm.unfound = sm.degenerate = 0;
+            sm.axes = sm.counted = 0;
+            if (sm.item >= 0) {
+                const int slot = level_slot(v, sm.item);
+                const orb_cell_t &h = v.heap[slot];
                 const uint2 rg = v.ranges[slot];
-                if (rg.y - rg.x > (uint32_t)kWarpKeys) continue;  // warp-uniform
-                warp_bisect_cell(v, slot, lane, bytes);
-                warp_partition_cell(v, slot, lane, bytes);
+                SubCell &sc = sm.cell[0][0];
+                sc.id = h.id;
+                sc.leaves = h.nLeafCells;
+                sc.axis = h.cutAxis;
+                for (int a = 0; a < 3; ++a) {
+                    sc.lower[a] = h.lower[a];
+                    sc.upper[a] = h.upper[a];
+                }
+                sc.b = 0;
+                sc.m = (uint16_t)(rg.y - rg.x);
+                sm.root = slot;
             }
-            __syncthreads();
-            cur ^= 1;
-            nq = 2 * nq;
+        }
+        sync();
+        const int c = sm.item;
+        if (c < 0) break;
+        const int root = sm.root, root_id = sm.cell[0][0].id;
+        const uint32_t n = sm.cell[0][0].m, first = v.ranges[root].x;
+        const int levels = levels_below(sm.cell[0][0].leaves);
+        // heap slot of a descendant: slot - id is the instance's heap base
+        const int heap0 = root - root_id;
+        uint32_t off = begin_load(axis_keys(v, eff_axis(sm.cell[0][0].axis)) + first, n);  // the root's keys
+        for (uint32_t p = ti; p < n; p += NT) order[p] = (uint16_t)p;
+        bool loading = true;  // a copy of an axis is under way
+        for (int l = 0; l < levels; ++l) {
+            SubCell *const cells = sm.cell[l & 1];
+            const uint32_t nq = 1u << l;
+            // cell q's warps: gs of them (at least one), this warp is number gw of cell q0 and,
+            // with more cells than warps, takes q0 + qs, ... too (then gs = 1)
+            const uint32_t gs = max(1u, (uint32_t)NW >> l), q0 = warp / gs, gw = warp % gs, qs = NW / gs;
+            const uint32_t nb = kBins >> l, lslots = kLists >> l, cap = min(kSubWindowList, lslots);
+            if (ti < nq) {
+                const SubCell &sc = cells[ti];
+                SubState &s = sm.state[ti];
+                const int a = eff_axis(sc.axis);
+                s.L = s.a = sc.lower[a];  // setCutMargin, src/cell.h:123-126
+                s.R = s.b = sc.upper[a];
+                s.mode = sc.m ? kSubOpen : kSubDone;  // no key: the first cut is found (count 0 of 0)
+                s.it = s.found = sc.m ? 0 : 1;
+                s.cand = 0xffffffffu;
+                s.nlist = s.s = 0;
+                s.i = sc.m;
+                atomicOr(&sm.axes, 1u << a);
+                if (sc.m > kSubDirect) atomicOr(&sm.counted, 1u << a);
+            }
+            sync();
+            const uint32_t axes = sm.axes, counted = sm.counted;
+            const float *kf = reinterpret_cast<const float *>(keys);
+            // f(word, key) for this warp's words of cell q, a run of consecutive ones (lanes past the
+            // cell's end hold NaN); a position's key is the one its order entry names
+            auto for_words = [&](uint32_t q, auto f) {
+                const uint32_t m = cells[q].m, W = (m + 31) / 32, run = (W + gs - 1) / gs;
+                uint32_t w = min(W, gw * run);
+                const uint32_t end = min(W, w + run), full = min(m / 32, end);
+                const uint16_t *ord = order + cells[q].b + lane + w * 32u;
+                for (; w + kU <= full; w += kU, ord += kU * 32) {
+                    uint32_t o[kU];
+                    float k[kU];
+#pragma unroll
+                    for (int u = 0; u < kU; ++u) o[u] = ord[u * 32];
+#pragma unroll
+                    for (int u = 0; u < kU; ++u) k[u] = kf[o[u]];
+#pragma unroll
+                    for (int u = 0; u < kU; ++u) f(w + (uint32_t)u, k[u], Flag<true>());
+                }
+                for (; w < full; ++w, ord += 32) f(w, kf[*ord], Flag<true>());
+                if (w < end) f(w, lane < (m & 31u) ? kf[*ord] : __int_as_float(0x7fc00000), Flag<false>());
+            };
+            // masks of cell q against lo and hi (see k_part_classify), the keys between listed;
+            // returns this lane's keys that are not below hi
+            auto classify = [&](uint32_t q, float lo, float hi) -> uint32_t {
+                uint2 *mk = mask + ((uint32_t)cells[q].b >> 5) + q;
+                const uint32_t vm = (1u << (cells[q].m & 31u)) - 1u;  // the partial word's positions
+                uint32_t above = 0;
+                for_words(q, [&](uint32_t w, float k, auto full) {
+                    constexpr bool kFull = decltype(full)::value;
+                    const uint32_t valid = kFull ? 0xffffffffu : vm;
+                    const bool not_below = !(k < hi);
+                    const uint32_t gb = __ballot_sync(0xffffffffu, not_below) & valid;
+                    const uint32_t lb = __ballot_sync(0xffffffffu, !(k >= lo)) & valid;
+                    above += not_below;
+                    if (lane == 0) mk[w] = make_uint2(gb, lb);
+                });
+                // the unresolved keys to the list, a lane a word
+                __syncwarp();
+                const uint32_t W = (cells[q].m + 31u) / 32u, run = (W + gs - 1) / gs;
+                const uint32_t w0 = min(W, gw * run), w1 = min(W, w0 + run);
+                for (uint32_t w = w0 + lane; w < w1; w += 32) {
+                    const uint2 x = mk[w];
+                    uint32_t e = ~(x.x | x.y) & (w * 32u + 32u <= cells[q].m ? 0xffffffffu : vm);
+                    if (!e) continue;
+                    uint32_t at = atomicAdd(&sm.state[q].nlist, (uint32_t)__popc(e));
+                    for (; e && at < lslots; e &= e - 1u, ++at) {
+                        const uint32_t p = w * 32u + (uint32_t)__ffs(e) - 1u;
+                        sm.lkey[q * lslots + at] = kf[order[cells[q].b + p]];
+                        sm.lpos[q * lslots + at] = (uint16_t)p;
+                    }
+                }
+                return above;
+            };
+            for (int ax = 0; ax < 3; ++ax) {
+                if (!((axes >> ax) & 1u)) continue;
+                if (!loading) off = begin_load(axis_keys(v, ax) + first, n);
+                loading = false;
+                kf = reinterpret_cast<const float *>(keys) + off;
+                bytes += 4ull * n;
+                auto mine = [&](uint32_t q) { return eff_axis(cells[q].axis) == ax; };
+                // rounds: histogram of the keys over the window (keys outside it in the end
+                // bins), then the window narrowed to the bins of the ranks around the target
+                auto counts = [&](uint32_t q) {
+                    return mine(q) && cells[q].m > kSubDirect && sm.state[q].mode == kSubOpen && sm.state[q].cand > cap;
+                };
+                if (ti == 0) sm.direct = 0;
+                if (!((counted >> ax) & 1u)) {
+                    end_load();
+                    sync();
+                }
+                for (int r = 0; (counted >> ax) & 1u; ++r) {
+                    for (uint32_t j = ti; j < kBins; j += NT) sm.bins[j] = 0u;
+                    if (ti == 0) sm.more = 0;
+                    if (r == 0) end_load();
+                    sync();
+                    bool any = false;
+                    for (uint32_t q = q0; q < nq; q += qs) {
+                        if (!counts(q)) continue;
+                        any = true;
+                        const float a = sm.state[q].a, scale = __frcp_rn(__fsub_rn(sm.state[q].b, a));
+                        const float top = (float)(nb - 1u);
+                        // the float 2^23 + g holds bin g in its low bits: 4 times its encoding plus
+                        // `at` is the bin's address
+                        const uint32_t at = (uint32_t)__cvta_generic_to_shared(sm.bins + q * nb) - 4u * 0x4b000000u;
+                        for_words(q, [&](uint32_t, float k, auto full) {
+                            const float t = __saturatef(__fmul_rn(__fsub_rn(k, a), scale));  // NaN: bin 0
+                            const uint32_t e = __float_as_uint(__fmaf_rn(t, top, 8388608.0f));
+                            if (decltype(full)::value || k == k)
+                                asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(4u * e + at) : "memory");
+                        });
+                    }
+                    sync();
+                    // the bins of the ranks m/2 - 4 and m/2 + 4: a cut the test accepts has a count
+                    // within 3 of half the keys
+                    const uint32_t per = nb / (gs * 32u);
+                    auto narrow = [&](uint32_t q, uint32_t j0, uint32_t run) {
+                        SubState &s = sm.state[q];
+                        const uint32_t half = cells[q].m / 2u, r0 = half - 4u, r1 = half + 4u;
+                        const float a = s.a, step = __fdiv_rn(__fsub_rn(s.b, a), (float)(nb - 1u));
+                        for (uint32_t j = j0; j < j0 + per; ++j) {
+                            const uint32_t h = sm.bins[q * nb + j];
+                            // bin j holds the keys rounded to j: [j - 1/2, j + 1/2) steps above a
+                            if (run <= r0 && r0 < run + h) {
+                                s.L = __fadd_rn(a, __fmul_rn((float)j - 0.53125f, step));
+                                s.cnt = run;
+                            }
+                            if (run <= r1 && r1 < run + h) {
+                                s.R = __fadd_rn(a, __fmul_rn((float)j + 0.53125f, step));
+                                s.cross = run + h;
+                            }
+                            run += h;
+                        }
+                    };
+                    // (s.L, s.R, s.cnt and s.cross carry the new window and its ranks here; the
+                    // bracket is set again below)
+                    if (gs == 1) {
+                        for (uint32_t q = q0; q < nq; q += qs) {
+                            if (!counts(q)) continue;
+                            uint32_t loc = 0, tot;
+                            for (uint32_t j = 0; j < per; ++j) loc += sm.bins[q * nb + lane * per + j];
+                            const uint32_t ex = warp_excl_scan(loc, &tot);
+                            if (lane == 0) {
+                                sm.state[q].L = sm.state[q].R = __int_as_float(0x7fc00000);
+                                sm.state[q].cnt = sm.state[q].cross = 0;
+                            }
+                            __syncwarp();
+                            narrow(q, lane * per, ex);
+                        }
+                    } else {
+                        uint32_t loc = 0, wtot;
+                        if (any)
+                            for (uint32_t j = 0; j < per; ++j) loc += sm.bins[q0 * nb + (gw * 32u + lane) * per + j];
+                        const uint32_t ex = warp_excl_scan(loc, &wtot);
+                        if (lane == 0) {
+                            sm.part[warp] = wtot;
+                            if (any && gw == 0) {
+                                sm.state[q0].L = sm.state[q0].R = __int_as_float(0x7fc00000);
+                                sm.state[q0].cnt = sm.state[q0].cross = 0;
+                            }
+                        }
+                        sync();
+                        const uint32_t before = __reduce_add_sync(0xffffffffu, lane < gw ? sm.part[warp - gw + lane] : 0u);
+                        if (any) narrow(q0, (gw * 32u + lane) * per, before + ex);
+                    }
+                    sync();
+                    for (uint32_t q = q0; q < nq; q += qs) {
+                        if (gw || lane || !counts(q)) continue;
+                        SubState &s = sm.state[q];
+                        const uint32_t cand = s.cross - s.cnt;
+                        const float na = s.L, nbnd = s.R;
+                        const int a = eff_axis(cells[q].axis);
+                        s.L = cells[q].lower[a];
+                        s.R = cells[q].upper[a];
+                        s.cnt = 0;  // (from here on: the classify pass's count)
+                        if (!(na < nbnd) || (cand > cap && (r == 3 || cand >= s.cand))) {
+                            s.mode = kSubCount;  // ranks outside the bins (NaN keys), or no narrowing
+                        } else {
+                            s.a = na;
+                            s.b = nbnd;
+                            s.cand = cand;
+                            if (cand > cap) sm.more = 1;
+                        }
+                    }
+                    sync();
+                    const bool again = sm.more != 0;
+                    sync();  // (more is cleared by the next round)
+                    if (!again) break;
+                }
+                // small cells: the whole loop by one warp, the keys in its registers; the others:
+                // masks and list against the window
+                for (uint32_t q = q0; q < nq; q += qs) {
+                    if (!mine(q)) continue;
+                    SubState &s = sm.state[q];
+                    const uint32_t m = cells[q].m;
+                    if (m <= kSubDirect) {
+                        if (gw || s.mode == kSubDone) continue;
+                        float kl[kSubDirect / 32], L = s.L, R = s.R;
+                        uint32_t it = 0;
+#pragma unroll
+                        for (int j = 0; j < (int)kSubDirect / 32; ++j) {
+                            const uint32_t p = (uint32_t)j * 32u + lane;
+                            kl[j] = p < m ? kf[order[cells[q].b + p]] : __int_as_float(0x7fc00000);  // NaN: never below
+                        }
+                        const int st = bisect_list(kl, 0u, m, 0.5f, L, R, it);
+                        __syncwarp();
+                        if (lane == 0) {
+                            s.L = L;
+                            s.R = R;
+                            s.it = (uint16_t)it;
+                            s.found = st == kFound;
+                            s.mode = kSubDone;
+                        }
+                    } else if (s.mode == kSubOpen) {
+                        uint32_t above = classify(q, s.a, s.b);
+                        // (lanes past the cell's end hold NaN, counted by the last word's warp)
+                        above = __reduce_add_sync(0xffffffffu, above);
+                        if (lane == 0 && above) atomicAdd(&s.cnt, above);
+                    }
+                }
+                sync();
+                // the window's exact counts, and the replay of the loop on the list
+                for (uint32_t q = q0; q < nq; q += qs) {
+                    SubState &s = sm.state[q];
+                    const uint32_t m = cells[q].m;
+                    if (gw || !mine(q) || m <= kSubDirect || s.mode == kSubDone) continue;
+                    uint32_t mode = s.mode;
+                    const uint32_t nl = s.nlist;
+                    if (mode == kSubOpen && nl <= cap) {
+                        const uint32_t wb = ((uint32_t)cells[q].b >> 5) + q;
+                        // keys at or above b, and NaN (without the partial word's empty lanes)
+                        const uint32_t g = s.cnt - ((m & 31u) ? 32u - (m & 31u) : 0u);
+                        const uint32_t below = m - g - nl;
+                        // NaN keys are in g and never below a cut: count(< b) = below + nl all the same
+                        const bool low = convergence(below, m, 0.5f) < 0, high = convergence(below + nl, m, 0.5f) > 0;
+                        const float a = s.a, b = s.b;
+                        float kl[kSubWindowList / 32], L = s.L, R = s.R;
+#pragma unroll
+                        for (int j = 0; j < (int)kSubWindowList / 32; ++j) {
+                            const uint32_t e = (uint32_t)j * 32u + lane;
+                            kl[j] = e < nl ? sm.lkey[q * lslots + e] : __int_as_float(0x7fc00000);
+                        }
+                        uint32_t it = 0;
+                        int st = kActive;
+                        while (st == kActive) {
+                            if (it >= (uint32_t)kMaxIterations) {
+                                st = kCapped;
+                                break;
+                            }
+                            const float cut = mid_cut(L, R);
+                            int dir;
+                            if (cut <= a) {
+                                if (!low) break;
+                                dir = -1;
+                            } else if (cut >= b) {
+                                if (!high) break;
+                                dir = 1;
+                            } else {
+                                uint32_t cc = 0;
+#pragma unroll
+                                for (int j = 0; j < (int)kSubWindowList / 32; ++j) cc += kl[j] < cut;
+                                dir = convergence(below + __reduce_add_sync(0xffffffffu, cc), m, 0.5f);
+                            }
+                            ++it;
+                            if (dir == 0)
+                                st = kFound;
+                            else if (dir > 0)
+                                R = cut;
+                            else
+                                L = cut;
+                        }
+                        const float cut = mid_cut(L, R);
+                        if (st != kActive && cut > a && cut < b) {
+                            // the listed keys' bits against the final cut
+#pragma unroll
+                            for (int j = 0; j < (int)kSubWindowList / 32; ++j) {
+                                const uint32_t e = (uint32_t)j * 32u + lane;
+                                if (e < nl) {
+                                    const uint32_t p = sm.lpos[q * lslots + e], bit = 1u << (p & 31u);
+                                    if (!(kl[j] < cut)) atomicOr(&mask[wb + (p >> 5)].x, bit);
+                                    if (!(kl[j] > cut)) atomicOr(&mask[wb + (p >> 5)].y, bit);
+                                }
+                            }
+                            mode = kSubWindow;
+                            if (lane == 0) {
+                                s.L = L;
+                                s.R = R;
+                                s.it = (uint16_t)it;
+                                s.found = st == kFound;
+                                s.mode = kSubWindow;
+                            }
+                        }
+                    }
+                    __syncwarp();
+                    if (mode != kSubWindow && lane == 0) {
+                        s.mode = kSubCount;
+                        sm.direct = 1;
+                    }
+                }
+                sync();
+                if (sm.direct) {
+                    // cells the window did not settle: every cut counted over all the keys
+                    for (int it = 0; it < kMaxIterations; ++it) {
+                        if (ti < nq) sm.state[ti].cnt = 0;
+                        if (ti == 0) sm.more = 0;
+                        sync();
+                        for (uint32_t q = q0; q < nq; q += qs) {
+                            if (!mine(q) || sm.state[q].mode != kSubCount) continue;
+                            const float cut = mid_cut(sm.state[q].L, sm.state[q].R);
+                            uint32_t cc = 0;
+                            for_words(q, [&](uint32_t, float k, auto) { cc += k < cut; });
+                            cc = __reduce_add_sync(0xffffffffu, cc);
+                            if (lane == 0 && cc) atomicAdd(&sm.state[q].cnt, cc);
+                        }
+                        sync();
+                        if (ti < nq && mine(ti) && sm.state[ti].mode == kSubCount) {
+                            SubState &s = sm.state[ti];
+                            const float cut = mid_cut(s.L, s.R);
+                            ++s.it;
+                            const int dir = convergence(s.cnt, cells[ti].m, 0.5f);
+                            if (dir == 0) {
+                                s.found = 1;
+                                s.mode = kSubDone;
+                            } else if (dir > 0) {
+                                s.R = cut;
+                            } else {
+                                s.L = cut;
+                            }
+                            if (dir != 0) sm.more = 1;
+                        }
+                        sync();
+                        const bool again = sm.more != 0;
+                        sync();
+                        if (!again) break;
+                    }
+                }
+                // masks against the final cut, where the window did not give them
+                for (uint32_t q = q0; q < nq; q += qs) {
+                    if (!mine(q) || sm.state[q].mode == kSubWindow) continue;
+                    const float cut = mid_cut(sm.state[q].L, sm.state[q].R);
+                    classify(q, next_above(cut), cut);
+                }
+                done_with_keys();
+                sync();
+            }
+            // prefixes of the masks' counts (>= in the low half of a word, <= in the high half)
+            // and the word where #{>= before} crosses #{<= after}
+            auto popcounts = [&](uint32_t wb, uint32_t w0, uint32_t w1) {
+                uint32_t t = 0;
+                for (uint32_t w = w0; w < w1; ++w) {
+                    const uint2 x = mask[wb + w];
+                    t += (uint32_t)__popc(x.x) + ((uint32_t)__popc(x.y) << 16);
+                }
+                return t;
+            };
+            auto prefix = [&](uint32_t q, uint32_t wb, uint32_t w0, uint32_t w1, uint32_t run, uint32_t le_tot) {
+                for (uint32_t w = w0; w < w1; ++w) {
+                    const bool was = w > 0 && (run & 0xffffu) >= le_tot - (run >> 16);
+                    const uint2 x = mask[wb + w];
+                    pre[wb + w] = run;
+                    run += (uint32_t)__popc(x.x) + ((uint32_t)__popc(x.y) << 16);
+                    if (!was && (run & 0xffffu) >= le_tot - (run >> 16)) sm.state[q].cross = w;
+                }
+            };
+            if (gs == 1) {
+                for (uint32_t q = q0; q < nq; q += qs) {
+                    const uint32_t W = ((uint32_t)cells[q].m + 31) / 32, pw = (W + 31) / 32, wb = ((uint32_t)cells[q].b >> 5) + q;
+                    const uint32_t w0 = min(W, lane * pw), w1 = min(W, w0 + pw);
+                    uint32_t tot;
+                    const uint32_t ex = warp_excl_scan(popcounts(wb, w0, w1), &tot);
+                    if (lane == 0) sm.state[q].tot = tot;
+                    prefix(q, wb, w0, w1, ex, tot >> 16);
+                }
+                __syncwarp();
+            } else {
+                const uint32_t W = ((uint32_t)cells[q0].m + 31) / 32, pw = (W + gs * 32u - 1) / (gs * 32u);
+                const uint32_t wb = ((uint32_t)cells[q0].b >> 5) + q0;
+                const uint32_t w0 = min(W, (gw * 32u + lane) * pw), w1 = min(W, w0 + pw);
+                uint32_t wtot;
+                const uint32_t ex = warp_excl_scan(popcounts(wb, w0, w1), &wtot);
+                if (lane == 0) sm.part[warp] = wtot;
+                sync();
+                const uint32_t pv = lane < gs ? sm.part[warp - gw + lane] : 0u;
+                const uint32_t before = __reduce_add_sync(0xffffffffu, lane < gw ? pv : 0u);
+                const uint32_t tot = __reduce_add_sync(0xffffffffu, pv);
+                if (gw == 0 && lane == 0) sm.state[q0].tot = tot;
+                prefix(q0, wb, w0, w1, before + ex, tot >> 16);
+                sync();
+            }
+            // The swap count s = max over x of min(#>= in [0,x), #<= in [x,m)): it lies in that word
+            // (every warp of the cell finds it). Then the pairs, a lane a word: left elements by
+            // rank (pair k: the key >= cut of rank k), right ones (the key <= cut of rank le-1-k),
+            // and the split index i = min(L_{s+1}, R_s). A word's 16 or so bits one after the other
+            // in a lane cost a sixth of the instructions of a warp a word.
+            for (uint32_t q = q0; q < nq; q += qs) {
+                SubState &s = sm.state[q];
+                const uint32_t b = cells[q].b, W = ((uint32_t)cells[q].m + 31) / 32, wb = (b >> 5) + q;
+                if (!W) continue;
+                const uint32_t x = s.cross, le_tot = s.tot >> 16;
+                const uint2 cw = mask[wb + x];
+                const uint32_t f = pre[wb + x] & 0xffffu, g = le_tot - (pre[wb + x] >> 16), upto = 0xffffffffu >> (31u - lane);
+                const uint32_t ns = __reduce_max_sync(
+                    0xffffffffu, max(min(f, g), min(f + __popc(cw.x & upto), g - __popc(cw.y & upto))));
+                if (gw == 0 && lane == 0) s.s = ns;
+                const uint32_t first_le = le_tot - ns;  // ranks from here on are partners
+                uint16_t *const pl = pairs + 2 * b, *const pr = pl + cells[q].m;
+                if (gw == 0) {  // the crossing word, a lane a bit: it can hold both kinds, and i
+                    const uint32_t kg = f + __popc(cw.x & lt), kl = le_tot - g + __popc(cw.y & lt);
+                    const bool isg = (cw.x >> lane) & 1u, isl = (cw.y >> lane) & 1u;
+                    if (isg && kg < ns) pl[kg] = (uint16_t)(b + x * 32u + lane);
+                    if (isl && kl >= first_le) pr[le_tot - 1u - kl] = (uint16_t)(b + x * 32u + lane);
+                    if ((isg && kg == ns) || (isl && kl == first_le && ns)) atomicMin(&s.i, x * 32u + lane);
+                }
+                // words before it: every key >= cut is a left element; words behind it: every key <=
+                // cut a partner. A lane takes words of its own run, each lane starting elsewhere in
+                // it, so the lanes' ranks (16 a word apart) fall on different banks.
+                const uint32_t run = (W + 31) / 32;
+                for (uint32_t j = gw, r0 = lane % run; j < run; j += gs) {
+                    uint32_t o = j + r0;
+                    if (o >= run) o -= run;
+                    const uint32_t w = lane * run + o;
+                    if (w >= W || w == x) continue;
+                    const uint2 k = mask[wb + w];
+                    const uint32_t at = pre[wb + w], rgt = at & 0xffffu, rl = at >> 16;
+                    const bool behind = w > x;
+                    uint32_t e = behind ? k.y : k.x;
+                    uint16_t *dst = behind ? pr + (le_tot - 1u - rl) : pl + rgt;
+                    const int step = behind ? -1 : 1;
+                    if (behind) {
+                        if (rgt <= ns && ns < rgt + (uint32_t)__popc(k.x))
+                            atomicMin(&s.i, w * 32u + select_in_word(k.x, ns - rgt));
+                        if (e && rl == first_le && ns) atomicMin(&s.i, w * 32u + (uint32_t)__ffs(e) - 1u);
+                    }
+                    const uint32_t base = b + w * 32u - 1u;
+                    for (; e; e &= e - 1u, dst += step) *dst = (uint16_t)(base + (uint32_t)__ffs(e));
+                }
+            }
+            sync();
+            // the swaps (the two sides' positions are disjoint)
+            for (uint32_t q = q0; q < nq; q += qs) {
+                const uint16_t *const pl = pairs + 2 * (uint32_t)cells[q].b, *const pr = pl + cells[q].m;
+                for (uint32_t k = gw * 32u + lane; k < sm.state[q].s; k += gs * 32u) {
+                    const uint32_t pa = pl[k], pb = pr[k];
+                    const uint16_t oa = order[pa], ob = order[pb];
+                    order[pa] = ob;
+                    order[pb] = oa;
+                }
+            }
+            done_with_keys();
+            sync();
+            if (l + 1 == levels) off = begin_load(v.x + first, n);  // for the final pass
+            // the final swap, the split (Cell::cut, src/cell.h:78-100) and the children, a thread a cell
+            if (ti < nq) {
+                const SubCell sc = cells[ti];
+                const SubState &s = sm.state[ti];
+                const uint32_t b = sc.b, m = sc.m, i = s.i;
+                if (i < m) {
+                    const uint16_t oa = order[b + i];
+                    order[b + i] = order[b + m - 1];
+                    order[b + m - 1] = oa;
+                } else {
+                    atomicAdd(&sm.degenerate, 1u);
+                }
+                orb_cell_t &h = v.heap[heap0 + sc.id];
+                h.cutMarginLeft = s.L;
+                h.cutMarginRight = s.R;
+                h.foundCut = (uint8_t)s.found;
+                atomicMax(&sm.max_it, (uint32_t)s.it);
+                if (!s.found) atomicAdd(&sm.unfound, 1u);
+                orb_cell_t cell;
+                cell.id = sc.id;
+                cell.nLeafCells = sc.leaves;
+                cell.cutAxis = sc.axis;
+                cell.cutMarginLeft = s.L;
+                cell.cutMarginRight = s.R;
+                for (int a = 0; a < 3; ++a) {
+                    cell.lower[a] = sc.lower[a];
+                    cell.upper[a] = sc.upper[a];
+                }
+                orb_cell_t kid[2];
+                split_cell(cell, kid[0], kid[1], v.counters);
+#pragma unroll
+                for (int w = 0; w < 2; ++w) {
+                    const int slot = heap0 + kid[w].id;
+                    const uint32_t kb = w ? b + i : b, km = w ? m - i : i;
+                    v.heap[slot] = kid[w];
+                    v.ranges[slot] = make_uint2(first + kb, first + kb + km);
+                    if (l + 1 < levels) {
+                        SubCell &o = sm.cell[(l + 1) & 1][2 * ti + w];
+                        o.id = kid[w].id;
+                        o.leaves = kid[w].nLeafCells;
+                        o.axis = kid[w].cutAxis;
+                        for (int a = 0; a < 3; ++a) {
+                            o.lower[a] = kid[w].lower[a];
+                            o.upper[a] = kid[w].upper[a];
+                        }
+                        o.b = (uint16_t)kb;
+                        o.m = (uint16_t)km;
+                    }
+                }
+            }
+            if (ti == 0) sm.axes = sm.counted = 0;
+            sync();
+        }
+        // the particles, one array after the other
+        uint32_t *const arr[4] = {reinterpret_cast<uint32_t *>(v.x), reinterpret_cast<uint32_t *>(v.y),
+                                  reinterpret_cast<uint32_t *>(v.z), v.idx};
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            if (!arr[a]) continue;
+            uint32_t *dst = arr[a] + first;
+            if (a > 0) off = begin_load(dst, n);
+            end_load();
+            sync();
+            const uint32_t *from = keys + off;
+            uint32_t p = ti;
+            for (; p + 7 * NT < n; p += 8 * NT) {
+                uint32_t x[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) x[u] = from[order[p + u * NT]];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) dst[p + u * NT] = x[u];
+            }
+            for (; p < n; p += NT) dst[p] = from[order[p]];
+            done_with_keys();
+            sync();
+            bytes += 8ull * n;
+        }
+        if (ti == 0) {
+            atomicMax(&v.counters->max_iters, sm.max_it);
+            if (sm.unfound) atomicAdd(&v.counters->unfound, sm.unfound);
+            if (sm.degenerate) atomicAdd(&v.counters->degenerate, sm.degenerate);
         }
         if (v.hwin) {
             // the cell is final: every thread's writes made visible beyond the GPU, then the
             // last cell of its window reports the window's particle range to the host
             __threadfence_system();
-            __syncthreads();
-            if (threadIdx.x == 0) {
+            sync();
+            if (ti == 0) {
                 const uint32_t w = (uint32_t)c / v.win_cells;
-                const uint32_t first = w * v.win_cells, last = min(first + v.win_cells, (uint32_t)v.C) - 1u;
-                if (atomicAdd(&v.win_cnt[w], 1u) == last - first) {
+                const uint32_t c0 = w * v.win_cells, c1 = min(c0 + v.win_cells, (uint32_t)v.C) - 1u;
+                if (atomicAdd(&v.win_cnt[w], 1u) == c1 - c0) {
                     __threadfence_system();
-                    const uint2 r = make_uint2(v.ranges[level_slot(v, (int)first)].x,
-                                               v.ranges[level_slot(v, (int)last)].y);
+                    const uint2 r = make_uint2(v.ranges[level_slot(v, (int)c0)].x,
+                                               v.ranges[level_slot(v, (int)c1)].y);
                     volatile uint32_t *hr = &v.hwin->range[w].x;
                     hr[0] = r.x;
                     hr[1] = r.y;
@@ -3254,8 +3474,31 @@ __global__ void __launch_bounds__(kSubThreads, 4) k_subtree(const __grid_constan
             }
         }
     }
-    // lane 0 of every warp counted the small cells its warp finished (thread 0 the rest too)
-    if (lane == 0 && bytes) add_bytes(v, kKSubtree, bytes);
+    if (ti == 0 && bytes) add_bytes(v, kKSubtree, bytes);
+}
+
+// The level's cells, largest class first: all of the CTA's warps on one cell, then groups of
+// 16, 8 and 2 warps on their own slices of its shared memory.
+__global__ void __launch_bounds__(kSubThreads) k_subtree(const __grid_constant__ Level v) {
+    pdl_enter();
+    if (*(volatile const uint32_t *)v.skip != 1u) return;  // the level kernels run instead
+    const uint32_t tid = threadIdx.x;
+    if (v.counters->sub_cells[0]) sub_group<32>(v, 0u, tid, 0);
+    __syncthreads();
+    if (v.counters->sub_cells[1]) {
+        const uint32_t k = tid / 512;
+        sub_group<16>(v, k * sub_bytes<16>(kSub16), tid % 512, 1 + (int)k);
+    }
+    __syncthreads();
+    if (v.counters->sub_cells[2]) {
+        const uint32_t k = tid / 256;
+        sub_group<8>(v, k * sub_bytes<8>(kSub8), tid % 256, 1 + (int)k);
+    }
+    __syncthreads();
+    if (v.counters->sub_cells[3]) {
+        const uint32_t k = tid / 64;
+        sub_group<2>(v, k * sub_bytes<2>(kSub2), tid % 64, (int)k);
+    }
 }
 
 // ------------------------------------------------------------------------------------
@@ -3707,12 +3950,7 @@ void launch_level_kernel(Kernel k, const Level &v, int grid, int arg, cudaStream
             break;
         case kKBisectTile: launch_kernel(p, k_bisect_tile, dim3(grid), T, 0, st, v); break;
         case kKSubtreeCheck: launch_kernel(p, k_subtree_check, dim3(1), dim3(1024), 0, st, v, arg); break;
-        case kKSubtree:  // arg: 1 when cells of at most kWarpKeys particles can occur
-            if (arg)
-                launch_kernel(p, k_subtree<true>, dim3(grid), dim3(kSubThreads), 0, st, v);
-            else
-                launch_kernel(p, k_subtree<false>, dim3(grid), dim3(kSubThreads), 0, st, v);
-            break;
+        case kKSubtree: launch_kernel(p, k_subtree, dim3(grid), dim3(kSubThreads), kSubBytes, st, v); break;
         case kKBisectCta:
             launch_kernel(p, k_bisect_cta, dim3(grid), dim3(kCtaThreads), kCtaSmemBytes, st, v);
             break;
@@ -3751,8 +3989,10 @@ void launch_level_kernel(Kernel k, const Level &v, int grid, int arg, cudaStream
 }
 
 cudaError_t configure_kernels() {
-    return cudaFuncSetAttribute(k_bisect_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kCtaSmemBytes);
+    const cudaError_t e = cudaFuncSetAttribute(k_bisect_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)kCtaSmemBytes);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSubBytes);
 }
 
 int swap_blocks_per_sm() {
