@@ -520,6 +520,11 @@ uint32_t small_cells(const orb_ctx *ctx, const Level &v, uint64_t max_n, size_t 
     return !v.slots && (max_n >> li) > 4ull * kTile ? 0u : (uint32_t)kTile;
 }
 
+// Histogram bins for the cells planned for a level of C cells: those with count tiles, or
+// (weighted builds) those of several tiles, all of them on a level of few cells (whose tiles
+// are dealt in pieces).
+uint32_t plan_bins(const orb_ctx *ctx, const Level &v, int C) { return !v.wt || C <= ctx->num_sms ? 1u : 0u; }
+
 // The level from which subtree CTAs finish the tree (-1: none): the first level whose cells
 // (at most max_n >> l particles plus a few per split: each split leaves a cell within 3 of
 // half) all fit one CTA and that is at most kSubMaxLevels above the leaves
@@ -565,7 +570,6 @@ orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, u
                       int sub_from, uint64_t n, uint64_t max_n, bool rest = false, size_t from = 0,
                       size_t to = SIZE_MAX, size_t hint_to = 0) {
     to = std::min(to, lv.size());
-    v.plan_bins = v.wt ? 0u : 1u;
     for (size_t li = rest ? (size_t)sub_from : from; li < to; ++li) {
         const LevelDesc &d = lv[li];
         v.base = d.base;
@@ -590,6 +594,7 @@ orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, u
         v.next_C = 0;  // nothing to plan below the last level or at the subtree level
         if (li + 1 < lv.size() && (rest || (int)li + 1 != sub_from)) {
             v.next_C = lv[li + 1].C;
+            v.plan_bins = plan_bins(ctx, v, lv[li + 1].C);
             v.child_map = d.child_map;
             v.small_next = small_cells(ctx, v, max_n, li + 1, lv[li + 1].C);
         }
@@ -597,15 +602,20 @@ orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, u
             // this level was not planned by the one above
             ORB_CUDA(cudaMemsetAsync(&ctx->counters.p->plan[0], 0, 2 * sizeof(PlanTotals), ctx->stream));
             v.plan_hint = hinted ? 1 : 0;
+            v.plan_bins = plan_bins(ctx, v, v.C);
             run_kernel(ctx, kKPlan, v, 1);
+            if (v.next_C) v.plan_bins = plan_bins(ctx, v, v.next_C);
         }
         v.plan_hint = v.hint && li + 1 < hint_to ? 1 : 0;
         if (v.wt) {
             // weighted build: every cell through the weighted passes (kWPasses reach the cap)
-            const uint64_t tiles = n / kTile + (uint64_t)v.C;
+            // levels of few cells: quarter tiles, so that the CTAs' shares are even
+            const int pieces = v.C <= ctx->num_sms ? 4 : 1;
+            const uint64_t tiles = (n / kTile + (uint64_t)v.C) * pieces;
+            v.last_pass = kWPasses - 1;
             for (int pass = 0; pass < kWPasses; ++pass) {
                 v.pass = pass;
-                run_kernel(ctx, kKWHist, v, (int)std::min<uint64_t>(pass_grid(ctx), tiles));
+                run_kernel(ctx, kKWHist, v, (int)std::min<uint64_t>(ctx->num_sms * 4, tiles), pieces);
                 ++*passes;
             }
         } else if (ctx->tune.cta_min_cells && !hinted && (uint32_t)v.C >= ctx->tune.cta_min_cells) {
@@ -880,7 +890,8 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     if (st != ORB_OK) return st;
     ORB_CUDA(ctx->idx.ensure(n + 1));
     if (weighted) {
-        ORB_CUDA(ctx->whist.ensure((size_t)max_cells * kWBins, true));  // all-zero between passes
+        // bins of cells of several tiles, all-zero between passes
+        ORB_CUDA(ctx->whist.ensure((size_t)(n / kTile + 2 + ctx->num_sms) << kMaxBinsLog2, true));
         ORB_CUDA(ctx->wbelow.ensure(max_cells));
         ORB_CUDA(ctx->wtot.ensure(max_cells));
         if (!dev) ORB_CUDA(ctx->w.ensure(n + 1));
@@ -963,7 +974,7 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     }
     v.C = lv.empty() ? 0 : lv[0].C;  // the init kernel plans the root
     v.small = small_cells(ctx, v, n, 0, v.C);
-    v.plan_bins = weighted ? 0u : 1u;
+    v.plan_bins = plan_bins(ctx, v, v.C);
     std::vector<uint64_t> key = level_key(ctx, v);
     key.push_back(0xB111D);  // single build
     key.push_back(n);

@@ -42,12 +42,9 @@ constexpr uint32_t kHintSubMax = 34816;
 constexpr uint32_t kSubDefaultLevels = 4;     // default of tune.subtree_levels
 constexpr int kSubMaxLevels = 6;              // deepest tree one subtree CTA finishes
 
-// Weighted builds: every active cell's bracket is binned into a midpoint tree of this depth
-// per pass (its weights summed per bin), so kWPasses passes reach the 32-iteration cap.
-constexpr int kWBinsLog2 = 8;
-constexpr int kWBins = 1 << kWBinsLog2;
-constexpr int kWPasses = 4;
-static_assert(kWPasses * kWBinsLog2 >= 32, "the weighted passes reach the iteration cap");
+// Weighted builds: launches of the weighted pass a level (11 iterations each for cells of more
+// than one tile; smaller cells are finished by the first).
+constexpr int kWPasses = 3;
 
 // kSmall: at most kWarpKeys keys (one warp bisects it); kOneTile: at most kTile keys (one CTA)
 // kReady: its bracket holds few enough keys for a list: the classify pass lists them and
@@ -208,8 +205,8 @@ struct Level {
     uint32_t *win_cnt;
     uint32_t win_cells;
     // weighted builds (null otherwise): an integer weight per particle, moved with it, and
-    // per cell of the level its weight bins (kWBins, kept all-zero between passes), the
-    // weight below its bracket and its total weight
+    // per cell of the level with several tiles its weight bins (at hist_off, kept all-zero
+    // between passes), the weight below its bracket and its total weight
     uint32_t *wt;
     unsigned long long *whist;
     unsigned long long *wbelow;

@@ -276,9 +276,10 @@ __device__ PlanCell plan_cell(const Level &v, PlanTotals *tot, uint32_t small, i
     }
     v.ptile_off[c] = p.t0;
     v.tile_off[c] = p.h0;
-    if (p.H && v.plan_bins) {
+    // (weighted builds: bins for cells of several tiles, on levels of few cells for all; no list)
+    if (v.wt ? p.H > (v.plan_bins ? 0u : 1u) : p.H && v.plan_bins) {
         const unsigned long long a =
-            atomicAdd(&tot->pools, (1ull << 32) | (unsigned long long)list_capacity(v, n));
+            atomicAdd(&tot->pools, (1ull << 32) | (v.wt ? 0ull : (unsigned long long)list_capacity(v, n)));
         v.hist_off[c] = (uint32_t)(a >> 32) << kMaxBinsLog2;
         v.cmp_off[c] = (uint32_t)a;
     }
@@ -3504,11 +3505,20 @@ __global__ void __launch_bounds__(kSubThreads) k_subtree(const __grid_constant__
 // ------------------------------------------------------------------------------------
 // Weighted builds: the reference's bisection loop on integer weight sums instead of counts
 // (the thesis's weighted ORB, documentation/notes.tex:259-271; never implemented by the
-// reference). Per level: every cell starts active; kWPasses passes each bin the weights of
-// every active cell's bracket into its midpoint tree of depth kWBinsLog2 (the exact
-// descent: the reference's own cuts) and sum the weights below the bracket; the CTA that
-// brings a cell's last tile replays up to kWBinsLog2 iterations of the loop on the prefix
-// sums with the weighted test. Integer sums: the same results in any order.
+// reference). A pass bins the weights of an active cell's bracket into its midpoint tree (the
+// reference's own cuts, binned exactly as in the count passes) and replays up to its depth of
+// iterations on the prefix sums with the weighted test; the first pass also sums the weights
+// below the bracket and the cell's total. Integer sums: the same results in any order.
+//
+// A cell whose tiles one CTA reads (all cells of at most one tile, but on levels of few cells)
+// is bisected to the end in one launch: up to kWDirect keys with the keys and weights in the
+// CTA's registers, every cut's weight summed (2.5 us a cell, against 12 with histograms),
+// more with the bins in shared memory. Larger cells take kWPasses launches, the CTA that brings
+// the last piece replaying; levels of few cells deal quarter tiles to the CTAs. A bin is two 32-bit sums, of the weights' low and high
+// halves (the high one is touched only by weights above 65535): shared memory has no 64-bit
+// add of its own, and an add that loops on compare-and-swap bound the passes (2^24 clustered
+// particles into 2^14 leaves: 4.0 ms of count passes with 64-bit bins, 256 a pass, four
+// launches a level and the descent for every key).
 // ------------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned long long block_sum_u64(unsigned long long x,
                                                             unsigned long long *sh) {
@@ -3522,150 +3532,420 @@ __device__ __forceinline__ unsigned long long block_sum_u64(unsigned long long x
     return t;
 }
 
-// The replay of up to kWBinsLog2 iterations of src/orbit.cpp:146-232 on cell c's finished
-// weight bins, with the weighted test, by the CTA that brought its last tile; the bins are
-// cleared for the next pass. (As a kernel of its own it took 9-10 us a pass.)
-__device__ __noinline__ void wresolve_cell(const Level &v, int c, bool whole, unsigned long long *s_pre,
-                                           unsigned long long *s_red) {
-    static_assert(kWBins == kThreads, "one bin a thread");
+// convergence_weighted() prepared for one cell: with W below 2^32 (k <= 2^30) the products fit
+// 64 bits, and n |D| < 3 k W is |D| < ceil(3 k W / n) for the integer |D|, one division a cell
+// in place of two 128-bit products a step (a third of the deep levels' passes).
+struct WeightTest {
+    unsigned long long W, half_w, limit;
+    uint32_t n;
+    int32_t k;
+    __device__ __forceinline__ WeightTest(unsigned long long w_cell, uint32_t n_, int32_t leaves)
+        : W(w_cell), half_w(0), limit(0), n(n_), k(leaves) {
+        if (!(W >> 32)) {
+            half_w = (unsigned long long)((k + 1) / 2) * W;
+            const unsigned long long b = 3ull * (unsigned long long)k * W;
+            limit = n ? (b + (n - 1)) / n : 0ull;
+            if (b + (n - 1) < b) limit = b / n + (b % n ? 1ull : 0ull);
+        }
+    }
+    __device__ __forceinline__ int dir(unsigned long long w_left) const {
+        if (W >> 32) return convergence_weighted(w_left, W, n, k);
+        const long long D = (long long)((unsigned long long)k * w_left) - (long long)half_w;
+        const unsigned long long ad = (unsigned long long)(D < 0 ? -D : D);
+        if (D == 0 || ad < limit) return 0;
+        return D > 0 ? 1 : -1;
+    }
+};
+
+// Tree depth of a pass over a cell of n keys that one CTA finishes: about two keys a bin, the
+// full depth for cells of more than a tile (so kWPasses launches reach the iteration cap; cells
+// dealt in pieces take it too).
+__device__ __forceinline__ int weighted_depth(uint32_t n) {
+    return max(4, min(kMaxBinsLog2, 30 - __clz(max(n, 1u))));
+}
+static_assert(kWPasses * kMaxBinsLog2 >= kMaxIterations, "the weighted passes reach the cap");
+constexpr uint32_t kWDirectPer = 8, kWDirect = kWDirectPer * kThreads;
+constexpr uint32_t kWFlush = 4;  // tiles whose low halves fit a 32-bit bin
+static_assert((unsigned long long)kWFlush * kTile * 0xffffull < (1ull << 32), "low halves of a run of tiles");
+
+// The cell a CTA is working on, in shared memory.
+struct WeightCell {
+    const float *keys;
+    float L, R;
+    int K;
+    uint32_t base, end, t0;
+    Guess gs;
+    unsigned long long below, tot;  // weight below L; the cell's weight
+    uint32_t it, state, last;
+};
+
+struct WeightSmem {
+    union {
+        uint32_t half[2][kHistBins];      // low and high halves' sums
+        unsigned long long pre[kHistBins];  // the replay's prefix sums
+    };
+    float edge[kHistBins + 1];
+    unsigned long long red[kThreads / 32];
+    uint32_t sum[2][2][kThreads / 32];  // direct sums by parity of the step: halves, a warp each
+    WeightCell cell;
+    uint32_t run[2];
+};
+
+// Replay of up to K iterations on the finished bins of cell c (in shared memory, or added up
+// in global memory by several CTAs), every thread; the cell's bracket and state in sm.cell.
+__device__ __noinline__ void weighted_replay(const Level &v, int c, bool global, WeightSmem &sm) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    unsigned long long *g = v.whist + (size_t)c * kWBins;
-    const unsigned long long x = whole ? s_pre[tid] : __ldcg(g + tid);
-    if (!whole) g[tid] = 0ull;
-    unsigned long long inc = x;
+    WeightCell &w = sm.cell;
+    const uint32_t nb = 1u << w.K, per = max(1u, nb / kThreads);
+    unsigned long long h[kHistBins / kThreads], run = 0;
+    unsigned long long *g = v.whist + v.hist_off[c];
+#pragma unroll
+    for (int j = 0; j < (int)(kHistBins / kThreads); ++j) {
+        h[j] = 0;
+        const uint32_t b = tid * per + (uint32_t)j;
+        if ((uint32_t)j < per && b < nb) {
+            if (global) {
+                h[j] = __ldcg(g + b);  // other CTAs' atomics: from L2
+                g[b] = 0ull;
+            } else {
+                h[j] = (unsigned long long)sm.half[0][b] + ((unsigned long long)sm.half[1][b] << 16);
+            }
+        }
+        run += h[j];
+    }
+    unsigned long long inc = run;
     for (int o = 1; o < 32; o <<= 1) {
         const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= (uint32_t)o) inc += t;
     }
-    if (lane == 31) s_red[warp] = inc;
+    if (lane == 31) sm.red[warp] = inc;
+    __syncthreads();  // (and every bin is read)
+    for (uint32_t k = 0; k < warp; ++k) inc += sm.red[k];
+    run = inc - run;
+#pragma unroll
+    for (int j = 0; j < (int)(kHistBins / kThreads); ++j) {
+        const uint32_t b = tid * per + (uint32_t)j;
+        if ((uint32_t)j < per && b < nb) sm.pre[b] = run;
+        run += h[j];
+    }
     __syncthreads();
-    for (uint32_t w = 0; w < warp; ++w) inc += s_red[w];
-    s_pre[tid] = inc - x;
+    if (tid == 0) {
+        const int slot = level_slot(v, c);
+        const int32_t leaves = v.heap[slot].nLeafCells;
+        const uint32_t n = w.end - w.base;
+        float L = w.L, R = w.R;
+        uint32_t it = w.it, pos = 0, width = nb;
+        uint8_t st = kActive;
+        const WeightTest test(w.tot, n, leaves);
+        for (int step = 0; step < w.K; ++step) {
+            if (it >= (uint32_t)kMaxIterations) break;
+            const uint32_t half = width >> 1;
+            ++it;
+            const int dir = test.dir(w.below + sm.pre[pos + half]);
+            if (dir == 0) {
+                st = kFound;
+                break;
+            }
+            const float cut = mid_cut(L, R);
+            if (dir > 0) {
+                R = cut;
+            } else {
+                L = cut;
+                pos += half;
+            }
+            width = half;
+        }
+        if (st == kActive && it >= (uint32_t)kMaxIterations) st = kCapped;
+        // the weight below the new bracket: below the old one plus the bins left of it
+        w.below += sm.pre[pos];
+        w.L = L;
+        w.R = R;
+        w.it = it;
+        w.state = st;
+        w.gs = make_guess(L, R, __fdiv_rn((float)nb, __fsub_rn(R, L)), nb);
+    }
     __syncthreads();
-    if (tid != 0) return;
-    const int slot = level_slot(v, c);
-    orb_cell_t &cell = v.heap[slot];
-    const uint2 rg = v.ranges[slot];
-    const uint32_t n = rg.y - rg.x;
-    const unsigned long long W = __ldcg(&v.wtot[c]), below = __ldcg(&v.wbelow[c]);
-    float L = cell.cutMarginLeft, R = cell.cutMarginRight;
-    uint32_t it = v.iters[c], pos = 0, width = kWBins;
-    uint8_t st = kActive;
-    for (int step = 0; step < kWBinsLog2; ++step) {
-        if (it >= (uint32_t)kMaxIterations) break;
-        const uint32_t half = width >> 1;
-        const unsigned long long wl = below + s_pre[pos + half];
-        ++it;
-        const int dir = convergence_weighted(wl, W, n, cell.nLeafCells);
-        if (dir == 0) {
-            st = kFound;
+}
+
+// The whole loop of a cell of at most kWDirect keys by the CTA, keys and weights in registers.
+__device__ __noinline__ void weighted_direct(const Level &v, int c, WeightSmem &sm) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    WeightCell &w = sm.cell;
+    const int32_t leaves = v.heap[level_slot(v, c)].nLeafCells;
+    const uint32_t n = w.end - w.base;
+    float k[kWDirectPer], L = w.L, R = w.R;
+    uint32_t x[kWDirectPer];
+#pragma unroll
+    for (int j = 0; j < (int)kWDirectPer; ++j) {
+        const uint32_t p = (uint32_t)j * kThreads + tid;
+        k[j] = p < n ? __ldg(w.keys + w.base + p) : __int_as_float(0x7fc00000);  // NaN: never below
+        x[j] = p < n ? __ldg(v.wt + w.base + p) : 0u;
+    }
+    // the CTA's sum of the weights of the keys below cut, in every thread; one barrier a step
+    uint32_t step = 0;
+    auto below = [&](float cut, bool all) -> unsigned long long {
+        uint32_t lo = 0, hi = 0;
+#pragma unroll
+        for (int j = 0; j < (int)kWDirectPer; ++j) {
+            const uint32_t y = all || k[j] < cut ? x[j] : 0u;
+            lo += y & 0xffffu;
+            hi += y >> 16;
+        }
+        lo = __reduce_add_sync(0xffffffffu, lo);
+        hi = __reduce_add_sync(0xffffffffu, hi);
+        uint32_t(*s)[kThreads / 32] = sm.sum[step++ & 1u];
+        if (lane == 0) {
+            s[0][warp] = lo;
+            s[1][warp] = hi;
+        }
+        __syncthreads();
+        lo = __reduce_add_sync(0xffffffffu, lane < kThreads / 32 ? s[0][lane] : 0u);
+        hi = __reduce_add_sync(0xffffffffu, lane < kThreads / 32 ? s[1][lane] : 0u);
+        return (unsigned long long)lo + ((unsigned long long)hi << 16);
+    };
+    const WeightTest test(below(0.f, true), n, leaves);
+    uint32_t it = 0;
+    int st = kActive;
+    while (st == kActive) {
+        if (it >= (uint32_t)kMaxIterations) {
+            st = kCapped;
             break;
         }
         const float cut = mid_cut(L, R);
-        if (dir > 0) {
+        ++it;
+        const int dir = test.dir(below(cut, false));
+        if (dir == 0)
+            st = kFound;
+        else if (dir > 0)
             R = cut;
-        } else {
+        else
             L = cut;
-            pos += half;
-        }
-        width = half;
     }
-    if (st == kActive && it >= (uint32_t)kMaxIterations) st = kCapped;
-    cell.cutMarginLeft = L;
-    cell.cutMarginRight = R;
-    cell.foundCut = st == kFound ? 1 : 0;
-    v.iters[c] = (uint8_t)it;
-    v.state[c] = st;
-    v.hdone[c] = 0;
-    // the weight below the new bracket [L, R): below the old one plus the bins left of it
-    v.wbelow[c] = below + s_pre[pos];
-    if (st != kActive) atomicMax(&v.counters->max_iters, it);
-    if (st == kCapped) atomicAdd(&v.counters->unfound, 1u);
+    __syncthreads();  // every thread has left the cell and the sums
+    if (tid == 0) {
+        w.L = L;
+        w.R = R;
+        w.it = it;
+        w.state = (uint32_t)st;
+        w.below = 0;
+    }
+    __syncthreads();
 }
 
-__global__ void __launch_bounds__(kThreads) k_whist(const __grid_constant__ Level v) {
+__global__ void __launch_bounds__(kThreads, 4) k_whist(const __grid_constant__ Level v, uint32_t pieces) {
     pdl_enter();
     if (level_failed(v)) return;
-    __shared__ unsigned long long s_bins[kWBins];
-    __shared__ unsigned long long s_red[kThreads / 32];
-    __shared__ uint32_t s_last;
-    const uint32_t total = (uint32_t)(v.tot->tiles >> 32);
-    unsigned long long bytes = 0, wkeys = 0;  // this thread's bracket weight reads; the CTA's keys
-    for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
-        const TileRef tr = tile_ref(v, t);
-        if (v.state[tr.c] != kActive) continue;  // block-uniform
-        const orb_cell_t &cell = v.heap[tr.slot];
-        const float L = cell.cutMarginLeft, R = cell.cutMarginRight;
-        const float *keys = axis_keys(v, eff_axis(cell.cutAxis));
-        for (uint32_t j = threadIdx.x; j < (uint32_t)kWBins; j += blockDim.x) s_bins[j] = 0ull;
+    __shared__ WeightSmem sm;
+    WeightCell &w = sm.cell;
+    const uint32_t tid = threadIdx.x;
+    const uint32_t piece = (uint32_t)kTile / pieces;  // keys of a piece; `pieces` of them a tile
+    unsigned long long bytes = 0;
+    if (tid == 0) {
+        const uint64_t total = (v.tot->tiles >> 32) * pieces;
+        sm.run[0] = (uint32_t)(total * blockIdx.x / gridDim.x);
+        sm.run[1] = (uint32_t)(total * (blockIdx.x + 1) / gridDim.x);
+    }
+    __syncthreads();
+    const uint32_t t_end = sm.run[1];
+    int cur = -1;
+    uint32_t ntiles = 0, held = 0;  // pieces of the cell so far; of them in the shared bins
+    bool flushed = false, direct = false;
+    unsigned long long below = 0, tot = 0;  // this thread's weights below L, and all (first pass)
+    auto clear = [&]() {
+        for (uint32_t j = tid; j < (1u << w.K); j += kThreads) sm.half[0][j] = sm.half[1][j] = 0u;
+    };
+    auto flush = [&]() {  // the shared bins to the cell's global ones
         __syncthreads();
-        unsigned long long below = 0, tot = 0;
-        // kWLoads keys of a thread in flight per round. The first pass reads every weight
-        // (the cell's total and the weight below its bracket); later passes read the weights
-        // of the keys inside the bracket only (the weight below it is carried by k_wresolve).
-        constexpr int kWLoads = 4;
-        const uint32_t nt = blockDim.x;
-        const bool first = v.pass == 0;
-        for (uint32_t p0 = tr.e0 + threadIdx.x; p0 < tr.e1; p0 += nt * kWLoads) {
-            float k[kWLoads];
-            uint32_t w[kWLoads];
-#pragma unroll
-            for (int u = 0; u < kWLoads; ++u) {
-                const uint32_t p = p0 + (uint32_t)u * nt;
-                k[u] = p < tr.e1 ? __ldg(keys + p) : L;
-                w[u] = first && p < tr.e1 ? __ldg(v.wt + p) : 0u;
-            }
-#pragma unroll
-            for (int u = 0; u < kWLoads; ++u) {
-                const uint32_t p = p0 + (uint32_t)u * nt;
-                if (p >= tr.e1) continue;
-                if (first) {
-                    tot += w[u];
-                    if (k[u] < L) below += w[u];
-                }
-                if (k[u] >= L && k[u] < R) {
-                    const uint32_t wk = first ? w[u] : __ldg(v.wt + p);
-                    if (wk) atomicAdd(&s_bins[tree_bin(k[u], L, R, kWBinsLog2)], (unsigned long long)wk);
-                    if (!first) ++bytes;  // a weight read (counted in 4-byte units below)
-                }
-            }
-        }
-        if (first) {
-            below = block_sum_u64(below, s_red);
-            tot = block_sum_u64(tot, s_red);
+        unsigned long long *g = v.whist + v.hist_off[cur];
+        for (uint32_t j = tid; j < (1u << w.K); j += kThreads) {
+            const unsigned long long x =
+                (unsigned long long)sm.half[0][j] + ((unsigned long long)sm.half[1][j] << 16);
+            if (x) atomicAdd(&g[j], x);
         }
         __syncthreads();
-        const uint2 rg = v.ranges[tr.slot];
-        const uint32_t tiles = (rg.y - rg.x + (uint32_t)kTile - 1) / (uint32_t)kTile;
-        if (threadIdx.x == 0) {
-            wkeys += tr.e1 - tr.e0;
-            s_last = tiles == 1 ? 1u : 0u;
-            if (first) {
-                if (below) atomicAdd(&v.wbelow[tr.c], below);
-                if (tot) atomicAdd(&v.wtot[tr.c], tot);
+        flushed = true;
+        held = 0;
+    };
+    // keys [e0, e1) of the cell; first: every weight is read (the total, the weight below L),
+    // later: those of the bracket's keys
+    auto tile = [&](uint32_t e0, uint32_t e1, bool first) {
+        const float *keys = w.keys;
+        const Guess gs = w.gs;
+        const float L = w.L, R = w.R;
+        const uint32_t top = (1u << w.K) - 1u;
+        auto add = [&](float k, uint32_t x) {
+            uint32_t b;
+            if (!guess_bin(gs, k, &b)) b = near_bin(k, gs, sm.edge, top);
+            atomicAdd(&sm.half[0][b], x & 0xffffu);
+            if (x >> 16) atomicAdd(&sm.half[1][b], x >> 16);
+        };
+        if (!first) {
+            // 16 keys of a thread in flight, the weights of the bracket's keys only
+            constexpr int kLoads = 16;
+            for (uint32_t p0 = e0 + tid; p0 < e1; p0 += kThreads * kLoads) {
+                float k[kLoads];
+#pragma unroll
+                for (int u = 0; u < kLoads; ++u) {
+                    const uint32_t p = p0 + (uint32_t)u * kThreads;
+                    k[u] = p < e1 ? __ldg(keys + p) : __int_as_float(0x7fc00000);  // NaN: not binned
+                }
+                uint32_t in = 0;
+#pragma unroll
+                for (int u = 0; u < kLoads; ++u) in |= (uint32_t)(k[u] >= L && k[u] < R) << u;
+                for (; in; in &= in - 1u) {
+                    const uint32_t p = p0 + ((uint32_t)__ffs(in) - 1u) * kThreads, y = __ldg(v.wt + p);
+                    if (y) add(__ldg(keys + p), y);
+                }
             }
+            if (tid == 0) bytes += 4ull * (e1 - e0);
+            return;
         }
-        if (tiles > 1) {
-            unsigned long long *g = v.whist + (size_t)tr.c * kWBins;
-            for (uint32_t j = threadIdx.x; j < (uint32_t)kWBins; j += blockDim.x)
-                if (s_bins[j]) atomicAdd(&g[j], s_bins[j]);
+        constexpr int kLoads = 8;
+        for (uint32_t p0 = e0 + tid; p0 < e1; p0 += kThreads * kLoads) {
+            float k[kLoads];
+            uint32_t x[kLoads], any = 0;
+#pragma unroll
+            for (int u = 0; u < kLoads; ++u) {
+                const uint32_t p = p0 + (uint32_t)u * kThreads;
+                k[u] = p < e1 ? __ldg(keys + p) : __int_as_float(0x7fc00000);
+                x[u] = p < e1 ? __ldg(v.wt + p) : 0u;
+            }
+#pragma unroll
+            for (int u = 0; u < kLoads; ++u) any |= x[u];
+            if (any < (1u << 29)) {  // eight weights below 2^29 add up in 32 bits
+                uint32_t all = 0, low = 0;
+#pragma unroll
+                for (int u = 0; u < kLoads; ++u) {
+                    all += x[u];
+                    low += k[u] < L ? x[u] : 0u;
+                }
+                tot += all;
+                below += low;
+            } else {
+#pragma unroll
+                for (int u = 0; u < kLoads; ++u) {
+                    tot += x[u];
+                    if (k[u] < L) below += x[u];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kLoads; ++u)
+                if (k[u] >= L && k[u] < R && x[u]) add(k[u], x[u]);
+        }
+        if (tid == 0) bytes += 8ull * (e1 - e0);
+    };
+    auto end_cell = [&]() {
+        const uint32_t tiles = (w.end - w.base + (uint32_t)kTile - 1) / (uint32_t)kTile * pieces;
+        const bool whole = ntiles == tiles && !flushed, first = v.pass == 0;
+        if (first && !direct) {
+            below = block_sum_u64(below, sm.red);
+            tot = block_sum_u64(tot, sm.red);
+        }
+        __syncthreads();
+        bool last = true;
+        if (direct) {
+            weighted_direct(v, cur, sm);
+        } else if (whole) {
+            if (tid == 0 && first) {
+                w.below = below;
+                w.tot = tot;
+            }
             __syncthreads();
-            if (threadIdx.x == 0) {
-                s_last = arrive_release(&v.hdone[tr.c], 1u) + 1u == tiles;
-                if (s_last) acquire();
+            weighted_replay(v, cur, false, sm);
+            while (w.state == kActive) {  // the rest of the loop, on this CTA's own cell
+                clear();
+                fill_edges(sm.edge, w.L, w.R, w.K, tid, kThreads);
+                __syncthreads();
+                tile(w.base, w.end, false);
+                __syncthreads();
+                weighted_replay(v, cur, false, sm);
             }
+        } else {
+            if (tid == 0 && first) {
+                if (below) atomicAdd(&v.wbelow[cur], below);
+                if (tot) atomicAdd(&v.wtot[cur], tot);
+            }
+            flush();
+            if (tid == 0) {
+                w.last = arrive_release(&v.hdone[cur], ntiles) + ntiles == tiles;
+                if (w.last) {
+                    acquire();
+                    w.below = __ldcg(&v.wbelow[cur]);
+                    w.tot = __ldcg(&v.wtot[cur]);
+                }
+            }
+            __syncthreads();
+            last = w.last != 0;
+            if (last) weighted_replay(v, cur, true, sm);
         }
-        __syncthreads();
-        if (s_last) wresolve_cell(v, tr.c, tiles == 1, s_bins, s_red);
-        __syncthreads();  // s_bins reused by the next tile
+        if (last && tid == 0) {
+            orb_cell_t &cell = v.heap[level_slot(v, cur)];
+            cell.cutMarginLeft = w.L;
+            cell.cutMarginRight = w.R;
+            cell.foundCut = w.state == kFound ? 1 : 0;
+            v.iters[cur] = (uint8_t)w.it;
+            v.state[cur] = (uint8_t)w.state;
+            v.wbelow[cur] = w.below;
+            v.hdone[cur] = 0;
+            if (w.state != kActive) atomicMax(&v.counters->max_iters, w.it);
+            if (w.state == kCapped) atomicAdd(&v.counters->unfound, 1u);
+            if (w.state == kActive && v.pass == v.last_pass) atomicExch(&v.counters->error, 1u);
+        }
+        __syncthreads();  // the cell and its bins are free for the next one
+        ntiles = 0;
+        below = tot = 0;
+        flushed = false;
+    };
+    int skip_c = -1;  // an inactive cell whose tiles are being passed over
+    for (uint32_t t = sm.run[0]; t < t_end; ++t) {
+        const int c = (int)v.htile_cell[t / pieces];
+        if (c == skip_c) continue;
+        if (c != cur) {
+            // a cell with a tile still to come is not resolved in this pass: its state stands
+            if (v.state[c] != kActive) {
+                skip_c = c;
+                continue;
+            }
+            if (cur >= 0) end_cell();
+            cur = c;
+            held = 0;
+            if (tid == 0) {
+                const int slot = level_slot(v, c);
+                const orb_cell_t &cell = v.heap[slot];
+                const uint2 rg = v.ranges[slot];
+                w.keys = axis_keys(v, eff_axis(cell.cutAxis));
+                w.L = cell.cutMarginLeft;
+                w.R = cell.cutMarginRight;
+                w.K = pieces > 1 ? kMaxBinsLog2 : weighted_depth(rg.y - rg.x);
+                w.base = rg.x;
+                w.end = rg.y;
+                w.t0 = v.tile_off[c];
+                w.it = v.iters[c];
+                w.below = v.pass ? v.wbelow[c] : 0ull;
+                w.tot = v.pass ? v.wtot[c] : 0ull;
+                const uint32_t nb = 1u << w.K;
+                w.gs = make_guess(w.L, w.R, __fdiv_rn((float)nb, __fsub_rn(w.R, w.L)), nb);
+            }
+            __syncthreads();
+            direct = pieces == 1 && w.end - w.base <= kWDirect;
+            if (!direct) {
+                clear();
+                fill_edges(sm.edge, w.L, w.R, w.K, tid, kThreads);
+                __syncthreads();
+            }
+        } else if (held == kWFlush * pieces) {
+            flush();
+            clear();
+            __syncthreads();
+        }
+        const uint32_t e0 = min(w.end, w.base + (t - w.t0 * pieces) * piece);
+        if (!direct) tile(e0, min(w.end, e0 + piece), v.pass == 0);
+        if (direct && tid == 0) bytes += 8ull * (w.end - w.base);
+        ++ntiles;
+        ++held;
     }
-    // 4 B per key read (every pass), 4 B per weight read (every key in the first pass, the
-    // bracket's keys after it): per thread in-bracket weight reads summed over the block
-    const unsigned long long wr = v.pass == 0 ? 0ull : block_sum_u64(bytes, s_red);
-    if (threadIdx.x == 0) {
-        const unsigned long long b = 4ull * wkeys * (v.pass == 0 ? 2ull : 1ull) + 4ull * wr;
-        if (b) add_bytes(v, kKWHist, b);
-    }
+    if (cur >= 0) end_cell();
+    if (tid == 0 && bytes) add_bytes(v, kKWHist, bytes);
 }
 
 // ------------------------------------------------------------------------------------
@@ -3975,7 +4255,7 @@ void launch_level_kernel(Kernel k, const Level &v, int grid, int arg, cudaStream
             else
                 launch_kernel(p, k_part_finish<false>, dim3(per_cell_warps), T, 0, st, v, arg);
             break;
-        case kKWHist: launch_kernel(p, k_whist, dim3(grid), T, 0, st, v); break;
+        case kKWHist: launch_kernel(p, k_whist, dim3(grid), T, 0, st, v, (uint32_t)arg); break;
         case kKCountLeft: launch_kernel(p, k_count_left, dim3(grid), T, 0, st, v); break;
         case kKSample:
             launch_kernel(p, k_sample_bin, dim3(kSampleMax / kSamplePerCta, (unsigned)min(v.C, 65535)),
