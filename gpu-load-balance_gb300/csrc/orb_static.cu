@@ -5,9 +5,9 @@
 // either fails or fragments the pool, and cudaMalloc/cudaFree synchronise the device, which
 // stalls the caller's other streams. orb_count_left needs a context whose buffers are
 // allocated on first use; this entry point needs no context and allocates nothing. Its
-// scratch (per-cell tile offsets and per-cell counters) is the file-scope device array
-// below, ORB_STATIC_MAX_CELLS cells large; every GPU that loads the library holds it
-// (2 * 65536 + 2 words, 512 KiB) until the process exits.
+// scratch (per-cell tile offsets and their chunks' totals) is the file-scope device array
+// below, for ORB_STATIC_MAX_CELLS cells; every GPU that loads the library holds it
+// (65536 + 64 words, 256 KiB) until the process exits.
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -17,12 +17,15 @@
 namespace {
 
 constexpr uint32_t kMaxCells = ORB_STATIC_MAX_CELLS;
-constexpr uint32_t kTileKeys = 8192;
+constexpr uint32_t kTileKeys = 2048;   // keys a warp counts at a time
+constexpr uint32_t kChunk = 1024;      // cells a plan CTA takes
+constexpr uint32_t kChunks = kMaxCells / kChunk;
+static_assert(kChunks <= 64, "two chunks a lane in k_static_count");
 constexpr int kMaxDevices = 64;
 
-// [0, C]: exclusive prefix of tiles per cell (entry C = total tiles);
-// [C+1, 2C+1): per-cell counts of keys below the cut.
-static __device__ __align__(256) uint32_t g_count_scratch[2 * kMaxCells + 2];
+// [0, kMaxCells): first tile of each cell within its chunk; [kMaxCells, kMaxCells + kChunks):
+// the chunks' tiles.
+static __device__ __align__(256) uint32_t g_count_scratch[kMaxCells + kChunks];
 
 struct DeviceSetup {
     bool done;
@@ -65,22 +68,19 @@ __device__ __forceinline__ uint2 cell_range(const orb_cell_t &c, const uint32_t 
     return make_uint2(b, e);
 }
 
-// One CTA: tiles per cell (none for found cells), exclusive scan into scratch[0..C],
-// counters scratch[C+1 ..] cleared (they keep the previous call's values otherwise).
-__global__ void __launch_bounds__(1024) k_static_plan(const orb_cell_t *cells, uint32_t C,
-                                                      const uint32_t *ranges, uint32_t n_ranges,
-                                                      uint64_t n, uint32_t *scratch) {
+// A CTA a chunk of cells, a thread a cell: its tiles (none for a found cell), their exclusive
+// prefix within the chunk, and a zero in the output of every cell that is counted.
+__global__ void __launch_bounds__(kChunk) k_static_plan(const orb_cell_t *cells, uint32_t C,
+                                                        const uint32_t *ranges, uint32_t n_ranges,
+                                                        uint64_t n, uint32_t *out, uint32_t *scratch) {
     __shared__ uint32_t warp_tot[32];
-    const uint32_t tid = threadIdx.x, per = (C + blockDim.x - 1) / blockDim.x;
-    const uint32_t c0 = min(C, tid * per), c1 = min(C, c0 + per);
+    const uint32_t tid = threadIdx.x, c = blockIdx.x * kChunk + tid;
     uint32_t mine = 0;
-    for (uint32_t c = c0; c < c1; ++c) {
-        scratch[C + 1 + c] = 0u;
-        if (cells[c].foundCut) continue;
+    if (c < C && !cells[c].foundCut) {
         const uint2 r = cell_range(cells[c], ranges, n_ranges, n);
-        mine += (r.y - r.x + kTileKeys - 1) / kTileKeys;
+        mine = (r.y - r.x + kTileKeys - 1) / kTileKeys;
+        out[c] = 0u;
     }
-    // block exclusive scan of `mine`
     const int lane = tid & 31, warp = tid >> 5;
     uint32_t inc = mine;
     for (int o = 1; o < 32; o <<= 1) {
@@ -89,63 +89,93 @@ __global__ void __launch_bounds__(1024) k_static_plan(const orb_cell_t *cells, u
     }
     if (lane == 31) warp_tot[warp] = inc;
     __syncthreads();
-    if (warp == 0) {
-        const uint32_t w = warp_tot[lane];
-        uint32_t s = w;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o) s += t;
-        }
-        warp_tot[lane] = s - w;
-    }
-    __syncthreads();
-    uint32_t off = warp_tot[warp] + inc - mine;
-    for (uint32_t c = c0; c < c1; ++c) {
-        scratch[c] = off;
-        if (cells[c].foundCut) continue;
-        const uint2 r = cell_range(cells[c], ranges, n_ranges, n);
-        off += (r.y - r.x + kTileKeys - 1) / kTileKeys;
-    }
-    if (tid == blockDim.x - 1) scratch[C] = off;
+    const uint32_t w = warp_tot[lane];
+    const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u);
+    if (c < C) scratch[c] = before + inc - mine;
+    if (tid == kChunk - 1) scratch[kMaxCells + blockIdx.x] = before + inc;
 }
 
+// A warp a tile, the CTA's eight warps on consecutive ones: two searches find its cell (the
+// chunk among the lanes' prefixes, then 32 cells a probe), 16-byte loads, and one add per cell
+// and CTA. Bound by HBM for many keys, by the chain of small loads ahead of them for few. The
+// former form (a scan by one CTA, a CTA a tile of 8192 keys with 4-byte loads and a binary
+// search, counters in scratch copied out by a third kernel) took 47 us for 2^24 clustered
+// particles in 1024 cells, a quarter of them found; this takes 18.
 __global__ void __launch_bounds__(256) k_static_count(const float *x, const float *y, const float *z,
                                                       const orb_cell_t *cells, uint32_t C,
                                                       const uint32_t *ranges, uint32_t n_ranges,
-                                                      uint64_t n, uint32_t *scratch) {
-    __shared__ uint32_t red[8];
-    const uint32_t total = scratch[C];
-    for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
-        uint32_t lo = 0, hi = C;  // largest c with scratch[c] <= t
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi + 1) >> 1;
-            if (scratch[mid] <= t) lo = mid; else hi = mid - 1;
+                                                      uint64_t n, uint32_t *out, const uint32_t *scratch) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __shared__ uint32_t s_cell[8], s_cnt[8];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t chunks = (C + kChunk - 1) / kChunk;
+    // first tile of chunks 2 lane and 2 lane + 1 (past the last chunk: all the tiles)
+    const uint32_t ta = 2 * lane < chunks ? scratch[kMaxCells + 2 * lane] : 0u;
+    const uint32_t tb = 2 * lane + 1 < chunks ? scratch[kMaxCells + 2 * lane + 1] : 0u;
+    unsigned long long inc = (unsigned long long)ta + tb;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o) inc += t;
+    }
+    const unsigned long long total = __shfl_sync(0xffffffffu, inc, 31);
+    const unsigned long long b0 = inc - ta - tb, b1 = b0 + ta;
+    for (unsigned long long g = 8ull * blockIdx.x; g < total; g += 8ull * gridDim.x) {
+        const unsigned long long t = g + warp;
+        uint32_t c = 0xffffffffu, cnt = 0;
+        if (t < total) {  // warp-uniform
+            const uint32_t below = (uint32_t)__popc(__ballot_sync(0xffffffffu, 2 * lane < chunks && b0 <= t)) +
+                                   (uint32_t)__popc(__ballot_sync(0xffffffffu, 2 * lane + 1 < chunks && b1 <= t));
+            const uint32_t chunk = below - 1u;  // the last chunk that starts at or before t
+            const unsigned long long base =
+                __shfl_sync(0xffffffffu, (chunk & 1u) ? b1 : b0, (int)(chunk >> 1));
+            const uint32_t local = (uint32_t)(t - base);
+            const uint32_t *off = scratch + chunk * kChunk;
+            const uint32_t len = min(kChunk, C - chunk * kChunk);
+            // the last cell that starts at or before `local`, 32 probes a round
+            uint32_t lo = 0;
+            for (uint32_t step = kChunk / 32; step; step = step > 1 ? 1 : 0) {
+                const uint32_t p = lo + lane * step;
+                const bool ok = p < len && off[p] <= local;
+                lo += ((uint32_t)__popc(__ballot_sync(0xffffffffu, ok)) - 1u) * step;
+            }
+            c = chunk * kChunk + lo;
+            const orb_cell_t &cell = cells[c];
+            const uint2 r = cell_range(cell, ranges, n_ranges, n);
+            const int axis = cell.cutAxis < 0 ? 0 : cell.cutAxis;
+            const float *keys = axis == 0 ? x : (axis == 1 ? y : z);
+            const float cut = orb::mid_cut(cell.cutMarginLeft, cell.cutMarginRight);  // getCut()
+            const uint32_t e0 = r.x + (local - off[lo]) * kTileKeys, e1 = min(r.y, e0 + kTileKeys);
+            const uintptr_t addr = reinterpret_cast<uintptr_t>(keys + e0);
+            const uint32_t a0 = min(e1, e0 + (uint32_t)(((16u - (addr & 15u)) & 15u) >> 2));
+            const uint32_t n4 = (e1 - a0) >> 2;
+            if (lane < a0 - e0) cnt += __ldg(keys + e0 + lane) < cut;
+            const float4 *k4 = reinterpret_cast<const float4 *>(keys + a0);
+#pragma unroll 8
+            for (uint32_t i = lane; i < n4; i += 32) {
+                const float4 q = __ldg(k4 + i);
+                cnt += (q.x < cut) + (q.y < cut) + (q.z < cut) + (q.w < cut);
+            }
+            const uint32_t tail = a0 + (n4 << 2);
+            if (lane < e1 - tail) cnt += __ldg(keys + tail + lane) < cut;
+            cnt = __reduce_add_sync(0xffffffffu, cnt);
         }
-        const orb_cell_t &cell = cells[lo];
-        const uint2 r = cell_range(cell, ranges, n_ranges, n);
-        const uint32_t e0 = r.x + (t - scratch[lo]) * kTileKeys;
-        const uint32_t e1 = min(r.y, e0 + kTileKeys);
-        const int axis = cell.cutAxis < 0 ? 0 : cell.cutAxis;
-        const float *keys = axis == 0 ? x : (axis == 1 ? y : z);
-        const float cut = orb::mid_cut(cell.cutMarginLeft, cell.cutMarginRight);  // getCut()
-        uint32_t cnt = 0;
-        for (uint32_t i = e0 + threadIdx.x; i < e1; i += blockDim.x) cnt += __ldg(keys + i) < cut;
-        for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = cnt;
+        if (lane == 0) {
+            s_cell[warp] = c;
+            s_cnt[warp] = cnt;
+        }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t s = 0;
-            for (int w = 0; w < 8; ++w) s += red[w];
-            if (s) atomicAdd(&scratch[C + 1 + lo], s);
+        if (warp == 0) {
+            // the warps' counts added up per cell, by each cell's first warp
+            const uint32_t mc = lane < 8 ? s_cell[lane] : 0xffffffffu;
+            const uint32_t peers = __match_any_sync(0xffffffffu, mc);
+            if (mc != 0xffffffffu && lane == (uint32_t)__ffs(peers) - 1u) {
+                uint32_t sum = 0;
+                for (uint32_t p = peers; p; p &= p - 1u) sum += s_cnt[__ffs(p) - 1];
+                if (sum) atomicAdd(&out[mc], sum);
+            }
         }
         __syncthreads();
     }
-}
-
-__global__ void k_static_store(const orb_cell_t *cells, uint32_t C, uint32_t *out,
-                               const uint32_t *scratch) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < C && !cells[c].foundCut) out[c] = scratch[C + 1 + c];
 }
 
 }  // namespace
@@ -163,8 +193,22 @@ extern "C" orb_status orb_count_left_static(const float *x, const float *y, cons
     DeviceSetup s;
     if (setup_device(dev, &s) != cudaSuccess) return ORB_ERR_CUDA;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    k_static_plan<<<1, 1024, 0, st>>>(cells, n_cells, ranges, n_ranges, n, s.scratch);
-    k_static_count<<<s.sms * 8, 256, 0, st>>>(x, y, z, cells, n_cells, ranges, n_ranges, n, s.scratch);
-    k_static_store<<<(n_cells + 255) / 256, 256, 0, st>>>(cells, n_cells, out, s.scratch);
+    k_static_plan<<<(n_cells + kChunk - 1) / kChunk, kChunk, 0, st>>>(cells, n_cells, ranges, n_ranges, n, out,
+                                                                     s.scratch);
+    // the count kernel's launch overlaps the plan's (it waits for it in griddepcontrol.wait)
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)s.sms * 8);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, k_static_count, x, y, z, cells, n_cells, ranges, n_ranges, n, out,
+                           (const uint32_t *)s.scratch) != cudaSuccess) {
+        cudaGetLastError();
+        return ORB_ERR_CUDA;
+    }
     return cudaGetLastError() == cudaSuccess ? ORB_OK : ORB_ERR_CUDA;
 }
