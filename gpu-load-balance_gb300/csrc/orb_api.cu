@@ -23,6 +23,10 @@
 #include <utility>
 #include <vector>
 
+#include <errno.h>
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include "orb_internal.cuh"
 
 using namespace orb;
@@ -113,6 +117,8 @@ struct orb_ctx {
     DevBuf<unsigned long long> whist, wbelow, wtot;  // weighted builds: per-cell weight sums
     BuildCounters *h_counters = nullptr;  // pinned
     uint32_t *h_sub_flag = nullptr;       // pinned: the subtree path was taken
+    char *h_tree = nullptr;               // pinned: small trees on their way to the caller
+    size_t h_tree_bytes = 0;
 
     // service layer state
     bool loaded = false;
@@ -183,6 +189,32 @@ bool is_device_ptr(const void *p) {
 
 // Levels of at most this many cells per SM send every cell through the count passes.
 constexpr int kCountCells = 1;
+
+}  // namespace
+
+namespace orb {
+// Results in ordinary host memory. A device-to-host copy into pages the process has never
+// written faults them in from the GPU's side, which was seen to take anything from 2.8 to 54 ms
+// for 64 MB in fresh pages (0.4 ms in resident ones): so results have their pages made
+// resident and writable first, in one call that leaves their bytes alone, while the device
+// works where there is work to wait for. (Reading and writing back a byte a page took 19 ms: the
+// read maps the shared zero page, whose replacement the GPU's address translation must see.)
+// Memory it does not apply to (page-locked, device-mapped) is left as it is.
+void touch_pages(void *ptr, size_t bytes) {
+    if (!ptr || !bytes) return;
+    static const uintptr_t page = [] {
+        const long v = sysconf(_SC_PAGESIZE);
+        return v > 0 ? (uintptr_t)v : (uintptr_t)4096;
+    }();
+    const uintptr_t a = reinterpret_cast<uintptr_t>(ptr) / page * page;
+    const uintptr_t e = (reinterpret_cast<uintptr_t>(ptr) + bytes + page - 1) / page * page;
+    constexpr int kPopulateWrite = 23;  // MADV_POPULATE_WRITE (Linux 5.14)
+    const int saved = errno;
+    if (madvise(reinterpret_cast<void *>(a), e - a, kPopulateWrite) != 0) errno = saved;
+}
+}  // namespace orb
+
+namespace {
 
 orb_status ensure_ptile_buffers(orb_ctx *ctx, uint64_t ptiles, uint64_t cells) {
     ORB_CUDA(ctx->ptile_cell.ensure(ptiles));
@@ -641,6 +673,55 @@ orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, u
     return ORB_OK;
 }
 
+// Where a build's heap and ranges go: into the caller's memory, or (small trees) through the
+// context's page-locked buffer.
+struct TreeOut {
+    orb_cell_t *heap;
+    uint32_t *ranges;
+    size_t cells;
+    char *staged;  // the page-locked buffer (null: straight to the caller)
+};
+constexpr size_t kStagedTreeBytes = 1u << 20;
+
+TreeOut tree_out(orb_ctx *ctx, orb_cell_t *heap, uint32_t *ranges, size_t cells) {
+    TreeOut t = {heap, ranges, cells, nullptr};
+    const size_t bytes = cells * (sizeof(orb_cell_t) + sizeof(uint2));
+    if (bytes > kStagedTreeBytes) return t;
+    if (ctx->h_tree_bytes < bytes) {
+        if (ctx->h_tree) cudaFreeHost(ctx->h_tree);
+        ctx->h_tree = nullptr;
+        ctx->h_tree_bytes = 0;
+        const size_t want = std::max<size_t>(bytes, 1u << 16);
+        if (cudaMallocHost(reinterpret_cast<void **>(&ctx->h_tree), want) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->h_tree = nullptr;
+            return t;
+        }
+        ctx->h_tree_bytes = want;
+    }
+    t.staged = ctx->h_tree;
+    return t;
+}
+
+// Queues the copies of the tree and the counters behind the build.
+orb_status queue_tree(orb_ctx *ctx, const TreeOut &t) {
+    const size_t hb = t.cells * sizeof(orb_cell_t), rb = t.cells * sizeof(uint2);
+    void *h = t.staged ? static_cast<void *>(t.staged) : t.heap, *r = t.staged ? static_cast<void *>(t.staged + hb) : t.ranges;
+    if (t.cells) {
+        ORB_CUDA(cudaMemcpyAsync(h, ctx->heap.p, hb, cudaMemcpyDeviceToHost, ctx->stream));
+        ORB_CUDA(cudaMemcpyAsync(r, ctx->ranges.p, rb, cudaMemcpyDeviceToHost, ctx->stream));
+    }
+    ORB_CUDA(cudaMemcpyAsync(ctx->h_counters, ctx->counters.p, sizeof(BuildCounters), cudaMemcpyDeviceToHost, ctx->stream));
+    return ORB_OK;
+}
+
+// After the copies have ended.
+void take_tree(const TreeOut &t) {
+    if (!t.staged) return;
+    std::memcpy(t.heap, t.staged, t.cells * sizeof(orb_cell_t));
+    std::memcpy(t.ranges, t.staged + t.cells * sizeof(orb_cell_t), t.cells * sizeof(uint2));
+}
+
 constexpr const char *kUnfinished = "a cell's tiles did not all report or a bisection did not finish";
 
 // After a build (its counters read back): no step flagged an error and every cell of the first
@@ -652,17 +733,23 @@ bool build_finished(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, size_t
     return true;
 }
 
-// After the main graph of a build that planned subtrees (sub_from >= 0): waits for it and
-// reads whether the device took the subtree path (*taken). When it refused (a cell too large
+// After the main graph of a build: queues the copies of its tree; of one that planned subtrees
+// (sub_from >= 0): waits for it and reads whether the device took the subtree path (*taken). When it refused (a cell too large
 // for one CTA), a second graph runs the level kernels of the levels from sub_from down. The
 // build's end event is recorded again after it.
 orb_status finish_subtree_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv,
                                  std::vector<uint64_t> key, uint32_t *passes, int sub_from,
-                                 uint64_t n, uint64_t max_n, size_t hint_to, bool *taken) {
+                                 uint64_t n, uint64_t max_n, size_t hint_to, const TreeOut &out, bool *taken) {
     *taken = false;
-    if (sub_from < 0) return ORB_OK;
+    if (!out.staged) {  // while the device builds
+        touch_pages(out.heap, out.cells * sizeof(orb_cell_t));
+        touch_pages(out.ranges, out.cells * sizeof(uint2));
+    }
+    if (sub_from < 0) return queue_tree(ctx, out);
     ORB_CUDA(cudaMemcpyAsync(ctx->h_sub_flag, ctx->sub_flag.p, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                              ctx->stream));
+    orb_status qst = queue_tree(ctx, out);  // (final when the subtree path was taken)
+    if (qst != ORB_OK) return qst;
     ORB_CUDA(cudaStreamSynchronize(ctx->stream));
     *taken = *ctx->h_sub_flag == 1u;
     if (*taken) return ORB_OK;
@@ -678,7 +765,7 @@ orb_status finish_subtree_levels(orb_ctx *ctx, Level v, const std::vector<LevelD
     });
     if (st != ORB_OK) return st;
     ORB_CUDA(cudaEventRecord(ctx->ev[1], ctx->stream));
-    return ORB_OK;
+    return queue_tree(ctx, out);
 }
 
 }  // namespace
@@ -806,6 +893,7 @@ orb_status orb_ctx_destroy(orb_ctx *ctx) {
     ctx->cmp_off.release(); ctx->cmp_cnt.release(); ctx->cmp_keys.release(); ctx->cmp_pos.release();
     if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
     if (ctx->h_sub_flag) cudaFreeHost(ctx->h_sub_flag);
+    if (ctx->h_tree) cudaFreeHost(ctx->h_tree);
     if (ctx->h_win) cudaFreeHost(ctx->h_win);
     ctx->win_cnt.release();
     collect_profile(ctx);
@@ -1086,10 +1174,12 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
         return ORB_OK;
     };
     ORB_CUDA(cudaEventRecord(ctx->ev[1], s));
+    if (!dev && perm) touch_pages(perm, n * sizeof(uint32_t));  // while the device builds
     bool streamed = false;
     if (windows && (st = stream_windows(&streamed)) != ORB_OK) return st;
     bool taken = false;  // the subtree kernel finished the tree
-    st = finish_subtree_levels(ctx, v, lv, key, &passes, sub_from, n, n, 0, &taken);
+    const TreeOut out = tree_out(ctx, heap, ranges, heap_cells);
+    st = finish_subtree_levels(ctx, v, lv, key, &passes, sub_from, n, n, 0, out, &taken);
     if (st != ORB_OK) return st;
     bool written = false;  // the particles are in the host arrays (or on their way there)
     if (!dev) {
@@ -1108,9 +1198,6 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     if (perm && n && !written)
         ORB_CUDA(cudaMemcpyAsync(perm, ctx->idx.p, n * sizeof(uint32_t),
                                  dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s));
-    ORB_CUDA(cudaMemcpyAsync(heap, ctx->heap.p, heap_cells * sizeof(orb_cell_t), cudaMemcpyDeviceToHost, s));
-    ORB_CUDA(cudaMemcpyAsync(ranges, ctx->ranges.p, heap_cells * sizeof(uint2), cudaMemcpyDeviceToHost, s));
-    ORB_CUDA(cudaMemcpyAsync(ctx->h_counters, ctx->counters.p, sizeof(BuildCounters), cudaMemcpyDeviceToHost, s));
     const bool on_cs = win_started;  // copies back on the copy stream
     if (on_cs && !written) {  // and some on the context stream after them: both timed
         ORB_CUDA(cudaEventRecord(ctx->ev[3], s));
@@ -1119,6 +1206,7 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     if (!dev) ORB_CUDA(cudaEventRecord(ctx->ev[3], on_cs ? ctx->copy_stream : s));
     ORB_CUDA(cudaStreamSynchronize(s));
     if (on_cs) ORB_CUDA(cudaStreamSynchronize(ctx->copy_stream));
+    take_tree(out);
     if (!build_finished(ctx, lv, taken ? (size_t)sub_from : lv.size()))
         return fail(ctx, ORB_ERR_TIMEOUT, kUnfinished);
     float dev_ms = 0.f;
@@ -1268,6 +1356,7 @@ orb_status orb_generate(orb_ctx *ctx, int kind, uint64_t seed, uint64_t n, float
     }
     ORB_CUDA(cudaGetLastError());
     if (!dev) {
+        for (void *p : {(void *)x, (void *)y, (void *)z}) touch_pages(p, n * sizeof(float));
         ORB_CUDA(cudaMemcpyAsync(x, dx, n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
         ORB_CUDA(cudaMemcpyAsync(y, dy, n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
         ORB_CUDA(cudaMemcpyAsync(z, dz, n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1302,9 +1391,8 @@ orb_status orb_load_particles(orb_ctx *ctx, const float *x, const float *y, cons
         ORB_CUDA(cudaMemcpyAsync(ctx->z.p, z, n * sizeof(float), k, s));
     }
     // identity permutation and range map {root = [0, n)} (src/services/init.cu:63-66)
-    std::vector<uint32_t> iota(n);
-    for (uint64_t i = 0; i < n; ++i) iota[i] = (uint32_t)i;
-    if (n) ORB_CUDA(cudaMemcpyAsync(ctx->idx.p, iota.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+    launch_iota_u32(ctx->idx.p, n, s);
+    ORB_CUDA(cudaGetLastError());
     ORB_CUDA(cudaMemsetAsync(ctx->ranges.p, 0, max_cells * sizeof(uint2), s));
     uint2 root = make_uint2(0u, (uint32_t)n);
     ORB_CUDA(cudaMemcpyAsync(ctx->ranges.p, &root, sizeof root, cudaMemcpyHostToDevice, s));
@@ -1327,6 +1415,8 @@ orb_status orb_store_particles(orb_ctx *ctx, float *x, float *y, float *z, uint3
     const cudaMemcpyKind k = (flags & ORB_DEVICE_POINTERS) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
     cudaStream_t s = ctx->stream;
     if (n) {
+        if (k == cudaMemcpyDeviceToHost)
+            for (void *p : {(void *)x, (void *)y, (void *)z, (void *)perm}) touch_pages(p, n * sizeof(float));
         ORB_CUDA(cudaMemcpyAsync(x, ctx->x.p, n * sizeof(float), k, s));
         ORB_CUDA(cudaMemcpyAsync(y, ctx->y.p, n * sizeof(float), k, s));
         ORB_CUDA(cudaMemcpyAsync(z, ctx->z.p, n * sizeof(float), k, s));
@@ -1375,15 +1465,16 @@ static orb_status service_prepare(orb_ctx *ctx, const orb_cell_t *cells, uint32_
     }
     // Each cell is placed at heap slot == id, so child slots are 2id+1 and 2id+2.
     if (n_cells) {
+        // (the plan kernel puts the cells at their slots: one copy, not one a cell)
         ORB_CUDA(cudaMemcpyAsync(ctx->slots.p, ids.data(), n_cells * sizeof(int), cudaMemcpyHostToDevice, s));
-        for (uint32_t i = 0; i < n_cells; ++i)
-            ORB_CUDA(cudaMemcpyAsync(ctx->heap.p + ids[i], cells + i, sizeof(orb_cell_t), cudaMemcpyHostToDevice, s));
+        ORB_CUDA(cudaMemcpyAsync(ctx->staging.p, cells, n_cells * sizeof(orb_cell_t), cudaMemcpyHostToDevice, s));
     }
     Level v = make_level(ctx, ctx->x.p, ctx->y.p, ctx->z.p);
     v.slots = ctx->slots.p;
     v.base = 0;
     v.C = (int)n_cells;
     v.plan_bins = 0;
+    v.cells_in = ctx->staging.p;
     *out = v;
     return ORB_OK;
 }
@@ -1687,8 +1778,10 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
     });
     if (st != ORB_OK) return st;
     ORB_CUDA(cudaEventRecord(ctx->ev[1], s));
+    if (!dev && perm) touch_pages(perm, n_total * sizeof(uint32_t));  // while the device builds
     bool taken = false;
-    st = finish_subtree_levels(ctx, v, lv, key, &passes, sub_from, n_total, max_n, hint_to, &taken);
+    const TreeOut out = tree_out(ctx, heaps, ranges, heap_cells);
+    st = finish_subtree_levels(ctx, v, lv, key, &passes, sub_from, n_total, max_n, hint_to, out, &taken);
     if (st != ORB_OK) return st;
     if (!dev) {
         ORB_CUDA(cudaStreamSynchronize(s));
@@ -1708,15 +1801,11 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
             ORB_CUDA(cudaMemcpyAsync(perm, ctx->idx.p, n_total * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         }
     }
-    if (heap_cells) {
-        ORB_CUDA(cudaMemcpyAsync(heaps, ctx->heap.p, heap_cells * sizeof(orb_cell_t), cudaMemcpyDeviceToHost, s));
-        ORB_CUDA(cudaMemcpyAsync(ranges, ctx->ranges.p, heap_cells * sizeof(uint2), cudaMemcpyDeviceToHost, s));
-    }
-    ORB_CUDA(cudaMemcpyAsync(ctx->h_counters, ctx->counters.p, sizeof(BuildCounters), cudaMemcpyDeviceToHost, s));
     if (!dev) ORB_CUDA(cudaEventRecord(ctx->ev[3], s));
     ORB_CUDA(cudaStreamSynchronize(s));
     if (!build_finished(ctx, lv, taken ? (size_t)sub_from : lv.size()))
         return fail(ctx, ORB_ERR_TIMEOUT, kUnfinished);
+    take_tree(out);
     // ranges relative to each instance (cells the build filled)
     for (uint32_t i = 0; i < k; ++i) {
         const uint64_t filled = Slices(inst[i].d).filled(lev[i]);

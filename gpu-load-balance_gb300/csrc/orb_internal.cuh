@@ -186,6 +186,7 @@ struct Level {
     int fuse;               // 1: the swap kernel finishes the cells (else k_part_finish)
     uint32_t done_start;    // what part_done starts from (0; the test hook's offset otherwise)
     uint32_t *out_counts;   // service calls: per-cell result
+    const orb_cell_t *cells_in;  // service calls: the cells, which k_plan puts at their slots
     uint32_t sparse_per_tile;  // a bracket of at most this many keys a count tile is listed
     int pdl;                // level kernels launched with programmatic dependent launch
     // warm builds (null otherwise): per heap slot the previous tree's cut and w x its extent
@@ -326,6 +327,9 @@ void launch_gen_xorshf96(const unsigned long long *starts, uint64_t draws, uint3
                          float *x, float *y, float *z, cudaStream_t st);
 void launch_gen_plummer(uint64_t seed, uint64_t n, const float *centres, const double *scales,
                         float *x, float *y, float *z, cudaStream_t st);
+
+// Makes the pages of a host buffer resident (its bytes keep their values), see orb_api.cu.
+void touch_pages(void *ptr, size_t bytes);
 
 // Context internals used by the request server (orb_server.cu).
 cudaStream_t ctx_stream(orb_ctx *ctx);

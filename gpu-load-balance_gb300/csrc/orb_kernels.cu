@@ -327,8 +327,13 @@ __global__ void __launch_bounds__(kThreads) k_plan(const __grid_constant__ Level
     const uint32_t lane = threadIdx.x & 31;
     if (c >= v.C) return;
     PlanCell p = {};
+    const int slot = level_slot(v, c);
+    if (v.cells_in) {
+        if (lane < 13)
+            reinterpret_cast<uint32_t *>(v.heap + slot)[lane] = reinterpret_cast<const uint32_t *>(v.cells_in + c)[lane];
+        __syncwarp();
+    }
     if (lane == 0) {
-        const int slot = level_slot(v, c);
         p = plan_cell(v, v.tot, v.small, c, slot, v.ranges[slot]);
     }
     p.c = c;
