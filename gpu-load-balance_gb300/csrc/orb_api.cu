@@ -562,8 +562,8 @@ uint32_t plan_bins(const orb_ctx *ctx, const Level &v, int C) { return !v.wt || 
 // half) all fit one CTA and that is at most kSubMaxLevels above the leaves
 // (tune.subtree_levels below its default: at most that many). As many levels as fit: a level
 // there takes 5-10 ps a particle where the level kernels take 7-12 (2^27 uniform, 2^26
-// clustered), and 20-30 us instead of 45 where the cells are few. full: every tree is built to
-// its leaves. from: the levels before it are level kernels' (staged builds).
+// clustered), and 20-30 us instead of 45 where the cells are few. full: every cell of every level
+// splits (batches: every tree is built to its leaves). from: the levels before it are level kernels' (staged builds).
 int subtree_from(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, uint64_t max_n, bool full, size_t from) {
     const uint32_t tuned = ctx->tune.subtree_levels;
     const uint32_t want = tuned < kSubDefaultLevels ? tuned : (uint32_t)kSubMaxLevels;
@@ -615,6 +615,7 @@ orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, u
             if (v.C == 0) break;
             v.skip = ctx->sub_flag.p;
             v.sub_list = ctx->sub_list.p;
+            v.sub_levels = v.slots ? 0 : (int)(lv.size() - li);  // (single builds: every cell alike)
             v.sub_wide = v.C <= ctx->num_sms ? 1 : 0;
             run_kernel(ctx, kKSubtreeCheck, v, 1, (int)(lv.size() - li));
             run_kernel(ctx, kKSubtree, v, std::min(v.C, ctx->num_sms));
@@ -1002,8 +1003,11 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     // runs on x and y while z arrives. Same cuts, same swaps: the result is the unstaged one.
     const float y_ext = upper[1] - lower[1], z_ext = upper[2] - lower[2];
     const bool staged = !dev && n && !weighted && ctx->use_stage && levels >= 2 && y_ext > 0.f && y_ext >= z_ext;
-    // subtrees finish complete unweighted trees only: d a power of two, built to its leaves
-    const int sub_from = subtree_from(ctx, lv, n, !weighted && sl.pow2 && levels == sl.depth, staged ? 2 : 0);
+    // subtrees split every cell of every level they take: not where a slice is partial (some
+    // leaf counts that are not powers of two), nor weighted builds
+    bool complete = !weighted;
+    for (uint32_t l = 1; l <= levels; ++l) complete = complete && (uint64_t)sl.count(l) == 1ull << (l - 1);
+    const int sub_from = subtree_from(ctx, lv, n, complete, staged ? 2 : 0);
     if (sub_from >= 0) {
         ORB_CUDA(ctx->sub_flag.ensure(1));
         ORB_CUDA(ctx->sub_list.ensure(4 * (size_t)lv[sub_from].C));

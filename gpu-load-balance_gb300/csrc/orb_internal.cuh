@@ -199,6 +199,7 @@ struct Level {
     // not attempted
     uint32_t *skip;
     int *sub_list;          // [4 C] the subtree kernel's cells by class
+    int sub_levels;         // levels below every cell (0: by its leaf count)
     int sub_wide;           // 1: all of a CTA's warps on every cell (levels of few cells)
     // window reports (null otherwise): the host-mapped reports, a finished-cell counter per
     // window, root cells per window

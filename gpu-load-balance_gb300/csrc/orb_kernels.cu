@@ -2693,6 +2693,7 @@ enum : uint32_t { kSubOpen = 0, kSubDone = 1, kSubWindow = 2, kSubCount = 3 };
 struct SubState {
     float L, R;          // the bisection's bracket
     float a, b;          // the window (kSubOpen: being narrowed; kSubWindow: classified)
+    float ratio;         // the test's share of the keys, leaf_ratio() of the cell
     uint32_t mode;       // kSubOpen, kSubWindow, kSubCount (counts every cut), kSubDone
     uint16_t it, found;
     uint32_t cand;       // keys in the window by the last histogram (~0: none yet)
@@ -2734,8 +2735,11 @@ static_assert(kSubBytes <= 232448, "a CTA's shared memory");
 static_assert(2 * sub_bytes<16>(kSub16) <= kSubBytes && 4 * sub_bytes<8>(kSub8) <= kSubBytes && 16 * sub_bytes<2>(kSub2) <= kSubBytes,
               "the smaller groups' slices");
 
-// Levels below a cell in a full build: log2 of its leaf count (d is a power of two).
-__device__ __forceinline__ int levels_below(int leaves) { return leaves > 1 ? 31 - __clz((uint32_t)leaves) : 0; }
+// Levels below a cell: the same for every cell of the level in a single build (v.sub_levels);
+// in a batch (powers of two, built to their leaves) log2 of its leaf count.
+__device__ __forceinline__ int levels_below(const Level &v, int leaves) {
+    return v.sub_levels ? v.sub_levels : (leaves > 1 ? 31 - __clz((uint32_t)leaves) : 0);
+}
 
 // Flag for k_subtree: every cell of the level fits a CTA and has at most `max_levels`
 // (<= kSubLevels) levels below it. Then the cells with levels below them, by class (all of
@@ -2749,7 +2753,7 @@ __global__ void __launch_bounds__(1024) k_subtree_check(const __grid_constant__ 
         const int slot = level_slot(v, c);
         const uint2 rg = v.ranges[slot];
         mx = max(mx, rg.y - rg.x);
-        ml = max(ml, (uint32_t)levels_below(v.heap[slot].nLeafCells));
+        ml = max(ml, (uint32_t)levels_below(v, v.heap[slot].nLeafCells));
     }
     mx = block_max(mx, sh);
     ml = block_max(ml, sh);
@@ -2918,7 +2922,7 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
         if (c < 0) break;
         const int root = sm.root, root_id = sm.cell[0][0].id;
         const uint32_t n = sm.cell[0][0].m, first = v.ranges[root].x;
-        const int levels = levels_below(sm.cell[0][0].leaves);
+        const int levels = levels_below(v, sm.cell[0][0].leaves);
         // heap slot of a descendant: slot - id is the instance's heap base
         const int heap0 = root - root_id;
         uint32_t off = begin_load(axis_keys(v, eff_axis(sm.cell[0][0].axis)) + first, n);  // the root's keys
@@ -2937,6 +2941,7 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
                 const int a = eff_axis(sc.axis);
                 s.L = s.a = sc.lower[a];  // setCutMargin, src/cell.h:123-126
                 s.R = s.b = sc.upper[a];
+                s.ratio = leaf_ratio(sc.leaves);  // src/orbit.cpp:204
                 s.mode = sc.m ? kSubOpen : kSubDone;  // no key: the first cut is found (count 0 of 0)
                 s.it = s.found = sc.m ? 0 : 1;
                 s.cand = 0xffffffffu;
@@ -3039,12 +3044,12 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
                         });
                     }
                     sync();
-                    // the bins of the ranks m/2 - 4 and m/2 + 4: a cut the test accepts has a count
-                    // within 3 of half the keys
+                    // the bins of the ranks 4 below and above ratio * m: a cut the test accepts has
+                    // a count within 3 of that
                     const uint32_t per = nb / (gs * 32u);
                     auto narrow = [&](uint32_t q, uint32_t j0, uint32_t run) {
                         SubState &s = sm.state[q];
-                        const uint32_t half = cells[q].m / 2u, r0 = half - 4u, r1 = half + 4u;
+                        const uint32_t target = (uint32_t)(s.ratio * (float)cells[q].m), r0 = target - 4u, r1 = target + 4u;
                         const float a = s.a, step = __fdiv_rn(__fsub_rn(s.b, a), (float)(nb - 1u));
                         for (uint32_t j = j0; j < j0 + per; ++j) {
                             const uint32_t h = sm.bins[q * nb + j];
@@ -3130,7 +3135,7 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
                             const uint32_t p = (uint32_t)j * 32u + lane;
                             kl[j] = p < m ? kf[order[cells[q].b + p]] : __int_as_float(0x7fc00000);  // NaN: never below
                         }
-                        const int st = bisect_list(kl, 0u, m, 0.5f, L, R, it);
+                        const int st = bisect_list(kl, 0u, m, s.ratio, L, R, it);
                         __syncwarp();
                         if (lane == 0) {
                             s.L = L;
@@ -3160,7 +3165,8 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
                         const uint32_t g = s.cnt - ((m & 31u) ? 32u - (m & 31u) : 0u);
                         const uint32_t below = m - g - nl;
                         // NaN keys are in g and never below a cut: count(< b) = below + nl all the same
-                        const bool low = convergence(below, m, 0.5f) < 0, high = convergence(below + nl, m, 0.5f) > 0;
+                        const float ratio = s.ratio;
+                        const bool low = convergence(below, m, ratio) < 0, high = convergence(below + nl, m, ratio) > 0;
                         const float a = s.a, b = s.b;
                         float kl[kSubWindowList / 32], L = s.L, R = s.R;
 #pragma unroll
@@ -3187,7 +3193,7 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
                                 uint32_t cc = 0;
 #pragma unroll
                                 for (int j = 0; j < (int)kSubWindowList / 32; ++j) cc += kl[j] < cut;
-                                dir = convergence(below + __reduce_add_sync(0xffffffffu, cc), m, 0.5f);
+                                dir = convergence(below + __reduce_add_sync(0xffffffffu, cc), m, ratio);
                             }
                             ++it;
                             if (dir == 0)
@@ -3245,7 +3251,7 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
                             SubState &s = sm.state[ti];
                             const float cut = mid_cut(s.L, s.R);
                             ++s.it;
-                            const int dir = convergence(s.cnt, cells[ti].m, 0.5f);
+                            const int dir = convergence(s.cnt, cells[ti].m, s.ratio);
                             if (dir == 0) {
                                 s.found = 1;
                                 s.mode = kSubDone;

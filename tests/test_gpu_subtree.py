@@ -13,13 +13,13 @@ pytestmark = pytest.mark.gpu
 SIZES = [33, 255, 257, 1088, 1089, 6656, 6657, 14848, 14849, 33023, 33024]
 
 
-def build_on_device(ctx, oracle, x, y, z, d):
+def build_on_device(ctx, oracle, x, y, z, d, levels=0):
     torch = pytest.importorskip("torch")
-    ref = oracle.build_tree(x, y, z, d)
+    ref = oracle.build_tree(x, y, z, d, levels=levels or None)
     dev = [torch.from_numpy(a.copy()).cuda() for a in (x, y, z)]
     perm = torch.empty(x.size, dtype=torch.int32, device="cuda")
     torch.cuda.synchronize()
-    res = ctx.build(*dev, d, perm=perm, device_pointers=True)
+    res = ctx.build(*dev, d, levels=levels, perm=perm, device_pointers=True)
     res.perm = perm.cpu().numpy().view(np.uint32)
     assert_same(res, ref, *(a.cpu().numpy() for a in dev))
 
@@ -28,8 +28,17 @@ def build_on_device(ctx, oracle, x, y, z, d):
 @pytest.mark.parametrize("n", SIZES)
 def test_one_cell_trees_match_oracle(ctx, oracle, kind, n):
     x, y, z = keys(kind, n, n + 1)
-    for d in (2, 16, 64):
+    for d in (2, 16, 64, 5, 50, 100):
         build_on_device(ctx, oracle, x, y, z, d)
+
+
+@pytest.mark.parametrize("d,levels", [(3, 0), (7, 0), (11, 0), (100, 3), (1000, 0), (1 << 10, 7), (96, 0)])
+def test_leaf_counts_and_level_bounds_match_oracle(ctx, oracle, d, levels):
+    """Leaf counts that are not powers of two (odd ratios in the test, partial slices that keep
+    the level kernels) and trees not built to their leaves."""
+    for n in (100, 30001, 200003):
+        x, y, z = oracle.gen_plummer(d + n, n)
+        build_on_device(ctx, oracle, x, y, z, d, levels)
 
 
 @pytest.mark.parametrize("cell", [300, 1087, 6650, 14840])
