@@ -187,9 +187,6 @@ bool is_device_ptr(const void *p) {
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
-// Levels of at most this many cells per SM send every cell through the count passes.
-constexpr int kCountCells = 1;
-
 }  // namespace
 
 namespace orb {
@@ -231,9 +228,8 @@ orb_status ensure_ptile_buffers(orb_ctx *ctx, uint64_t ptiles, uint64_t cells) {
 // Level buffers for up to `max_cells` cells per level over n particles.
 orb_status ensure_level_buffers(orb_ctx *ctx, uint64_t n, uint32_t max_cells, uint32_t heap_cells) {
     const uint64_t max_ptiles = n / kPTile + max_cells + 2;
-    // histogram cells of a level: cells of more than kTile particles, or every cell on levels of
-    // few or large cells (small_cells)
-    const uint64_t max_hist = n / kTile + (uint64_t)(kCountCells * ctx->num_sms) + 2;
+    // histogram cells of a level: cells of more than kTile particles
+    const uint64_t max_hist = n / kTile + 2;
     const uint64_t max_bins = max_hist << kMaxBinsLog2;
     ORB_CUDA(ctx->heap.ensure(heap_cells));
     ORB_CUDA(ctx->ranges.ensure(heap_cells));
@@ -251,8 +247,9 @@ orb_status ensure_level_buffers(orb_ctx *ctx, uint64_t n, uint32_t max_cells, ui
     ORB_CUDA(ctx->cmp_off.ensure(max_cells));
     ORB_CUDA(ctx->cmp_cnt.ensure(max_cells));
     ORB_CUDA(ctx->pred.ensure(max_cells));
-    // lists of bracket keys: at most max(2048, n/64) per histogram cell (list_capacity)
-    const uint64_t max_list = n / 64 + 2048ull * max_hist;
+    // lists of bracket keys: at most max(2048, n/64) of a cell of several tiles, an eighth of the
+    // keys of a smaller one (list_capacity)
+    const uint64_t max_list = n / 64 + 2048ull * max_hist + n / 8;
     ORB_CUDA(ctx->cmp_keys.ensure(max_list));
     ORB_CUDA(ctx->cmp_pos.ensure(max_list));
     ORB_CUDA(ctx->slots.ensure(max_cells));
@@ -542,20 +539,17 @@ struct LevelDesc {
     const int *child_map;
 };
 
-// Cells of at most this many particles take the one-tile bisection (a warp a cell) on a level
-// of C cells; larger ones the count passes. A level of large cells (one instance, more than
-// 4 tiles expected a cell) or of few cells sends every cell through the count passes: a warp
-// takes 36-42 us for a cell of 2^14 particles where the passes' CTAs take 10, so the
-// one-tile bisection pays only where its warps fill the GPU.
+// Cells of at most this many particles take the one-warp bisection on a level of C cells;
+// larger ones the count passes. Levels of few cells, or (one instance) of cells expected well
+// above that size, send every cell through the count passes and save that launch.
 uint32_t small_cells(const orb_ctx *ctx, const Level &v, uint64_t max_n, size_t li, int C) {
-    if (v.wt || C <= kCountCells * ctx->num_sms) return 0;
-    return !v.slots && (max_n >> li) > 4ull * kTile ? 0u : (uint32_t)kTile;
+    if (v.wt || C <= ctx->num_sms) return 0;
+    return !v.slots && (max_n >> li) > 4ull * kWarpKeys ? 0u : (uint32_t)kWarpKeys;
 }
 
-// Histogram bins for the cells planned for a level of C cells: those with count tiles, or
-// (weighted builds) those of several tiles, all of them on a level of few cells (whose tiles
-// are dealt in pieces).
-uint32_t plan_bins(const orb_ctx *ctx, const Level &v, int C) { return !v.wt || C <= ctx->num_sms ? 1u : 0u; }
+// Histogram bins for the cells planned for a level of C cells: those of several tiles, but all
+// of them on a weighted level of few cells, whose tiles are dealt in pieces.
+uint32_t plan_bins(const orb_ctx *ctx, const Level &v, int C) { return v.wt && C <= ctx->num_sms ? 2u : 1u; }
 
 // The level from which subtree CTAs finish the tree (-1: none): the first level whose cells
 // (at most max_n >> l particles plus a few per split: each split leaves a cell within 3 of

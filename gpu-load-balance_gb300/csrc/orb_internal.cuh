@@ -32,7 +32,7 @@ constexpr int kThreads = 256;
 #define ORB_HIST_BLOCKS_PER_SM 6
 #endif
 constexpr int kHistBlocksPerSm = ORB_HIST_BLOCKS_PER_SM;
-constexpr int kTileBlocksPerSm = 4;  // resident CTAs of the one-tile cell bisection
+constexpr int kTileBlocksPerSm = 4;  // resident CTAs of the one-warp cell bisection
 constexpr uint32_t kSubMaxParticles = 33024;  // largest cell one subtree CTA takes (2^15 + 256)
 // Warm builds: hints apply to the levels above the first one of at least two cells per SM whose
 // cells have at most this many particles and that is at most tune.subtree_levels above the
@@ -46,10 +46,10 @@ constexpr int kSubMaxLevels = 6;              // deepest tree one subtree CTA fi
 // than one tile; smaller cells are finished by the first).
 constexpr int kWPasses = 3;
 
-// kSmall: at most kWarpKeys keys (one warp bisects it); kOneTile: at most kTile keys (one CTA)
+// kSmall: at most kWarpKeys keys, one warp bisects it
 // kReady: its bracket holds few enough keys for a list: the classify pass lists them and
 // k_part_cells finishes the bisection on the list
-enum CellState : uint8_t { kActive = 0, kFound = 1, kCapped = 2, kSmall = 3, kOneTile = 4, kReady = 5 };
+enum CellState : uint8_t { kActive = 0, kFound = 1, kCapped = 2, kSmall = 3, kReady = 4 };
 constexpr int kWarpKeys = 1024;      // cells up to this size bisect in one warp's registers
 constexpr int kMaxLevels = 30;       // d is at most 2^30
 
@@ -142,14 +142,15 @@ struct Level {
     uint32_t depth;         // index of the level within the build (0: the root's)
     // the next level: its cells (0: none is planned), where a cell's children stand among
     // them (child_map[c] = 4 x index of the first child | bit per child in the level; null:
-    // 2c and 2c+1) and the cells the one-tile bisection takes there (up to small_next
+    // 2c and 2c+1) and the cells the one-warp bisection takes there (up to small_next
     // particles; larger ones get count tiles)
     int next_C;
     const int *child_map;
     const int *next_slots;  // heap slots of the next level's cells (null: implied)
     uint32_t small_next;
     uint32_t small;         // ... on this level (k_plan, k_init)
-    uint32_t plan_bins;     // 1: cells with count tiles get histogram bins and a list
+    uint32_t plan_bins;     // cells with count tiles get a list and, with several tiles, bins (1);
+                            // bins for all (2); neither (0)
     // plan
     PlanTotals *tot, *tot_next;
     uint32_t *tile_off;     // [C] first count tile of each cell

@@ -213,12 +213,12 @@ __device__ __forceinline__ TileRef tile_ref(const Level &v, uint32_t t) {
 }
 
 // Slots of a cell's list: a cell whose bracket holds at most that many keys is finished on
-// the list (sparse_per_tile a count tile; the lists of a level fit n/8 + n/64 slots and 2048
-// a cell).
+// the list (sparse_per_tile a count tile, at most an eighth of a one-tile cell's keys and
+// max(2048, n/64) of a larger one's, so that a level's lists have a bound: ensure_level_buffers).
 __device__ __forceinline__ uint32_t list_capacity(const Level &v, uint32_t n) {
     const unsigned long long want =
         (unsigned long long)v.sparse_per_tile * ((n + (uint32_t)kTile - 1) / (uint32_t)kTile);
-    return (uint32_t)min(want, (unsigned long long)max(2048u, n / 64));
+    return (uint32_t)min(want, (unsigned long long)(n <= (uint32_t)kTile ? n / 8 : max(2048u, n / 64)));
 }
 
 static_assert(kColdHistPasses * kMaxBinsLog2 >= kMaxIterations, "3 cold passes reach the cap");
@@ -276,17 +276,19 @@ __device__ PlanCell plan_cell(const Level &v, PlanTotals *tot, uint32_t small, i
     }
     v.ptile_off[c] = p.t0;
     v.tile_off[c] = p.h0;
-    // (weighted builds: bins for cells of several tiles, on levels of few cells for all; no list)
-    if (v.wt ? p.H > (v.plan_bins ? 0u : 1u) : p.H && v.plan_bins) {
+    if (p.H && v.plan_bins) {
+        // bins for cells of several tiles (one CTA reads a one-tile cell and keeps its bins in
+        // shared memory), for all where a tile is dealt in pieces; a list unless weighted
+        const unsigned long long bins = p.H > 1 || v.plan_bins > 1 ? 1ull : 0ull;
         const unsigned long long a =
-            atomicAdd(&tot->pools, (1ull << 32) | (v.wt ? 0ull : (unsigned long long)list_capacity(v, n)));
+            atomicAdd(&tot->pools, (bins << 32) | (v.wt ? 0ull : (unsigned long long)list_capacity(v, n)));
         v.hist_off[c] = (uint32_t)(a >> 32) << kMaxBinsLog2;
         v.cmp_off[c] = (uint32_t)a;
     }
     uint8_t st = kActive;
     uint32_t it = 0;
     if (n <= small && small) {
-        st = n <= (uint32_t)kWarpKeys ? kSmall : kOneTile;
+        st = kSmall;
     } else if (n == 0) {
         // no key: the first cut is found (src/orbit.cpp:204-213 with count 0)
         st = kFound;
@@ -1293,13 +1295,8 @@ __global__ void __launch_bounds__(kThreads, kHistBlocksPerSm) k_hist(const __gri
 }
 
 // ------------------------------------------------------------------------------------
-// Bisection of one-tile cells (kWarpKeys < n <= kTile keys): one warp per cell, the whole
-// reference loop (src/orbit.cpp:146-232) in one launch. Histogram rounds over the midpoint
-// tree of the current bracket (about 16 keys a bin, warp-private shared-memory bins) each
-// replay up to K iterations on the prefix counts; once the bracket holds at most
-// kListKeys keys they are gathered into registers and every remaining iteration is a
-// register count plus a warp sum. Every round streams the cell's keys (L2-resident after
-// the first).
+// Bisection of small cells (at most kWarpKeys keys): one warp per cell, the whole reference
+// loop (src/orbit.cpp:146-232) in one launch.
 // ------------------------------------------------------------------------------------
 constexpr int kWarpKeysPerLane = kWarpKeys / 32;
 
@@ -1369,167 +1366,16 @@ __device__ __forceinline__ void bisect_small(const Level &v, int c, uint32_t lan
     }
 }
 
-constexpr int kTileBinsLog2 = 9;
-constexpr int kTileBins = 1 << kTileBinsLog2;
-constexpr int kListPerLane = 8;     // bracket keys a lane can hold
-constexpr uint32_t kListKeys = 64;  // bracket size that switches to the register list
-
+// A warp a cell. (Cells of up to a whole tile took this kernel before, in histogram rounds of a
+// warp: 36-42 us a cell of 2^14 keys, 1.3 of the 11 ms of a batch of 128 instances; a CTA of the
+// count passes takes about 7.)
 __global__ void __launch_bounds__(kThreads, kTileBlocksPerSm) k_bisect_tile(const __grid_constant__ Level v) {
     pdl_enter();
     if (level_failed(v)) return;
-    __shared__ uint32_t s_bins[kThreads / 32][kTileBins];
-    __shared__ float s_edges[kThreads / 32][kTileBins + 1];
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t *bins = s_bins[warp];
-    float *edges = s_edges[warp];
+    const uint32_t lane = threadIdx.x & 31;
     const int nwarps = (int)(gridDim.x * (blockDim.x >> 5));
-    unsigned long long bytes = 0;
-    for (int c = (int)(blockIdx.x * (blockDim.x >> 5) + warp); c < v.C; c += nwarps) {
-        const uint8_t state = v.state[c];
-        if (state == kSmall) {
-            bisect_small(v, c, lane);
-            continue;
-        }
-        if (state != kOneTile) continue;
-        const int slot = level_slot(v, c);
-        orb_cell_t &cell = v.heap[slot];
-        const uint2 rg = v.ranges[slot];
-        const uint32_t n = rg.y - rg.x;
-        const float ratio = leaf_ratio(cell.nLeafCells);  // src/orbit.cpp:204
-        const float *keys = axis_keys(v, eff_axis(cell.cutAxis));
-        float L = cell.cutMarginLeft, R = cell.cutMarginRight;
-        uint32_t it = 0, cand = n;
-        int st = kActive;
-        bool warm = v.warm && v.warm[c];  // hinted bracket, checked by the first round
-        while (st == kActive) {
-            bytes += 4ull * n;
-            if (cand <= kListKeys) {
-                // the bracket's keys into registers (each lane keeps its own), keys below L
-                float kl[kListPerLane];
-                uint32_t nk = 0, below = 0;
-                bool over = false;
-                auto gather = [&](float k) {
-                    if (k < L) {
-                        ++below;
-                    } else if (k < R) {
-                        if (nk < (uint32_t)kListPerLane) {
-#pragma unroll
-                            for (int q = 0; q < kListPerLane; ++q)
-                                if (q == (int)nk) kl[q] = k;
-                        } else {
-                            over = true;
-                        }
-                        ++nk;
-                    }
-                };
-                visit_keys(keys, rg.x, rg.y, R, lane, 32, gather, each(gather));
-                if (!__any_sync(0xffffffffu, over)) {
-                    below = warp_sum(below);
-                    while (st == kActive) {
-                        if (it >= (uint32_t)kMaxIterations) {
-                            st = kCapped;
-                            break;
-                        }
-                        const float cut = mid_cut(L, R);
-                        uint32_t cnt = 0;
-#pragma unroll
-                        for (int q = 0; q < kListPerLane; ++q) cnt += (q < (int)nk) && kl[q] < cut;
-                        const uint32_t cl = below + warp_sum(cnt);
-                        ++it;
-                        const int dir = convergence(cl, n, ratio);
-                        if (dir == 0)
-                            st = kFound;
-                        else if (dir > 0)
-                            R = cut;
-                        else
-                            L = cut;
-                    }
-                    break;
-                }
-                // a lane met more than it can hold: one more histogram round instead
-            }
-            const int K = max(1, min(kTileBinsLog2, 28 - __clz(max(cand, 1u))));
-            const uint32_t nb = 1u << K;
-            for (uint32_t j = lane; j < nb; j += 32) bins[j] = 0u;
-            fill_edges(edges, L, R, K, lane, 32);
-            __syncwarp();
-            const float scale = __fdiv_rn((float)nb, __fsub_rn(R, L));
-            const Guess gs = make_guess(L, R, scale, nb);
-            const int top = (int)nb - 1;
-            uint32_t below = 0;
-            auto one = [&](float k) {
-                if (k < L)
-                    ++below;
-                else if (k < R)
-                    atomicAdd(&bins[fast_bin(k, gs, top, edges)], 1u);
-            };
-            visit_keys(keys, rg.x, rg.y, R, lane, 32, one, each(one));
-            __syncwarp();
-            below = warp_sum(below);
-            // exclusive prefix of the bins in place (each lane its own run of bins)
-            const uint32_t per = max(1u, nb >> 5), j0 = lane * per, j1 = min(nb, j0 + per);
-            uint32_t loc = 0;
-            for (uint32_t j = j0; j < j1; ++j) loc += bins[j];
-            uint32_t tot;
-            uint32_t run = warp_excl_scan(loc, &tot);
-            for (uint32_t j = j0; j < j1; ++j) {
-                const uint32_t h = bins[j];
-                bins[j] = run;
-                run += h;
-            }
-            __syncwarp();
-            if (warm) {
-                warm = false;
-                if (!warm_bracket_holds(below, below + tot, n, ratio)) {  // restart on the extent
-                    const int a = eff_axis(cell.cutAxis);
-                    L = cell.lower[a];
-                    R = cell.upper[a];
-                    cand = n;
-                    if (lane == 0) atomicAdd(&v.counters->warm_resets, 1u);
-                    __syncwarp();
-                    continue;
-                }
-            }
-            // replay up to K iterations (identically in every lane)
-            uint32_t pos = 0, width = nb;
-            for (int step = 0; step < K; ++step) {
-                if (it >= (uint32_t)kMaxIterations) {
-                    st = kCapped;
-                    break;
-                }
-                const uint32_t half = width >> 1;
-                const uint32_t cl = below + bins[pos + half];
-                ++it;
-                const int dir = convergence(cl, n, ratio);
-                if (dir == 0) {
-                    st = kFound;
-                    break;
-                }
-                const float cut = mid_cut(L, R);
-                if (dir > 0) {
-                    R = cut;
-                } else {
-                    L = cut;
-                    pos += half;
-                }
-                width = half;
-            }
-            if (st == kActive && it >= (uint32_t)kMaxIterations) st = kCapped;
-            if (st == kActive) cand = (pos + 1 < nb ? bins[pos + 1] : tot) - bins[pos];
-            __syncwarp();  // the bins are rewritten by the next round
-        }
-        if (lane == 0) {
-            cell.cutMarginLeft = L;
-            cell.cutMarginRight = R;
-            cell.foundCut = st == kFound ? 1 : 0;
-            v.iters[c] = (uint8_t)it;
-            v.state[c] = (uint8_t)st;
-            if (v.warm) v.warm[c] = 0;
-            atomicMax(&v.counters->max_iters, it);
-            if (st == kCapped) atomicAdd(&v.counters->unfound, 1u);
-        }
-    }
-    if (lane == 0 && bytes) add_bytes(v, kKBisectTile, bytes);
+    for (int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); c < v.C; c += nwarps)
+        if (v.state[c] == kSmall) bisect_small(v, c, lane);
 }
 
 // ------------------------------------------------------------------------------------

@@ -49,3 +49,12 @@ def test_many_listed_keys_in_one_cell(tuned, oracle):
     for n in ((1 << 22) + 3, 300001):
         x, y, z = keys("uniform", n, n)
         run_both(tuned, oracle, x, y, z, 8)
+
+
+@pytest.mark.parametrize("n", [256 * 1024 - 7, 256 * 1024 + 300, 256 * 4096 + 5, 256 * 16384 + 300])
+def test_many_cells_about_a_warp_and_a_tile(tuned, oracle, n):
+    """256 cells of 1024 keys (the most a warp bisects) and of 16384 (a count tile), and a few
+    more or less."""
+    x, y, z = keys("narrow", n, n)
+    tuned.set_tuning(subtree_levels=0)
+    run_both(tuned, oracle, x, y, z, 512)
