@@ -221,7 +221,8 @@ orb_status ensure_ptile_buffers(orb_ctx *ctx, uint64_t ptiles, uint64_t cells) {
     ORB_CUDA(ctx->pt_le.ensure(ptiles));
     ORB_CUDA(ctx->pt_ge_pre.ensure(ptiles + 1));
     ORB_CUDA(ctx->pt_le_pre.ensure(ptiles + 1));
-    ORB_CUDA(ctx->swap_list.ensure(ptiles + cells));  // left tiles, or one empty item a cell
+    // the pieces of the left tiles (few of them are split, see partition_level), or one empty item a cell
+    ORB_CUDA(ctx->swap_list.ensure(ptiles + cells + 4ull * ctx->num_sms * swap_blocks_per_sm()));
     return ORB_OK;
 }
 
@@ -499,13 +500,16 @@ void partition_level(orb_ctx *ctx, Level v, uint64_t n, bool do_split) {
     // at most one swap tile a CTA (about half of the tiles hold left elements): the swap also
     // finishes the cells
     v.fuse = tiles <= 2 * swap_ctas ? 1 : 0;
+    // few tiles: the pairs of each in 2 or 4 CTAs as far as the GPU holds them at once (2^20
+    // particles, 128 left tiles: 27 -> 20 us a level, most of it the chains of loads a CTA waits for)
+    v.piece_log2 = 2 * tiles <= swap_ctas ? 2 : (tiles <= swap_ctas ? 1 : 0);
     run_kernel(ctx, kKPartClassify, v, (int)std::min<uint64_t>(pass_grid(ctx), tiles / (kThreads / 32) + 1));
     run_kernel(ctx, kKPartCells, v, ctx->num_sms);
     if (ctx->yz_pending) {  // the first kernel that reads y and z
         cudaStreamWaitEvent(ctx->stream, ctx->yz_ready, ctx->capturing ? cudaEventWaitExternal : 0);
         ctx->yz_pending = false;
     }
-    run_kernel(ctx, kKPartSwap, v, (int)std::min<uint64_t>(swap_ctas, tiles), do_split ? 1 : 0);
+    run_kernel(ctx, kKPartSwap, v, (int)std::min<uint64_t>(swap_ctas, tiles << v.piece_log2), do_split ? 1 : 0);
     if (!v.fuse) run_kernel(ctx, kKPartFinish, v, ctx->num_sms, do_split ? 1 : 0);
 }
 
@@ -519,11 +523,14 @@ orb_status run_bisection(orb_ctx *ctx, Level v, uint64_t n, uint32_t *passes, in
     const int npasses = first == 1 ? kColdHistPasses : kHistPasses;
     const uint64_t tiles = n / kTile + (uint64_t)v.C;
     v.last_pass = npasses - 1;
+    // few tiles: larger CTAs, at most one tile each (a level of 2^20 particles, 64 tiles: 15.4 ->
+    // 12.3 us with 1024 threads; of 4.1 million, 250 tiles: 26 -> 19.5 us with 512)
+    v.hist_threads = tiles <= (uint64_t)ctx->num_sms ? 1024 : (tiles <= kHistBlocks512 * (uint64_t)ctx->num_sms ? 512 : kThreads);
+    if (first == 2) v.hist_threads = kThreads;
     for (int pass = 0; pass < npasses; ++pass) {
         v.pass = pass;
-        run_kernel(ctx, kKHist, v,
-                   (int)std::min<uint64_t>(ctx->num_sms * (uint64_t)ctx->tune.hist_blocks_per_sm, tiles),
-                   pass == 0 ? first : 0);
+        const uint64_t ctas = v.hist_threads == kThreads ? ctx->num_sms * (uint64_t)ctx->tune.hist_blocks_per_sm : tiles;
+        run_kernel(ctx, kKHist, v, (int)std::min(ctas, tiles), pass == 0 ? first : 0);
         ++*passes;
     }
     ORB_CUDA(cudaGetLastError());

@@ -32,6 +32,7 @@ constexpr int kThreads = 256;
 #define ORB_HIST_BLOCKS_PER_SM 6
 #endif
 constexpr int kHistBlocksPerSm = ORB_HIST_BLOCKS_PER_SM;
+constexpr int kHistBlocks512 = 3;  // ... and of its CTAs of 512 threads
 constexpr int kTileBlocksPerSm = 4;  // resident CTAs of the one-warp cell bisection
 constexpr uint32_t kSubMaxParticles = 33024;  // largest cell one subtree CTA takes (2^15 + 256)
 // Warm builds: hints apply to the levels above the first one of at least two cells per SM whose
@@ -149,6 +150,7 @@ struct Level {
     const int *next_slots;  // heap slots of the next level's cells (null: implied)
     uint32_t small_next;
     uint32_t small;         // ... on this level (k_plan, k_init)
+    uint32_t hist_threads;  // threads of a count pass's CTA (kThreads, 512 or 1024)
     uint32_t plan_bins;     // cells with count tiles get a list and, with several tiles, bins (1);
                             // bins for all (2); neither (0)
     // plan
@@ -182,7 +184,9 @@ struct Level {
     uint32_t *pt_ge_pre;    // [ptiles] exclusive prefix within the cell
     uint32_t *pt_le_pre;
     CellPart *part;         // [C]
-    uint2 *swap_list;       // [ptiles] (cell, tile within the cell) of the swap's tiles
+    uint2 *swap_list;       // [ptiles + cells] (cell, piece within the cell) of the swap's work: the
+                            // tiles with left elements, each in 2^piece_log2 pieces
+    uint32_t piece_log2;
     uint32_t *part_done;    // [C] tiles swapped
     int fuse;               // 1: the swap kernel finishes the cells (else k_part_finish)
     uint32_t done_start;    // what part_done starts from (0; the test hook's offset otherwise)

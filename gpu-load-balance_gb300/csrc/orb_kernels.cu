@@ -21,6 +21,7 @@
 // the subtree kernel (one CTA finishes a cell's last levels with its particles in L2), the
 // optional sampled first pass, the service count-left, seeded generators and the batched
 // and served forms' helpers.
+#include <type_traits>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -259,32 +260,40 @@ __device__ __forceinline__ void warm_start_cell(const Level &v, int c, int slot,
     v.warm[c] = w;
 }
 
-// One thread: plans cell c (heap slot `slot`, particles [rg.x, rg.y)) with the totals `tot`;
-// cells of at most `small` particles get no count tiles.
-__device__ PlanCell plan_cell(const Level &v, PlanTotals *tot, uint32_t small, int c, int slot, uint2 rg) {
+// The tiles of cell c of n particles (c < 0: none); cells of at most `small` particles get no
+// count tiles.
+__device__ __forceinline__ PlanCell plan_sizes(uint32_t small, int c, uint32_t n) {
     PlanCell p;
-    const uint32_t n = rg.y - rg.x;
     p.c = c;
-    p.T = (n + (uint32_t)kPTile - 1) / (uint32_t)kPTile;
-    p.H = n > small ? (n + (uint32_t)kTile - 1) / (uint32_t)kTile : 0u;
+    p.T = c < 0 ? 0u : (n + (uint32_t)kPTile - 1) / (uint32_t)kPTile;
+    p.H = c >= 0 && n > small ? (n + (uint32_t)kTile - 1) / (uint32_t)kTile : 0u;
     p.t0 = p.h0 = 0;
+    return p;
+}
+// Its share of the level's tiles (count << 32 | partition), and of the pools (bins << 32 | list):
+// bins for cells of several tiles (one CTA reads a one-tile cell and keeps its bins in shared
+// memory), for all where a tile is dealt in pieces; a list unless weighted.
+__device__ __forceinline__ unsigned long long plan_tiles(const PlanCell &p) {
+    return ((unsigned long long)p.H << 32) | (unsigned long long)p.T;
+}
+__device__ __forceinline__ unsigned long long plan_pools(const Level &v, const PlanCell &p, uint32_t n) {
+    if (!p.H || !v.plan_bins) return 0ull;
+    const unsigned long long bins = p.H > 1 || v.plan_bins > 1 ? 1ull : 0ull;
+    return (bins << 32) | (v.wt ? 0ull : (unsigned long long)list_capacity(v, n));
+}
+
+// The plan of a cell (heap slot `slot`) of n particles whose shares start at `tiles` and `pools`.
+__device__ __forceinline__ void plan_store(const Level &v, PlanCell &p, unsigned long long tiles,
+                                           unsigned long long pools, uint32_t small, int slot, uint32_t n) {
+    const int c = p.c;
     if (p.T) {
-        const unsigned long long a =
-            atomicAdd(&tot->tiles, ((unsigned long long)p.H << 32) | (unsigned long long)p.T);
-        p.t0 = (uint32_t)a;
-        p.h0 = (uint32_t)(a >> 32);
+        p.t0 = (uint32_t)tiles;
+        p.h0 = (uint32_t)(tiles >> 32);
     }
     v.ptile_off[c] = p.t0;
     v.tile_off[c] = p.h0;
-    if (p.H && v.plan_bins) {
-        // bins for cells of several tiles (one CTA reads a one-tile cell and keeps its bins in
-        // shared memory), for all where a tile is dealt in pieces; a list unless weighted
-        const unsigned long long bins = p.H > 1 || v.plan_bins > 1 ? 1ull : 0ull;
-        const unsigned long long a =
-            atomicAdd(&tot->pools, (bins << 32) | (v.wt ? 0ull : (unsigned long long)list_capacity(v, n)));
-        v.hist_off[c] = (uint32_t)(a >> 32) << kMaxBinsLog2;
-        v.cmp_off[c] = (uint32_t)a;
-    }
+    v.hist_off[c] = (uint32_t)(pools >> 32) << kMaxBinsLog2;
+    v.cmp_off[c] = (uint32_t)pools;
     uint8_t st = kActive;
     uint32_t it = 0;
     if (n <= small && small) {
@@ -311,6 +320,14 @@ __device__ PlanCell plan_cell(const Level &v, PlanTotals *tot, uint32_t small, i
         v.warm[c] = 0;
         if (v.plan_hint) warm_start_cell(v, c, slot, n);
     }
+}
+
+// One thread: plans cell c (heap slot `slot`, n particles) with the totals `tot`.
+__device__ PlanCell plan_cell(const Level &v, PlanTotals *tot, uint32_t small, int c, int slot, uint32_t n) {
+    PlanCell p = plan_sizes(small, c, n);
+    const unsigned long long ti = plan_tiles(p), po = plan_pools(v, p, n);
+    const unsigned long long a = ti ? atomicAdd(&tot->tiles, ti) : 0ull, b = po ? atomicAdd(&tot->pools, po) : 0ull;
+    plan_store(v, p, a, b, small, slot, n);
     return p;
 }
 
@@ -336,7 +353,8 @@ __global__ void __launch_bounds__(kThreads) k_plan(const __grid_constant__ Level
         __syncwarp();
     }
     if (lane == 0) {
-        p = plan_cell(v, v.tot, v.small, c, slot, v.ranges[slot]);
+        const uint2 rg = v.ranges[slot];
+        p = plan_cell(v, v.tot, v.small, c, slot, rg.y - rg.x);
     }
     p.c = c;
     p.t0 = __shfl_sync(0xffffffffu, p.t0, 0);
@@ -382,7 +400,7 @@ __global__ void k_init(const __grid_constant__ Level v, uint32_t n, float lo0, f
         v.ranges[0] = make_uint2(0u, n);
         BuildCounters z = {};
         *v.counters = z;
-        if (v.C) plan_cell(v, v.tot, v.small, 0, 0, make_uint2(0u, n));
+        if (v.C) plan_cell(v, v.tot, v.small, 0, 0, n);
     }
 }
 
@@ -411,7 +429,7 @@ __global__ void k_init_batch(const __grid_constant__ Level v, const BatchRoot *r
             const uint2 rg = make_uint2(r.offset, r.offset + r.n);
             v.ranges[r.heap_base] = rg;
             s_plan.c = -1;
-            if (r.cell >= 0) s_plan = plan_cell(v, v.tot, v.small, r.cell, (int)r.heap_base, rg);
+            if (r.cell >= 0) s_plan = plan_cell(v, v.tot, v.small, r.cell, (int)r.heap_base, r.n);
         }
         if (blockIdx.x == 0) {
             __syncthreads();
@@ -782,6 +800,7 @@ __device__ __forceinline__ void visit_keys(const float *keys, uint32_t e0, uint3
 // scaled guess into the CTA's shared bins (a key the guess does not settle counted in the
 // lane's spare bin and binned exactly right after its round). Rounds of kHistVec float4
 // loads a thread; the unaligned head and tail and a last partial round key by key.
+template <uint32_t NT>
 __device__ __forceinline__ void dense_tile(const float *keys, uint32_t e0, uint32_t e1, const Guess gs,
                                            uint32_t *s_hist, HistCell *hc, const float *s_edge) {
     const uint32_t ti = threadIdx.x;
@@ -795,16 +814,16 @@ __device__ __forceinline__ void dense_tile(const float *keys, uint32_t e0, uint3
     };
     const uintptr_t addr = reinterpret_cast<uintptr_t>(keys + e0);
     const uint32_t a0 = min(e1, e0 + (uint32_t)(((16u - (addr & 15u)) & 15u) >> 2));
-    for (uint32_t i = e0 + ti; i < a0; i += kThreads) one(__ldg(keys + i));
+    for (uint32_t i = e0 + ti; i < a0; i += NT) one(__ldg(keys + i));
     const uint32_t n4 = (e1 - a0) >> 2;
     const float4 *k4 = reinterpret_cast<const float4 *>(keys + a0);
     const float *kb = keys + a0;
     uint32_t j0 = 0;
 #pragma unroll 1
-    for (; j0 + kHistVec * kThreads <= n4; j0 += kHistVec * kThreads) {
+    for (; j0 + kHistVec * NT <= n4; j0 += kHistVec * NT) {
         float4 q[kHistVec];
 #pragma unroll
-        for (int u = 0; u < kHistVec; ++u) q[u] = __ldg(k4 + j0 + u * kThreads + ti);
+        for (int u = 0; u < kHistVec; ++u) q[u] = __ldg(k4 + j0 + u * NT + ti);
         uint32_t miss = 0;
 #pragma unroll
         for (int u = 0; u < kHistVec; ++u) {
@@ -820,17 +839,17 @@ __device__ __forceinline__ void dense_tile(const float *keys, uint32_t e0, uint3
         while (miss) {
             const uint32_t b = (uint32_t)__ffs(miss) - 1u;
             miss &= miss - 1u;
-            dense_exact(__ldg(kb + 4 * (j0 + (b >> 2) * kThreads + ti) + (b & 3u)), hc, s_hist, s_edge);
+            dense_exact(__ldg(kb + 4 * (j0 + (b >> 2) * NT + ti) + (b & 3u)), hc, s_hist, s_edge);
         }
     }
-    for (uint32_t j = j0 + ti; j < n4; j += kThreads) {
+    for (uint32_t j = j0 + ti; j < n4; j += NT) {
         const float4 q = __ldg(k4 + j);
         one(q.x);
         one(q.y);
         one(q.z);
         one(q.w);
     }
-    for (uint32_t i = a0 + (n4 << 2) + ti; i < e1; i += kThreads) one(__ldg(keys + i));
+    for (uint32_t i = a0 + (n4 << 2) + ti; i < e1; i += NT) one(__ldg(keys + i));
 }
 
 // A later pass's tile [e0, e1): keys below L counted in `below`, keys inside [L, R) binned by
@@ -838,6 +857,7 @@ __device__ __forceinline__ void dense_tile(const float *keys, uint32_t e0, uint3
 // or above R and NaN ignored. Same rounds as dense_tile; a key outside the bracket costs its
 // comparisons only (the dense loop would send each one through the exact path: clustered
 // cells' second passes ran at 1.7 TB/s that way).
+template <uint32_t NT>
 __device__ __forceinline__ void bracket_tile(const float *keys, uint32_t e0, uint32_t e1, const Guess gs, float L,
                                              float R, uint32_t &below, uint32_t *s_hist, const float *s_edge) {
     const uint32_t ti = threadIdx.x;
@@ -852,16 +872,16 @@ __device__ __forceinline__ void bracket_tile(const float *keys, uint32_t e0, uin
     };
     const uintptr_t addr = reinterpret_cast<uintptr_t>(keys + e0);
     const uint32_t a0 = min(e1, e0 + (uint32_t)(((16u - (addr & 15u)) & 15u) >> 2));
-    for (uint32_t i = e0 + ti; i < a0; i += kThreads) one(__ldg(keys + i));
+    for (uint32_t i = e0 + ti; i < a0; i += NT) one(__ldg(keys + i));
     const uint32_t n4 = (e1 - a0) >> 2;
     const float4 *k4 = reinterpret_cast<const float4 *>(keys + a0);
     const float *kb = keys + a0;
     uint32_t j0 = 0;
 #pragma unroll 1
-    for (; j0 + kHistVec * kThreads <= n4; j0 += kHistVec * kThreads) {
+    for (; j0 + kHistVec * NT <= n4; j0 += kHistVec * NT) {
         float4 q[kHistVec];
 #pragma unroll
-        for (int u = 0; u < kHistVec; ++u) q[u] = __ldg(k4 + j0 + u * kThreads + ti);
+        for (int u = 0; u < kHistVec; ++u) q[u] = __ldg(k4 + j0 + u * NT + ti);
         uint32_t miss = 0;
 #pragma unroll
         for (int u = 0; u < kHistVec; ++u) {
@@ -878,18 +898,18 @@ __device__ __forceinline__ void bracket_tile(const float *keys, uint32_t e0, uin
         while (miss) {
             const uint32_t b = (uint32_t)__ffs(miss) - 1u;
             miss &= miss - 1u;
-            const float k = __ldg(kb + 4 * (j0 + (b >> 2) * kThreads + ti) + (b & 3u));
+            const float k = __ldg(kb + 4 * (j0 + (b >> 2) * NT + ti) + (b & 3u));
             atomicAdd(&s_hist[near_bin(k, gs, s_edge, kHistBins - 1u)], 1u);
         }
     }
-    for (uint32_t j = j0 + ti; j < n4; j += kThreads) {
+    for (uint32_t j = j0 + ti; j < n4; j += NT) {
         const float4 q = __ldg(k4 + j);
         one(q.x);
         one(q.y);
         one(q.z);
         one(q.w);
     }
-    for (uint32_t i = a0 + (n4 << 2) + ti; i < e1; i += kThreads) one(__ldg(keys + i));
+    for (uint32_t i = a0 + (n4 << 2) + ti; i < e1; i += NT) one(__ldg(keys + i));
 }
 
 // ------------------------------------------------------------------------------------
@@ -1044,29 +1064,39 @@ __global__ void __launch_bounds__(kPickThreads) k_sample_pick(const __grid_const
 // keys fit a list: the classify pass lists them, k_part_cells goes on) or active for the next
 // pass. Fused here: as a kernel of its own behind every pass it took 9-10 us a launch, three
 // times a level, most of it launch and load latency.
+template <uint32_t NT>
 __device__ __noinline__ void resolve_cell(const Level &v, int c, const HistCell *hc, uint32_t *s_hist, uint32_t *s_red) {
-    static_assert(kHistBins == 8 * kThreads, "8 bins a thread");
+    constexpr uint32_t kPer = kHistBins / NT;  // bins a thread
+    static_assert(kPer == 2 || kPer == 4 || kPer == 8, "vector loads");
     const uint32_t tid = threadIdx.x;
-    uint4 a, b;
-    if (hc->whole) {
-        a = reinterpret_cast<const uint4 *>(s_hist)[2 * tid];
-        b = reinterpret_cast<const uint4 *>(s_hist)[2 * tid + 1];
-    } else {
-        uint4 *g4 = reinterpret_cast<uint4 *>(hc->gh) + 2 * tid;
-        a = __ldcg(g4);  // other CTAs' atomics: from L2
-        b = __ldcg(g4 + 1);
-        g4[0] = make_uint4(0u, 0u, 0u, 0u);
-        g4[1] = make_uint4(0u, 0u, 0u, 0u);
+    uint32_t h[kPer];
+    using Vec = typename std::conditional<kPer == 2, uint2, uint4>::type;
+    constexpr uint32_t kVecs = kPer * sizeof(uint32_t) / sizeof(Vec);
+#pragma unroll
+    for (uint32_t q = 0; q < kVecs; ++q) {
+        Vec a;
+        if (hc->whole) {
+            a = reinterpret_cast<const Vec *>(s_hist)[kVecs * tid + q];
+        } else {
+            Vec *g = reinterpret_cast<Vec *>(hc->gh) + kVecs * tid + q;
+            a = __ldcg(g);  // other CTAs' atomics: from L2
+            *g = Vec{};
+        }
+        h[q * kPer / kVecs] = a.x;
+        h[q * kPer / kVecs + 1] = a.y;
+        if constexpr (kPer > 2) {
+            h[q * 4 + 2] = a.z;
+            h[q * 4 + 3] = a.w;
+        }
     }
-    const uint32_t h[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     uint32_t loc = 0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) loc += h[j];
+    for (uint32_t j = 0; j < kPer; ++j) loc += h[j];
     uint32_t tot, unused;
     uint32_t run = block_excl_scan2(loc, 0u, s_red, &tot, &unused).x;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        s_hist[8 * tid + j] = run;
+    for (uint32_t j = 0; j < kPer; ++j) {
+        s_hist[kPer * tid + j] = run;
         run += h[j];
     }
     __syncthreads();
@@ -1160,8 +1190,8 @@ __device__ __noinline__ void resolve_cell(const Level &v, int c, const HistCell 
 constexpr uint32_t kHFirstDense = kHDense;
 constexpr uint32_t kHFirstSampled = kHDense | kHPred;
 constexpr uint32_t kHRest = kHDense | kHBracket;
-template <uint32_t Allowed>
-__global__ void __launch_bounds__(kThreads, kHistBlocksPerSm) k_hist(const __grid_constant__ Level v) {
+template <uint32_t Allowed, uint32_t NT>
+__global__ void __launch_bounds__(NT, NT == kThreads ? kHistBlocksPerSm : (NT == 512 ? kHistBlocks512 : 1)) k_hist(const __grid_constant__ Level v) {
     pdl_enter();
     __shared__ __align__(16) uint32_t s_hist[kHistBins + 32];  // + the dense loop's spare bins
     __shared__ float s_edge[kHistBins + 1];                    // the tree's edges
@@ -1196,7 +1226,7 @@ __global__ void __launch_bounds__(kThreads, kHistBlocksPerSm) k_hist(const __gri
         }
         if (!whole) {
             uint32_t *gh = s_hc.gh;
-            for (uint32_t b = threadIdx.x; b < kHistBins; b += kThreads) {
+            for (uint32_t b = threadIdx.x; b < kHistBins; b += NT) {
                 const uint32_t h = s_hist[b];
                 if (h) atomicAdd(&gh[b], h);
             }
@@ -1207,7 +1237,7 @@ __global__ void __launch_bounds__(kThreads, kHistBlocksPerSm) k_hist(const __gri
             }
         }
         __syncthreads();
-        if (s_hc.last) resolve_cell(v, cur, &s_hc, s_hist, s_red);
+        if (s_hc.last) resolve_cell<NT>(v, cur, &s_hc, s_hist, s_red);
         __syncthreads();  // s_hc and s_hist free for the next cell
         below = 0;
         ntiles = 0;
@@ -1254,8 +1284,8 @@ __global__ void __launch_bounds__(kThreads, kHistBlocksPerSm) k_hist(const __gri
                 s_hc.gs = make_guess(L, R, __fdiv_rn((float)kHistBins, __fsub_rn(R, L)), kHistBins);
             }
             __syncthreads();
-            for (uint32_t j = threadIdx.x; j < kHistBins; j += kThreads) s_hist[j] = 0u;
-            fill_edges(s_edge, s_hc.L, s_hc.R, kHistK, threadIdx.x, kThreads);
+            for (uint32_t j = threadIdx.x; j < kHistBins; j += NT) s_hist[j] = 0u;
+            fill_edges(s_edge, s_hc.L, s_hc.R, kHistK, threadIdx.x, NT);
             __syncthreads();
         }
         ++ntiles;
@@ -1268,7 +1298,7 @@ __global__ void __launch_bounds__(kThreads, kHistBlocksPerSm) k_hist(const __gri
             // binned afterwards, keys above it and NaN ignored
             const float pa = s_hc.pa, pb = s_hc.pb;
             auto key = [&](float k) { pred_key(k, &s_hc, s_hist, s_edge); };
-            scan_tile<kThreads>(
+            scan_tile<NT>(
                 keys, e0, e1, s_hc.R,
                 [&](float k) {
                     below += k < pa;
@@ -1282,11 +1312,11 @@ __global__ void __launch_bounds__(kThreads, kHistBlocksPerSm) k_hist(const __gri
                         key(k);
                 });
         } else if ((Allowed & kHBracket) && (mode & kHBracket)) {
-            bracket_tile(keys, e0, e1, s_hc.gs, s_hc.L, s_hc.R, below, s_hist, s_edge);
+            bracket_tile<NT>(keys, e0, e1, s_hc.gs, s_hc.L, s_hc.R, below, s_hist, s_edge);
         } else {
             // every key by the scaled guess (no range test: guess_bin fails keys outside
             // [L, R) and NaN, which dense_exact then counts or ignores)
-            dense_tile(keys, e0, e1, s_hc.gs, s_hist, &s_hc, s_edge);
+            dense_tile<NT>(keys, e0, e1, s_hc.gs, s_hist, &s_hc, s_edge);
         }
         if (threadIdx.x == 0) s_bytes += 4ull * (e1 - e0);
     }
@@ -1779,28 +1809,42 @@ __device__ uint32_t warp_select(const uint32_t *bits, const uint32_t *pre, uint3
 
 // (y or z null: that array is not moved at this level; builds from host memory reorder it
 // later through the permutation, see orb_build.) Read from L2: in the swap kernel other CTAs
-// wrote these particles.
+// wrote these particles. Every load is issued before the first store.
 __device__ __forceinline__ void swap_particles(const Level &v, uint32_t a, uint32_t b) {
+    float ya = 0.f, yb = 0.f, za = 0.f, zb = 0.f;
+    uint32_t ia = 0, ib = 0, wa = 0, wb = 0;
     const float xa = __ldcg(v.x + a), xb = __ldcg(v.x + b);
+    if (v.y) {
+        ya = __ldcg(v.y + a);
+        yb = __ldcg(v.y + b);
+    }
+    if (v.z) {
+        za = __ldcg(v.z + a);
+        zb = __ldcg(v.z + b);
+    }
+    if (v.idx) {
+        ia = __ldcg(v.idx + a);
+        ib = __ldcg(v.idx + b);
+    }
+    if (v.wt) {
+        wa = __ldcg(v.wt + a);
+        wb = __ldcg(v.wt + b);
+    }
     v.x[a] = xb;
     v.x[b] = xa;
     if (v.y) {
-        const float ya = __ldcg(v.y + a), yb = __ldcg(v.y + b);
         v.y[a] = yb;
         v.y[b] = ya;
     }
     if (v.z) {
-        const float za = __ldcg(v.z + a), zb = __ldcg(v.z + b);
         v.z[a] = zb;
         v.z[b] = za;
     }
     if (v.idx) {
-        const uint32_t ia = __ldcg(v.idx + a), ib = __ldcg(v.idx + b);
         v.idx[a] = ib;
         v.idx[b] = ia;
     }
     if (v.wt) {
-        const uint32_t wa = __ldcg(v.wt + a), wb = __ldcg(v.wt + b);
         v.wt[a] = wb;
         v.wt[b] = wa;
     }
@@ -1847,46 +1891,61 @@ __device__ __forceinline__ void split_cell(const orb_cell_t &cell, orb_cell_t &l
     set_axis_and_margin(lc, ctr);
 }
 
-// Final swap(i, n-1) of a partitioned cell (src/services/partition.cpp:52), its children's
-// ranges and (optionally) its children's cells.
-__device__ void finish_cell(const Level &v, int slot, uint32_t i, bool do_split) {
-    const orb_cell_t cell = v.heap[slot];
-    const uint2 rg = v.ranges[slot];
-    const uint32_t n = rg.y - rg.x;
+// What finishing cell c reads besides its split point; the swap's CTAs load it before their
+// last arrival (it does not change while the level's particles move).
+struct FinishIn {
+    orb_cell_t cell;
+    int slot;
+    int map;  // where the children stand in the next level (see Level::child_map)
+};
+__device__ __forceinline__ FinishIn finish_in(const Level &v, int c) {
+    FinishIn f;
+    f.slot = level_slot(v, c);
+    f.cell = v.heap[f.slot];
+    f.map = !v.next_C ? 0
+            : v.child_map ? v.child_map[c]
+                          : 8 * c + (2 * c < v.next_C ? 1 : 0) + (2 * c + 1 < v.next_C ? 2 : 0);
+    return f;
+}
+
+// One thread: the final swap(i, n-1) of partitioned cell c of the level
+// (src/services/partition.cpp:52), its children's ranges, (optionally) their cells, and their
+// plan for the next level. One chain of dependent accesses, which a level of few cells waits
+// for: both children's shares of the level's totals in one atomic each, issued ahead of the
+// swap's loads (4.7 us where the atomics and the arrays followed one another).
+struct Kids {
+    PlanCell p[2];
+};
+__device__ __noinline__ Kids finish_and_plan(const Level &v, const FinishIn &f, const CellPart &P, bool do_split) {
+    const uint32_t n = P.n, i = P.i, nk[2] = {i, n - i};
+    const int first = f.map >> 2;
+    Kids k;
+    unsigned long long ti[2], po[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        k.p[q] = plan_sizes(v.small_next, (f.map >> q) & 1 ? first + q : -1, nk[q]);
+        ti[q] = plan_tiles(k.p[q]);
+        po[q] = plan_pools(v, k.p[q], nk[q]);
+    }
+    const unsigned long long a = ti[0] + ti[1] ? atomicAdd(&v.tot_next->tiles, ti[0] + ti[1]) : 0ull;
+    const unsigned long long b = po[0] + po[1] ? atomicAdd(&v.tot_next->pools, po[0] + po[1]) : 0ull;
     if (i < n) {
-        if (i != n - 1) swap_particles(v, rg.x + i, rg.x + n - 1);
+        if (i != n - 1) swap_particles(v, P.b + i, P.b + n - 1);
     } else {
         atomicAdd(&v.counters->degenerate, 1u);
     }
     // children slots: slot - id is the instance's heap base
-    const int lslot = slot + cell.id + 1, rslot = slot + cell.id + 2;
-    v.ranges[lslot] = make_uint2(rg.x, rg.x + i);
-    v.ranges[rslot] = make_uint2(rg.x + i, rg.y);
-    if (!do_split) return;
-    orb_cell_t lc, rc;
-    split_cell(cell, lc, rc, v.counters);
-    v.heap[lslot] = lc;
-    v.heap[rslot] = rc;
-}
-
-// One thread: finish_cell for cell c of the level, its children planned for the next one.
-struct Kids {
-    PlanCell p[2];
-};
-__device__ __noinline__ Kids finish_and_plan(const Level &v, int c, uint32_t i, bool do_split) {
-    const int slot = level_slot(v, c);
-    const uint2 rg = v.ranges[slot];
-    const int id = v.heap[slot].id;
-    finish_cell(v, slot, i, do_split);
-    Kids k;
-    k.p[0].c = k.p[1].c = -1;
-    if (v.next_C) {
-        const int m = v.child_map ? v.child_map[c]
-                                  : 8 * c + (2 * c < v.next_C ? 1 : 0) + (2 * c + 1 < v.next_C ? 2 : 0);
-        const int first = m >> 2, lslot = slot + id + 1;
-        if (m & 1) k.p[0] = plan_cell(v, v.tot_next, v.small_next, first, lslot, make_uint2(rg.x, rg.x + i));
-        if (m & 2) k.p[1] = plan_cell(v, v.tot_next, v.small_next, first + 1, lslot + 1, make_uint2(rg.x + i, rg.y));
+    const int lslot = f.slot + f.cell.id + 1;
+    v.ranges[lslot] = make_uint2(P.b, P.b + i);
+    v.ranges[lslot + 1] = make_uint2(P.b + i, P.b + n);
+    if (do_split) {
+        orb_cell_t lc, rc;
+        split_cell(f.cell, lc, rc, v.counters);
+        v.heap[lslot] = lc;
+        v.heap[lslot + 1] = rc;
     }
+    if (k.p[0].c >= 0) plan_store(v, k.p[0], a, b, v.small_next, lslot, nk[0]);
+    if (k.p[1].c >= 0) plan_store(v, k.p[1], a + ti[0], b + po[0], v.small_next, lslot + 1, nk[1]);
     atomicAdd(&v.counters->done[v.depth], 1u);
     return k;
 }
@@ -2023,7 +2082,7 @@ __device__ void cell_split_point(const Level &v, int c, uint2 rg, uint32_t t0, u
         if (ge_tot > s) i = min(i, warp_select(v.ge_bits, v.pt_ge_pre, t0, t0 + T, s));
         if (s >= 1) i = min(i, warp_select(v.le_bits, v.pt_le_pre, t0, t0 + T, le_tot - s));
     }
-    const uint32_t left = s ? min(T, (i + (uint32_t)kPTile - 1) / (uint32_t)kPTile) : 1u;
+    const uint32_t left = s ? min(T, (i + (uint32_t)kPTile - 1) / (uint32_t)kPTile) << v.piece_log2 : 1u;
     uint32_t at = 0;
     if (lane == 0) {
         CellPart p;
@@ -2357,20 +2416,27 @@ __global__ void __launch_bounds__(kSwapThreads, ORB_SWAP_MIN_BLOCKS) k_part_swap
     __shared__ uint32_t posL[kPTile];
     __shared__ uint32_t posR[kPTile];
     __shared__ uint32_t sh[96];
+    __shared__ FinishIn s_in;
     const uint32_t total = v.tot->swaps;
     unsigned long long bytes = 0;  // pairs swapped by this CTA
     for (uint32_t w = blockIdx.x; w < total; w += gridDim.x) {
         const uint2 item = v.swap_list[w];
         const int c = (int)item.x;
         const CellPart P = v.part[c];
-        const uint32_t t0 = P.t0, t1 = t0 + P.T, t = t0 + item.y;
+        const uint32_t tile = item.y >> v.piece_log2, t0 = P.t0, t1 = t0 + P.T, t = t0 + tile;
         const uint32_t s = P.s, le_tot = P.le, b = P.b;
-        const uint32_t ka = s ? v.pt_ge_pre[t] : 0u;  // (a cell without pairs has one empty item)
-        const uint32_t kb = s ? max(ka, min(s, ka + v.pt_ge[t])) : 0u;
+        const uint32_t kt = s ? v.pt_ge_pre[t] : 0u;  // (a cell without pairs has one empty item)
+        uint32_t ka = kt, kb = s ? max(kt, min(s, kt + v.pt_ge[t])) : 0u;
+        if (v.piece_log2) {  // the item's share of the tile's pairs
+            const uint32_t per = ((kb - ka) + (1u << v.piece_log2) - 1u) >> v.piece_log2;
+            ka = min(kb, kt + (item.y - (tile << v.piece_log2)) * per);
+            kb = min(kb, ka + per);
+        }
         const uint32_t cnt = kb - ka;
+        if (kFuse && threadIdx.x == 0) s_in = finish_in(v, c);
         if (cnt) {
             // left elements: ranks [ka, kb) of this tile's >= mask, in order
-            emit_positions(v.ge_bits + (size_t)t * kPWords, ka, ka, kb, item.y * (uint32_t)kPTile, false, 0u,
+            emit_positions(v.ge_bits + (size_t)t * kPWords, kt, ka, kb, tile * (uint32_t)kPTile, false, 0u,
                            posL, sh);
             // right partners: left-to-right <= ranks [le_tot-kb, le_tot-ka); rank r pairs with
             // k = le_tot-1-r, stored at posR[k - ka] = posR[(le_tot-1-ka) - r]
@@ -2446,7 +2512,7 @@ __global__ void __launch_bounds__(kSwapThreads, ORB_SWAP_MIN_BLOCKS) k_part_swap
                 s_last = arrive_release(&v.part_done[c], 1u) + 1u == P.left;
                 if (s_last) {
                     acquire();
-                    s_kids = finish_and_plan(v, c, P.i, do_split != 0);
+                    s_kids = finish_and_plan(v, s_in, P, do_split != 0);
                 }
             }
             __syncthreads();
@@ -2480,7 +2546,8 @@ __global__ void __launch_bounds__(kThreads) k_part_finish(const __grid_constant_
     if (c < v.C && ti == 0) {
         const CellPart P = v.part[c];
         k.p[0].c = k.p[1].c = -1;
-        if (v.part_done[c] == P.left) k = finish_and_plan(v, c, P.i, do_split != 0);
+        const FinishIn in = finish_in(v, c);
+        if (v.part_done[c] == P.left) k = finish_and_plan(v, in, P, do_split != 0);
     }
     if (kPerCell)
         __syncthreads();
@@ -2726,15 +2793,22 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
         if (e > a)
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((uint32_t)(e - a)) : "memory");
     };
+    // A group takes its next cell while it works on one, unless there are no more cells than
+    // groups: the first groups to start then took two each, and the others, a few microseconds
+    // later, none (2^20 particles, 32 cells of 2^15 on 32 CTAs: 142 or 270 us).
+    const bool ahead = ncells > gridDim.x * (32 / NW);
     int next = -1;  // thread 0: the cell after this one
     bool started = false;
     for (;;) {
         if (ti == 0) {
             // this cell, and the next one, whose particles start their way into L2 meanwhile
-            if (!started) next = take();
+            if (NW == 32 && !ahead)
+                next = !started && blockIdx.x < ncells ? list[blockIdx.x] : -1;
+            else if (!started || !ahead)
+                next = take();
             started = true;
             sm.item = next;
-            if (next >= 0) {
+            if (ahead && next >= 0) {
                 next = take();
                 if (next >= 0) {
                     const uint2 r = v.ranges[level_slot(v, next)];
@@ -4078,12 +4152,14 @@ void launch_level_kernel(Kernel k, const Level &v, int grid, int arg, cudaStream
     switch (k) {
         case kKPlan: launch_kernel(p, k_plan, dim3(per_cell_warps), T, 0, st, v); break;
         case kKHist:  // arg: 1 first pass, all cells dense; 2 first pass of a sampled level
-            if (arg == 1)
-                launch_kernel(p, k_hist<kHFirstDense>, dim3(grid), T, 0, st, v);
-            else if (arg == 2)
-                launch_kernel(p, k_hist<kHFirstSampled>, dim3(grid), T, 0, st, v);
+            if (arg == 2)
+                launch_kernel(p, k_hist<kHFirstSampled, kThreads>, dim3(grid), T, 0, st, v);
+            else if (v.hist_threads == 1024)
+                launch_kernel(p, arg ? k_hist<kHFirstDense, 1024> : k_hist<kHRest, 1024>, dim3(grid), dim3(1024), 0, st, v);
+            else if (v.hist_threads == 512)
+                launch_kernel(p, arg ? k_hist<kHFirstDense, 512> : k_hist<kHRest, 512>, dim3(grid), dim3(512), 0, st, v);
             else
-                launch_kernel(p, k_hist<kHRest>, dim3(grid), T, 0, st, v);
+                launch_kernel(p, arg ? k_hist<kHFirstDense, kThreads> : k_hist<kHRest, kThreads>, dim3(grid), T, 0, st, v);
             break;
         case kKBisectTile: launch_kernel(p, k_bisect_tile, dim3(grid), T, 0, st, v); break;
         case kKSubtreeCheck: launch_kernel(p, k_subtree_check, dim3(1), dim3(1024), 0, st, v, arg); break;

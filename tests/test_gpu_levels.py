@@ -58,3 +58,11 @@ def test_many_cells_about_a_warp_and_a_tile(tuned, oracle, n):
     x, y, z = keys("narrow", n, n)
     tuned.set_tuning(subtree_levels=0)
     run_both(tuned, oracle, x, y, z, 512)
+
+
+@pytest.mark.parametrize("n", [1_240_003, 1_250_001, 2_480_001, 2_500_003, 7_450_001])
+def test_sizes_where_launch_shapes_change(tuned, oracle, n):
+    """A swap tile's pairs go to 4, 2 or 1 CTAs, a count tile to 1024, 512 or 256 threads."""
+    x, y, z = keys("ends", n, n)
+    tuned.set_tuning(subtree_levels=0)
+    run_both(tuned, oracle, x, y, z, 6)
