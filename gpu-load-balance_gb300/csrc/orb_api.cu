@@ -503,7 +503,8 @@ void partition_level(orb_ctx *ctx, Level v, uint64_t n, bool do_split) {
     // few tiles: the pairs of each in 2 or 4 CTAs as far as the GPU holds them at once (2^20
     // particles, 128 left tiles: 27 -> 20 us a level, most of it the chains of loads a CTA waits for)
     v.piece_log2 = 2 * tiles <= swap_ctas ? 2 : (tiles <= swap_ctas ? 1 : 0);
-    run_kernel(ctx, kKPartClassify, v, (int)std::min<uint64_t>(pass_grid(ctx), tiles / (kThreads / 32) + 1));
+    const int parts = tiles <= (uint64_t)pass_grid(ctx) ? 4 : 1;
+    run_kernel(ctx, kKPartClassify, v, (int)std::min<uint64_t>(pass_grid(ctx), tiles / (kThreads / 32 / parts) + 1), parts);
     run_kernel(ctx, kKPartCells, v, ctx->num_sms);
     if (ctx->yz_pending) {  // the first kernel that reads y and z
         cudaStreamWaitEvent(ctx->stream, ctx->yz_ready, ctx->capturing ? cudaEventWaitExternal : 0);

@@ -1614,6 +1614,9 @@ __device__ __forceinline__ float next_above(float c) {
 constexpr int kClassifyLoads = 16;
 constexpr uint32_t kListStage = 128;  // listed keys a warp stages before it appends them
 
+// kParts: warps a tile (consecutive ones of a CTA, each a run of its words). 4 on levels of few
+// tiles, where one warp's eight rounds of loads are all the launch lasts.
+template <int kParts>
 __global__ void __launch_bounds__(kThreads) k_part_classify(const __grid_constant__ Level v) {
     pdl_enter();
     if (blockIdx.x == 0 && threadIdx.x < 4) {
@@ -1634,7 +1637,10 @@ __global__ void __launch_bounds__(kThreads) k_part_classify(const __grid_constan
     uint32_t(*sw)[kPWords] = s_words[threadIdx.x >> 5];
     float *lkey = s_lkey[threadIdx.x >> 5];
     uint32_t *lpos = s_lpos[threadIdx.x >> 5];
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    constexpr int kWords = kPWords / kParts;  // mask words of a warp's part of a tile
+    const int part = kParts > 1 ? (int)(threadIdx.x >> 5) % kParts : 0, w_at = part * kWords;
+    __shared__ uint32_t s_cnt[kThreads / 32][2];
+    const uint32_t nwarps = gridDim.x * (kThreads / 32 / kParts), warp = (blockIdx.x * kThreads + threadIdx.x) / (32 * kParts);
     unsigned long long bytes = 0;
     // a run of consecutive tiles a warp: a cell's bracket and its staged keys stay with it
     const uint32_t t_end = (uint32_t)(total * (warp + 1) / nwarps);
@@ -1716,21 +1722,36 @@ __global__ void __launch_bounds__(kThreads) k_part_classify(const __grid_constan
         };
         if (m == (uint32_t)kPTile) {
 #pragma unroll 1
-            for (int r = 0; r < kPWords; r += kClassifyLoads) round(r, Flag<true>());
+            for (int r = w_at; r < w_at + kWords; r += kClassifyLoads) round(r, Flag<true>());
         } else {
 #pragma unroll 1
-            for (int r = 0; r < kPWords; r += kClassifyLoads) round(r, Flag<false>());
+            for (int r = w_at; r < w_at + kWords; r += kClassifyLoads) round(r, Flag<false>());
         }
         uint32_t *gw = v.ge_bits + (size_t)t * kPWords;
         uint32_t *lw = v.le_bits + (size_t)t * kPWords;
         __syncwarp();
 #pragma unroll
-        for (int q = 0; q < kPWords / 32; ++q) {
-            gw[q * 32 + lane] = sw[0][q * 32 + lane];
-            lw[q * 32 + lane] = sw[1][q * 32 + lane];
+        for (int q = 0; q < kWords / 32; ++q) {
+            gw[w_at + q * 32 + lane] = sw[0][w_at + q * 32 + lane];
+            lw[w_at + q * 32 + lane] = sw[1][w_at + q * 32 + lane];
         }
         __syncwarp();
-        if (lane == 0) {
+        if constexpr (kParts > 1) {
+            // the parts' counts (the tile's warps walk the same tiles)
+            const int bar = 1 + (int)(threadIdx.x / (32 * kParts)), w0 = (int)(threadIdx.x >> 5) - part;
+            if (lane == 0) {
+                s_cnt[threadIdx.x >> 5][0] = cg;
+                s_cnt[threadIdx.x >> 5][1] = cl;
+            }
+            asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(32 * kParts) : "memory");
+            cg = cl = 0;
+            for (int q = 0; q < kParts; ++q) {
+                cg += s_cnt[w0 + q][0];
+                cl += s_cnt[w0 + q][1];
+            }
+            asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(32 * kParts) : "memory");
+        }
+        if (lane == 0 && part == 0) {
             v.pt_ge[t] = cg;
             v.pt_le[t] = cl;
             bytes += 4ull * m + 8ull * kPWords + 8ull;
@@ -1772,39 +1793,61 @@ __device__ __forceinline__ uint32_t warp_last_at_most(const uint32_t *pre, uint3
     return lo;
 }
 
-// Position (cell-relative) of the set bit with in-cell rank `rank` among the bitmasks of
-// tiles [t0, t1), `pre` the cell's exclusive tile prefix (warp-cooperative; every lane
-// returns the answer). The masks are read from L2 (atomics may have set bits).
-__device__ uint32_t warp_select(const uint32_t *bits, const uint32_t *pre, uint32_t t0, uint32_t t1,
-                                uint32_t rank) {
+// Largest u in [lo, hi] with pre[u] <= r for two arrays at once, each as in warp_last_at_most:
+// the loads of a round are in flight together.
+__device__ __forceinline__ uint2 warp_last_at_most2(const uint32_t *pa, const uint32_t *pb, uint32_t lo, uint32_t hi,
+                                                    uint32_t ra, uint32_t rb) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t lo = warp_last_at_most(pre, t0, t1 - 1, rank);
-    const uint32_t r = rank - pre[lo];
+    uint2 l = make_uint2(lo, lo), h = make_uint2(hi, hi);
+    while (l.x < h.x || l.y < h.y) {
+        const uint32_t sa = (h.x - l.x + 31) / 32, sb = (h.y - l.y + 31) / 32;
+        const uint32_t ua = l.x + (lane + 1) * sa, ub = l.y + (lane + 1) * sb;
+        const uint32_t va = sa && ua <= h.x ? pa[ua] : 0xffffffffu, vb = sb && ub <= h.y ? pb[ub] : 0xffffffffu;
+        const bool oka = sa && ua <= h.x && va <= ra, okb = sb && ub <= h.y && vb <= rb;
+        l.x += (uint32_t)__popc(__ballot_sync(0xffffffffu, oka)) * sa;
+        l.y += (uint32_t)__popc(__ballot_sync(0xffffffffu, okb)) * sb;
+        if (sa) h.x = min(h.x, l.x + sa - 1);
+        if (sb) h.y = min(h.y, l.y + sb - 1);
+    }
+    return l;
+}
+
+// The smaller position (cell-relative; ~0: none) of two set bits among the masks of tiles
+// [t0, t1): the one of in-cell rank rg of the >= masks (if g), of rank rl of the <= masks (if l).
+// Warp-cooperative; every lane returns the answer. The masks are read from L2 (atomics may have
+// set bits). Both searches step by step together: one after the other they were a quarter of
+// k_part_cells' chain on levels of few cells.
+__device__ uint32_t warp_select2(const Level &v, uint32_t t0, uint32_t t1, bool g, uint32_t rg, bool l, uint32_t rl) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint2 at = warp_last_at_most2(v.pt_ge_pre, v.pt_le_pre, t0, t1 - 1, g ? rg : 0u, l ? rl : 0u);
     static_assert(kPWords == 128, "four mask words a lane");
-    const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(bits + (size_t)lo * kPWords) + lane);
-    const uint32_t words[4] = {q.x, q.y, q.z, q.w};
-    uint32_t cnt = 0;
+    const uint4 qg = __ldcg(reinterpret_cast<const uint4 *>(v.ge_bits + (size_t)at.x * kPWords) + lane);
+    const uint4 ql = __ldcg(reinterpret_cast<const uint4 *>(v.le_bits + (size_t)at.y * kPWords) + lane);
+    const uint32_t r[2] = {rg - v.pt_ge_pre[at.x], rl - v.pt_le_pre[at.y]}, tile[2] = {at.x, at.y};
+    const uint32_t words[2][4] = {{qg.x, qg.y, qg.z, qg.w}, {ql.x, ql.y, ql.z, ql.w}};
+    uint32_t pos = 0xffffffffu;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) cnt += __popc(words[j]);
-    uint32_t tot;
-    const uint32_t ex = warp_excl_scan(cnt, &tot);
-    const bool mine = r >= ex && r < ex + cnt;
-    uint32_t pos = 0;
-    if (mine) {
-        uint32_t rr = r - ex;
+    for (int k = 0; k < 2; ++k) {
+        uint32_t cnt = 0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t pc = __popc(words[j]);
-            if (rr < pc) {
-                pos = (lo - t0) * (uint32_t)kPTile + (lane * 4 + (uint32_t)j) * 32u +
-                      select_in_word(words[j], rr);
-                break;
+        for (int j = 0; j < 4; ++j) cnt += __popc(words[k][j]);
+        uint32_t tot;
+        const uint32_t ex = warp_excl_scan(cnt, &tot);
+        if ((k ? l : g) && r[k] >= ex && r[k] < ex + cnt) {
+            uint32_t rr = r[k] - ex;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t pc = __popc(words[k][j]);
+                if (rr < pc) {
+                    pos = min(pos, (tile[k] - t0) * (uint32_t)kPTile + (lane * 4 + (uint32_t)j) * 32u +
+                                       select_in_word(words[k][j], rr));
+                    break;
+                }
+                rr -= pc;
             }
-            rr -= pc;
         }
     }
-    const uint32_t who = __ballot_sync(0xffffffffu, mine);
-    return __shfl_sync(0xffffffffu, pos, __ffs(who) - 1);
+    return __reduce_min_sync(0xffffffffu, pos);
 }
 
 // (y or z null: that array is not moved at this level; builds from host memory reorder it
@@ -2079,8 +2122,7 @@ __device__ void cell_split_point(const Level &v, int c, uint2 rg, uint32_t t0, u
         const uint32_t upto = 0xffffffffu >> (31u - lane);
         s = max(min(wf, wg), min(wf + __popc(wa & upto), wg - __popc(wb & upto)));
         s = __reduce_max_sync(0xffffffffu, s);
-        if (ge_tot > s) i = min(i, warp_select(v.ge_bits, v.pt_ge_pre, t0, t0 + T, s));
-        if (s >= 1) i = min(i, warp_select(v.le_bits, v.pt_le_pre, t0, t0 + T, le_tot - s));
+        i = min(i, warp_select2(v, t0, t0 + T, ge_tot > s, s, s >= 1, le_tot - s));
     }
     const uint32_t left = s ? min(T, (i + (uint32_t)kPTile - 1) / (uint32_t)kPTile) << v.piece_log2 : 1u;
     uint32_t at = 0;
@@ -4167,7 +4209,7 @@ void launch_level_kernel(Kernel k, const Level &v, int grid, int arg, cudaStream
         case kKBisectCta:
             launch_kernel(p, k_bisect_cta, dim3(grid), dim3(kCtaThreads), kCtaSmemBytes, st, v);
             break;
-        case kKPartClassify: launch_kernel(p, k_part_classify, dim3(grid), T, 0, st, v); break;
+        case kKPartClassify: launch_kernel(p, arg == 4 ? k_part_classify<4> : k_part_classify<1>, dim3(grid), T, 0, st, v); break;
         case kKPartCells:
             // grid = the SM count: levels of few cells take large CTAs, several a cell
             if (v.C <= grid)
