@@ -796,13 +796,31 @@ __device__ __forceinline__ void visit_keys(const float *keys, uint32_t e0, uint3
     for (uint32_t i = a0 + (n4 << 2) + ti; i < e1; i += nt) visit(ld(keys + i));
 }
 
+// A dense pass's key, its guess corrected by the edges either side of it: exact while the guess
+// errs by less than a bin (bin_margin below 1; see make_guess for the form of the guess). Returns 1
+// for a key below L, which it does not bin.
+__device__ __forceinline__ uint32_t edges_key(float k, const Guess &gs, float R, uint32_t *s_hist, const float *s_edge) {
+    const uint32_t t = __float_as_uint(__fmaf_rn(__fsub_rn(k, gs.L), gs.scale, 2048.0f)) - 0x45000000u;
+    const uint32_t g = min(t >> 12, kHistBins - 1u);  // (a key outside [L, R): not used)
+    const float a = s_edge[g], b = s_edge[g + 1];
+    if (k >= gs.L && k < R) atomicAdd(&s_hist[g + (k >= b ? 1u : 0u) - (k < a ? 1u : 0u)], 1u);
+    return k < gs.L ? 1u : 0u;
+}
+
 // The dense pass's tile [e0, e1) in the first pass of a cold level: every key binned by the
 // scaled guess into the CTA's shared bins (a key the guess does not settle counted in the
-// lane's spare bin and binned exactly right after its round). Rounds of kHistVec float4
-// loads a thread; the unaligned head and tail and a last partial round key by key.
+// lane's spare bin and binned exactly right after its round). Where a round leaves a warp many
+// keys (many equal ones on an edge, or a cell thin for its distance from the origin) the warp
+// bins every key of the cell's later rounds by its guess and two edges (by_edges): 1.4 times a
+// clean round's time, where key by key a pass over 2^26 clustered particles took 160-300 us on
+// levels with such cells, 80 on the others. Rounds of kHistVec float4 loads a thread; the
+// unaligned head and tail and a last partial round key by key.
+constexpr uint32_t kByEdges = 32;  // many: more of a warp's 512
+constexpr int kEdgeVec = 2;        // float4 loads of a round by edges
 template <uint32_t NT>
 __device__ __forceinline__ void dense_tile(const float *keys, uint32_t e0, uint32_t e1, const Guess gs,
-                                           uint32_t *s_hist, HistCell *hc, const float *s_edge) {
+                                           uint32_t *s_hist, HistCell *hc, const float *s_edge, uint32_t &below,
+                                           bool &by_edges) {
     const uint32_t ti = threadIdx.x;
     const uint32_t spare = (gs.lim >> 12) + (ti & 31u);
     auto one = [&](float k) {
@@ -820,7 +838,7 @@ __device__ __forceinline__ void dense_tile(const float *keys, uint32_t e0, uint3
     const float *kb = keys + a0;
     uint32_t j0 = 0;
 #pragma unroll 1
-    for (; j0 + kHistVec * NT <= n4; j0 += kHistVec * NT) {
+    for (; !by_edges && j0 + kHistVec * NT <= n4; j0 += kHistVec * NT) {
         float4 q[kHistVec];
 #pragma unroll
         for (int u = 0; u < kHistVec; ++u) q[u] = __ldg(k4 + j0 + u * NT + ti);
@@ -836,10 +854,24 @@ __device__ __forceinline__ void dense_tile(const float *keys, uint32_t e0, uint3
                 if (!ok) miss |= 1u << (4 * u + c);
             }
         }
+        if (__reduce_add_sync(0xffffffffu, (uint32_t)__popc(miss)) > kByEdges) by_edges = gs.span != 0u;
         while (miss) {
             const uint32_t b = (uint32_t)__ffs(miss) - 1u;
             miss &= miss - 1u;
             dense_exact(__ldg(kb + 4 * (j0 + (b >> 2) * NT + ti) + (b & 3u)), hc, s_hist, s_edge);
+        }
+    }
+#pragma unroll 1
+    for (; by_edges && j0 + kEdgeVec * NT <= n4; j0 += kEdgeVec * NT) {
+        const float R = hc->R;
+        float4 q[kEdgeVec];
+#pragma unroll
+        for (int u = 0; u < kEdgeVec; ++u) q[u] = __ldg(k4 + j0 + u * NT + ti);
+#pragma unroll
+        for (int u = 0; u < kEdgeVec; ++u) {
+            const float kk[4] = {q[u].x, q[u].y, q[u].z, q[u].w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) below += edges_key(kk[c], gs, R, s_hist, s_edge);
         }
     }
     for (uint32_t j = j0 + ti; j < n4; j += NT) {
@@ -1212,6 +1244,7 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? kHistBlocksPerSm : (NT ==
     int cur = -1;         // the cell s_hc describes (every thread follows it)
     uint32_t ntiles = 0;  // the CTA's tiles of it so far
     uint32_t below = 0;   // this thread's keys below L in them
+    bool by_edges = false;  // (dense) the warp's keys by their edges, see dense_tile
     // the current cell's count below L and its shared bins to the global ones; then, with the
     // cell's last tile, its replay
     auto end_cell = [&]() {
@@ -1259,6 +1292,7 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? kHistBlocksPerSm : (NT ==
             }
             if (cur >= 0) end_cell();
             cur = c;
+            by_edges = false;
             if (threadIdx.x == 0) {
                 const int slot = level_slot(v, c);
                 const orb_cell_t &cell = v.heap[slot];
@@ -1316,7 +1350,7 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? kHistBlocksPerSm : (NT ==
         } else {
             // every key by the scaled guess (no range test: guess_bin fails keys outside
             // [L, R) and NaN, which dense_exact then counts or ignores)
-            dense_tile<NT>(keys, e0, e1, s_hc.gs, s_hist, &s_hc, s_edge);
+            dense_tile<NT>(keys, e0, e1, s_hc.gs, s_hist, &s_hc, s_edge, below, by_edges);
         }
         if (threadIdx.x == 0) s_bytes += 4ull * (e1 - e0);
     }

@@ -66,3 +66,20 @@ def test_sizes_where_launch_shapes_change(tuned, oracle, n):
     x, y, z = keys("ends", n, n)
     tuned.set_tuning(subtree_levels=0)
     run_both(tuned, oracle, x, y, z, 6)
+
+
+@pytest.mark.parametrize("width", [2.0**-6, 2.0**-9, 2.0**-10, 2.0**-14])
+@pytest.mark.parametrize("n", [70_001, 1 << 20])
+def test_thin_box_far_from_the_origin(tuned, oracle, n, width):
+    """Boxes whose bins are a few floats wide, with keys on their ends, outside them and NaN: a
+    warp's keys binned by guess alone, by guess and edges (margins below half a bin), by search."""
+    rng = np.random.default_rng(n)
+    x, y, z = (np.float32(0.3) + np.float32(width) * (rng.random((3, n), dtype=np.float32) - np.float32(0.01))).astype(np.float32)
+    hi = np.float32(0.3) + np.float32(width)
+    pick = rng.integers(0, 12, (3, n))
+    for a, p in zip((x, y, z), pick):
+        a[p == 0] = np.float32(0.3)
+        a[p == 1] = hi
+        a[(p == 2) & (rng.random(n) < 0.01)] = np.nan
+    tuned.set_tuning(subtree_levels=0)
+    run_both(tuned, oracle, x, y, z, 8, lower=(np.float32(0.3),) * 3, upper=(hi,) * 3)
