@@ -2662,13 +2662,15 @@ __global__ void __launch_bounds__(kThreads) k_part_finish(const __grid_constant_
 // its keys instead. Same cuts, same integer counts, same iterations on every path.
 //
 // A group is the CTA's 32 warps, or 16, 8 or 2 of them for smaller cells (by size): small
-// cells are bound by the latency of their steps, so an SM keeps 2, 4 or 16 in flight.
+// cells are bound by the latency of their steps, so an SM keeps 2, 4 or 16 in flight. (Cells of
+// 2^14, the common size above 2^8 particles a leaf: 2^26 clustered particles into 2^18, six
+// levels, 4.00 ms with one on an SM, 2.48 with two. So a group of 16 has half the bins, and the list
+// holds positions only.)
 // ------------------------------------------------------------------------------------
 constexpr int kSubLevels = kSubMaxLevels;
 constexpr int kSubCells = 1 << (kSubLevels - 1);  // cells of the deepest level split
 constexpr int kSubThreads = 1024;                 // of the CTA, one on an SM
 constexpr uint32_t kSubSpins = 1u << 20;           // polls of one copy's wait (each waits in hardware)
-constexpr uint32_t kSubDirect = 256;              // cells up to this size: one warp's registers
 constexpr uint32_t kSubWindowList = 256;          // most listed keys of a cell (8 a lane)
 
 struct SubCell {
@@ -2694,13 +2696,15 @@ struct SubState {
 
 template <int NW>
 struct SubSmem {
-    static constexpr uint32_t kBins = NW >= 16 ? 2048 : (NW == 8 ? 1024 : 256);   // a level's cells together
-    static constexpr uint32_t kLists = NW >= 16 ? 1024 : (NW == 8 ? 512 : 256);
+    // a level's cells together (16 warps: what two cells of 2^14 on an SM leave room for)
+    static constexpr uint32_t kBins = NW == 32 ? 2048 : (NW >= 8 ? 1024 : 256);
+    static constexpr uint32_t kLists = NW == 32 ? 1024 : (NW == 16 ? 1280 : (NW == 8 ? 512 : 256));
+    // cells up to this size: one warp's registers
+    static constexpr uint32_t kDirect = NW == 16 ? 768 : 256;
     SubCell cell[2][kSubCells];
     SubState state[kSubCells];
     uint32_t bins[kBins];
-    float lkey[kLists];
-    uint16_t lpos[kLists];
+    uint16_t lpos[kLists];  // the listed keys' positions within their cell
     uint32_t part[NW];
     uint32_t axes;    // axes the level's cells cut along
     uint32_t counted; // ... those of cells too large for one warp's registers
@@ -2718,10 +2722,9 @@ __host__ __device__ constexpr uint32_t sub_bytes(uint32_t nmax) {
     return ((uint32_t)((sizeof(SubSmem<NW>) + 15) / 16 * 16) + (nmax + 4) * 4 + sub_words(nmax) * 12 + nmax * 2 + 15) / 16 * 16;
 }
 // particles of a cell a group of 32, 16, 8, 2 warps takes
-constexpr uint32_t kSub32 = kSubMaxParticles, kSub16 = 14848, kSub8 = 6656, kSub2 = 1088;
-constexpr uint32_t kSubBytes = sub_bytes<32>(kSub32);
-static_assert(kSubBytes <= 232448, "a CTA's shared memory");
-static_assert(2 * sub_bytes<16>(kSub16) <= kSubBytes && 4 * sub_bytes<8>(kSub8) <= kSubBytes && 16 * sub_bytes<2>(kSub2) <= kSubBytes,
+constexpr uint32_t kSub32 = kSubMaxParticles, kSub16 = 16400, kSub8 = 6656, kSub2 = 1088;
+constexpr uint32_t kSubBytes = 232448;  // all of a CTA's shared memory
+static_assert(sub_bytes<32>(kSub32) <= kSubBytes && 2 * sub_bytes<16>(kSub16) <= kSubBytes && 4 * sub_bytes<8>(kSub8) <= kSubBytes && 16 * sub_bytes<2>(kSub2) <= kSubBytes,
               "the smaller groups' slices");
 
 // Levels below a cell: the same for every cell of the level in a single build (v.sub_levels);
@@ -2798,7 +2801,7 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
     unsigned char *const mem = sub_mem + slice;
     constexpr int kClass = NW == 32 ? 0 : (NW == 16 ? 1 : (NW == 8 ? 2 : 3));
     constexpr uint32_t NT = NW * 32, nmax = NW == 32 ? kSub32 : (NW == 16 ? kSub16 : (NW == 8 ? kSub8 : kSub2)), nwords = sub_words(nmax);
-    constexpr uint32_t kBins = SubSmem<NW>::kBins, kLists = SubSmem<NW>::kLists;
+    constexpr uint32_t kBins = SubSmem<NW>::kBins, kLists = SubSmem<NW>::kLists, kSubDirect = SubSmem<NW>::kDirect;
     constexpr int kU = 8;  // words of a warp in flight
     auto sync = [&]() {
         if (NW == 32)
@@ -2995,7 +2998,6 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
                     uint32_t at = atomicAdd(&sm.state[q].nlist, (uint32_t)__popc(e));
                     for (; e && at < lslots; e &= e - 1u, ++at) {
                         const uint32_t p = w * 32u + (uint32_t)__ffs(e) - 1u;
-                        sm.lkey[q * lslots + at] = kf[order[cells[q].b + p]];
                         sm.lpos[q * lslots + at] = (uint16_t)p;
                     }
                 }
@@ -3168,7 +3170,7 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
 #pragma unroll
                         for (int j = 0; j < (int)kSubWindowList / 32; ++j) {
                             const uint32_t e = (uint32_t)j * 32u + lane;
-                            kl[j] = e < nl ? sm.lkey[q * lslots + e] : __int_as_float(0x7fc00000);
+                            kl[j] = e < nl ? kf[order[cells[q].b + sm.lpos[q * lslots + e]]] : __int_as_float(0x7fc00000);
                         }
                         uint32_t it = 0;
                         int st = kActive;

@@ -76,3 +76,12 @@ def test_batch_of_every_class_matches_oracle(ctx, oracle, kind):
         assert np.array_equal(perm[o:e], ref.perm)
         for got, want in zip(b, (ref.x, ref.y, ref.z)):
             assert np.array_equal(got[o:e].view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("kind", ["uniform", "plummer", "narrow", "ends"])
+def test_two_cells_of_an_sm_match_oracle(ctx, oracle, kind):
+    """256 cells of about 16396 particles, on both sides of the most two cells of an SM can have,
+    six levels each (their descendants of 512 end in one warp's registers, those of 1025 do not)."""
+    n = 256 * 16396
+    x, y, z = oracle.gen_plummer(3, n) if kind == "plummer" else keys(kind, n, 3)
+    run_both(ctx, oracle, x, y, z, 256 * 64)
