@@ -3521,7 +3521,8 @@ __global__ void __launch_bounds__(kSubThreads) k_subtree(const __grid_constant__
 //
 // A cell whose tiles one CTA reads (all cells of at most one tile, but on levels of few cells)
 // is bisected to the end in one launch: up to kWDirect keys with the keys and weights in the
-// CTA's registers, every cut's weight summed (2.5 us a cell, against 12 with histograms),
+// CTA's registers, every cut's weight summed (2.5 us a cell of 2^11 keys, against 12 with
+// histograms; 4096 cells of 3900: 120 us, against 160),
 // more with the bins in shared memory. Larger cells take kWPasses launches, the CTA that brings
 // the last piece replaying; levels of few cells deal quarter tiles to the CTAs. A bin is two 32-bit sums, of the weights' low and high
 // halves (the high one is touched only by weights above 65535): shared memory has no 64-bit
@@ -3573,7 +3574,7 @@ __device__ __forceinline__ int weighted_depth(uint32_t n) {
     return max(4, min(kMaxBinsLog2, 30 - __clz(max(n, 1u))));
 }
 static_assert(kWPasses * kMaxBinsLog2 >= kMaxIterations, "the weighted passes reach the cap");
-constexpr uint32_t kWDirectPer = 8, kWDirect = kWDirectPer * kThreads;
+constexpr uint32_t kWDirect = 16 * kThreads;
 constexpr uint32_t kWFlush = 4;  // tiles whose low halves fit a 32-bit bin
 static_assert((unsigned long long)kWFlush * kTile * 0xffffull < (1ull << 32), "low halves of a run of tiles");
 
@@ -3676,16 +3677,17 @@ __device__ __noinline__ void weighted_replay(const Level &v, int c, bool global,
     __syncthreads();
 }
 
-// The whole loop of a cell of at most kWDirect keys by the CTA, keys and weights in registers.
+// The whole loop of a cell of at most kPer keys a thread by the CTA, keys and weights in registers.
+template <uint32_t kPer>
 __device__ __noinline__ void weighted_direct(const Level &v, int c, WeightSmem &sm) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     WeightCell &w = sm.cell;
     const int32_t leaves = v.heap[level_slot(v, c)].nLeafCells;
     const uint32_t n = w.end - w.base;
-    float k[kWDirectPer], L = w.L, R = w.R;
-    uint32_t x[kWDirectPer];
+    float k[kPer], L = w.L, R = w.R;
+    uint32_t x[kPer];
 #pragma unroll
-    for (int j = 0; j < (int)kWDirectPer; ++j) {
+    for (int j = 0; j < (int)kPer; ++j) {
         const uint32_t p = (uint32_t)j * kThreads + tid;
         k[j] = p < n ? __ldg(w.keys + w.base + p) : __int_as_float(0x7fc00000);  // NaN: never below
         x[j] = p < n ? __ldg(v.wt + w.base + p) : 0u;
@@ -3695,7 +3697,7 @@ __device__ __noinline__ void weighted_direct(const Level &v, int c, WeightSmem &
     auto below = [&](float cut, bool all) -> unsigned long long {
         uint32_t lo = 0, hi = 0;
 #pragma unroll
-        for (int j = 0; j < (int)kWDirectPer; ++j) {
+        for (int j = 0; j < (int)kPer; ++j) {
             const uint32_t y = all || k[j] < cut ? x[j] : 0u;
             lo += y & 0xffffu;
             hi += y >> 16;
@@ -3743,8 +3745,10 @@ __device__ __noinline__ void weighted_direct(const Level &v, int c, WeightSmem &
 
 __global__ void __launch_bounds__(kThreads, 4) k_whist(const __grid_constant__ Level v, uint32_t pieces) {
     pdl_enter();
-    if (level_failed(v)) return;
     __shared__ WeightSmem sm;
+    if (v.pass == 0 && level_failed(v)) return;
+    // every cell of the level finished in an earlier pass
+    if (v.pass > 0 && *(volatile uint32_t *)&v.counters->any_active[v.pass - 1] == 0u) return;
     WeightCell &w = sm.cell;
     const uint32_t tid = threadIdx.x;
     const uint32_t piece = (uint32_t)kTile / pieces;  // keys of a piece; `pieces` of them a tile
@@ -3837,6 +3841,20 @@ __global__ void __launch_bounds__(kThreads, 4) k_whist(const __grid_constant__ L
                     if (k[u] < L) below += x[u];
                 }
             }
+            if (gs.span) {  // each guess corrected by the edges either side of it, as in edges_key
+#pragma unroll
+                for (int u = 0; u < kLoads; ++u) {
+                    const uint32_t t = __float_as_uint(__fmaf_rn(__fsub_rn(k[u], gs.L), gs.scale, 2048.0f)) - 0x45000000u;
+                    const uint32_t g = min(t >> 12, top);
+                    const float a = sm.edge[g], b = sm.edge[g + 1];
+                    const uint32_t bin = g + (k[u] >= b ? 1u : 0u) - (k[u] < a ? 1u : 0u);
+                    if (k[u] >= L && k[u] < R) {
+                        atomicAdd(&sm.half[0][bin], x[u] & 0xffffu);
+                        if (x[u] >> 16) atomicAdd(&sm.half[1][bin], x[u] >> 16);
+                    }
+                }
+                continue;
+            }
 #pragma unroll
             for (int u = 0; u < kLoads; ++u)
                 if (k[u] >= L && k[u] < R && x[u]) add(k[u], x[u]);
@@ -3853,7 +3871,10 @@ __global__ void __launch_bounds__(kThreads, 4) k_whist(const __grid_constant__ L
         __syncthreads();
         bool last = true;
         if (direct) {
-            weighted_direct(v, cur, sm);
+            if (w.end - w.base <= 8 * kThreads)
+                weighted_direct<8>(v, cur, sm);
+            else
+                weighted_direct<16>(v, cur, sm);
         } else if (whole) {
             if (tid == 0 && first) {
                 w.below = below;
@@ -3898,7 +3919,10 @@ __global__ void __launch_bounds__(kThreads, 4) k_whist(const __grid_constant__ L
             v.hdone[cur] = 0;
             if (w.state != kActive) atomicMax(&v.counters->max_iters, w.it);
             if (w.state == kCapped) atomicAdd(&v.counters->unfound, 1u);
-            if (w.state == kActive && v.pass == v.last_pass) atomicExch(&v.counters->error, 1u);
+            if (w.state == kActive) {
+                v.counters->any_active[v.pass] = 1u;
+                if (v.pass == v.last_pass) atomicExch(&v.counters->error, 1u);
+            }
         }
         __syncthreads();  // the cell and its bins are free for the next one
         ntiles = 0;

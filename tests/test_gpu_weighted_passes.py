@@ -26,3 +26,12 @@ def test_weighted_many_small_cells(ctx, oracle):
     x, y, z = oracle.gen_plummer(5, n)
     w = np.random.default_rng(3).integers(1, 100, n).astype(np.uint32)
     check(ctx, oracle, x, y, z, w, 1 << 13)
+
+
+@pytest.mark.parametrize("n", [256 * 2048 + 99, 256 * 4096 - 99, 256 * 4096 + 99])
+def test_cells_a_cta_holds_match_oracle(ctx, oracle, n):
+    """256 cells about the most keys a CTA holds at 8 and at 16 a thread."""
+    rng = np.random.default_rng(n)
+    w = rng.integers(0, 1 << 17, n, dtype=np.uint64).astype(np.uint32)
+    for kind in ("uniform", "ends", "narrow"):
+        check(ctx, oracle, *keys(kind, n, n), w, 1 << 9)
