@@ -1884,47 +1884,20 @@ __device__ uint32_t warp_select2(const Level &v, uint32_t t0, uint32_t t1, bool 
     return __reduce_min_sync(0xffffffffu, pos);
 }
 
-// (y or z null: that array is not moved at this level; builds from host memory reorder it
-// later through the permutation, see orb_build.) Read from L2: in the swap kernel other CTAs
-// wrote these particles. Every load is issued before the first store.
-__device__ __forceinline__ void swap_particles(const Level &v, uint32_t a, uint32_t b) {
-    float ya = 0.f, yb = 0.f, za = 0.f, zb = 0.f;
-    uint32_t ia = 0, ib = 0, wa = 0, wb = 0;
-    const float xa = __ldcg(v.x + a), xb = __ldcg(v.x + b);
-    if (v.y) {
-        ya = __ldcg(v.y + a);
-        yb = __ldcg(v.y + b);
-    }
-    if (v.z) {
-        za = __ldcg(v.z + a);
-        zb = __ldcg(v.z + b);
-    }
-    if (v.idx) {
-        ia = __ldcg(v.idx + a);
-        ib = __ldcg(v.idx + b);
-    }
-    if (v.wt) {
-        wa = __ldcg(v.wt + a);
-        wb = __ldcg(v.wt + b);
-    }
-    v.x[a] = xb;
-    v.x[b] = xa;
-    if (v.y) {
-        v.y[a] = yb;
-        v.y[b] = ya;
-    }
-    if (v.z) {
-        v.z[a] = zb;
-        v.z[b] = za;
-    }
-    if (v.idx) {
-        v.idx[a] = ib;
-        v.idx[b] = ia;
-    }
-    if (v.wt) {
-        v.wt[a] = wb;
-        v.wt[b] = wa;
-    }
+// By a warp, a lane an array (y or z null: that array is not moved at this level; builds from host
+// memory reorder it later through the permutation, see orb_build). Read from L2: in the swap
+// kernel other CTAs wrote these particles.
+__device__ __forceinline__ void swap_particles(const Level &v, uint32_t a, uint32_t b, uint32_t lane) {
+    uint32_t *p = nullptr;
+    if (lane == 0) p = reinterpret_cast<uint32_t *>(v.x);
+    if (lane == 1) p = reinterpret_cast<uint32_t *>(v.y);
+    if (lane == 2) p = reinterpret_cast<uint32_t *>(v.z);
+    if (lane == 3) p = v.idx;
+    if (lane == 4) p = v.wt;
+    if (!p) return;
+    const uint32_t xa = __ldcg(p + a), xb = __ldcg(p + b);
+    p[a] = xb;
+    p[b] = xa;
 }
 
 __device__ void set_axis_and_margin(orb_cell_t &c, BuildCounters *ctr) {
@@ -1945,27 +1918,21 @@ __device__ void set_axis_and_margin(orb_cell_t &c, BuildCounters *ctr) {
     c.cutMarginRight = c.upper[a];
 }
 
-// The children of a cell at its cut: Cell::cut (src/cell.h:78-100) and src/orbit.cpp:238-246.
-__device__ __forceinline__ void split_cell(const orb_cell_t &cell, orb_cell_t &lc, orb_cell_t &rc,
-                                           BuildCounters *ctr) {
+// Child q of a cell at its cut: Cell::cut (src/cell.h:78-100) and src/orbit.cpp:238-246.
+__device__ __forceinline__ void split_child(const orb_cell_t &cell, int q, orb_cell_t &kid, BuildCounters *ctr) {
     const float cut = cell_cut(cell);
     const int a = eff_axis(cell.cutAxis);
     const int n_left = (cell.nLeafCells + 1) / 2;
-    lc.id = 2 * cell.id + 1;
-    rc.id = 2 * cell.id + 2;
-    lc.nLeafCells = n_left;
-    rc.nLeafCells = cell.nLeafCells - n_left;
-    lc.prevCutAxis = rc.prevCutAxis = cell.cutAxis;
-    lc.foundCut = rc.foundCut = 0;
-    lc.pad_[0] = lc.pad_[1] = lc.pad_[2] = 0;
-    rc.pad_[0] = rc.pad_[1] = rc.pad_[2] = 0;
+    kid.id = 2 * cell.id + 1 + q;
+    kid.nLeafCells = q ? cell.nLeafCells - n_left : n_left;
+    kid.prevCutAxis = cell.cutAxis;
+    kid.foundCut = 0;
+    kid.pad_[0] = kid.pad_[1] = kid.pad_[2] = 0;
     for (int k = 0; k < 3; ++k) {
-        lc.lower[k] = rc.lower[k] = cell.lower[k];
-        lc.upper[k] = rc.upper[k] = cell.upper[k];
-        if (k == a) lc.upper[k] = rc.lower[k] = cut;
+        kid.lower[k] = k == a && q ? cut : cell.lower[k];
+        kid.upper[k] = k == a && !q ? cut : cell.upper[k];
     }
-    set_axis_and_margin(rc, ctr);
-    set_axis_and_margin(lc, ctr);
+    set_axis_and_margin(kid, ctr);
 }
 
 // What finishing cell c reads besides its split point; the swap's CTAs load it before their
@@ -1985,46 +1952,48 @@ __device__ __forceinline__ FinishIn finish_in(const Level &v, int c) {
     return f;
 }
 
-// One thread: the final swap(i, n-1) of partitioned cell c of the level
+// One warp: the final swap(i, n-1) of partitioned cell c of the level
 // (src/services/partition.cpp:52), its children's ranges, (optionally) their cells, and their
-// plan for the next level. One chain of dependent accesses, which a level of few cells waits
-// for: both children's shares of the level's totals in one atomic each, issued ahead of the
-// swap's loads (4.7 us where the atomics and the arrays followed one another).
+// plan for the next level, lane q for child q. One chain of dependent accesses, which a level of
+// few cells waits for: both children's shares of the level's totals in one atomic each, issued
+// ahead of the swap's loads (one thread doing all of it, an access after the other, took 6 us).
 struct Kids {
     PlanCell p[2];
 };
-__device__ __noinline__ Kids finish_and_plan(const Level &v, const FinishIn &f, const CellPart &P, bool do_split) {
-    const uint32_t n = P.n, i = P.i, nk[2] = {i, n - i};
-    const int first = f.map >> 2;
-    Kids k;
-    unsigned long long ti[2], po[2];
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        k.p[q] = plan_sizes(v.small_next, (f.map >> q) & 1 ? first + q : -1, nk[q]);
-        ti[q] = plan_tiles(k.p[q]);
-        po[q] = plan_pools(v, k.p[q], nk[q]);
-    }
-    const unsigned long long a = ti[0] + ti[1] ? atomicAdd(&v.tot_next->tiles, ti[0] + ti[1]) : 0ull;
-    const unsigned long long b = po[0] + po[1] ? atomicAdd(&v.tot_next->pools, po[0] + po[1]) : 0ull;
+__device__ __noinline__ void finish_and_plan(const Level &v, const FinishIn &f, const CellPart &P, bool do_split, Kids &out) {
+    const uint32_t lane = threadIdx.x & 31u, n = P.n, i = P.i;
+    const int q = (int)(lane & 1u);
+    const uint32_t nq = q ? n - i : i;
+    PlanCell p = plan_sizes(v.small_next, (f.map >> q) & 1 ? (f.map >> 2) + q : -1, nq);
+    const unsigned long long ti = plan_tiles(p), po = plan_pools(v, p, nq);
+    const unsigned long long t0 = __shfl_sync(0xffffffffu, ti, 0), p0 = __shfl_sync(0xffffffffu, po, 0);
+    const unsigned long long ts = t0 + __shfl_sync(0xffffffffu, ti, 1), ps = p0 + __shfl_sync(0xffffffffu, po, 1);
+    unsigned long long at = 0;
+    if (lane == 0 && ts) at = atomicAdd(&v.tot_next->tiles, ts);
+    if (lane == 1 && ps) at = atomicAdd(&v.tot_next->pools, ps);
     if (i < n) {
-        if (i != n - 1) swap_particles(v, P.b + i, P.b + n - 1);
-    } else {
+        if (i != n - 1) swap_particles(v, P.b + i, P.b + n - 1, lane);
+    } else if (lane == 0) {
         atomicAdd(&v.counters->degenerate, 1u);
     }
     // children slots: slot - id is the instance's heap base
-    const int lslot = f.slot + f.cell.id + 1;
-    v.ranges[lslot] = make_uint2(P.b, P.b + i);
-    v.ranges[lslot + 1] = make_uint2(P.b + i, P.b + n);
-    if (do_split) {
-        orb_cell_t lc, rc;
-        split_cell(f.cell, lc, rc, v.counters);
-        v.heap[lslot] = lc;
-        v.heap[lslot + 1] = rc;
+    const int slot = f.slot + f.cell.id + 1 + q;
+    if (lane < 2) {
+        v.ranges[slot] = make_uint2(P.b + (q ? i : 0u), P.b + (q ? n : i));
+        if (do_split) {
+            orb_cell_t kid;
+            split_child(f.cell, q, kid, v.counters);
+            v.heap[slot] = kid;
+        }
     }
-    if (k.p[0].c >= 0) plan_store(v, k.p[0], a, b, v.small_next, lslot, nk[0]);
-    if (k.p[1].c >= 0) plan_store(v, k.p[1], a + ti[0], b + po[0], v.small_next, lslot + 1, nk[1]);
-    atomicAdd(&v.counters->done[v.depth], 1u);
-    return k;
+    const unsigned long long a = __shfl_sync(0xffffffffu, at, 0) + (q ? t0 : 0ull);
+    const unsigned long long b = __shfl_sync(0xffffffffu, at, 1) + (q ? p0 : 0ull);
+    if (lane < 2) {
+        if (p.c >= 0) plan_store(v, p, a, b, v.small_next, slot, nq);
+        out.p[q] = p;
+        if (lane == 0) atomicAdd(&v.counters->done[v.depth], 1u);
+    }
+    __syncwarp();
 }
 
 // P2: per cell: the bisection of a kReady cell finished on its list, the tile prefixes, the
@@ -2584,12 +2553,14 @@ __global__ void __launch_bounds__(kSwapThreads, ORB_SWAP_MIN_BLOCKS) k_part_swap
         if constexpr (kFuse) {
             __shared__ Kids s_kids;
             __shared__ bool s_last;
-            if (threadIdx.x == 0) {
-                s_last = arrive_release(&v.part_done[c], 1u) + 1u == P.left;
-                if (s_last) {
-                    acquire();
-                    s_kids = finish_and_plan(v, s_in, P, do_split != 0);
+            if (threadIdx.x < 32) {
+                uint32_t last = 0;
+                if (threadIdx.x == 0) {
+                    last = arrive_release(&v.part_done[c], 1u) + 1u == P.left ? 1u : 0u;
+                    s_last = last != 0;
+                    if (last) acquire();
                 }
+                if (__shfl_sync(0xffffffffu, last, 0)) finish_and_plan(v, s_in, P, do_split != 0, s_kids);
             }
             __syncthreads();
             if (s_last) {
@@ -2615,15 +2586,20 @@ __global__ void __launch_bounds__(kThreads) k_part_finish(const __grid_constant_
     pdl_enter();
     if (level_failed(v)) return;
     __shared__ Kids s_kids[kThreads / 32];
+    __shared__ FinishIn s_in[kThreads / 32];
     const uint32_t warp = threadIdx.x >> 5, nt = kPerCell ? kThreads : 32u;
     const uint32_t ti = kPerCell ? threadIdx.x : threadIdx.x & 31u;
     const int c = kPerCell ? (int)blockIdx.x : (int)(blockIdx.x * (kThreads / 32) + warp);
     Kids &k = s_kids[kPerCell ? 0 : warp];
-    if (c < v.C && ti == 0) {
+    if (c < v.C && ti < 32) {
         const CellPart P = v.part[c];
-        k.p[0].c = k.p[1].c = -1;
-        const FinishIn in = finish_in(v, c);
-        if (v.part_done[c] == P.left) k = finish_and_plan(v, in, P, do_split != 0);
+        const uint32_t done = v.part_done[c];
+        if (ti == 0) {
+            s_in[warp] = finish_in(v, c);
+            k.p[0].c = k.p[1].c = -1;
+        }
+        __syncwarp();
+        if (done == P.left) finish_and_plan(v, s_in[warp], P, do_split != 0, k);
     }
     if (kPerCell)
         __syncthreads();
@@ -3410,7 +3386,8 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
                     cell.upper[a] = sc.upper[a];
                 }
                 orb_cell_t kid[2];
-                split_cell(cell, kid[0], kid[1], v.counters);
+                split_child(cell, 0, kid[0], v.counters);
+                split_child(cell, 1, kid[1], v.counters);
 #pragma unroll
                 for (int w = 0; w < 2; ++w) {
                     const int slot = heap0 + kid[w].id;
