@@ -270,7 +270,7 @@ def check_parity(job):
 def effective_count_left(count_left: dict, kernels: dict, parity, peak: float):
     """The count-left aggregate's reference-equivalent rate: 4 B x the keys the reference's
     plain scan would read on the levels the count passes run, over their measured time. It
-    can exceed the peak: the engine reads far fewer keys (compaction, one pass bins several
+    can exceed the peak: the engine reads far fewer keys (lists, one pass bins several
     sweeps)."""
     if not parity or "ref_key_reads_per_level" not in parity or not count_left.get("ms_per_step"):
         return
@@ -445,7 +445,7 @@ def run_plain(ctx, E, torch, dev, args, kind: str, n: int, d: int, seed: int, pe
                   "peak_source": f"{peak_kind} hbm_gbs",
                   "timed": f"CUDA events around every count-left launch of {args.steps} steps "
                            "after the headline's timed region (same inputs and tuning)",
-                  "bytes": "4 B per key read + 4 B per key compacted (algorithmic, engine counters)",
+                  "bytes": "4 B per key read (algorithmic, engine counters)",
                   "excluded": "the bisection inside k_subtree (the last levels' bisection and "
                               "partition run fused in one kernel, timed as `subtree`)"
                               if "subtree" in warm else None}

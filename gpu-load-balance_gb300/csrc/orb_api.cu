@@ -564,7 +564,7 @@ uint32_t plan_bins(const orb_ctx *ctx, const Level &v, int C) { return v.wt && C
 // half) all fit one CTA and that is at most kSubMaxLevels above the leaves
 // (tune.subtree_levels below its default: at most that many). As many levels as fit: a level
 // there takes 5-10 ps a particle where the level kernels take 7-12 (2^27 uniform, 2^26
-// clustered), and 20-30 us instead of 45 where the cells are few. full: every cell of every level
+// clustered), and 20-30 us instead of 55 where the cells are few. full: every cell of every level
 // splits (batches: every tree is built to its leaves). from: the levels before it are level kernels' (staged builds).
 int subtree_from(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, uint64_t max_n, bool full, size_t from) {
     const uint32_t tuned = ctx->tune.subtree_levels;
@@ -587,8 +587,7 @@ size_t hint_levels(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, uint64_
 }
 
 // The reference's level loop (src/orbit.cpp:102-275) over every cell of every level: the
-// bisection (one warp for cells of at most one tile, the histogram passes for the rest, or one
-// CTA per cell), then the partition, which also splits the cells and plans the next level.
+// bisection (one warp for small cells, the histogram passes for the rest, or one CTA per cell), then the partition, which also splits the cells and plans the next level.
 // The first level's cells are planned by the init kernel.
 // sub_from >= 0: from level lv[sub_from] down, one CTA per cell finishes the tree when every
 // cell of that level fits one (k_subtree_check decides on the device).

@@ -17,8 +17,8 @@
 //   swap       the pairs; whoever finishes a cell's last tile does the final swap and the split
 //              (src/cell.h:78-126, src/orbit.cpp:235-250) and plans the children for the
 //              next level.
-// Beside them: the bisection of cells of at most one tile in one launch (a warp per cell),
-// the subtree kernel (one CTA finishes a cell's last levels with its particles in L2), the
+// Beside them: the bisection of small cells in one launch (a warp per cell), the subtree kernel
+// (a group of warps finishes a cell's last levels in shared memory), the
 // optional sampled first pass, the service count-left, seeded generators and the batched
 // and served forms' helpers.
 #include <type_traits>
@@ -2622,9 +2622,8 @@ __global__ void __launch_bounds__(kThreads) k_part_finish(const __grid_constant_
 // side by side, the group's warps divided evenly among them, all in step.
 //
 // Measured (GB300): the last four levels of 2^27 uniform particles into 2^16 leaves (cells of
-// 2^15) take 2.68 ms, against 3.88 ms for a CTA of 256 threads that moved the particles in
-// global memory at every level (four such CTAs an SM, its cells re-read from L2); 2^26
-// clustered into 2^18, the last four levels: 2.12 against 3.69 ms.
+// 2^15) take 2.71 ms, against 3.88 ms for a CTA of 256 threads that moved the particles in
+// global memory at every level (four such CTAs an SM, its cells re-read from L2).
 //
 // The kernel is bound by instructions and shared memory, so the bisection avoids exact binning: a histogram by
 // the rounded scaled key finds a window [a, b) of floats around the target rank (a few dozen

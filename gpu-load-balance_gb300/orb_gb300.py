@@ -465,7 +465,7 @@ class Context:
         return arr, heap_cells, bases
 
     def test_set_scan_wait(self, spin_limit: int = 0, ticket_start: int = 0):
-        """Test hook of the tile scan's bounded look-back wait (orb_test_set_scan_wait)."""
+        """Test hook: a cell's partition tiles never all arrive (orb_test_set_scan_wait)."""
         self._check(self.lib.orb_test_set_scan_wait(self.h, spin_limit, ticket_start))
 
     # launch tuning -----------------------------------------------------------------

@@ -217,10 +217,10 @@ typedef struct orb_tuning {
     uint32_t hist_blocks_per_sm;   /* count-left pass: CTAs per SM, 1..8 (default 8) */
     uint32_t part_blocks_per_sm;   /* partition passes: CTAs per SM, 1..16 (default 8) */
     uint32_t tile_blocks_per_sm;   /* one-warp cell bisection: CTAs per SM, 1..8 (default 4) */
-    uint32_t sparse_keys_per_tile; /* compaction threshold: a count pass sends a cell's bracket
-                                      keys straight to its global bins (instead of binning all
-                                      keys in shared memory) once the bracket holds at most
-                                      this many keys per tile, 1..16384 (default 64) */
+    uint32_t sparse_keys_per_tile; /* list threshold: a cell's bisection is finished on the list
+                                      of its bracket's keys (instead of another count pass) once
+                                      the bracket holds at most this many keys per tile of 16384,
+                                      1..16384 (default 64) */
     uint32_t cta_min_cells;        /* levels with at least this many cells bisect one cell per
                                       CTA; 0 = never (default) */
     uint32_t subtree_levels;       /* the last levels are finished by one CTA per cell once every
