@@ -2021,6 +2021,7 @@ struct CellsSmem {
     float L, R;
     uint32_t it, st;
     uint32_t cross;      // the tile where f crosses g
+    uint2 swaps;         // the cell's pieces on the swap's list
     uint32_t last;       // the cell's other CTAs have arrived
 };
 
@@ -2084,9 +2085,9 @@ __device__ __noinline__ void patch_upper(const Level &v, const orb_cell_t &cell,
         }
 }
 
-// One warp: s and i of a cell from its tile prefixes and the crossing tile (see P2), its
-// record, and its tiles on the swap's list.
-__device__ void cell_split_point(const Level &v, int c, uint2 rg, uint32_t t0, uint32_t T, uint32_t cross,
+// One warp: s and i of a cell from its tile prefixes and the crossing tile (see P2) and its
+// record. Returns where its pieces start on the swap's list, and their number (fill_swaps).
+__device__ uint2 cell_split_point(const Level &v, int c, uint2 rg, uint32_t t0, uint32_t T, uint32_t cross,
                                  uint32_t ge_tot, uint32_t le_tot) {
     const uint32_t lane = threadIdx.x & 31, n = rg.y - rg.x;
     uint32_t s = 0, i = n;
@@ -2143,8 +2144,10 @@ __device__ void cell_split_point(const Level &v, int c, uint2 rg, uint32_t t0, u
         v.part_done[c] = v.done_start;
         at = atomicAdd(&v.tot->swaps, left);
     }
-    at = __shfl_sync(0xffffffffu, at, 0);
-    for (uint32_t j = lane; j < left; j += 32) v.swap_list[at + j] = make_uint2((uint32_t)c, j);
+    return make_uint2(__shfl_sync(0xffffffffu, at, 0), left);
+}
+__device__ __forceinline__ void fill_swaps(const Level &v, int c, uint2 w, uint32_t ti, uint32_t nt) {
+    for (uint32_t j = ti; j < w.y; j += nt) v.swap_list[w.x + j] = make_uint2((uint32_t)c, j);
 }
 
 // A cell of at most kWarpTiles tiles and kWarpList listed keys, by one warp.
@@ -2211,7 +2214,7 @@ __device__ void cells_warp(const Level &v, int c) {
         const uint32_t b = __ballot_sync(0xffffffffu, u < T && pg[q] + g[q] >= le_tot - pl[q] - l[q]);
         if (b) cross = (uint32_t)q * 32u + (uint32_t)__ffs(b) - 1u;
     }
-    cell_split_point(v, c, rg, t0, T, t0 + cross, ge_tot, le_tot);
+    fill_swaps(v, c, cell_split_point(v, c, rg, t0, T, t0 + cross, ge_tot, le_tot), lane, 32);
 }
 
 // A larger cell, by the CTA, or by nchunks CTAs of which this is number `chunk`.
@@ -2239,14 +2242,20 @@ __device__ void cells_cta(const Level &v, int c, uint32_t chunk, uint32_t nchunk
             fill_edges(sm.edges, L, R, K, tid, NT);
             __syncthreads();
             const Guess gs = make_guess(L, R, __fdiv_rn((float)nb, __fsub_rn(R, L)), nb);
-#pragma unroll 4
-            for (uint32_t j = tid; j < m; j += NT) {
-                const float k = keys[j];
-                if (k >= L && k < R) {
-                    uint32_t g;
-                    if (!guess_bin(gs, k, &g)) g = near_bin(k, gs, sm.edges, nb - 1u);
-                    atomicAdd(&sm.bins[g], 1u);
-                }
+            // (with the loads a round at a time, and the wide cells' lists below filled by the CTA,
+            // the root of 2^27 particles takes 54 us here, 74 before)
+            constexpr int kLoads = 8;
+            for (uint32_t j0 = tid; j0 < m; j0 += kLoads * NT) {
+                float k[kLoads];
+#pragma unroll
+                for (int q = 0; q < kLoads; ++q) k[q] = j0 + q * NT < m ? keys[j0 + q * NT] : __int_as_float(0x7fc00000);
+#pragma unroll
+                for (int q = 0; q < kLoads; ++q)
+                    if (k[q] >= L && k[q] < R) {
+                        uint32_t g;
+                        if (!guess_bin(gs, k[q], &g)) g = near_bin(k[q], gs, sm.edges, nb - 1u);
+                        atomicAdd(&sm.bins[g], 1u);
+                    }
             }
             __syncthreads();
             constexpr uint32_t kPer = kHistBins / NT;  // bins a thread
@@ -2297,7 +2306,7 @@ __device__ void cells_cta(const Level &v, int c, uint32_t chunk, uint32_t nchunk
             // the bracket's keys gathered; warp 0 finishes
             if (tid == 0) sm.count = 0;
             __syncthreads();
-#pragma unroll 4
+#pragma unroll 8
             for (uint32_t j = tid; j < m; j += NT) {
                 const float k = keys[j];
                 if (k >= L && k < R) sm.list[atomicAdd(&sm.count, 1u)] = k;
@@ -2353,24 +2362,44 @@ __device__ void cells_cta(const Level &v, int c, uint32_t chunk, uint32_t nchunk
     uint32_t f = __shfl_sync(0xffffffffu, ex.x, 0), l = __shfl_sync(0xffffffffu, ex.y, 0);
     if (tid == 0) sm.cross = 0xffffffffu;
     __syncthreads();
-    for (uint32_t b = u0; b < u1; b += 32) {
-        const uint32_t u = b + lane;
-        const uint32_t g1 = u < u1 ? __ldcg(&v.pt_ge[t0 + u]) : 0u, l1 = u < u1 ? __ldcg(&v.pt_le[t0 + u]) : 0u;
-        uint32_t tg, tl;
-        const uint32_t pf = f + warp_excl_scan(g1, &tg), pl = l + warp_excl_scan(l1, &tl);
-        if (u < u1) {
-            v.pt_ge_pre[t0 + u] = pf;
-            v.pt_le_pre[t0 + u] = pl;
+    constexpr int kAhead = 4;  // rounds of 32 tiles whose counts are loaded together
+    for (uint32_t b0 = u0; b0 < u1; b0 += 32 * kAhead) {
+        uint32_t gs[kAhead], ls[kAhead];
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) {
+            const uint32_t u = b0 + (uint32_t)q * 32u + lane;
+            gs[q] = u < u1 ? __ldcg(&v.pt_ge[t0 + u]) : 0u;
+            ls[q] = u < u1 ? __ldcg(&v.pt_le[t0 + u]) : 0u;
         }
-        // crossing tile: the first whose end has f >= g (the last always does)
-        const uint32_t x = __ballot_sync(0xffffffffu, u < u1 && pf + g1 >= le_tot - pl - l1);
-        if (lane == 0 && x) atomicMin(&sm.cross, t0 + b + (uint32_t)__ffs(x) - 1u);
-        f += tg;
-        l += tl;
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) {
+            const uint32_t b = b0 + (uint32_t)q * 32u, u = b + lane;
+            if (b >= u1) break;
+            uint32_t tg, tl;
+            const uint32_t pf = f + warp_excl_scan(gs[q], &tg), pl = l + warp_excl_scan(ls[q], &tl);
+            if (u < u1) {
+                v.pt_ge_pre[t0 + u] = pf;
+                v.pt_le_pre[t0 + u] = pl;
+            }
+            // crossing tile: the first whose end has f >= g (the last always does)
+            const uint32_t x = __ballot_sync(0xffffffffu, u < u1 && pf + gs[q] >= le_tot - pl - ls[q]);
+            if (lane == 0 && x) atomicMin(&sm.cross, t0 + b + (uint32_t)__ffs(x) - 1u);
+            f += tg;
+            l += tl;
+        }
     }
     __syncthreads();
-    if (tid < 32) cell_split_point(v, c, rg, t0, T, sm.cross, ge_tot, le_tot);
+    const bool wide = T > 1024;  // a list worth the CTA's threads
+    if (tid < 32) {
+        const uint2 w = cell_split_point(v, c, rg, t0, T, sm.cross, ge_tot, le_tot);
+        if (!wide) fill_swaps(v, c, w, lane, 32);
+        if (tid == 0) sm.swaps = w;
+    }
     __syncthreads();  // sm reused by the next cell
+    if (wide) {
+        fill_swaps(v, c, sm.swaps, tid, NT);
+        __syncthreads();
+    }
 }
 
 // kPerCell: gridDim.x CTAs a cell (levels of few cells); else a warp a cell, the larger ones
