@@ -578,11 +578,12 @@ __device__ __forceinline__ int edge_bin(float k, float L, float scale, int top, 
 // t = fl(fl(k-L) * scale), scale = fl(2^K / fl(R-L)), is within 1.01 u S + 2^K 2^-22 of the
 // exact (k-L) S, S = 2^K/(R-L). A fractional part of t farther than
 // m = 8 u scale + 2^K 2^-21 from 0 and 1 therefore puts k strictly between the edges of
-// bin floor(t). Returns 1 (guess never trusted) for non-finite or tiny brackets.
+// bin floor(t). Returns 1 (guess never trusted) for tiny brackets and where an end lies at or past
+// 2^127: midpoints can overflow there (edges are then infinite, not linear), and R - L.
 __device__ __forceinline__ float bin_margin(float L, float R, float scale, uint32_t nb) {
     const float M = fmaxf(fabsf(L), fabsf(R));
     const int e = (__float_as_int(M) >> 23) & 0xff;
-    if (e < 24 || e == 0xff) return 1.0f;
+    if (e < 24 || e >= 0xfe) return 1.0f;
     const float u = __int_as_float((e - 23) << 23);
     return __fadd_ru(__fmul_ru(__fmul_ru(8.0f, u), scale), __fmul_ru((float)nb, 0x1p-21f));
 }
@@ -1194,7 +1195,8 @@ __device__ __noinline__ void resolve_cell(const Level &v, int c, const HistCell 
         // keys in the bracket the next step looks at, and keys below it
         const uint32_t inb = (pos + 1 < kHistBins ? s_hist[pos + 1] : tot) - s_hist[pos];
         v.inb[c] = inb;
-        if (inb <= list_capacity(v, n)) {
+        // (no list where a midpoint can overflow: the cut can then leave the bracket)
+        if (inb <= list_capacity(v, n) && fmaxf(fabsf(L), fabsf(R)) < 0x1p127f) {
             st = kReady;
             v.below[c] = below + s_hist[pos];
         } else {
@@ -1589,12 +1591,14 @@ __global__ void __launch_bounds__(kCtaThreads) k_bisect_cta(const __grid_constan
                 for_keys(keys, rg.x, rg.y, [&](float k) {
                     if (k < L)
                         ++blw;
-                    else if (k < R)
-                        list[atomicAdd(&s_fill, 1u)] = k;
+                    else if (k < R) {
+                        const uint32_t q = atomicAdd(&s_fill, 1u);
+                        if (q < kListCap) list[q] = k;
+                    }
                 });
                 bytes += 4ull * n;
                 base = block_sum(blw, sh);
-                m = s_fill;
+                m = min(s_fill, kListCap);
                 in_list = true;
             }
             __syncthreads();
@@ -1687,10 +1691,16 @@ __global__ void __launch_bounds__(kThreads) k_part_classify(const __grid_constan
         __syncwarp();
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(&v.cmp_cnt[c], nl);
-        base = v.cmp_off[c] + __shfl_sync(0xffffffffu, base, 0);
-        for (uint32_t j = lane; j < nl; j += 32) {
-            v.cmp_keys[base + j] = lkey[j];
-            v.cmp_pos[base + j] = lpos[j];
+        base = __shfl_sync(0xffffffffu, base, 0);
+        // (the count pass saw to it that they fit)
+        if (base + nl > list_capacity(v, rg.y - rg.x)) {
+            if (lane == 0) atomicExch(&v.counters->error, 1u);
+        } else {
+            base += v.cmp_off[c];
+            for (uint32_t j = lane; j < nl; j += 32) {
+                v.cmp_keys[base + j] = lkey[j];
+                v.cmp_pos[base + j] = lpos[j];
+            }
         }
         __syncwarp();
         nl = 0;
@@ -2309,7 +2319,10 @@ __device__ void cells_cta(const Level &v, int c, uint32_t chunk, uint32_t nchunk
 #pragma unroll 8
             for (uint32_t j = tid; j < m; j += NT) {
                 const float k = keys[j];
-                if (k >= L && k < R) sm.list[atomicAdd(&sm.count, 1u)] = k;
+                if (k >= L && k < R) {
+                    const uint32_t q = atomicAdd(&sm.count, 1u);
+                    if (q < kWarpList) sm.list[q] = k;
+                }
             }
             __syncthreads();
             if (tid < 32) {

@@ -83,3 +83,15 @@ def test_thin_box_far_from_the_origin(tuned, oracle, n, width):
         a[(p == 2) & (rng.random(n) < 0.01)] = np.nan
     tuned.set_tuning(subtree_levels=0)
     run_both(tuned, oracle, x, y, z, 8, lower=(np.float32(0.3),) * 3, upper=(hi,) * 3)
+
+
+@pytest.mark.parametrize("subtree", [0, 4])
+@pytest.mark.parametrize("n", [3001, 70_001, 300_001])
+@pytest.mark.parametrize("box,spread", [(1.8e38, 1e38), (3.2e38, 3.2e38)])
+def test_box_wider_than_the_largest_float(tuned, oracle, box, spread, n, subtree):
+    """Extents whose difference overflows, and cells whose midpoints do: no guess of a bin holds,
+    and a cut can leave its bracket."""
+    rng = np.random.default_rng(n)
+    x, y, z = ((rng.random((3, n)) * 2 - 1) * spread).astype(np.float32)
+    tuned.set_tuning(subtree_levels=subtree)
+    run_both(tuned, oracle, x, y, z, 16, lower=(-box,) * 3, upper=(box,) * 3)
