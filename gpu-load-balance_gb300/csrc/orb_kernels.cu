@@ -645,15 +645,6 @@ __device__ __forceinline__ uint32_t near_bin(float k, const Guess &gs, const flo
     return (uint32_t)edge_bin_slow(k, gs.L, gs.scale, (int)top, e);
 }
 
-// edge_bin() with the guess accepted outright when guess_bin() proves it; L <= k < R.
-__device__ __forceinline__ int fast_bin(float k, const Guess &g, int top, const float *e) {
-    uint32_t b;
-    if (guess_bin(g, k, &b)) return (int)b;
-    return edge_bin_slow(k, g.L, g.scale, top, e);
-}
-
-
-
 // The cell a count pass's CTA is working on, in shared memory (thread 0 fills it when the
 // CTA's tiles move to a new cell): the rare paths read it there, so the streaming loop keeps
 // only what it needs in registers.
@@ -702,8 +693,6 @@ struct Flag {
 // Keys per thread per round of the histogram pass (float4 loads issued together).
 constexpr int kHistVec = 4;
 
-constexpr int kGroup = 4 * kHistVec;  // keys a thread holds per round
-
 // The keys [e0, e1) of one tile (at most kTile keys), visited by the CTA's threads, for a
 // pass that leaves a few percent of its keys (the sampled pass). The 16-byte aligned body is
 // read in rounds of kHistVec float4 loads a thread (all issued before any key is used); each
@@ -750,51 +739,6 @@ __device__ __forceinline__ void scan_tile(const float *keys, uint32_t e0, uint32
     for (; j0 + kHistVec * NT <= n4; j0 += kHistVec * NT) round(Flag<true>());
     if (j0 < n4) round(Flag<false>());
     for (uint32_t i = a0 + (n4 << 2) + ti; i < e1; i += NT) visit(__ldg(keys + i));
-}
-
-// Group visitor that applies a per-key visitor to each key in order.
-template <class Visit>
-__device__ __forceinline__ auto each(Visit &visit) {
-    return [&visit](const float (&k)[kGroup]) {
-#pragma unroll
-        for (int i = 0; i < kGroup; ++i) visit(k[i]);
-    };
-}
-
-// Keys [e0, e1) of one axis, visited by `nt` threads (ti = this thread's index): scalar
-// head to 16-byte alignment and scalar tail through visit(k), float4 body (kHistVec loads
-// in flight a thread) through group(k[kGroup]). `pad` fills the body's missing lanes and
-// must be a value the visitors ignore.
-// NC: read-only loads (keys not written during the kernel); false: coherent loads, for a
-// kernel that moves the keys it reads (k_subtree).
-template <bool NC = true, class Visit, class Group>
-__device__ __forceinline__ void visit_keys(const float *keys, uint32_t e0, uint32_t e1, float pad,
-                                           uint32_t ti, uint32_t nt, Visit visit, Group group) {
-    auto ld = [](const float *p) { return NC ? __ldg(p) : *p; };
-    auto ld4 = [](const float4 *p) { return NC ? __ldg(p) : *p; };
-    const uintptr_t addr = reinterpret_cast<uintptr_t>(keys + e0);
-    const uint32_t a0 = min(e1, e0 + (uint32_t)(((16u - (addr & 15u)) & 15u) >> 2));
-    for (uint32_t i = e0 + ti; i < a0; i += nt) visit(ld(keys + i));
-    const uint32_t n4 = (e1 - a0) >> 2;
-    const float4 *k4 = reinterpret_cast<const float4 *>(keys + a0);
-    for (uint32_t j0 = 0; j0 < n4; j0 += kHistVec * nt) {
-        float4 q[kHistVec];
-#pragma unroll
-        for (int u = 0; u < kHistVec; ++u) {
-            const uint32_t j = j0 + u * nt + ti;
-            q[u] = j < n4 ? ld4(k4 + j) : make_float4(pad, pad, pad, pad);
-        }
-        float k[kGroup];
-#pragma unroll
-        for (int u = 0; u < kHistVec; ++u) {
-            k[4 * u] = q[u].x;
-            k[4 * u + 1] = q[u].y;
-            k[4 * u + 2] = q[u].z;
-            k[4 * u + 3] = q[u].w;
-        }
-        group(k);
-    }
-    for (uint32_t i = a0 + (n4 << 2) + ti; i < e1; i += nt) visit(ld(keys + i));
 }
 
 // A dense pass's key, its guess corrected by the edges either side of it: exact while the guess
