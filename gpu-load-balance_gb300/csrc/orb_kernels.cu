@@ -3341,7 +3341,7 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
             }
             done_with_keys();
             sync();
-            if (l + 1 == levels) off = begin_load(v.x + first, n);  // for the final pass
+            if (l + 1 == levels && n) off = begin_load(v.x + first, n);  // for the final pass
             // the final swap, the split (Cell::cut, src/cell.h:78-100) and the children, a thread a cell
             if (ti < nq) {
                 const SubCell sc = cells[ti];
@@ -3401,7 +3401,7 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
                                   reinterpret_cast<uint32_t *>(v.z), v.idx};
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            if (!arr[a]) continue;
+            if (!n || !arr[a]) continue;  // (without particles the coordinates may be null)
             uint32_t *dst = arr[a] + first;
             if (a > 0) off = begin_load(dst, n);
             end_load();
