@@ -53,15 +53,14 @@ __device__ __forceinline__ void pdl_enter() {
 
 // A level may not start when a cell of the level above was never finished (its arrivals
 // never completed) or an earlier step flagged an error: the build is flagged and its
-// remaining kernels do nothing (ORB_ERR_TIMEOUT).
+// remaining kernels do nothing (ORB_ERR_TIMEOUT). Every thread of the CTA calls it and all get
+// the same answer: another CTA of the same kernel may flag the error meanwhile, and a warp that
+// left alone would leave the others at a barrier.
 __device__ __forceinline__ bool level_failed(const Level &v) {
     const volatile BuildCounters *ctr = v.counters;
-    if (ctr->error) return true;
-    if (v.prev_C && ctr->done[v.depth - 1] != v.prev_C) {
-        if (threadIdx.x == 0) atomicExch(&v.counters->error, 1u);
-        return true;
-    }
-    return false;
+    const bool late = v.prev_C && ctr->done[v.depth - 1] != v.prev_C;
+    if (late && threadIdx.x == 0) atomicExch(&v.counters->error, 1u);
+    return __syncthreads_or(late || ctr->error) != 0;
 }
 
 // Arrival at a counter, by one thread after a barrier of its CTA: the CTA's writes before the

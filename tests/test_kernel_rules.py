@@ -1,0 +1,34 @@
+"""Rules of the device code that no run can show safely, checked on its source: what a broken one
+would cost is a hang or a read of freed memory."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gpu-load-balance_gb300", "csrc")
+
+
+def source(name):
+    text = open(os.path.join(CSRC, name)).read()
+    text = re.sub(r"/\*.*?\*/", "", text, flags=re.S)
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def body(text, start):
+    """The brace block that opens after the match of `start`."""
+    i = text.index("{", re.search(start, text).end())
+    depth = 0
+    for j in range(i, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[j], 0)
+        if depth == 0:
+            return text[i:j + 1]
+    raise AssertionError("unbalanced braces")
+
+
+def test_a_cta_leaves_a_failed_level_as_a_whole():
+    """The error flag can be set while a kernel runs; a CTA whose threads each decided for
+    themselves could lose some of a named barrier's warps. So the one test of the flag ends in a
+    vote of the CTA, and is its only way out."""
+    text = source("orb_kernels.cu")
+    fail = body(text, r"bool level_failed\(const Level &v\)")
+    assert re.findall(r"return\b[^;]*;", fail) == ["return __syncthreads_or(late || ctr->error) != 0;"]
+    # and nothing else decides on the flag
+    assert not re.search(r"if \([^)]*error\b", text)
