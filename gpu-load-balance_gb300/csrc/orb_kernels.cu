@@ -2545,6 +2545,7 @@ __global__ void __launch_bounds__(kSwapThreads, ORB_SWAP_MIN_BLOCKS) k_part_swap
                     s_last = last != 0;
                     if (last) acquire();
                 }
+                __syncwarp();  // (the other lanes read the cell's particles too)
                 if (__shfl_sync(0xffffffffu, last, 0)) finish_and_plan(v, s_in, P, do_split != 0, s_kids);
             }
             __syncthreads();

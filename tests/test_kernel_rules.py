@@ -32,3 +32,13 @@ def test_a_cta_leaves_a_failed_level_as_a_whole():
     assert re.findall(r"return\b[^;]*;", fail) == ["return __syncthreads_or(late || ctr->error) != 0;"]
     # and nothing else decides on the flag
     assert not re.search(r"if \([^)]*error\b", text)
+
+
+def test_an_acquire_is_followed_by_a_barrier():
+    """One thread acquires the other CTAs' writes; the threads that read them are ordered behind
+    it by a barrier (a shuffle orders no memory)."""
+    text = source("orb_kernels.cu")
+    calls = [m.end() for m in re.finditer(r"\bacquire\(\);", text)]
+    assert len(calls) == 4
+    for at in calls:
+        assert re.search(r"__sync(threads|warp)\b|__shfl_sync", text[at:]).group() != "__shfl_sync"
