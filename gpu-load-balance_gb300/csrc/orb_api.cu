@@ -94,6 +94,9 @@ struct orb_ctx {
     // test hook (orb_test_set_scan_wait): what the arrivals of a cell's partition tiles start
     // from below zero (0 normally; otherwise the last arrival never comes)
     uint32_t done_offset = 0;
+    // test hooks of the subtree kernel's waits (orb_test_set_scan_wait, orb_test_drop_copies)
+    uint32_t copy_polls = kCopyPolls;
+    bool drop_copies = false;
     // launch tuning (orb_set_tuning / orb_autotune_batch); cta_min_cells = 0 means never
     orb_tuning tune = {(uint32_t)kHistBlocksPerSm, 8u, (uint32_t)kTileBlocksPerSm, 64u, 0u, kSubDefaultLevels, 0u};
     DevBuf<uint8_t> state, iters;
@@ -299,6 +302,8 @@ Level make_level(orb_ctx *ctx, float *x, float *y, float *z) {
     v.swap_list = ctx->swap_list.p;
     v.part_done = ctx->part_done.p;
     v.done_start = 0u - ctx->done_offset;
+    v.copy_polls = ctx->copy_polls;
+    v.drop_copies = ctx->drop_copies ? 1 : 0;
     v.out_counts = ctx->out_counts.p;
     v.sparse_per_tile = ctx->tune.sparse_keys_per_tile;
     v.pdl = ctx->use_pdl ? 1 : 0;
@@ -484,6 +489,8 @@ std::vector<uint64_t> level_key(orb_ctx *ctx, const Level &v) {
     key_add(key, ctx->sub_list.p);
     key.push_back(ctx->prof_mask);
     key.push_back(ctx->done_offset);
+    key.push_back(ctx->copy_polls);
+    key.push_back(ctx->drop_copies ? 1u : 0u);
     key.push_back(ctx->use_pdl ? 1u : 0u);
     for (uint32_t t : {ctx->tune.hist_blocks_per_sm, ctx->tune.part_blocks_per_sm, ctx->tune.tile_blocks_per_sm,
                        ctx->tune.sparse_keys_per_tile, ctx->tune.cta_min_cells, ctx->tune.subtree_levels,
@@ -724,7 +731,8 @@ void take_tree(const TreeOut &t) {
     std::memcpy(t.ranges, t.staged + t.cells * sizeof(orb_cell_t), t.cells * sizeof(uint2));
 }
 
-constexpr const char *kUnfinished = "a cell's tiles did not all report or a bisection did not finish";
+constexpr const char *kUnfinished =
+    "a cell's tiles did not all report, a copy of keys did not come or a bisection did not finish";
 
 // After a build (its counters read back): no step flagged an error and every cell of the first
 // `levels` levels, the ones the level kernels ran, was finished.
@@ -1894,8 +1902,15 @@ orb_status orb_test_set_scan_wait(orb_ctx *ctx, uint32_t spin_limit, uint32_t ti
     if (!ctx) return ORB_ERR_INVALID_ARGUMENT;
     ctx->err.clear();
     if (ticket_start > 255) return fail(ctx, ORB_ERR_INVALID_ARGUMENT, "ticket_start above 255");
-    (void)spin_limit;  // no device wait polls (see orb.h)
+    ctx->copy_polls = spin_limit ? spin_limit : kCopyPolls;
     ctx->done_offset = ticket_start;
+    return ORB_OK;
+}
+
+orb_status orb_test_drop_copies(orb_ctx *ctx, int on) {
+    if (!ctx) return ORB_ERR_INVALID_ARGUMENT;
+    ctx->err.clear();
+    ctx->drop_copies = on != 0;
     return ORB_OK;
 }
 

@@ -53,6 +53,9 @@ constexpr int kWPasses = 3;
 enum CellState : uint8_t { kActive = 0, kFound = 1, kCapped = 2, kSmall = 3, kReady = 4 };
 constexpr int kWarpKeys = 1024;      // cells up to this size bisect in one warp's registers
 constexpr int kMaxLevels = 30;       // d is at most 2^30
+// The subtree kernel's wait for a copy of keys: its polls at most, and the nanoseconds after which
+// the hardware is asked to end one (2^20 of them were measured to take 3.8 s, 2^18 a second).
+constexpr uint32_t kCopyPolls = 1u << 18, kCopyPollNs = 1000;
 
 // Kernel kinds, for launch counting, event timing and algorithmic-byte accounting.
 enum Kernel : int {
@@ -206,6 +209,8 @@ struct Level {
     int *sub_list;          // [4 C] the subtree kernel's cells by class
     int sub_levels;         // levels below every cell (0: by its leaf count)
     int sub_wide;           // 1: all of a CTA's warps on every cell (levels of few cells)
+    uint32_t copy_polls;    // most polls of a wait for a copy of keys
+    int drop_copies;        // test hook: no copy of keys is made
     // window reports (null otherwise): the host-mapped reports, a finished-cell counter per
     // window, root cells per window
     HostWindows *hwin;

@@ -2631,7 +2631,6 @@ __global__ void __launch_bounds__(kThreads) k_part_finish(const __grid_constant_
 constexpr int kSubLevels = kSubMaxLevels;
 constexpr int kSubCells = 1 << (kSubLevels - 1);  // cells of the deepest level split
 constexpr int kSubThreads = 1024;                 // of the CTA, one on an SM
-constexpr uint32_t kSubSpins = 1u << 20;           // polls of one copy's wait (each waits in hardware)
 constexpr uint32_t kSubWindowList = 256;          // most listed keys of a cell (8 a lane)
 
 struct SubCell {
@@ -2672,6 +2671,7 @@ struct SubSmem {
     uint32_t more, direct;
     uint32_t max_it, unfound, degenerate;
     int item, root;
+    uint32_t lost;    // a copy's wait ran out
     alignas(8) unsigned long long arrived;  // mbarrier of the key copies
 };
 
@@ -2756,9 +2756,10 @@ extern __shared__ __align__(16) unsigned char sub_mem[];
 
 // One group of NW warps: the cells of one class, from its work queue. `slice`: where the
 // group's shared memory starts (named here, not passed as a pointer, so that every access is a
-// shared-memory one); ti: thread of the group; bar: its named barrier.
+// shared-memory one); ti: thread of the group; bar: its named barrier. False: a copy did not come;
+// the build is flagged and the group has left its queue and this shared memory.
 template <int NW>
-__device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32_t ti, int bar) {
+__device__ __forceinline__ bool sub_group(const Level &v, uint32_t slice, uint32_t ti, int bar) {
     unsigned char *const mem = sub_mem + slice;
     constexpr int kClass = NW == 32 ? 0 : (NW == 16 ? 1 : (NW == 8 ? 2 : 3));
     constexpr uint32_t NT = NW * 32, nmax = NW == 32 ? kSub32 : (NW == 16 ? kSub16 : (NW == 8 ? kSub8 : kSub2)), nwords = sub_words(nmax);
@@ -2785,10 +2786,13 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
     // Copies the n words at src into keys[off ...] (off: src's misalignment in words, so that
     // 16-byte pieces stay aligned on both sides): one bulk copy for the whole pieces, plain loads
     // for the rest. begin_load after a barrier that ends the keys' last use; end_load, then a
-    // barrier, before they are read. The wait is bounded; a copy that does not come flags the build.
+    // barrier, before they are read, and the group leaves where any of its threads' waits ran out
+    // (sm.lost, read after that barrier). A wait polls at most v.copy_polls times (kCopyPolls: about
+    // a second, far beyond any copy).
     const uint32_t arrived = (uint32_t)__cvta_generic_to_shared(&sm.arrived);
     uint32_t parity = 0;
     if (ti == 0) {
+        sm.lost = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(arrived) : "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -2799,7 +2803,7 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
         const uint32_t *src = reinterpret_cast<const uint32_t *>(from);
         const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(src) >> 2) & 3u;
         const uint32_t head = min(n, (4u - off) & 3u), body = (n - head) & ~3u;
-        if (ti == 0) {
+        if (ti == 0 && !v.drop_copies) {
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(arrived), "r"(4u * body) : "memory");
             if (body)
                 asm volatile(
@@ -2812,16 +2816,26 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
         if (ti >= 32 && ti - 32 < n - head - body) keys[off + head + body + ti - 32] = __ldcg(src + head + body + ti - 32);
         return off;
     };
-    auto end_load = [&]() {
+    auto wait_copy = [&](uint32_t phase, uint32_t polls) -> bool {
         uint32_t ok = 0;
-        for (uint32_t spins = 0; !ok && spins < kSubSpins; ++spins)
+        for (uint32_t spins = 0; !ok && spins < polls; ++spins)
             asm volatile(
-                "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.b32 %0, 1, 0, p;\n}"
+                "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.b32 %0, 1, 0, p;\n}"
                 : "=r"(ok)
-                : "r"(arrived), "r"(parity)
+                : "r"(arrived), "r"(phase), "r"(kCopyPollNs)
                 : "memory");
-        if (!ok) atomicExch(&v.counters->error, 1u);
+        return ok != 0;
+    };
+    auto end_load = [&]() {
+        if (!wait_copy(parity, v.copy_polls)) sm.lost = 1;
         parity ^= 1u;
+    };
+    // After the barrier behind end_load: the group leaves, its own copy (if one is under way after
+    // all) waited for once more.
+    auto leave = [&]() {
+        if (ti == 0) atomicExch(&v.counters->error, 1u);
+        if (!v.drop_copies) wait_copy(parity ^ 1u, kCopyPolls);
+        return false;
     };
     auto take = [&]() -> int {
         const uint32_t k = atomicAdd(&v.counters->sub_next[kClass], 1u);
@@ -2980,12 +2994,14 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
                 if (!((counted >> ax) & 1u)) {
                     end_load();
                     sync();
+                    if (sm.lost) return leave();
                 }
                 for (int r = 0; (counted >> ax) & 1u; ++r) {
                     for (uint32_t j = ti; j < kBins; j += NT) sm.bins[j] = 0u;
                     if (ti == 0) sm.more = 0;
                     if (r == 0) end_load();
                     sync();
+                    if (r == 0 && sm.lost) return leave();
                     bool any = false;
                     for (uint32_t q = q0; q < nq; q += qs) {
                         if (!counts(q)) continue;
@@ -3406,6 +3422,7 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
             if (a > 0) off = begin_load(dst, n);
             end_load();
             sync();
+            if (sm.lost) return leave();
             const uint32_t *from = keys + off;
             uint32_t p = ti;
             for (; p + 7 * NT < n; p += 8 * NT) {
@@ -3447,26 +3464,29 @@ __device__ __forceinline__ void sub_group(const Level &v, uint32_t slice, uint32
         }
     }
     if (ti == 0 && bytes) add_bytes(v, kKSubtree, bytes);
+    return true;
 }
 
 // The level's cells, largest class first: all of the CTA's warps on one cell, then groups of
-// 16, 8 and 2 warps on their own slices of its shared memory.
+// 16, 8 and 2 warps on their own slices of its shared memory. A class is not begun by a CTA one of
+// whose groups left the one before.
 __global__ void __launch_bounds__(kSubThreads) k_subtree(const __grid_constant__ Level v) {
     pdl_enter();
     if (*(volatile const uint32_t *)v.skip != 1u) return;  // the level kernels run instead
     const uint32_t tid = threadIdx.x;
-    if (v.counters->sub_cells[0]) sub_group<32>(v, 0u, tid, 0);
-    __syncthreads();
+    bool ok = true;
+    if (v.counters->sub_cells[0]) ok = sub_group<32>(v, 0u, tid, 0);
+    if (!__syncthreads_and(ok)) return;
     if (v.counters->sub_cells[1]) {
         const uint32_t k = tid / 512;
-        sub_group<16>(v, k * sub_bytes<16>(kSub16), tid % 512, 1 + (int)k);
+        ok = sub_group<16>(v, k * sub_bytes<16>(kSub16), tid % 512, 1 + (int)k);
     }
-    __syncthreads();
+    if (!__syncthreads_and(ok)) return;
     if (v.counters->sub_cells[2]) {
         const uint32_t k = tid / 256;
-        sub_group<8>(v, k * sub_bytes<8>(kSub8), tid % 256, 1 + (int)k);
+        ok = sub_group<8>(v, k * sub_bytes<8>(kSub8), tid % 256, 1 + (int)k);
     }
-    __syncthreads();
+    if (!__syncthreads_and(ok)) return;
     if (v.counters->sub_cells[3]) {
         const uint32_t k = tid / 64;
         sub_group<2>(v, k * sub_bytes<2>(kSub2), tid % 64, (int)k);

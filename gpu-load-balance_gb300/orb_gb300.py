@@ -70,6 +70,7 @@ EXPORTS = [
     "orb_server_fetch", "orb_server_release", "orb_server_get_stats", "orb_get_tuning",
     "orb_set_tuning", "orb_autotune_batch", "orb_build_batch_warm", "orb_build_warm",
     "orb_server_submit_rebalance_warm", "orb_test_set_scan_wait", "orb_build_weighted",
+    "orb_test_drop_copies",
 ]
 
 ORB_STATIC_MAX_CELLS = 65536
@@ -293,6 +294,8 @@ def load(path: str | None = None):
     L.orb_server_get_stats.argtypes = [vp, ctypes.POINTER(ServerStats)]
     L.orb_test_set_scan_wait.restype = ctypes.c_int
     L.orb_test_set_scan_wait.argtypes = [vp, u32, u32]
+    L.orb_test_drop_copies.restype = ctypes.c_int
+    L.orb_test_drop_copies.argtypes = [vp, ctypes.c_int]
     L.orb_count_left_static.restype = ctypes.c_int
     L.orb_count_left_static.argtypes = [vp, vp, vp, u64, vp, u32, vp, u32, vp, vp]
     _lib = L
@@ -465,8 +468,13 @@ class Context:
         return arr, heap_cells, bases
 
     def test_set_scan_wait(self, spin_limit: int = 0, ticket_start: int = 0):
-        """Test hook: a cell's partition tiles never all arrive (orb_test_set_scan_wait)."""
+        """Test hook: the polls of the subtree kernel's waits for its copies; a cell's partition
+        tiles never all arrive (orb_test_set_scan_wait)."""
         self._check(self.lib.orb_test_set_scan_wait(self.h, spin_limit, ticket_start))
+
+    def test_drop_copies(self, on: bool):
+        """Test hook: the subtree kernel's waits run out (orb_test_drop_copies)."""
+        self._check(self.lib.orb_test_drop_copies(self.h, int(on)))
 
     # launch tuning -----------------------------------------------------------------
     def get_tuning(self) -> dict:

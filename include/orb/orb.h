@@ -407,17 +407,21 @@ orb_status orb_count_left_static(const float *x, const float *y, const float *z,
                                  void *stream);
 
 /*
- * Test hook of the device's failure detection (no counterpart in the reference, whose errors
+ * Test hooks of the device's failure detection (no counterpart in the reference, whose errors
  * end the process, src/constants.h:19-23). No kernel of the engine waits for another CTA: the
  * partition's tiles count their arrivals per cell and whoever brings a cell's last one
  * finishes the cell. A cell whose last arrival never comes is found by the next level's
  * kernels, which then do nothing, and by the host at the build's end: the build returns
  * ORB_ERR_TIMEOUT and the context stays usable. ticket_start (0..255, normally 0) makes every
  * cell's arrivals start that far below zero, so that with 1 the last one is never counted.
- * spin_limit: accepted for callers of earlier versions, which polled with that bound.
- * Settings stay until changed; (0, 0) restores the defaults.
+ * spin_limit: the most polls (of about a microsecond) of the one device wait there is, the
+ * subtree kernel's for its own copies of keys (0: the default, about a second). A wait that
+ * runs out flags the build, which returns ORB_ERR_TIMEOUT; the context stays usable.
+ * orb_test_drop_copies(on = 1) leaves those copies out, so that every such wait runs out with
+ * nothing under way. Settings stay until changed; (0, 0) and on = 0 restore the defaults.
  */
 orb_status orb_test_set_scan_wait(orb_ctx *ctx, uint32_t spin_limit, uint32_t ticket_start);
+orb_status orb_test_drop_copies(orb_ctx *ctx, int on);
 
 #ifdef __cplusplus
 }

@@ -42,3 +42,16 @@ def test_an_acquire_is_followed_by_a_barrier():
     assert len(calls) == 4
     for at in calls:
         assert re.search(r"__sync(threads|warp)\b|__shfl_sync", text[at:]).group() != "__shfl_sync"
+
+
+def test_a_lost_copy_ends_its_group():
+    """A wait for a copy that ran out leaves its barrier in a phase that must not be armed again:
+    the barrier behind every wait is followed by the group's way out."""
+    text = source("orb_kernels.cu")
+    group = body(text, r"bool sub_group\(")
+    waits = [m.end() for m in re.finditer(r"\bend_load\(\);", group)]
+    assert len(waits) == 3
+    for at in waits:
+        assert re.match(r"\s*sync\(\);\s*if \((r == 0 && )?sm\.lost\) return leave\(\);", group[at:])
+    kernel = body(text, r"void __launch_bounds__\(kSubThreads\) k_subtree\(")
+    assert kernel.count("if (!__syncthreads_and(ok)) return;") == 3
