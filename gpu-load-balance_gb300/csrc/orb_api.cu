@@ -1740,6 +1740,7 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
     std::vector<uint64_t> key = level_key(ctx, v);
     key.push_back(warm ? 0xBA7C4A : 0xBA7C4);  // batched build (warm)
     key_add(key, v.hint);
+    key_add(key, v.hint_axis);
     key_add(key, v.warm);
     key.push_back(n_total);
     key_add(key, ctx->batch_roots.p);

@@ -150,7 +150,6 @@ struct Level {
     // particles; larger ones get count tiles)
     int next_C;
     const int *child_map;
-    const int *next_slots;  // heap slots of the next level's cells (null: implied)
     uint32_t small_next;
     uint32_t small;         // ... on this level (k_plan, k_init)
     uint32_t hist_threads;  // threads of a count pass's CTA (kThreads, 512 or 1024)

@@ -55,3 +55,20 @@ def test_a_lost_copy_ends_its_group():
         assert re.match(r"\s*sync\(\);\s*if \((r == 0 && )?sm\.lost\) return leave\(\);", group[at:])
     kernel = body(text, r"void __launch_bounds__\(kSubThreads\) k_subtree\(")
     assert kernel.count("if (!__syncthreads_and(ok)) return;") == 3
+
+
+def test_a_graph_is_replayed_with_the_buffers_it_was_captured_with():
+    """Every device address a captured kernel can read stands in the graph's key: a buffer that
+    was freed and allocated elsewhere must not be reached through an older graph."""
+    level = body(source("orb_internal.cuh"), r"struct Level ")
+    pointers = set(re.findall(r"\*\s*(\w+)(?=\s*[,;])", level))
+    assert {"x", "hint", "hint_axis", "win_cnt", "wtot"} <= pointers
+    api = source("orb_api.cu")
+    keyed = set(re.findall(r"\(const void \*\)v\.(\w+)", body(api, r"level_key\(orb_ctx \*ctx, const Level &v\)")))
+    keyed |= set(re.findall(r"key_add\(key, v\.(\w+)\)", api))
+    for name, buffer in {"skip": "sub_flag", "sub_list": "sub_list", "slots": "batch_slots", "child_map": "batch_child"}.items():
+        assert f"key_add(key, ctx->{buffer}.p)" in api
+        keyed.add(name)
+    keyed |= {"tot", "tot_next"}  # inside the counters
+    keyed |= {"out_counts", "cells_in"}  # service calls, which are not captured
+    assert pointers - keyed == set()
