@@ -499,6 +499,13 @@ std::vector<uint64_t> level_key(orb_ctx *ctx, const Level &v) {
     return key;
 }
 
+// Boxes with an end at or past 2^127 (or none at all): midpoints of their cells can overflow.
+bool wide_box(const float lower[3], const float upper[3]) {
+    for (int a = 0; a < 3; ++a)
+        if (!(std::fabs(lower[a]) < 0x1p127f) || !(std::fabs(upper[a]) < 0x1p127f)) return true;
+    return false;
+}
+
 // Most partition tiles of a level of v.C cells over n particles.
 uint64_t ptiles_of(const Level &v, uint64_t n) { return n / kPTile + (uint64_t)v.C; }
 
@@ -534,7 +541,7 @@ orb_status run_bisection(orb_ctx *ctx, Level v, uint64_t n, uint32_t *passes, in
     // few tiles: larger CTAs, at most one tile each (a level of 2^20 particles, 64 tiles: 15.4 ->
     // 12.3 us with 1024 threads; of 4.1 million, 250 tiles: 26 -> 19.5 us with 512)
     v.hist_threads = tiles <= (uint64_t)ctx->num_sms ? 1024 : (tiles <= kHistBlocks512 * (uint64_t)ctx->num_sms ? 512 : kThreads);
-    if (first == 2) v.hist_threads = kThreads;
+    if (first == 2 || v.wide) v.hist_threads = kThreads;
     for (int pass = 0; pass < npasses; ++pass) {
         v.pass = pass;
         const uint64_t ctas = v.hist_threads == kThreads ? ctx->num_sms * (uint64_t)ctx->tune.hist_blocks_per_sm : tiles;
@@ -1073,6 +1080,7 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
         v.wbelow = ctx->wbelow.p;
         v.wtot = ctx->wtot.p;
     }
+    v.wide = wide_box(lower, upper) ? 1 : 0;
     v.C = lv.empty() ? 0 : lv[0].C;  // the init kernel plans the root
     v.small = small_cells(ctx, v, n, 0, v.C);
     v.plan_bins = plan_bins(ctx, v, v.C);
@@ -1763,6 +1771,7 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
         const Slices sl(inst[i].d);
         full = full && sl.pow2 && lev[i] == sl.depth;
         max_n = std::max<uint64_t>(max_n, inst[i].n);
+        if (wide_box(inst[i].lower, inst[i].upper)) v.wide = 1;
     }
     // warm: the subtree kernel only on levels that take no hints
     const size_t hint_to = warm ? hint_levels(ctx, lv, max_n, full) : 0;

@@ -1033,6 +1033,68 @@ __global__ void __launch_bounds__(kPickThreads) k_sample_pick(const __grid_const
     }
 }
 
+// Midpoints overflow in brackets with an end at or past 2^127: the cut is then infinite and not in
+// its bracket, and its count is over all the cell's keys (none below -inf, those below +inf), which
+// the bins do not hold.
+__device__ __forceinline__ bool may_overflow(float L, float R) { return !(fmaxf(fabsf(L), fabsf(R)) < 0x1p127f); }
+__device__ __forceinline__ bool overflowed(float cut) { return fabsf(cut) == __int_as_float(0x7f800000); }
+// Keys (of [e0, e1)) below +inf, by the CTA. `sh` holds >= 32 words.
+__device__ __noinline__ uint32_t finite_keys(const float *keys, uint32_t e0, uint32_t e1, uint32_t *sh) {
+    uint32_t cnt = 0;
+    for_keys(keys, e0, e1, [&](float k) { cnt += k < __int_as_float(0x7f800000); });
+    return block_sum(cnt, sh);
+}
+
+// Up to K iterations of the reference loop (src/orbit.cpp:146-232) on the prefix counts pre[] of a
+// midpoint tree's leaves over [L, R): leaf `pos` starts the new bracket. kWide: cuts can be infinite;
+// `finite` is then the cell's keys below +inf, and the result false if one comes up while that is
+// not known (~0).
+template <bool kWide>
+__device__ __forceinline__ bool replay(const uint32_t *pre, int K, uint32_t below, uint32_t n, float ratio,
+                                       uint32_t finite, float &L, float &R, uint32_t &it, uint32_t &pos, uint8_t &st) {
+    uint32_t width = 1u << K;
+    for (int step = 0; step < K; ++step) {
+        if (it >= (uint32_t)kMaxIterations) break;
+        const uint32_t half = width >> 1;
+        uint32_t cl = below + pre[pos + half];
+        if (kWide && overflowed(mid_cut(L, R))) {
+            if (finite == 0xffffffffu) return false;
+            cl = mid_cut(L, R) > 0.f ? finite : 0u;
+        }
+        ++it;
+        const int dir = convergence(cl, n, ratio);
+        if (dir == 0) {
+            st = kFound;
+            break;
+        }
+        const float cut = mid_cut(L, R);
+        if (dir > 0) {
+            R = cut;
+        } else {
+            L = cut;
+            pos += half;
+        }
+        width = half;
+    }
+    if (st == kActive && it >= (uint32_t)kMaxIterations) st = kCapped;
+    return true;
+}
+
+// `finite` for the replay of cell c (described by hc; pre: its prefix counts), by the CTA, if a trial
+// run by every thread meets an infinite cut.
+__device__ __noinline__ uint32_t infinite_cut_count(const Level &v, int c, const HistCell *hc, const uint32_t *pre,
+                                                    uint32_t *sh) {
+    uint32_t finite = 0xffffffffu;
+    const float ratio = leaf_ratio(v.heap[level_slot(v, c)].nLeafCells);
+    float L = hc->L, R = hc->R;
+    uint32_t it = v.iters[c], pos = 0;
+    uint8_t st = kActive;
+    if (!replay<true>(pre, kHistK, hc->whole ? hc->below : __ldcg(&v.below[c]), hc->end - hc->base, ratio, finite, L, R, it, pos, st))
+        finite = finite_keys(hc->keys, hc->base, hc->end, sh);
+    __syncthreads();  // every thread has read the cell
+    return finite;
+}
+
 // Replay of up to 11 iterations of the reference loop (src/orbit.cpp:146-232) on the finished
 // histogram of cell c, by the CTA that finished its last tile (every thread; hc describes the
 // cell). The bins are read, cleared and turned into prefix counts in shared memory, so a step
@@ -1040,7 +1102,9 @@ __global__ void __launch_bounds__(kPickThreads) k_sample_pick(const __grid_const
 // keys fit a list: the classify pass lists them, k_part_cells goes on) or active for the next
 // pass. Fused here: as a kernel of its own behind every pass it took 9-10 us a launch, three
 // times a level, most of it launch and load latency.
-template <uint32_t NT>
+// kWide: midpoints can overflow (builds whose box reaches 2^127 have their own instances of the
+// passes: the registers this takes made the others 0.7% slower).
+template <uint32_t NT, bool kWide>
 __device__ __noinline__ void resolve_cell(const Level &v, int c, const HistCell *hc, uint32_t *s_hist, uint32_t *s_red) {
     constexpr uint32_t kPer = kHistBins / NT;  // bins a thread
     static_assert(kPer == 2 || kPer == 4 || kPer == 8, "vector loads");
@@ -1076,6 +1140,7 @@ __device__ __noinline__ void resolve_cell(const Level &v, int c, const HistCell 
         run += h[j];
     }
     __syncthreads();
+    const uint32_t finite = kWide ? infinite_cut_count(v, c, hc, s_hist, s_red) : 0xffffffffu;
     if (tid >= 32) return;  // one warp replays (identically in every lane)
     const int slot = level_slot(v, c);
     orb_cell_t &cell = v.heap[slot];
@@ -1105,28 +1170,9 @@ __device__ __noinline__ void resolve_cell(const Level &v, int c, const HistCell 
         }
         return;
     }
-    uint32_t pos = 0, width = kHistBins;
+    uint32_t pos = 0;
     uint8_t st = kActive;
-    for (int step = 0; step < kHistK; ++step) {
-        if (it >= (uint32_t)kMaxIterations) break;
-        const uint32_t half = width >> 1;
-        const uint32_t cl = below + s_hist[pos + half];
-        ++it;
-        const int dir = convergence(cl, n, ratio);
-        if (dir == 0) {
-            st = kFound;
-            break;
-        }
-        const float cut = mid_cut(L, R);
-        if (dir > 0) {
-            R = cut;
-        } else {
-            L = cut;
-            pos += half;
-        }
-        width = half;
-    }
-    if (st == kActive && it >= (uint32_t)kMaxIterations) st = kCapped;
+    replay<kWide>(s_hist, kHistK, below, n, ratio, finite, L, R, it, pos, st);
     if (tid != 0) return;
     cell.cutMarginLeft = L;
     cell.cutMarginRight = R;
@@ -1139,7 +1185,7 @@ __device__ __noinline__ void resolve_cell(const Level &v, int c, const HistCell 
         const uint32_t inb = (pos + 1 < kHistBins ? s_hist[pos + 1] : tot) - s_hist[pos];
         v.inb[c] = inb;
         // (no list where a midpoint can overflow: the cut can then leave the bracket)
-        if (inb <= list_capacity(v, n) && fmaxf(fabsf(L), fabsf(R)) < 0x1p127f) {
+        if (inb <= list_capacity(v, n) && !(kWide && may_overflow(L, R))) {
             st = kReady;
             v.below[c] = below + s_hist[pos];
         } else {
@@ -1167,7 +1213,7 @@ __device__ __noinline__ void resolve_cell(const Level &v, int c, const HistCell 
 constexpr uint32_t kHFirstDense = kHDense;
 constexpr uint32_t kHFirstSampled = kHDense | kHPred;
 constexpr uint32_t kHRest = kHDense | kHBracket;
-template <uint32_t Allowed, uint32_t NT>
+template <uint32_t Allowed, uint32_t NT, bool kWide = false>
 __global__ void __launch_bounds__(NT, NT == kThreads ? kHistBlocksPerSm : (NT == 512 ? kHistBlocks512 : 1)) k_hist(const __grid_constant__ Level v) {
     pdl_enter();
     __shared__ __align__(16) uint32_t s_hist[kHistBins + 32];  // + the dense loop's spare bins
@@ -1215,7 +1261,7 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? kHistBlocksPerSm : (NT ==
             }
         }
         __syncthreads();
-        if (s_hc.last) resolve_cell<NT>(v, cur, &s_hc, s_hist, s_red);
+        if (s_hc.last) resolve_cell<NT, kWide>(v, cur, &s_hc, s_hist, s_red);
         __syncthreads();  // s_hc and s_hist free for the next cell
         below = 0;
         ntiles = 0;
@@ -1423,8 +1469,8 @@ __global__ void __launch_bounds__(kCtaThreads) k_bisect_cta(const __grid_constan
         const float ratio = leaf_ratio(cell.nLeafCells);  // src/orbit.cpp:204
         const float *keys = axis_keys(v, eff_axis(cell.cutAxis));
         float L = cell.cutMarginLeft, R = cell.cutMarginRight;
-        uint32_t it = 0, base = 0, m = n, inb = n;
-        int st = kActive;
+        uint32_t it = 0, base = 0, m = n, inb = n, finite = 0xffffffffu;
+        uint8_t st = kActive;
         bool in_list = n <= kListCap;
         unsigned long long bytes = 0;
         if (in_list) {
@@ -1473,30 +1519,18 @@ __global__ void __launch_bounds__(kCtaThreads) k_bisect_cta(const __grid_constan
             }
             __syncthreads();
             // ---- replay up to K iterations (identically in every thread)
-            uint32_t pos = 0, width = nb;
-            for (int step = 0; step < K; ++step) {
-                if (it >= (uint32_t)kMaxIterations) {
-                    st = kCapped;
-                    break;
-                }
-                const uint32_t half = width >> 1;
-                const uint32_t cl = below + s_hist[pos + half];
-                ++it;
-                const int dir = convergence(cl, n, ratio);
-                if (dir == 0) {
-                    st = kFound;
-                    break;
-                }
-                const float cut = mid_cut(L, R);
-                if (dir > 0) {
-                    R = cut;
-                } else {
-                    L = cut;
-                    pos += half;
-                }
-                width = half;
+            uint32_t pos = 0;
+            float l = L, r = R;
+            uint32_t i0 = it;
+            if (!replay<true>(s_hist, K, below, n, ratio, finite, l, r, i0, pos, st)) {
+                finite = finite_keys(keys, rg.x, rg.y, sh);
+                bytes += 4ull * n;
+                l = L, r = R, i0 = it, pos = 0, st = kActive;
+                replay<true>(s_hist, K, below, n, ratio, finite, l, r, i0, pos, st);
             }
-            if (st == kActive && it >= (uint32_t)kMaxIterations) st = kCapped;
+            L = l;
+            R = r;
+            it = i0;
             if (st != kActive) break;
             // keys in the new bracket [L, R) (entry nb of the prefix is the round's total)
             inb = (pos + 1 < nb ? s_hist[pos + 1] : tot_a) - s_hist[pos];
@@ -1551,7 +1585,7 @@ __global__ void __launch_bounds__(kCtaThreads) k_bisect_cta(const __grid_constan
             cell.cutMarginRight = R;
             cell.foundCut = st == kFound ? 1 : 0;
             v.iters[c] = (uint8_t)it;
-            v.state[c] = (uint8_t)st;
+            v.state[c] = st;
             atomicMax(&v.counters->max_iters, it);
             if (st == kCapped) atomicAdd(&v.counters->unfound, 1u);
             add_bytes(v, kKBisectCta, bytes);
@@ -2186,7 +2220,7 @@ __device__ void cells_cta(const Level &v, int c, uint32_t chunk, uint32_t nchunk
         float L = cell.cutMarginLeft, R = cell.cutMarginRight;
         const float hi = R;
         uint32_t it = v.iters[c], cand = m, below = v.below[c];  // keys below L
-        int st = kActive;
+        uint8_t st = kActive;
         // histogram rounds over the bracket's midpoint tree, until the bracket fits a warp
         while (st == kActive && cand > kWarpList) {
             const int K = min(kMaxBinsLog2, 32 - __clz(cand));
@@ -2226,29 +2260,8 @@ __device__ void cells_cta(const Level &v, int c, uint32_t chunk, uint32_t nchunk
                 run += h[j];
             }
             __syncthreads();
-            uint32_t p = 0, width = nb;
-            for (int step = 0; step < K; ++step) {
-                if (it >= (uint32_t)kMaxIterations) {
-                    st = kCapped;
-                    break;
-                }
-                const uint32_t half = width >> 1;
-                ++it;
-                const int dir = convergence(below + sm.bins[p + half], n, ratio);
-                if (dir == 0) {
-                    st = kFound;
-                    break;
-                }
-                const float cut = mid_cut(L, R);
-                if (dir > 0) {
-                    R = cut;
-                } else {
-                    L = cut;
-                    p += half;
-                }
-                width = half;
-            }
-            if (st == kActive && it >= (uint32_t)kMaxIterations) st = kCapped;
+            uint32_t p = 0;
+            replay<false>(sm.bins, K, below, n, ratio, 0u, L, R, it, p, st);
             if (st == kActive) {
                 cand = (p + 1 < nb ? sm.bins[p + 1] : tot) - sm.bins[p];
                 below += sm.bins[p];
@@ -2275,14 +2288,14 @@ __device__ void cells_cta(const Level &v, int c, uint32_t chunk, uint32_t nchunk
                     const uint32_t j = (uint32_t)q * 32u + lane;
                     kl[q] = j < cand ? sm.list[j] : R;
                 }
-                st = bisect_list(kl, below, n, ratio, L, R, it);
+                st = (uint8_t)bisect_list(kl, below, n, ratio, L, R, it);
             }
         }
         if (tid == 0) {
             sm.L = L;
             sm.R = R;
             sm.it = it;
-            sm.st = (uint32_t)st;
+            sm.st = st;
         }
         __syncthreads();
         const float cut = mid_cut(sm.L, sm.R);
@@ -3585,6 +3598,7 @@ struct WeightSmem {
 
 // Replay of up to K iterations on the finished bins of cell c (in shared memory, or added up
 // in global memory by several CTAs), every thread; the cell's bracket and state in sm.cell.
+template <bool kWide>
 __device__ __noinline__ void weighted_replay(const Level &v, int c, bool global, WeightSmem &sm) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     WeightCell &w = sm.cell;
@@ -3621,19 +3635,24 @@ __device__ __noinline__ void weighted_replay(const Level &v, int c, bool global,
         run += h[j];
     }
     __syncthreads();
-    if (tid == 0) {
-        const int slot = level_slot(v, c);
-        const int32_t leaves = v.heap[slot].nLeafCells;
-        const uint32_t n = w.end - w.base;
-        float L = w.L, R = w.R;
-        uint32_t it = w.it, pos = 0, width = nb;
-        uint8_t st = kActive;
-        const WeightTest test(w.tot, n, leaves);
+    const uint32_t n = w.end - w.base;
+    float L = w.L, R = w.R;
+    uint32_t it = w.it, pos = 0;
+    uint8_t st = kActive;
+    unsigned long long finite = ~0ull;  // (kWide) the weight of the keys below +inf, see replay()
+    auto attempt = [&]() -> bool {
+        const WeightTest test(w.tot, n, v.heap[level_slot(v, c)].nLeafCells);
+        uint32_t width = nb;
         for (int step = 0; step < w.K; ++step) {
             if (it >= (uint32_t)kMaxIterations) break;
             const uint32_t half = width >> 1;
+            unsigned long long wl = w.below + sm.pre[pos + half];
+            if (kWide && overflowed(mid_cut(L, R))) {
+                if (finite == ~0ull) return false;
+                wl = mid_cut(L, R) > 0.f ? finite : 0ull;
+            }
             ++it;
-            const int dir = test.dir(w.below + sm.pre[pos + half]);
+            const int dir = test.dir(wl);
             if (dir == 0) {
                 st = kFound;
                 break;
@@ -3648,6 +3667,20 @@ __device__ __noinline__ void weighted_replay(const Level &v, int c, bool global,
             width = half;
         }
         if (st == kActive && it >= (uint32_t)kMaxIterations) st = kCapped;
+        return true;
+    };
+    if (kWide) {  // a trial run by every thread
+        if (!attempt()) {
+            finite = 0;
+            for (uint32_t p = w.base + tid; p < w.end; p += kThreads)
+                if (__ldg(w.keys + p) < __int_as_float(0x7f800000)) finite += __ldg(v.wt + p);
+            finite = block_sum_u64(finite, sm.red);
+        }
+        L = w.L, R = w.R, it = w.it, pos = 0, st = kActive;
+        __syncthreads();
+    }
+    if (tid == 0) {
+        attempt();
         // the weight below the new bracket: below the old one plus the bins left of it
         w.below += sm.pre[pos];
         w.L = L;
@@ -3725,6 +3758,7 @@ __device__ __noinline__ void weighted_direct(const Level &v, int c, WeightSmem &
     __syncthreads();
 }
 
+template <bool kWide>
 __global__ void __launch_bounds__(kThreads, 4) k_whist(const __grid_constant__ Level v, uint32_t pieces) {
     pdl_enter();
     __shared__ WeightSmem sm;
@@ -3863,14 +3897,14 @@ __global__ void __launch_bounds__(kThreads, 4) k_whist(const __grid_constant__ L
                 w.tot = tot;
             }
             __syncthreads();
-            weighted_replay(v, cur, false, sm);
+            weighted_replay<kWide>(v, cur, false, sm);
             while (w.state == kActive) {  // the rest of the loop, on this CTA's own cell
                 clear();
                 fill_edges(sm.edge, w.L, w.R, w.K, tid, kThreads);
                 __syncthreads();
                 tile(w.base, w.end, false);
                 __syncthreads();
-                weighted_replay(v, cur, false, sm);
+                weighted_replay<kWide>(v, cur, false, sm);
             }
         } else {
             if (tid == 0 && first) {
@@ -3888,7 +3922,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_whist(const __grid_constant__ L
             }
             __syncthreads();
             last = w.last != 0;
-            if (last) weighted_replay(v, cur, true, sm);
+            if (last) weighted_replay<kWide>(v, cur, true, sm);
         }
         if (last && tid == 0) {
             orb_cell_t &cell = v.heap[level_slot(v, cur)];
@@ -4236,7 +4270,9 @@ void launch_level_kernel(Kernel k, const Level &v, int grid, int arg, cudaStream
     switch (k) {
         case kKPlan: launch_kernel(p, k_plan, dim3(per_cell_warps), T, 0, st, v); break;
         case kKHist:  // arg: 1 first pass, all cells dense; 2 first pass of a sampled level
-            if (arg == 2)
+            if (v.wide)
+                launch_kernel(p, arg == 2 ? k_hist<kHFirstSampled, kThreads, true> : k_hist<kHRest, kThreads, true>, dim3(grid), T, 0, st, v);
+            else if (arg == 2)
                 launch_kernel(p, k_hist<kHFirstSampled, kThreads>, dim3(grid), T, 0, st, v);
             else if (v.hist_threads == 1024)
                 launch_kernel(p, arg ? k_hist<kHFirstDense, 1024> : k_hist<kHRest, 1024>, dim3(grid), dim3(1024), 0, st, v);
@@ -4272,7 +4308,7 @@ void launch_level_kernel(Kernel k, const Level &v, int grid, int arg, cudaStream
             else
                 launch_kernel(p, k_part_finish<false>, dim3(per_cell_warps), T, 0, st, v, arg);
             break;
-        case kKWHist: launch_kernel(p, k_whist, dim3(grid), T, 0, st, v, (uint32_t)arg); break;
+        case kKWHist: launch_kernel(p, v.wide ? k_whist<true> : k_whist<false>, dim3(grid), T, 0, st, v, (uint32_t)arg); break;
         case kKCountLeft: launch_kernel(p, k_count_left, dim3(grid), T, 0, st, v); break;
         case kKSample:
             launch_kernel(p, k_sample_bin, dim3(kSampleMax / kSamplePerCta, (unsigned)min(v.C, 65535)),
