@@ -53,14 +53,19 @@ __device__ __forceinline__ void pdl_enter() {
 
 // A level may not start when a cell of the level above was never finished (its arrivals
 // never completed) or an earlier step flagged an error: the build is flagged and its
-// remaining kernels do nothing (ORB_ERR_TIMEOUT). Every thread of the CTA calls it and all get
-// the same answer: another CTA of the same kernel may flag the error meanwhile, and a warp that
-// left alone would leave the others at a barrier.
+// remaining kernels do nothing (ORB_ERR_TIMEOUT). The threads of a CTA decide alike without a vote
+// (one in every kernel cost a level 0.5 us): nothing counted in done[] changes below its level, and
+// the one kernel that can flag an error while its other CTAs start, k_part_classify, looks at
+// level_late() alone; a warp that left there without the others would leave them at a barrier.
+__device__ __forceinline__ bool level_late(const Level &v) {
+    if (v.prev_C && *(volatile const uint32_t *)&v.counters->done[v.depth - 1] != v.prev_C) {
+        if (threadIdx.x == 0) atomicExch(&v.counters->error, 1u);
+        return true;
+    }
+    return false;
+}
 __device__ __forceinline__ bool level_failed(const Level &v) {
-    const volatile BuildCounters *ctr = v.counters;
-    const bool late = v.prev_C && ctr->done[v.depth - 1] != v.prev_C;
-    if (late && threadIdx.x == 0) atomicExch(&v.counters->error, 1u);
-    return __syncthreads_or(late || ctr->error) != 0;
+    return *(volatile const uint32_t *)&v.counters->error || level_late(v);
 }
 
 // Arrival at a counter, by one thread after a barrier of its CTA: the CTA's writes before the
@@ -1643,7 +1648,7 @@ __global__ void __launch_bounds__(kThreads) k_part_classify(const __grid_constan
             v.tot_next->swaps = 0u;
         }
     }
-    if (level_failed(v)) return;
+    if (level_late(v)) return;  // (an error found meanwhile stops the next kernel)
     __shared__ uint32_t s_words[kThreads / 32][2][kPWords];
     __shared__ float s_lkey[kThreads / 32][kListStage];
     __shared__ uint32_t s_lpos[kThreads / 32][kListStage];
@@ -2684,7 +2689,6 @@ struct SubSmem {
     uint32_t more, direct;
     uint32_t max_it, unfound, degenerate;
     int item, root;
-    uint32_t lost;    // a copy's wait ran out
     alignas(8) unsigned long long arrived;  // mbarrier of the key copies
 };
 
@@ -2799,13 +2803,12 @@ __device__ __forceinline__ bool sub_group(const Level &v, uint32_t slice, uint32
     // Copies the n words at src into keys[off ...] (off: src's misalignment in words, so that
     // 16-byte pieces stay aligned on both sides): one bulk copy for the whole pieces, plain loads
     // for the rest. begin_load after a barrier that ends the keys' last use; end_load, then a
-    // barrier, before they are read, and the group leaves where any of its threads' waits ran out
-    // (sm.lost, read after that barrier). A wait polls at most v.copy_polls times (kCopyPolls: about
-    // a second, far beyond any copy).
+    // barrier, before they are read, and the group leaves if any of its threads' waits ran out
+    // (come_all). A wait polls at most v.copy_polls times (kCopyPolls: about a second, far beyond
+    // any copy).
     const uint32_t arrived = (uint32_t)__cvta_generic_to_shared(&sm.arrived);
     uint32_t parity = 0;
     if (ti == 0) {
-        sm.lost = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(arrived) : "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -2839,12 +2842,24 @@ __device__ __forceinline__ bool sub_group(const Level &v, uint32_t slice, uint32
                 : "memory");
         return ok != 0;
     };
-    auto end_load = [&]() {
-        if (!wait_copy(parity, v.copy_polls)) sm.lost = 1;
+    auto end_load = [&]() -> bool {
+        const bool ok = wait_copy(parity, v.copy_polls);
         parity ^= 1u;
+        return ok;
     };
-    // After the barrier behind end_load: the group leaves, its own copy (if one is under way after
-    // all) waited for once more.
+    // The barrier, and whether every thread came with `ok` (a vote in the barrier: a flag in shared
+    // memory made a tree of six levels 1% slower).
+    auto come_all = [&](bool ok) -> bool {
+        if (NW == 32) return __syncthreads_and(ok) != 0;
+        uint32_t all;
+        asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.and.pred q, %2, %3, p;\n selp.b32 %0, 1, 0, q;\n}"
+                     : "=r"(all)
+                     : "r"((uint32_t)ok), "r"(bar), "n"((int)NT)
+                     : "memory");
+        return all != 0;
+    };
+    // Where not all copies came: the group leaves, its own copy (if one is under way after all)
+    // waited for once more.
     auto leave = [&]() {
         if (ti == 0) atomicExch(&v.counters->error, 1u);
         if (!v.drop_copies) wait_copy(parity ^ 1u, kCopyPolls);
@@ -3005,16 +3020,12 @@ __device__ __forceinline__ bool sub_group(const Level &v, uint32_t slice, uint32
                 };
                 if (ti == 0) sm.direct = 0;
                 if (!((counted >> ax) & 1u)) {
-                    end_load();
-                    sync();
-                    if (sm.lost) return leave();
+                    if (!come_all(end_load())) return leave();
                 }
                 for (int r = 0; (counted >> ax) & 1u; ++r) {
                     for (uint32_t j = ti; j < kBins; j += NT) sm.bins[j] = 0u;
                     if (ti == 0) sm.more = 0;
-                    if (r == 0) end_load();
-                    sync();
-                    if (r == 0 && sm.lost) return leave();
+                    if (!come_all(r > 0 || end_load())) return leave();
                     bool any = false;
                     for (uint32_t q = q0; q < nq; q += qs) {
                         if (!counts(q)) continue;
@@ -3433,9 +3444,7 @@ __device__ __forceinline__ bool sub_group(const Level &v, uint32_t slice, uint32
             if (!n || !arr[a]) continue;  // (without particles the coordinates may be null)
             uint32_t *dst = arr[a] + first;
             if (a > 0) off = begin_load(dst, n);
-            end_load();
-            sync();
-            if (sm.lost) return leave();
+            if (!come_all(end_load())) return leave();
             const uint32_t *from = keys + off;
             uint32_t p = ti;
             for (; p + 7 * NT < n; p += 8 * NT) {

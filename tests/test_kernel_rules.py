@@ -24,14 +24,27 @@ def body(text, start):
 
 
 def test_a_cta_leaves_a_failed_level_as_a_whole():
-    """The error flag can be set while a kernel runs; a CTA whose threads each decided for
-    themselves could lose some of a named barrier's warps. So the one test of the flag ends in a
-    vote of the CTA, and is its only way out."""
+    """The classify pass sets the error flag while its other CTAs start, and its warps meet at named
+    barriers, which wait for warps that have left: it decides on the level above's count alone,
+    which no CTA of it changes. Every other kernel that flags an error is through with its own test
+    of the flag: the last of several passes does it, the first one tests."""
     text = source("orb_kernels.cu")
-    fail = body(text, r"bool level_failed\(const Level &v\)")
-    assert re.findall(r"return\b[^;]*;", fail) == ["return __syncthreads_or(late || ctr->error) != 0;"]
-    # and nothing else decides on the flag
-    assert not re.search(r"if \([^)]*error\b", text)
+    late = body(text, r"bool level_late\(const Level &v\)")
+    assert "done[v.depth - 1]" in late and late.count("error") == 1 and "atomicExch(&v.counters->error" in late
+    classify = body(text, r"k_part_classify\(const __grid_constant__ Level v\)")
+    assert "if (level_late(v)) return;" in classify and "level_failed" not in classify
+    flag = "atomicExch(&v.counters->error, 1u)"
+    setters = {m.start() for m in re.finditer(re.escape(flag), text)}
+    known = 0
+    for start, guard in [(r"bool level_late\(", "threadIdx.x == 0"), (r"k_part_classify\(", "lane == 0"),
+                         (r"void resolve_cell\(", "v.pass == v.last_pass"), (r"void __launch_bounds__\(kThreads, 4\) k_whist\(", "v.pass == v.last_pass"),
+                         (r"bool sub_group\(", "ti == 0")]:
+        block = body(text, start)
+        assert re.findall(r"if \(([^()]*)\) " + re.escape(flag), block) == [guard]
+        known += 1
+    assert len(setters) == known
+    for kernel in (r"void __launch_bounds__\(kThreads, 4\) k_whist\(", r"kHistBlocks512 : 1\)\) k_hist\("):
+        assert "if (v.pass == 0 && level_failed(v)) return;" in body(text, kernel)
 
 
 def test_an_acquire_is_followed_by_a_barrier():
@@ -46,13 +59,11 @@ def test_an_acquire_is_followed_by_a_barrier():
 
 def test_a_lost_copy_ends_its_group():
     """A wait for a copy that ran out leaves its barrier in a phase that must not be armed again:
-    the barrier behind every wait is followed by the group's way out."""
+    the barrier behind every wait is the group's way out."""
     text = source("orb_kernels.cu")
     group = body(text, r"bool sub_group\(")
-    waits = [m.end() for m in re.finditer(r"\bend_load\(\);", group)]
-    assert len(waits) == 3
-    for at in waits:
-        assert re.match(r"\s*sync\(\);\s*if \((r == 0 && )?sm\.lost\) return leave\(\);", group[at:])
+    assert len(re.findall(r"\bend_load\(\)", group)) == 3
+    assert len(re.findall(r"if \(!come_all\((r > 0 \|\| )?end_load\(\)\)\) return leave\(\);", group)) == 3
     kernel = body(text, r"void __launch_bounds__\(kSubThreads\) k_subtree\(")
     assert kernel.count("if (!__syncthreads_and(ok)) return;") == 3
 
