@@ -1179,6 +1179,32 @@ __device__ __noinline__ void resolve_cell(const Level &v, int c, const HistCell 
     uint8_t st = kActive;
     replay<kWide>(s_hist, kHistK, below, n, ratio, finite, L, R, it, pos, st);
     if (tid != 0) return;
+    uint32_t inb = 0;
+    bool inside = false;  // the later cuts lie in the bracket (where no midpoint can overflow)
+    if (st == kActive) {
+        // keys in the bracket the next step looks at, and keys below it
+        inb = (pos + 1 < kHistBins ? s_hist[pos + 1] : tot) - s_hist[pos];
+        inside = !(kWide && may_overflow(L, R));
+        // Where the bracket's lowest and highest counts give the same answer, so does every cut in
+        // it (the test is monotone in the count) and the loop ends without another count: many keys
+        // on or beyond the box's end, whose bracket narrows towards that end.
+        const int dir = convergence(below + s_hist[pos], n, ratio);
+        if (inside && dir == convergence(below + s_hist[pos] + inb, n, ratio)) {
+            while (st == kActive) {
+                if (it >= (uint32_t)kMaxIterations) {
+                    st = kCapped;
+                    break;
+                }
+                ++it;
+                if (dir == 0)
+                    st = kFound;
+                else if (dir > 0)
+                    R = mid_cut(L, R);
+                else
+                    L = mid_cut(L, R);
+            }
+        }
+    }
     cell.cutMarginLeft = L;
     cell.cutMarginRight = R;
     cell.foundCut = st == kFound ? 1 : 0;
@@ -1186,11 +1212,8 @@ __device__ __noinline__ void resolve_cell(const Level &v, int c, const HistCell 
     v.hdone[c] = 0;
     if (warm) v.warm[c] = 0;
     if (st == kActive) {
-        // keys in the bracket the next step looks at, and keys below it
-        const uint32_t inb = (pos + 1 < kHistBins ? s_hist[pos + 1] : tot) - s_hist[pos];
         v.inb[c] = inb;
-        // (no list where a midpoint can overflow: the cut can then leave the bracket)
-        if (inb <= list_capacity(v, n) && !(kWide && may_overflow(L, R))) {
+        if (inb <= list_capacity(v, n) && inside) {
             st = kReady;
             v.below[c] = below + s_hist[pos];
         } else {
@@ -2015,6 +2038,8 @@ struct CellsSmem {
     uint32_t cross;      // the tile where f crosses g
     uint2 swaps;         // the cell's pieces on the swap's list
     uint32_t last;       // the cell's other CTAs have arrived
+    int upper[32];       // each warp's cell that needs patch_upper (-1: none), and its cut
+    float cuts[32];
 };
 
 // The rest of the reference loop on at most 32 N bracket keys, N a lane (slots past them
@@ -2065,16 +2090,28 @@ __device__ __forceinline__ void patch_key(const Level &v, uint32_t t0, uint32_t 
 }
 
 // The final cut is the classify pass's upper bracket end: keys equal to it are <= cut too.
-// (Only a bracket a few floats wide ends there.) Sets their bits; threads ti of nt.
-__device__ __noinline__ void patch_upper(const Level &v, const orb_cell_t &cell, uint2 rg, uint32_t t0, float cut,
-                                         uint32_t ti, uint32_t nt) {
-    const float *keys = axis_keys(v, eff_axis(cell.cutAxis));
-    for (uint32_t p = rg.x + ti; p < rg.y; p += nt)
-        if (keys[p] == cut) {
-            const uint32_t rel = p - rg.x, t = t0 + rel / (uint32_t)kPTile, in = rel % (uint32_t)kPTile;
-            atomicOr(&v.le_bits[(size_t)t * kPWords + (in >> 5)], 1u << (in & 31u));
-            atomicAdd(&v.pt_le[t], 1u);
+// (Only a bracket a few floats wide ends there.) Sets their bits: a second read of the cell's
+// keys, warp `w` of `nw` taking every nw-th run of kUpperWords mask words, a lane a key.
+constexpr int kUpperWords = 16;
+__device__ __noinline__ void patch_upper(const Level &v, const float *keys, uint2 rg, uint32_t t0, float cut,
+                                         uint32_t w, uint32_t nw) {
+    const uint32_t lane = threadIdx.x & 31u, n = rg.y - rg.x, words = (n + 31u) / 32u;
+    for (uint32_t w0 = w * kUpperWords; w0 < words; w0 += nw * kUpperWords) {
+        float k[kUpperWords];
+#pragma unroll
+        for (int u = 0; u < kUpperWords; ++u) {
+            const uint32_t p = (w0 + (uint32_t)u) * 32u + lane;
+            k[u] = p < n ? __ldg(keys + rg.x + p) : __int_as_float(0x7fc00000);
         }
+#pragma unroll
+        for (int u = 0; u < kUpperWords; ++u) {
+            const uint32_t eq = __ballot_sync(0xffffffffu, k[u] == cut), word = w0 + (uint32_t)u;
+            if (eq && lane == 0) {  // (a cell's tiles are kPWords words each, one after the other)
+                atomicOr(&v.le_bits[(size_t)t0 * kPWords + word], eq);
+                atomicAdd(&v.pt_le[t0 + word / (uint32_t)kPWords], (uint32_t)__popc(eq));
+            }
+        }
+    }
 }
 
 // One warp: s and i of a cell from its tile prefixes and the crossing tile (see P2) and its
@@ -2142,14 +2179,21 @@ __device__ __forceinline__ void fill_swaps(const Level &v, int c, uint2 w, uint3
     for (uint32_t j = ti; j < w.y; j += nt) v.swap_list[w.x + j] = make_uint2((uint32_t)c, j);
 }
 
-// A cell of at most kWarpTiles tiles and kWarpList listed keys, by one warp.
-__device__ void cells_warp(const Level &v, int c) {
-    const uint32_t lane = threadIdx.x & 31;
+// A cell of at most kWarpTiles tiles and kWarpList listed keys, by one warp. Every warp of the CTA
+// calls it (c < 0: without a cell): cells that need patch_upper get it from all of them (by the
+// cell's own warp, 2^20 keys outside a box without extent took 29 ms; 1 ms with the CTA and the
+// loop ended by resolve_cell).
+__device__ void cells_warp(const Level &v, int c, CellsSmem &sm) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const bool any = c >= 0;
+    if (!any) c = 0;
     const int slot = level_slot(v, c);
     orb_cell_t &cell = v.heap[slot];
     const uint2 rg = v.ranges[slot];
     const uint32_t n = rg.y - rg.x, t0 = v.ptile_off[c], T = (n + (uint32_t)kPTile - 1) / (uint32_t)kPTile;
-    if (v.state[c] == kReady) {
+    bool upper = false;
+    float cut = 0.f;
+    if (any && v.state[c] == kReady) {
         const uint32_t m = v.cmp_cnt[c], off = v.cmp_off[c];
         const float ratio = leaf_ratio(cell.nLeafCells);  // src/orbit.cpp:204
         float L = cell.cutMarginLeft, R = cell.cutMarginRight;
@@ -2164,16 +2208,32 @@ __device__ void cells_warp(const Level &v, int c) {
         const int st = bisect_list(kl, v.below[c], n, ratio, L, R, it);
         __syncwarp();
         if (lane == 0) store_bisection(v, c, cell, L, R, it, st);
-        const float cut = mid_cut(L, R);
+        cut = mid_cut(L, R);
+        upper = cut == hi;
 #pragma unroll
         for (int q = 0; q < (int)kWarpList / 32; ++q) {
             const uint32_t j = (uint32_t)q * 32u + lane;
             if (j < m) patch_key(v, t0, v.cmp_pos[off + j] - rg.x, kl[q], cut);
         }
-        if (cut == hi) patch_upper(v, cell, rg, t0, cut, lane, 32);
         __threadfence();
         __syncwarp();
     }
+    if (__syncthreads_or(upper)) {
+        if (lane == 0) {
+            sm.upper[warp] = upper ? c : -1;
+            sm.cuts[warp] = cut;
+        }
+        __syncthreads();
+        for (uint32_t q = 0; q < nw; ++q) {
+            const int cq = sm.upper[q];
+            if (cq < 0) continue;
+            const int sq = level_slot(v, cq);
+            patch_upper(v, axis_keys(v, eff_axis(v.heap[sq].cutAxis)), v.ranges[sq], v.ptile_off[cq], sm.cuts[q], warp, nw);
+        }
+        __threadfence();
+        __syncthreads();
+    }
+    if (!any) return;
     // prefixes within the cell, tiles lane, 32 + lane, ... in a lane
     constexpr int kPer = (int)kWarpTiles / 32;
     uint32_t g[kPer], l[kPer], pg[kPer], pl[kPer];
@@ -2305,7 +2365,8 @@ __device__ void cells_cta(const Level &v, int c, uint32_t chunk, uint32_t nchunk
         __syncthreads();
         const float cut = mid_cut(sm.L, sm.R);
         for (uint32_t j = chunk * NT + tid; j < m; j += nchunks * NT) patch_key(v, t0, pos[j] - rg.x, keys[j], cut);
-        if (cut == hi) patch_upper(v, cell, rg, t0, cut, chunk * NT + tid, nchunks * NT);
+        if (cut == hi)
+            patch_upper(v, axis_keys(v, eff_axis(cell.cutAxis)), rg, t0, cut, chunk * (NT / 32) + tid / 32, nchunks * (NT / 32));
         __threadfence();
         __syncthreads();
     }
@@ -2394,8 +2455,8 @@ __global__ void __launch_bounds__(NT) k_part_cells(const __grid_constant__ Level
         __syncthreads();  // every thread has looked before the state changes
         if (!fits)
             cells_cta<NT>(v, c, blockIdx.x, gridDim.x, sm);
-        else if (warp == 0 && (gridDim.x == 1 || blockIdx.x == 0))
-            cells_warp(v, c);
+        else if (blockIdx.x == 0)
+            cells_warp(v, warp == 0 ? c : -1, sm);
         if (threadIdx.x == 0 && blockIdx.x == 0) add_bytes(v, kKPartCells, 512ull);
         return;
     }
@@ -2407,7 +2468,7 @@ __global__ void __launch_bounds__(NT) k_part_cells(const __grid_constant__ Level
     if ((threadIdx.x & 31) == 0 && c0 + warp < v.C && !fits_warp(c0 + warp)) atomicOr(&s_big, 1u << warp);
     __syncthreads();
     uint32_t big = s_big;
-    if (c0 + warp < v.C && !((big >> warp) & 1u)) cells_warp(v, c0 + warp);
+    cells_warp(v, c0 + warp < v.C && !((big >> warp) & 1u) ? c0 + warp : -1, sm);
     for (; big; big &= big - 1u) cells_cta<NT>(v, c0 + __ffs(big) - 1, 0u, 1u, sm);
     if (threadIdx.x == 0 && c0 < v.C) add_bytes(v, kKPartCells, 512ull * (unsigned)min(kW, v.C - c0));
 }
