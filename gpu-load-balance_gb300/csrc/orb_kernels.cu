@@ -837,7 +837,12 @@ __device__ __forceinline__ void dense_tile(const float *keys, uint32_t e0, uint3
 // the scaled guess (a key the guess does not settle exactly right after its round), keys at
 // or above R and NaN ignored. Same rounds as dense_tile; a key outside the bracket costs its
 // comparisons only (the dense loop would send each one through the exact path: clustered
-// cells' second passes ran at 1.7 TB/s that way).
+// cells' second passes ran at 1.7 TB/s that way). Where a round leaves a warp many keys they are
+// mostly equal ones, which kept their cell's bracket full (its bins are a few floats wide by then):
+// 32 at a time, the first one's bin is found once and takes all its equals in one addition. (Half
+// of 2^24 particles on one point, 2^13 leaves: passes two and three of a level 135 and 240 us with a
+// search and an addition a key.)
+constexpr uint32_t kTies = 64;  // many: more of a warp's 512
 template <uint32_t NT>
 __device__ __forceinline__ void bracket_tile(const float *keys, uint32_t e0, uint32_t e1, const Guess gs, float L,
                                              float R, uint32_t &below, uint32_t *s_hist, const float *s_edge) {
@@ -875,6 +880,28 @@ __device__ __forceinline__ void bracket_tile(const float *keys, uint32_t e0, uin
                 if (ok) atomicAdd(&s_hist[g], 1u);
                 if (!ok && kk[c] >= L && kk[c] < R) miss |= 1u << (4 * u + c);
             }
+        }
+        if (__reduce_add_sync(0xffffffffu, (uint32_t)__popc(miss)) > kTies) {
+            const uint32_t lane = ti & 31u;
+            float tie = __int_as_float(0x7fc00000);
+            uint32_t bin = 0;
+#pragma unroll 1
+            for (uint32_t b = 0; b < 4u * kHistVec; ++b) {
+                const bool in = (miss >> b) & 1u;
+                const uint32_t m = __ballot_sync(0xffffffffu, in);
+                if (!m) continue;
+                const float k = in ? __ldg(kb + 4 * (j0 + (b >> 2) * NT + ti) + (b & 3u)) : 0.0f;
+                const uint32_t first = (uint32_t)__ffs(m) - 1u;
+                const float t = __shfl_sync(0xffffffffu, k, (int)first);
+                if (t != tie) bin = near_bin(t, gs, s_edge, kHistBins - 1u);
+                tie = t;
+                const uint32_t same = __ballot_sync(0xffffffffu, in && k == t);
+                if (lane == first)
+                    atomicAdd(&s_hist[bin], (uint32_t)__popc(same));
+                else if (in && k != t)
+                    atomicAdd(&s_hist[near_bin(k, gs, s_edge, kHistBins - 1u)], 1u);
+            }
+            continue;
         }
         while (miss) {
             const uint32_t b = (uint32_t)__ffs(miss) - 1u;
