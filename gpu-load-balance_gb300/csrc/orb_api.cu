@@ -1745,6 +1745,23 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
         const size_t a = lv_off[l - 1], b = l < max_levels ? lv_off[l] : slots.size();
         lv.push_back({0, ctx->batch_slots.p + a, (int)(b - a), ctx->batch_child.p + a});
     }
+    // subtrees when every instance is built to its leaves; in warm builds the subtree levels
+    // bisect from each cell's extent (hints apply to the levels above them)
+    bool full = true;
+    uint64_t max_n = 0;
+    for (uint32_t i = 0; i < k; ++i) {
+        const Slices sl(inst[i].d);
+        full = full && sl.pow2 && lev[i] == sl.depth;
+        max_n = std::max<uint64_t>(max_n, inst[i].n);
+        if (wide_box(inst[i].lower, inst[i].upper)) v.wide = 1;
+    }
+    // warm: the subtree kernel only on levels that take no hints
+    const size_t hint_to = warm ? hint_levels(ctx, lv, max_n, full) : 0;
+    const int sub_from = hint_to == SIZE_MAX ? -1 : subtree_from(ctx, lv, max_n, full, hint_to);
+    if (sub_from >= 0) {
+        ORB_CUDA(ctx->sub_flag.ensure(1));
+        ORB_CUDA(ctx->sub_list.ensure(4 * (size_t)lv[sub_from].C));
+    }
     std::vector<uint64_t> key = level_key(ctx, v);
     key.push_back(warm ? 0xBA7C4A : 0xBA7C4);  // batched build (warm)
     key_add(key, v.hint);
@@ -1763,24 +1780,7 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
             key_add_f(key, inst[i].upper[a]);
         }
     }
-    // subtrees when every instance is built to its leaves; in warm builds the subtree levels
-    // bisect from each cell's extent (hints apply to the levels above them)
-    bool full = true;
-    uint64_t max_n = 0;
-    for (uint32_t i = 0; i < k; ++i) {
-        const Slices sl(inst[i].d);
-        full = full && sl.pow2 && lev[i] == sl.depth;
-        max_n = std::max<uint64_t>(max_n, inst[i].n);
-        if (wide_box(inst[i].lower, inst[i].upper)) v.wide = 1;
-    }
-    // warm: the subtree kernel only on levels that take no hints
-    const size_t hint_to = warm ? hint_levels(ctx, lv, max_n, full) : 0;
-    const int sub_from = hint_to == SIZE_MAX ? -1 : subtree_from(ctx, lv, max_n, full, hint_to);
     key.push_back((uint64_t)hint_to);
-    if (sub_from >= 0) {
-        ORB_CUDA(ctx->sub_flag.ensure(1));
-        ORB_CUDA(ctx->sub_list.ensure(4 * (size_t)lv[sub_from].C));
-    }
     key.push_back((uint64_t)(int64_t)sub_from);
     uint32_t passes = 0;
     st = run_graphed(ctx, key, &passes, [&](uint32_t *pp) -> orb_status {

@@ -83,3 +83,13 @@ def test_a_graph_is_replayed_with_the_buffers_it_was_captured_with():
     keyed |= {"tot", "tot_next"}  # inside the counters
     keyed |= {"out_counts", "cells_in"}  # service calls, which are not captured
     assert pointers - keyed == set()
+
+
+def test_buffers_are_sized_before_the_key_is_taken():
+    """A buffer that grows after its address went into the key would leave a graph under the key
+    of the buffer that was freed."""
+    api = source("orb_api.cu")
+    for build in (r"orb_status build_single\([^;{]*(?=\{)", r"orb_status build_batch_impl\([^;{]*(?=\{)"):
+        block = body(api, build)
+        key, run = block.index("level_key("), block.index("run_graphed(")
+        assert not [b for b in re.findall(r"ctx->(\w+)\.ensure\(", block[key:run]) if f"v.{b}" not in block[key:run]]
