@@ -113,13 +113,13 @@ struct orb_ctx {
     DevBuf<float2> hint;      // warm builds: starting bracket per heap slot
     DevBuf<int> hint_axis;
     DevBuf<uint8_t> warm;
-    DevBuf<uint32_t> sub_flag;  // subtree path taken (one word)
+    DevBuf<uint32_t> sub_flag;  // subtree path taken, largest cell (Level::skip)
     DevBuf<int> sub_list;       // the subtree kernel's cells by class
     DevBuf<uint32_t> w;         // weighted builds from host memory: the weights
     DevBuf<unsigned long long> gen_starts;  // xorshf96 generator: chunk start states
     DevBuf<unsigned long long> whist, wbelow, wtot;  // weighted builds: per-cell weight sums
     BuildCounters *h_counters = nullptr;  // pinned
-    uint32_t *h_sub_flag = nullptr;       // pinned: the subtree path was taken
+    uint32_t *h_sub_flag = nullptr;       // pinned: the two words of sub_flag
     char *h_tree = nullptr;               // pinned: small trees on their way to the caller
     size_t h_tree_bytes = 0;
 
@@ -580,9 +580,12 @@ uint32_t plan_bins(const orb_ctx *ctx, const Level &v, int C) { return v.wt && C
 // there takes 5-10 ps a particle where the level kernels take 7-12 (2^27 uniform, 2^26
 // clustered), and 20-30 us instead of 55 where the cells are few. full: every cell of every level
 // splits (batches: every tree is built to its leaves). from: the levels before it are level kernels' (staged builds).
-int subtree_from(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, uint64_t max_n, bool full, size_t from) {
+uint32_t most_subtree_levels(const orb_ctx *ctx) {
     const uint32_t tuned = ctx->tune.subtree_levels;
-    const uint32_t want = tuned < kSubDefaultLevels ? tuned : (uint32_t)kSubMaxLevels;
+    return tuned < kSubDefaultLevels ? tuned : (uint32_t)kSubMaxLevels;
+}
+int subtree_from(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, uint64_t max_n, bool full, size_t from) {
+    const uint32_t want = most_subtree_levels(ctx);
     if (!full || want == 0) return -1;
     for (size_t li = from; li < lv.size(); ++li) {
         if ((max_n >> li) + 1 + 8ull * li <= kSubMaxParticles && lv.size() - li <= want) return (int)li;
@@ -608,16 +611,14 @@ size_t hint_levels(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, uint64_
 // n: all particles; max_n: the largest instance's (cells of level l hold about max_n >> l;
 // levels whose cells can be large enough get a sampled first count pass (k_sample_bin,
 // k_sample_pick)).
-// rest = false: the levels above sub_from, then (sub_from >= 0) the subtree check and the
-// subtree kernel for the levels from sub_from down; rest = true: the levels from sub_from
-// down one by one, for builds whose subtree path the device refused.
-// [from, to): only those levels (staged builds run the levels in pieces).
+// [from, to): only those levels (staged builds run the levels in pieces); replan: the first of them
+// was not planned by the one above (builds whose subtree path the device refused).
 // v.hint set: levels below hint_to start from their hints (warm builds).
 orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, uint32_t *passes,
-                      int sub_from, uint64_t n, uint64_t max_n, bool rest = false, size_t from = 0,
-                      size_t to = SIZE_MAX, size_t hint_to = 0) {
+                      int sub_from, uint64_t n, uint64_t max_n, size_t from = 0, size_t to = SIZE_MAX,
+                      size_t hint_to = 0, bool replan = false) {
     to = std::min(to, lv.size());
-    for (size_t li = rest ? (size_t)sub_from : from; li < to; ++li) {
+    for (size_t li = from; li < to; ++li) {
         const LevelDesc &d = lv[li];
         v.base = d.base;
         v.slots = d.slots;
@@ -626,7 +627,7 @@ orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, u
         v.prev_C = li ? (uint32_t)lv[li - 1].C : 0u;
         v.tot = &ctx->counters.p->plan[li & 1];
         v.tot_next = &ctx->counters.p->plan[(li + 1) & 1];
-        if (!rest && (int)li == sub_from) {
+        if ((int)li == sub_from) {
             if (v.C == 0) break;
             v.skip = ctx->sub_flag.p;
             v.sub_list = ctx->sub_list.p;
@@ -640,14 +641,13 @@ orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, u
         v.small = small_cells(ctx, v, max_n, li, d.C);
         const bool hinted = v.hint && li < hint_to;
         v.next_C = 0;  // nothing to plan below the last level or at the subtree level
-        if (li + 1 < lv.size() && (rest || (int)li + 1 != sub_from)) {
+        if (li + 1 < lv.size() && (int)li + 1 != sub_from) {
             v.next_C = lv[li + 1].C;
             v.plan_bins = plan_bins(ctx, v, lv[li + 1].C);
             v.child_map = d.child_map;
             v.small_next = small_cells(ctx, v, max_n, li + 1, lv[li + 1].C);
         }
-        if (rest && (int)li == sub_from) {
-            // this level was not planned by the one above
+        if (replan && li == from) {
             ORB_CUDA(cudaMemsetAsync(&ctx->counters.p->plan[0], 0, 2 * sizeof(PlanTotals), ctx->stream));
             v.plan_hint = hinted ? 1 : 0;
             v.plan_bins = plan_bins(ctx, v, v.C);
@@ -750,39 +750,65 @@ bool build_finished(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, size_t
     return true;
 }
 
+// The level after `at`, whose largest cell of `largest` particles the subtree kernel refused, from
+// which it can try again (-1: none).
+int subtree_below(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, size_t at, uint32_t largest) {
+    if (largest == 0xffffffffu) return -1;
+    for (size_t li = at + 1; li < lv.size(); ++li)
+        if (((uint64_t)largest >> (li - at)) + 1 + 8ull * (li - at) <= kSubMaxParticles &&
+            lv.size() - li <= most_subtree_levels(ctx))
+            return (int)li;
+    return -1;
+}
+
 // After the main graph of a build: queues the copies of its tree; of one that planned subtrees
-// (sub_from >= 0): waits for it and reads whether the device took the subtree path (*taken). When it refused (a cell too large
-// for one CTA), a second graph runs the level kernels of the levels from sub_from down. The
-// build's end event is recorded again after it.
+// (*sub_from >= 0): waits for it and reads whether the device took the subtree path. When it refused
+// (a cell too large for one CTA), a second graph runs the level kernels from there down, and the
+// subtree kernel at the first level whose cells fit if the largest one halves (uneven cells: 2^24
+// particles on 1000 sites, 2^16 leaves, fit four levels above the leaves and not six); and so on
+// while the largest cell shrinks. The build's end event is recorded again after each. *sub_from: the
+// level the subtree kernel took (-1: none).
 orb_status finish_subtree_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv,
-                                 std::vector<uint64_t> key, uint32_t *passes, int sub_from,
-                                 uint64_t n, uint64_t max_n, size_t hint_to, const TreeOut &out, bool *taken) {
-    *taken = false;
+                                 const std::vector<uint64_t> &main_key, uint32_t *passes, int *sub_from,
+                                 uint64_t n, uint64_t max_n, size_t hint_to, const TreeOut &out) {
     if (!out.staged) {  // while the device builds
         touch_pages(out.heap, out.cells * sizeof(orb_cell_t));
         touch_pages(out.ranges, out.cells * sizeof(uint2));
     }
-    if (sub_from < 0) return queue_tree(ctx, out);
-    ORB_CUDA(cudaMemcpyAsync(ctx->h_sub_flag, ctx->sub_flag.p, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                             ctx->stream));
-    orb_status qst = queue_tree(ctx, out);  // (final when the subtree path was taken)
-    if (qst != ORB_OK) return qst;
-    ORB_CUDA(cudaStreamSynchronize(ctx->stream));
-    *taken = *ctx->h_sub_flag == 1u;
-    if (*taken) return ORB_OK;
-    if (ctx->use_graphs) collect_graph_profile(ctx);  // the main graph's kernel events
-    key.push_back(0x5E57u);  // the levels from sub_from down
-    v.skip = nullptr;
-    // warm builds: a refusal for another reason than the subtree kernel's shared memory leaves
-    // the levels to their hints
-    if (v.hint && *ctx->h_sub_flag == 0u) hint_to = SIZE_MAX;
-    key.push_back(hint_to == SIZE_MAX ? 1u : 0u);
-    orb_status st = run_graphed(ctx, key, passes, [&](uint32_t *pp) -> orb_status {
-        return run_levels(ctx, v, lv, pp, sub_from, n, max_n, true, 0, SIZE_MAX, hint_to);
-    });
-    if (st != ORB_OK) return st;
-    ORB_CUDA(cudaEventRecord(ctx->ev[1], ctx->stream));
-    return queue_tree(ctx, out);
+    uint32_t before = 0xffffffffu;  // the largest cell where the subtree kernel last refused
+    for (;;) {
+        if (*sub_from < 0) return queue_tree(ctx, out);
+        ORB_CUDA(cudaMemcpyAsync(ctx->h_sub_flag, ctx->sub_flag.p, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                 ctx->stream));
+        orb_status st = queue_tree(ctx, out);  // (final when the subtree path was taken)
+        if (st != ORB_OK) return st;
+        ORB_CUDA(cudaStreamSynchronize(ctx->stream));
+        if (ctx->h_sub_flag[0] == 1u) return ORB_OK;
+        if (ctx->use_graphs) collect_graph_profile(ctx);  // the graph's kernel events
+        const size_t at = (size_t)*sub_from;
+        const uint32_t largest = ctx->h_sub_flag[1];
+        v.skip = nullptr;
+        v.hwin = nullptr;
+        v.win_cnt = nullptr;
+        // warm builds: a refusal for another reason than the subtree kernel's shared memory leaves
+        // the levels to their hints
+        if (v.hint && before == 0xffffffffu && largest > kHintSubMax) hint_to = SIZE_MAX;
+        const bool hinted = v.hint && hint_to == SIZE_MAX;
+        *sub_from = hinted || largest >= before - before / 8 ? -1 : subtree_below(ctx, lv, at, largest);
+        before = largest;
+        if (*sub_from >= 0) ORB_CUDA(ctx->sub_list.ensure(4 * (size_t)lv[*sub_from].C));
+        std::vector<uint64_t> key = main_key;
+        key.push_back(0x5E57u);  // the levels from `at` down
+        key.push_back((uint64_t)at);
+        key.push_back((uint64_t)(int64_t)*sub_from);
+        key.push_back(hint_to == SIZE_MAX ? 1u : 0u);
+        key_add(key, ctx->sub_list.p);
+        st = run_graphed(ctx, key, passes, [&](uint32_t *pp) -> orb_status {
+            return run_levels(ctx, v, lv, pp, *sub_from, n, max_n, at, SIZE_MAX, hint_to, true);
+        });
+        if (st != ORB_OK) return st;
+        ORB_CUDA(cudaEventRecord(ctx->ev[1], ctx->stream));
+    }
 }
 
 }  // namespace
@@ -858,7 +884,7 @@ orb_status orb_ctx_create(int device, const orb_opts *opts, orb_ctx **out) {
             if (ew && ew[0]) ctx->e2e_windows = (uint32_t)std::min<long>(std::max<long>(0, std::atol(ew)), kMaxWindows);
         }
         if ((e = cudaMallocHost(reinterpret_cast<void **>(&ctx->h_counters), sizeof(BuildCounters))) != cudaSuccess ||
-            (e = cudaMallocHost(reinterpret_cast<void **>(&ctx->h_sub_flag), sizeof(uint32_t))) != cudaSuccess ||
+            (e = cudaMallocHost(reinterpret_cast<void **>(&ctx->h_sub_flag), 2 * sizeof(uint32_t))) != cudaSuccess ||
             (e = cudaHostAlloc(reinterpret_cast<void **>(&ctx->h_win), sizeof(HostWindows), cudaHostAllocMapped)) !=
                 cudaSuccess ||
             (e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&ctx->d_win), ctx->h_win, 0)) != cudaSuccess) {
@@ -1025,7 +1051,7 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     for (uint32_t l = 1; l <= levels; ++l) complete = complete && (uint64_t)sl.count(l) == 1ull << (l - 1);
     const int sub_from = subtree_from(ctx, lv, n, complete, staged ? 2 : 0);
     if (sub_from >= 0) {
-        ORB_CUDA(ctx->sub_flag.ensure(1));
+        ORB_CUDA(ctx->sub_flag.ensure(2));
         ORB_CUDA(ctx->sub_list.ensure(4 * (size_t)lv[sub_from].C));
     }
     if (!dev) {
@@ -1131,17 +1157,17 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
         v1.idx = ctx->idx.p;
         launch_init(v1, n, lower, upper, d, (int)heap_cells, s);
         ORB_CUDA(cudaGetLastError());
-        orb_status ls = run_levels(ctx, v1, lv, pp, sub_from, n, n, false, 0, 1);
+        orb_status ls = run_levels(ctx, v1, lv, pp, sub_from, n, n, 0, 1);
         if (ls != ORB_OK) return ls;
         ORB_CUDA(cudaStreamWaitEvent(s, ctx->y_ready, wf));
         run_stage_gather(ctx, dy, ctx->yraw.p, n);
         Level v2 = v1;  // level 2: x, y and the permutation
         v2.y = dy;
-        if ((ls = run_levels(ctx, v2, lv, pp, sub_from, n, n, false, 1, 2)) != ORB_OK) return ls;
+        if ((ls = run_levels(ctx, v2, lv, pp, sub_from, n, n, 1, 2)) != ORB_OK) return ls;
         ORB_CUDA(cudaStreamWaitEvent(s, ctx->yz_ready, wf));
         run_stage_gather(ctx, dz, ctx->zraw.p, n);
         ORB_CUDA(cudaGetLastError());
-        return run_levels(ctx, v, lv, pp, sub_from, n, n, false, 2);  // the rest
+        return run_levels(ctx, v, lv, pp, sub_from, n, n, 2);  // the rest
     });
     if (st != ORB_OK) return st;
     if (ctx->yz_pending || (!dev && n)) {
@@ -1198,15 +1224,15 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     if (!dev && perm) touch_pages(perm, n * sizeof(uint32_t));  // while the device builds
     bool streamed = false;
     if (windows && (st = stream_windows(&streamed)) != ORB_OK) return st;
-    bool taken = false;  // the subtree kernel finished the tree
+    int sub_taken = sub_from;  // the level from which the subtree kernel finished the tree
     const TreeOut out = tree_out(ctx, heap, ranges, heap_cells);
-    st = finish_subtree_levels(ctx, v, lv, key, &passes, sub_from, n, n, 0, out, &taken);
+    st = finish_subtree_levels(ctx, v, lv, key, &passes, &sub_taken, n, n, 0, out);
     if (st != ORB_OK) return st;
     bool written = false;  // the particles are in the host arrays (or on their way there)
     if (!dev) {
         ORB_CUDA(cudaStreamSynchronize(s));
         if (!win_started) ORB_CUDA(cudaEventElapsedTime(&h2d_ms, ctx->ev[2], ctx->ev[3]));
-        written = streamed && taken;
+        written = streamed && sub_taken == sub_from;
         if (!win_started) ORB_CUDA(cudaEventRecord(ctx->ev[2], s));
         if (n && !written) {
             ORB_CUDA(cudaMemcpyAsync(x, dx, n * sizeof(float), cudaMemcpyDeviceToHost, s));
@@ -1228,7 +1254,7 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     ORB_CUDA(cudaStreamSynchronize(s));
     if (on_cs) ORB_CUDA(cudaStreamSynchronize(ctx->copy_stream));
     take_tree(out);
-    if (!build_finished(ctx, lv, taken ? (size_t)sub_from : lv.size()))
+    if (!build_finished(ctx, lv, sub_taken >= 0 ? (size_t)sub_taken : lv.size()))
         return fail(ctx, ORB_ERR_TIMEOUT, kUnfinished);
     float dev_ms = 0.f;
     ORB_CUDA(cudaEventElapsedTime(&dev_ms, ctx->ev[0], ctx->ev[1]));
@@ -1759,7 +1785,7 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
     const size_t hint_to = warm ? hint_levels(ctx, lv, max_n, full) : 0;
     const int sub_from = hint_to == SIZE_MAX ? -1 : subtree_from(ctx, lv, max_n, full, hint_to);
     if (sub_from >= 0) {
-        ORB_CUDA(ctx->sub_flag.ensure(1));
+        ORB_CUDA(ctx->sub_flag.ensure(2));
         ORB_CUDA(ctx->sub_list.ensure(4 * (size_t)lv[sub_from].C));
     }
     std::vector<uint64_t> key = level_key(ctx, v);
@@ -1797,14 +1823,14 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
         v0.plan_hint = warm && hint_to > 0 ? 1 : 0;
         launch_init_batch(v0, ctx->batch_roots.p, (int)k, n_total, s);
         ORB_CUDA(cudaGetLastError());
-        return run_levels(ctx, v, lv, pp, sub_from, n_total, max_n, false, 0, SIZE_MAX, hint_to);
+        return run_levels(ctx, v, lv, pp, sub_from, n_total, max_n, 0, SIZE_MAX, hint_to);
     });
     if (st != ORB_OK) return st;
     ORB_CUDA(cudaEventRecord(ctx->ev[1], s));
     if (!dev && perm) touch_pages(perm, n_total * sizeof(uint32_t));  // while the device builds
-    bool taken = false;
+    int sub_taken = sub_from;
     const TreeOut out = tree_out(ctx, heaps, ranges, heap_cells);
-    st = finish_subtree_levels(ctx, v, lv, key, &passes, sub_from, n_total, max_n, hint_to, out, &taken);
+    st = finish_subtree_levels(ctx, v, lv, key, &passes, &sub_taken, n_total, max_n, hint_to, out);
     if (st != ORB_OK) return st;
     if (!dev) {
         ORB_CUDA(cudaStreamSynchronize(s));
@@ -1826,7 +1852,7 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
     }
     if (!dev) ORB_CUDA(cudaEventRecord(ctx->ev[3], s));
     ORB_CUDA(cudaStreamSynchronize(s));
-    if (!build_finished(ctx, lv, taken ? (size_t)sub_from : lv.size()))
+    if (!build_finished(ctx, lv, sub_taken >= 0 ? (size_t)sub_taken : lv.size()))
         return fail(ctx, ORB_ERR_TIMEOUT, kUnfinished);
     take_tree(out);
     // ranges relative to each instance (cells the build filled)

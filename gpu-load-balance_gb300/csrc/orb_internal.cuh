@@ -203,8 +203,8 @@ struct Level {
     const int *hint_axis;
     uint8_t *warm;          // [C] 1 while a hinted bracket is not yet checked
     int plan_hint;          // 1: the cells being planned start from their hints
-    // subtrees: 1 when one CTA per cell finishes the tree from this level down; null when
-    // not attempted
+    // subtrees: [0] 1 when one CTA per cell finishes the tree from this level down, [1] the level's
+    // largest cell (~0: no subtree would help); null when not attempted
     uint32_t *skip;
     int *sub_list;          // [4 C] the subtree kernel's cells by class
     int sub_levels;         // levels below every cell (0: by its leaf count)

@@ -2800,7 +2800,7 @@ __device__ __forceinline__ int levels_below(const Level &v, int leaves) {
 }
 
 // Flag for k_subtree: every cell of the level fits a CTA and has at most `max_levels`
-// (<= kSubLevels) levels below it. Then the cells with levels below them, by class (all of
+// (<= kSubLevels) levels below it; for the host, the largest cell. Then the cells with levels below them, by class (all of
 // the first class on levels of few cells, v.sub_wide), in order. One CTA.
 __global__ void __launch_bounds__(1024) k_subtree_check(const __grid_constant__ Level v, int max_levels) {
     pdl_enter();
@@ -2843,8 +2843,8 @@ __global__ void __launch_bounds__(1024) k_subtree_check(const __grid_constant__ 
     if (v.win_cnt)
         for (int w = threadIdx.x; w < kMaxWindows; w += blockDim.x) v.win_cnt[w] = 0u;
     if (threadIdx.x == 0) {
-        // 2: refused for this kernel's shared memory alone (see kHintSubMax)
-        *v.skip = take ? 1u : (!failed && mx <= kHintSubMax ? 2u : 0u);
+        v.skip[0] = take ? 1u : 0u;
+        v.skip[1] = failed || (int)ml > min(max_levels, kSubLevels) ? 0xffffffffu : mx;
         v.counters->sub_cells[0] = n0;
         v.counters->sub_cells[1] = n1;
         v.counters->sub_cells[2] = n2;
