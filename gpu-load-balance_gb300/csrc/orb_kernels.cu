@@ -3337,6 +3337,7 @@ __device__ __forceinline__ bool sub_group(const Level &v, uint32_t slice, uint32
                         if (ti < nq && mine(ti) && sm.state[ti].mode == kSubCount) {
                             SubState &s = sm.state[ti];
                             const float cut = mid_cut(s.L, s.R);
+                            const uint32_t was_l = __float_as_uint(s.L), was_r = __float_as_uint(s.R);
                             ++s.it;
                             const int dir = convergence(s.cnt, cells[ti].m, s.ratio);
                             if (dir == 0) {
@@ -3347,7 +3348,13 @@ __device__ __forceinline__ bool sub_group(const Level &v, uint32_t slice, uint32
                             } else {
                                 s.L = cut;
                             }
-                            if (dir != 0) sm.more = 1;
+                            // a bracket that stays as it is gives the same cut up to the cap
+                            if (dir != 0 && was_l == __float_as_uint(s.L) && was_r == __float_as_uint(s.R)) {
+                                s.it = kMaxIterations;
+                                s.mode = kSubDone;
+                            } else if (dir != 0) {
+                                sm.more = 1;
+                            }
                         }
                         sync();
                         const bool again = sm.more != 0;

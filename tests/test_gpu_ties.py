@@ -55,3 +55,14 @@ def test_a_box_without_extent_is_not_slow(fresh, oracle):
         return min(times[1:])
 
     assert ms(lower=(0, 0, 0), upper=(0, 0, 0)) < 10 * ms()
+
+
+@pytest.mark.parametrize("value", [0.123, 0.0, -0.5, 0.49999997])
+@pytest.mark.parametrize("n", [900, 5000, 15_000, 32_768])
+def test_equal_keys_in_a_subtree_match_oracle(fresh, oracle, n, value):
+    """Every cut is counted over all the keys, until the bracket is two neighbouring floats."""
+    x, y, z = (np.full(n, value, np.float32) for _ in range(3))
+    run_both(fresh, oracle, x, y, z, 64)
+    z = np.where(np.arange(n) % 3 == 0, np.nextafter(np.float32(value), np.float32(1)), z).astype(np.float32)
+    run_both(fresh, oracle, x, z, y, 64)
+    run_both(fresh, oracle, x, y, z, 64, lower=(-1.0, -2.0, -3.0), upper=(1.0, 2.0, 3.0))
