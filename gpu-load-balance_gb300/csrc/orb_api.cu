@@ -573,9 +573,17 @@ uint32_t small_cells(const orb_ctx *ctx, const Level &v, uint64_t max_n, size_t 
 // of them on a weighted level of few cells, whose tiles are dealt in pieces.
 uint32_t plan_bins(const orb_ctx *ctx, const Level &v, int C) { return v.wt && C <= ctx->num_sms ? 2u : 1u; }
 
+// Particles expected in the largest cell `down` levels below one of n particles and d leaves: its
+// share of the leaves (each split gives the left child the larger half, src/cell.h:88-92) plus a
+// few per split, which leaves a cell within 3 of its share. d = 0: halves (powers of two).
+uint64_t largest_cell(uint64_t n, uint32_t d, size_t down) {
+    uint64_t leaves = d;
+    for (size_t i = 0; i < down; ++i) leaves = (leaves + 1) / 2;
+    return (d ? (n * leaves + d - 1) / d : n >> down) + 1 + 8ull * down;
+}
+
 // The level from which subtree CTAs finish the tree (-1: none): the first level whose cells
-// (at most max_n >> l particles plus a few per split: each split leaves a cell within 3 of
-// half) all fit one CTA and that is at most kSubMaxLevels above the leaves
+// are expected to fit one CTA all and that is at most kSubMaxLevels above the leaves
 // (tune.subtree_levels below its default: at most that many). As many levels as fit: a level
 // there takes 5-10 ps a particle where the level kernels take 7-12 (2^27 uniform, 2^26
 // clustered), and 20-30 us instead of 55 where the cells are few. full: every cell of every level
@@ -584,11 +592,11 @@ uint32_t most_subtree_levels(const orb_ctx *ctx) {
     const uint32_t tuned = ctx->tune.subtree_levels;
     return tuned < kSubDefaultLevels ? tuned : (uint32_t)kSubMaxLevels;
 }
-int subtree_from(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, uint64_t max_n, bool full, size_t from) {
+int subtree_from(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, uint64_t max_n, uint32_t d, bool full, size_t from) {
     const uint32_t want = most_subtree_levels(ctx);
     if (!full || want == 0) return -1;
     for (size_t li = from; li < lv.size(); ++li) {
-        if ((max_n >> li) + 1 + 8ull * li <= kSubMaxParticles && lv.size() - li <= want) return (int)li;
+        if (largest_cell(max_n, d, li) <= kSubMaxParticles && lv.size() - li <= want) return (int)li;
     }
     return -1;
 }
@@ -752,10 +760,12 @@ bool build_finished(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, size_t
 
 // The level after `at`, whose largest cell of `largest` particles the subtree kernel refused, from
 // which it can try again (-1: none).
-int subtree_below(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, size_t at, uint32_t largest) {
+int subtree_below(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, size_t at, uint32_t largest, uint32_t d) {
     if (largest == 0xffffffffu) return -1;
+    uint32_t leaves = d;  // of a cell of that level
+    for (size_t i = 0; i < at; ++i) leaves = (leaves + 1) / 2;
     for (size_t li = at + 1; li < lv.size(); ++li)
-        if (((uint64_t)largest >> (li - at)) + 1 + 8ull * (li - at) <= kSubMaxParticles &&
+        if (largest_cell(largest, leaves, li - at) <= kSubMaxParticles &&
             lv.size() - li <= most_subtree_levels(ctx))
             return (int)li;
     return -1;
@@ -770,7 +780,7 @@ int subtree_below(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, size_t a
 // level the subtree kernel took (-1: none).
 orb_status finish_subtree_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv,
                                  const std::vector<uint64_t> &main_key, uint32_t *passes, int *sub_from,
-                                 uint64_t n, uint64_t max_n, size_t hint_to, const TreeOut &out) {
+                                 uint64_t n, uint64_t max_n, uint32_t d, size_t hint_to, const TreeOut &out) {
     if (!out.staged) {  // while the device builds
         touch_pages(out.heap, out.cells * sizeof(orb_cell_t));
         touch_pages(out.ranges, out.cells * sizeof(uint2));
@@ -794,7 +804,7 @@ orb_status finish_subtree_levels(orb_ctx *ctx, Level v, const std::vector<LevelD
         // the levels to their hints
         if (v.hint && before == 0xffffffffu && largest > kHintSubMax) hint_to = SIZE_MAX;
         const bool hinted = v.hint && hint_to == SIZE_MAX;
-        *sub_from = hinted || largest >= before - before / 8 ? -1 : subtree_below(ctx, lv, at, largest);
+        *sub_from = hinted || largest >= before - before / 8 ? -1 : subtree_below(ctx, lv, at, largest, d);
         before = largest;
         if (*sub_from >= 0) ORB_CUDA(ctx->sub_list.ensure(4 * (size_t)lv[*sub_from].C));
         std::vector<uint64_t> key = main_key;
@@ -1049,7 +1059,7 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     // leaf counts that are not powers of two), nor weighted builds
     bool complete = !weighted;
     for (uint32_t l = 1; l <= levels; ++l) complete = complete && (uint64_t)sl.count(l) == 1ull << (l - 1);
-    const int sub_from = subtree_from(ctx, lv, n, complete, staged ? 2 : 0);
+    const int sub_from = subtree_from(ctx, lv, n, sl.pow2 ? 0 : d, complete, staged ? 2 : 0);
     if (sub_from >= 0) {
         ORB_CUDA(ctx->sub_flag.ensure(2));
         ORB_CUDA(ctx->sub_list.ensure(4 * (size_t)lv[sub_from].C));
@@ -1226,7 +1236,7 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     if (windows && (st = stream_windows(&streamed)) != ORB_OK) return st;
     int sub_taken = sub_from;  // the level from which the subtree kernel finished the tree
     const TreeOut out = tree_out(ctx, heap, ranges, heap_cells);
-    st = finish_subtree_levels(ctx, v, lv, key, &passes, &sub_taken, n, n, 0, out);
+    st = finish_subtree_levels(ctx, v, lv, key, &passes, &sub_taken, n, n, sl.pow2 ? 0 : d, 0, out);
     if (st != ORB_OK) return st;
     bool written = false;  // the particles are in the host arrays (or on their way there)
     if (!dev) {
@@ -1783,7 +1793,7 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
     }
     // warm: the subtree kernel only on levels that take no hints
     const size_t hint_to = warm ? hint_levels(ctx, lv, max_n, full) : 0;
-    const int sub_from = hint_to == SIZE_MAX ? -1 : subtree_from(ctx, lv, max_n, full, hint_to);
+    const int sub_from = hint_to == SIZE_MAX ? -1 : subtree_from(ctx, lv, max_n, 0, full, hint_to);
     if (sub_from >= 0) {
         ORB_CUDA(ctx->sub_flag.ensure(2));
         ORB_CUDA(ctx->sub_list.ensure(4 * (size_t)lv[sub_from].C));
@@ -1830,7 +1840,7 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
     if (!dev && perm) touch_pages(perm, n_total * sizeof(uint32_t));  // while the device builds
     int sub_taken = sub_from;
     const TreeOut out = tree_out(ctx, heaps, ranges, heap_cells);
-    st = finish_subtree_levels(ctx, v, lv, key, &passes, &sub_taken, n_total, max_n, hint_to, out);
+    st = finish_subtree_levels(ctx, v, lv, key, &passes, &sub_taken, n_total, max_n, 0, hint_to, out);
     if (st != ORB_OK) return st;
     if (!dev) {
         ORB_CUDA(cudaStreamSynchronize(s));

@@ -73,3 +73,18 @@ def test_the_subtree_kernel_is_tried_again(fresh):
     x, y, z = sites(1 << 21, 130, (1 << 21) + 130)
     launches, levels = subtree_launches(fresh, x, y, z, 1 << 12)
     assert launches >= 2 and levels < 12
+
+
+@pytest.mark.parametrize("n,d", [(57_700, 7), (57_900, 7), (66_000, 7), (120_000, 13), (130_000, 9), (33_024 * 2 - 40, 3), (1 << 20, 65), (264_000, 33)])
+def test_odd_leaf_counts_are_not_refused(fresh, oracle, n, d):
+    """The larger children of odd leaf counts have more than half of the particles (4/7, 7/13, ...):
+    the level planned for the subtree kernel is one whose largest cell fits, so spread particles are
+    never refused (one check, one subtree launch, and no second graph)."""
+    x, y, z = oracle.gen_uniform(d, n)
+    run_both(fresh, oracle, x, y, z, d)
+    fresh.profile_reset()
+    gx, gy, gz = x.copy(), y.copy(), z.copy()
+    fresh.build(gx, gy, gz, d)
+    p = fresh.profile()
+    assert "plan" not in p  # launched by a second graph alone
+    assert p.get("subtree", {"launches": 0})["launches"] <= 1
