@@ -1791,9 +1791,12 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
         max_n = std::max<uint64_t>(max_n, inst[i].n);
         if (wide_box(inst[i].lower, inst[i].upper)) v.wide = 1;
     }
-    // warm: the subtree kernel only on levels that take no hints
+    // warm: the subtree kernel only on levels that take no hints; the first of them is where the
+    // device looks at the cells (kHintSubMax), fit for the kernel or not
     const size_t hint_to = warm ? hint_levels(ctx, lv, max_n, full) : 0;
-    const int sub_from = hint_to == SIZE_MAX ? -1 : subtree_from(ctx, lv, max_n, 0, full, hint_to);
+    const int sub_from = !warm                ? subtree_from(ctx, lv, max_n, 0, full, 0)
+                         : hint_to == SIZE_MAX ? -1
+                                               : (int)hint_to;
     if (sub_from >= 0) {
         ORB_CUDA(ctx->sub_flag.ensure(2));
         ORB_CUDA(ctx->sub_list.ensure(4 * (size_t)lv[sub_from].C));

@@ -36,9 +36,9 @@ constexpr int kHistBlocks512 = 3;  // ... and of its CTAs of 512 threads
 constexpr int kTileBlocksPerSm = 4;  // resident CTAs of the one-warp cell bisection
 constexpr uint32_t kSubMaxParticles = 33024;  // largest cell one subtree CTA takes (2^15 + 256)
 // Warm builds: hints apply to the levels above the first one of at least two cells per SM whose
-// cells have at most this many particles and that is at most tune.subtree_levels above the
-// leaves (which levels start from hints decides the trees, so the line stays where it was
-// whatever the subtree kernel takes).
+// cells are expected to have at most this many particles and that is at most tune.subtree_levels
+// above the leaves; where the device finds a larger cell there, to all levels. (Which levels start
+// from hints decides the trees, so the line stays where it was whatever the subtree kernel takes.)
 constexpr uint32_t kHintSubMax = 34816;
 constexpr uint32_t kSubDefaultLevels = 4;     // default of tune.subtree_levels
 constexpr int kSubMaxLevels = 6;              // deepest tree one subtree CTA finishes
