@@ -97,8 +97,10 @@ struct orb_ctx {
     // test hooks of the subtree kernel's waits (orb_test_set_scan_wait, orb_test_drop_copies)
     uint32_t copy_polls = kCopyPolls;
     bool drop_copies = false;
-    // launch tuning (orb_set_tuning / orb_autotune_batch); cta_min_cells = 0 means never
+    // launch tuning (orb_set_tuning / orb_autotune_batch); cta_min_cells = 0 means never.
+    // tuned: it was set; until then the subtree kernel takes as many levels as fit
     orb_tuning tune = {(uint32_t)kHistBlocksPerSm, 8u, (uint32_t)kTileBlocksPerSm, 64u, 0u, kSubDefaultLevels, 0u};
+    bool tuned = false;
     DevBuf<uint8_t> state, iters;
     DevBuf<uint32_t> cmp_off, cmp_cnt, cmp_pos, pred;
     DevBuf<float> cmp_keys;
@@ -492,6 +494,7 @@ std::vector<uint64_t> level_key(orb_ctx *ctx, const Level &v) {
     key.push_back(ctx->copy_polls);
     key.push_back(ctx->drop_copies ? 1u : 0u);
     key.push_back(ctx->use_pdl ? 1u : 0u);
+    key.push_back(ctx->tuned ? 1u : 0u);
     for (uint32_t t : {ctx->tune.hist_blocks_per_sm, ctx->tune.part_blocks_per_sm, ctx->tune.tile_blocks_per_sm,
                        ctx->tune.sparse_keys_per_tile, ctx->tune.cta_min_cells, ctx->tune.subtree_levels,
                        ctx->tune.predict_sigmas})
@@ -584,13 +587,12 @@ uint64_t largest_cell(uint64_t n, uint32_t d, size_t down) {
 
 // The level from which subtree CTAs finish the tree (-1: none): the first level whose cells
 // are expected to fit one CTA all and that is at most kSubMaxLevels above the leaves
-// (tune.subtree_levels below its default: at most that many). As many levels as fit: a level
+// (tune.subtree_levels where it was set). As many levels as fit: a level
 // there takes 5-10 ps a particle where the level kernels take 7-12 (2^27 uniform, 2^26
 // clustered), and 20-30 us instead of 55 where the cells are few. full: every cell of every level
 // splits (batches: every tree is built to its leaves). from: the levels before it are level kernels' (staged builds).
 uint32_t most_subtree_levels(const orb_ctx *ctx) {
-    const uint32_t tuned = ctx->tune.subtree_levels;
-    return tuned < kSubDefaultLevels ? tuned : (uint32_t)kSubMaxLevels;
+    return ctx->tuned ? ctx->tune.subtree_levels : (uint32_t)kSubMaxLevels;
 }
 int subtree_from(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, uint64_t max_n, uint32_t d, bool full, size_t from) {
     const uint32_t want = most_subtree_levels(ctx);
@@ -1982,6 +1984,7 @@ orb_status orb_set_tuning(orb_ctx *ctx, const orb_tuning *t) {
     ctx->err.clear();
     if (!t || !tuning_valid(*t)) return fail(ctx, ORB_ERR_INVALID_ARGUMENT, "tuning parameter out of range");
     ctx->tune = *t;
+    ctx->tuned = true;
     return ORB_OK;
 }
 
@@ -2018,6 +2021,7 @@ orb_status orb_autotune_batch(orb_ctx *ctx, const float *x, const float *y, cons
     // median device time of `reps` builds (after one untimed build: graph capture)
     auto trial = [&](const orb_tuning &t, float *ms) -> orb_status {
         ctx->tune = t;
+        ctx->tuned = true;
         std::vector<float> times;
         for (uint32_t r = 0; r <= reps; ++r) {
             for (int a = 0; a < 3; ++a)
@@ -2046,11 +2050,14 @@ orb_status orb_autotune_batch(orb_ctx *ctx, const float *x, const float *y, cons
         return ORB_OK;
     };
     const orb_tuning start = ctx->tune;
+    const bool was_tuned = ctx->tuned;
     orb_tuning cur = start;
+    cur.subtree_levels = most_subtree_levels(ctx);  // what builds do now
     float cur_ms = 0.f;
     orb_status st = trial(cur, &cur_ms);
     if (st != ORB_OK) {
         ctx->tune = start;
+        ctx->tuned = was_tuned;
         return st;
     }
     // coordinate descent over result-invariant parameters
@@ -2079,6 +2086,7 @@ orb_status orb_autotune_batch(orb_ctx *ctx, const float *x, const float *y, cons
             st = trial(t, &ms);
             if (st != ORB_OK) {
                 ctx->tune = start;
+                ctx->tuned = was_tuned;
                 return st;
             }
             if (ms < 0.98f * cur_ms) {  // keep a candidate only for a clear gain

@@ -223,10 +223,10 @@ typedef struct orb_tuning {
                                       1..16384 (default 64) */
     uint32_t cta_min_cells;        /* levels with at least this many cells bisect one cell per
                                       CTA; 0 = never (default) */
-    uint32_t subtree_levels;       /* the last levels are finished by one CTA per cell once every
-                                      cell of a level fits one (at most 33024 particles): 0 never,
-                                      1..3 at most that many levels, 4 (default) and more as many
-                                      as fit, at most 6 */
+    uint32_t subtree_levels;       /* the last levels (at most this many, 0..6) are finished by one
+                                      CTA per cell once every cell of a level fits one (at most
+                                      33024 particles); 0 = never. Reads 4 until a tuning is set
+                                      and, until then, stands for as many as fit, at most 6 */
     uint32_t predict_sigmas;       /* first count pass of cells of at least 2^18 particles: the
                                       keys are binned only inside a bracket predicted from a
                                       strided sample (its median +- this many standard errors),
