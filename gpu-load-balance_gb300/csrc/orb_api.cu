@@ -543,7 +543,8 @@ orb_status run_bisection(orb_ctx *ctx, Level v, uint64_t n, uint32_t *passes, in
     v.last_pass = npasses - 1;
     // few tiles: larger CTAs, at most one tile each (a level of 2^20 particles, 64 tiles: 15.4 ->
     // 12.3 us with 1024 threads; of 4.1 million, 250 tiles: 26 -> 19.5 us with 512)
-    v.hist_threads = tiles <= (uint64_t)ctx->num_sms ? 1024 : (tiles <= kHistBlocks512 * (uint64_t)ctx->num_sms ? 512 : kThreads);
+    const uint64_t most = std::min<uint32_t>(kHistBlocks512, ctx->tune.hist_blocks_per_sm);  // CTAs per SM
+    v.hist_threads = tiles <= (uint64_t)ctx->num_sms ? 1024 : (tiles <= most * (uint64_t)ctx->num_sms ? 512 : kThreads);
     if (first == 2 || v.wide) v.hist_threads = kThreads;
     for (int pass = 0; pass < npasses; ++pass) {
         v.pass = pass;

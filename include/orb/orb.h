@@ -214,7 +214,8 @@ orb_status orb_build_warm(orb_ctx *ctx, float *x, float *y, float *z, uint64_t n
  * order are the same under any valid setting.
  */
 typedef struct orb_tuning {
-    uint32_t hist_blocks_per_sm;   /* count-left pass: CTAs per SM, 1..8 (default 6) */
+    uint32_t hist_blocks_per_sm;   /* count-left pass: CTAs per SM at most, 1..8 (default 6); levels
+                                      of few tiles take fewer and larger ones */
     uint32_t part_blocks_per_sm;   /* partition passes: CTAs per SM, 1..16 (default 8) */
     uint32_t tile_blocks_per_sm;   /* one-warp cell bisection: CTAs per SM, 1..8 (default 4) */
     uint32_t sparse_keys_per_tile; /* list threshold: a cell's bisection is finished on the list

@@ -93,3 +93,11 @@ def test_buffers_are_sized_before_the_key_is_taken():
         block = body(api, build)
         key, run = block.index("level_key("), block.index("run_graphed(")
         assert not [b for b in re.findall(r"ctx->(\w+)\.ensure\(", block[key:run]) if f"v.{b}" not in block[key:run]]
+
+
+def test_the_count_passes_keep_to_their_ctas_per_sm():
+    """hist_blocks_per_sm bounds the count passes' CTAs on every level, those of few tiles too, whose
+    CTAs are larger and take a tile each."""
+    block = body(source("orb_api.cu"), r"orb_status run_bisection\([^{]*(?=\{)")
+    most = re.search(r"most = std::min<uint32_t>\(kHistBlocks512, ctx->tune\.hist_blocks_per_sm\);", block)
+    assert most and "tiles <= (uint64_t)ctx->num_sms ? 1024 : (tiles <= most * (uint64_t)ctx->num_sms ? 512 : kThreads)" in block
