@@ -201,9 +201,12 @@ namespace orb {
 // resident and writable first, in one call that leaves their bytes alone, while the device
 // works where there is work to wait for. (Reading and writing back a byte a page took 19 ms: the
 // read maps the shared zero page, whose replacement the GPU's address translation must see.)
-// Memory it does not apply to (page-locked, device-mapped) is left as it is.
-void touch_pages(void *ptr, size_t bytes) {
-    if (!ptr || !bytes) return;
+// Memory it does not apply to (page-locked, device-mapped) is left as it is. Where no device work
+// hides the call (meanwhile = false), arrays below 1 MiB go without: an allocator mostly hands out
+// resident pages up to that size, and four calls took 4-6 us of a store's 40-54.
+constexpr size_t kTouchBytes = 1u << 20;
+void touch_pages(void *ptr, size_t bytes, bool meanwhile) {
+    if (!ptr || !bytes || (!meanwhile && bytes < kTouchBytes)) return;
     static const uintptr_t page = [] {
         const long v = sysconf(_SC_PAGESIZE);
         return v > 0 ? (uintptr_t)v : (uintptr_t)4096;
@@ -785,8 +788,8 @@ orb_status finish_subtree_levels(orb_ctx *ctx, Level v, const std::vector<LevelD
                                  const std::vector<uint64_t> &main_key, uint32_t *passes, int *sub_from,
                                  uint64_t n, uint64_t max_n, uint32_t d, size_t hint_to, const TreeOut &out) {
     if (!out.staged) {  // while the device builds
-        touch_pages(out.heap, out.cells * sizeof(orb_cell_t));
-        touch_pages(out.ranges, out.cells * sizeof(uint2));
+        touch_pages(out.heap, out.cells * sizeof(orb_cell_t), true);
+        touch_pages(out.ranges, out.cells * sizeof(uint2), true);
     }
     uint32_t before = 0xffffffffu;  // the largest cell where the subtree kernel last refused
     for (;;) {
@@ -1234,7 +1237,7 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
         return ORB_OK;
     };
     ORB_CUDA(cudaEventRecord(ctx->ev[1], s));
-    if (!dev && perm) touch_pages(perm, n * sizeof(uint32_t));  // while the device builds
+    if (!dev && perm) touch_pages(perm, n * sizeof(uint32_t), true);  // while the device builds
     bool streamed = false;
     if (windows && (st = stream_windows(&streamed)) != ORB_OK) return st;
     int sub_taken = sub_from;  // the level from which the subtree kernel finished the tree
@@ -1416,7 +1419,7 @@ orb_status orb_generate(orb_ctx *ctx, int kind, uint64_t seed, uint64_t n, float
     }
     ORB_CUDA(cudaGetLastError());
     if (!dev) {
-        for (void *p : {(void *)x, (void *)y, (void *)z}) touch_pages(p, n * sizeof(float));
+        for (void *p : {(void *)x, (void *)y, (void *)z}) touch_pages(p, n * sizeof(float), false);
         ORB_CUDA(cudaMemcpyAsync(x, dx, n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
         ORB_CUDA(cudaMemcpyAsync(y, dy, n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
         ORB_CUDA(cudaMemcpyAsync(z, dz, n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1476,7 +1479,7 @@ orb_status orb_store_particles(orb_ctx *ctx, float *x, float *y, float *z, uint3
     cudaStream_t s = ctx->stream;
     if (n) {
         if (k == cudaMemcpyDeviceToHost)
-            for (void *p : {(void *)x, (void *)y, (void *)z, (void *)perm}) touch_pages(p, n * sizeof(float));
+            for (void *p : {(void *)x, (void *)y, (void *)z, (void *)perm}) touch_pages(p, n * sizeof(float), false);
         ORB_CUDA(cudaMemcpyAsync(x, ctx->x.p, n * sizeof(float), k, s));
         ORB_CUDA(cudaMemcpyAsync(y, ctx->y.p, n * sizeof(float), k, s));
         ORB_CUDA(cudaMemcpyAsync(z, ctx->z.p, n * sizeof(float), k, s));
@@ -1843,7 +1846,7 @@ static orb_status build_batch_impl(orb_ctx *ctx, float *x, float *y, float *z, u
     });
     if (st != ORB_OK) return st;
     ORB_CUDA(cudaEventRecord(ctx->ev[1], s));
-    if (!dev && perm) touch_pages(perm, n_total * sizeof(uint32_t));  // while the device builds
+    if (!dev && perm) touch_pages(perm, n_total * sizeof(uint32_t), true);  // while the device builds
     int sub_taken = sub_from;
     const TreeOut out = tree_out(ctx, heaps, ranges, heap_cells);
     st = finish_subtree_levels(ctx, v, lv, key, &passes, &sub_taken, n_total, max_n, 0, hint_to, out);

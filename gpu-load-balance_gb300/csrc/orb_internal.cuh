@@ -340,7 +340,7 @@ void launch_gen_plummer(uint64_t seed, uint64_t n, const float *centres, const d
                         float *x, float *y, float *z, cudaStream_t st);
 
 // Makes the pages of a host buffer resident (its bytes keep their values), see orb_api.cu.
-void touch_pages(void *ptr, size_t bytes);
+void touch_pages(void *ptr, size_t bytes, bool meanwhile);
 
 // Context internals used by the request server (orb_server.cu).
 cudaStream_t ctx_stream(orb_ctx *ctx);

@@ -530,7 +530,7 @@ orb_status orb_server_fetch(orb_server *sv, uint64_t instance_id, orb_cell_t *he
     cudaSetDevice(sv->device);
     cudaError_t e = cudaSuccess;
     if (n) {
-        for (void *p : {(void *)x, (void *)y, (void *)z, (void *)ident}) orb::touch_pages(p, n * 4);
+        for (void *p : {(void *)x, (void *)y, (void *)z, (void *)ident}) orb::touch_pages(p, n * 4, false);
         if (x && !e) e = cudaMemcpy(x, sv->ax + off, n * 4, cudaMemcpyDeviceToHost);
         if (y && !e) e = cudaMemcpy(y, sv->ay + off, n * 4, cudaMemcpyDeviceToHost);
         if (z && !e) e = cudaMemcpy(z, sv->az + off, n * 4, cudaMemcpyDeviceToHost);
