@@ -56,7 +56,7 @@ TRAFFIC_PROFILE = "dram_traffic_part_swap_hist_classify_subtree_2p24_2p13.txt"
 # every kernel kind that counts keys below a cut (the count-left family)
 COUNT_LEFT_KERNELS = ("count_left_hist", "bisect_tile", "bisect_cta", "count_left_sample",
                       "count_left_sample_pick")
-PARTITION_KERNELS = ("part_classify", "part_scan", "part_cells", "part_swap", "part_finish")
+PARTITION_KERNELS = ("part_classify", "part_cells", "part_swap", "part_finish")
 
 
 def workload_name(kind: str, n: int, d: int) -> str:

@@ -1,10 +1,10 @@
 // Host driver and C ABI of the ORB engine (include/orb/orb.h).
 //
 // orb_build runs the reference's master() level loop (src/orbit.cpp:102-275) with every
-// step on the device: per level a plan, histogram/resolve passes that replay the
-// bisection, the parallel Hoare partition and the split, and the last levels one CTA per
-// cell. The work is captured in CUDA graphs and replayed; the host reads one flag per build
-// (whether the device took the subtree path for the last levels).
+// step on the device: per level the histogram passes that replay the bisection, the parallel
+// Hoare partition and the split, which plans the next level, and the last levels one CTA per
+// cell. The work is captured in CUDA graphs and replayed; the host reads two words per build
+// (whether the device took the subtree path for the last levels, else its largest cell).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -594,7 +594,8 @@ uint64_t largest_cell(uint64_t n, uint32_t d, size_t down) {
 // (tune.subtree_levels where it was set). As many levels as fit: a level
 // there takes 5-10 ps a particle where the level kernels take 7-12 (2^27 uniform, 2^26
 // clustered), and 20-30 us instead of 55 where the cells are few. full: every cell of every level
-// splits (batches: every tree is built to its leaves). from: the levels before it are level kernels' (staged builds).
+// splits (batches: every tree is built to its leaves). from: the levels before it are the level
+// kernels' (staged builds). d as in largest_cell().
 uint32_t most_subtree_levels(const orb_ctx *ctx) {
     return ctx->tuned ? ctx->tune.subtree_levels : (uint32_t)kSubMaxLevels;
 }
@@ -618,7 +619,8 @@ size_t hint_levels(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, uint64_
 }
 
 // The reference's level loop (src/orbit.cpp:102-275) over every cell of every level: the
-// bisection (one warp for small cells, the histogram passes for the rest, or one CTA per cell), then the partition, which also splits the cells and plans the next level.
+// bisection (one warp for small cells, the histogram passes for the rest, or one CTA per cell),
+// then the partition, which also splits the cells and plans the next level.
 // The first level's cells are planned by the init kernel.
 // sub_from >= 0: from level lv[sub_from] down, one CTA per cell finishes the tree when every
 // cell of that level fits one (k_subtree_check decides on the device).
@@ -765,7 +767,7 @@ bool build_finished(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, size_t
 }
 
 // The level after `at`, whose largest cell of `largest` particles the subtree kernel refused, from
-// which it can try again (-1: none).
+// which it can try again (-1: none). d as in largest_cell().
 int subtree_below(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, size_t at, uint32_t largest, uint32_t d) {
     if (largest == 0xffffffffu) return -1;
     uint32_t leaves = d;  // of a cell of that level

@@ -19,9 +19,8 @@ constexpr int kTile = 16384;         // keys per tile of the count-left passes
 constexpr int kPTile = 4096;         // positions per tile of the partition passes
 constexpr int kPWords = kPTile / 32; // bitmask words per partition tile
 constexpr int kMaxBinsLog2 = 11;     // deepest midpoint tree one histogram pass resolves
-// Histogram passes per level. The count passes bisect cells of more than kTile keys, whose
-// trees have depth 11 (tree_depth), so 3 passes (33 iterations) reach the 32-iteration cap
-// of every cell. A first pass that is discarded (a warm or sampled bracket that missed the
+// Histogram passes per level: their midpoint trees have depth 11, so 3 passes (33 iterations)
+// reach the 32-iteration cap of every cell. A first pass that is discarded (a warm or sampled bracket that missed the
 // cut) costs one more, hence 4 for levels that may have one.
 constexpr int kHistPasses = 4;
 constexpr int kColdHistPasses = 3;
@@ -106,7 +105,7 @@ struct BuildCounters {
     uint32_t unfound;
     uint32_t max_iters;
     uint32_t any_active[4];  // histogram pass p left a cell active
-    uint32_t error;       // set when a bounded device wait gave up
+    uint32_t error;       // set when a step could not be finished (see level_late, k_subtree's waits)
     uint32_t done[kMaxLevels + 1];  // cells whose children (or leaves) are final, per level
     PlanTotals plan[2];   // levels 1, 3, ... and 2, 4, ...
     uint32_t warm_cells;  // warm builds: cells that started from a hinted bracket

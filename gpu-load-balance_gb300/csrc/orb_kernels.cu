@@ -95,7 +95,7 @@ __device__ __forceinline__ uint32_t warp_max(uint32_t v) {
     return v;
 }
 
-// Sum over the block; every thread gets the total. `sh` holds >= 32 words.
+// Exclusive scan over the warp (lane order); every lane gets the total.
 __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, uint32_t *total) {
     const int lane = threadIdx.x & 31;
     uint32_t inc = v;
@@ -108,6 +108,7 @@ __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, uint32_t *total) 
     return inc - v;
 }
 
+// Sum over the block; every thread gets the total. `sh` holds >= 32 words.
 __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t *sh) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     v = warp_sum(v);
@@ -2726,7 +2727,7 @@ __global__ void __launch_bounds__(kThreads) k_part_finish(const __grid_constant_
 // loop moves that margin (the float test is monotone in the count), and a cut inside the
 // window gets its exact count from the list. A cell whose replay meets a cut the window
 // cannot settle (many equal keys, a box far wider than its keys) counts every cut over all
-// its keys instead. Same cuts, same integer counts, same iterations on every path.
+// its keys instead, until its bracket is two neighbouring floats. Same cuts, same integer counts, same iterations on every path.
 //
 // A group is the CTA's 32 warps, or 16, 8 or 2 of them for smaller cells (by size): small
 // cells are bound by the latency of their steps, so an SM keeps 2, 4 or 16 in flight. (Cells of

@@ -415,7 +415,7 @@ orb_status orb_count_left_static(const float *x, const float *y, const float *z,
  * kernels, which then do nothing, and by the host at the build's end: the build returns
  * ORB_ERR_TIMEOUT and the context stays usable. ticket_start (0..255, normally 0) makes every
  * cell's arrivals start that far below zero, so that with 1 the last one is never counted.
- * spin_limit: the most polls (of about a microsecond) of the one device wait there is, the
+ * spin_limit: the most polls (of about 4 microseconds) of the one device wait there is, the
  * subtree kernel's for its own copies of keys (0: the default, about a second). A wait that
  * runs out flags the build, which returns ORB_ERR_TIMEOUT; the context stays usable.
  * orb_test_drop_copies(on = 1) leaves those copies out, so that every such wait runs out with

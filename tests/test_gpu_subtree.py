@@ -1,5 +1,5 @@
-"""The subtree kernel at the cell sizes where its groups of warps change (1088, 6656, 14848 and
-33024 particles), one to six levels deep, on keys that its key windows settle and on keys that
+"""The subtree kernel at the cell sizes where its groups of warps change (1088, 6656 and 33024
+particles; the fourth edge, 16400, is in test_gpu_subtree_levels.py), one to six levels deep, on keys that its key windows settle and on keys that
 they do not (a few neighbouring floats, many keys on the box ends and on cuts, NaN, a box far
 wider than its keys). Alone and with every size in one batch. Bit for bit against the oracle."""
 import numpy as np

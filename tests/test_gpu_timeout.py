@@ -1,12 +1,12 @@
-"""Failure detection without a GPU fault: a bounded device wait that runs out.
+"""Failure detection without a GPU fault: cells whose tiles never all report.
 
-The partition's tile scan chains its blocks with a decoupled look-back, each wait bounded
-(orb_test_set_scan_wait sets the bound). Starting the scan's block ticket at 1 leaves the
-first status slot unpublished, so the next block's wait can only end by giving up. It must
-give up within its bound, flag the build (the kernels that read the scan's prefixes then do
-nothing) and orb_build must return ORB_ERR_TIMEOUT; the same context must then build the
-oracle's tree bit for bit. The reference has no such path: its errors end the process
-(src/constants.h:19-23)."""
+The partition's tiles count their arrivals per cell and whoever brings the last one finishes the
+cell. orb_test_set_scan_wait(.., 1) starts the counts one below zero, so that the last arrival is
+never counted (its first argument, the polls of the subtree kernel's waits, plays no part here: see
+test_gpu_copy_wait.py). The next level's kernels see the missing cell and do nothing, and orb_build
+must return ORB_ERR_TIMEOUT; the same context must then build the oracle's tree bit for bit. (The
+names below are from a scan with a look-back wait, which this replaced.) The reference has no such
+path: its errors end the process (src/constants.h:19-23)."""
 import numpy as np
 import pytest
 

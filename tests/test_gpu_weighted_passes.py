@@ -1,5 +1,5 @@
 """The weighted pass where its ways of bisecting a cell change: cells one CTA holds in registers
-(up to 2048 keys), in shared bins (one tile), in several tiles and in pieces dealt to several
+(up to 4096 keys), in shared bins (one tile), in several tiles and in pieces dealt to several
 CTAs, weights on both sides of what their 16-bit halves and 32-bit sums take, and totals on both
 sides of 2^32 (the 64-bit and the 128-bit form of the test). Bit for bit against the oracle."""
 import numpy as np
