@@ -789,19 +789,42 @@ int subtree_below(const orb_ctx *ctx, const std::vector<LevelDesc> &lv, size_t a
 orb_status finish_subtree_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv,
                                  const std::vector<uint64_t> &main_key, uint32_t *passes, int *sub_from,
                                  uint64_t n, uint64_t max_n, uint32_t d, size_t hint_to, const TreeOut &out) {
-    if (!out.staged) {  // while the device builds
-        touch_pages(out.heap, out.cells * sizeof(orb_cell_t), true);
-        touch_pages(out.ranges, out.cells * sizeof(uint2), true);
-    }
+    // the result's pages are made resident while the device builds, a few MiB at a time: the host
+    // goes on as soon as the device has decided
+    size_t touched = 0;
+    const size_t heap_bytes = out.cells * sizeof(orb_cell_t), bytes = out.staged ? 0 : heap_bytes + out.cells * sizeof(uint2);
+    auto touch_some = [&]() -> bool {  // false: all of them are
+        const size_t at = touched, in_heap = at < heap_bytes ? heap_bytes - at : 0;
+        if (at >= bytes) return false;
+        const size_t k = std::min<size_t>(in_heap ? in_heap : bytes - at, 4u << 20);
+        touch_pages(in_heap ? reinterpret_cast<char *>(out.heap) + at : reinterpret_cast<char *>(out.ranges) + (at - heap_bytes), k, true);
+        touched += k;
+        return true;
+    };
     uint32_t before = 0xffffffffu;  // the largest cell where the subtree kernel last refused
     for (;;) {
-        if (*sub_from < 0) return queue_tree(ctx, out);
+        if (*sub_from < 0) {
+            while (touch_some()) {
+            }
+            return queue_tree(ctx, out);
+        }
         ORB_CUDA(cudaMemcpyAsync(ctx->h_sub_flag, ctx->sub_flag.p, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                  ctx->stream));
-        orb_status st = queue_tree(ctx, out);  // (final when the subtree path was taken)
+        // small trees are copied behind the flag, final when the subtree path was taken; larger ones
+        // once that is known (168 MB of a refused tree made resident and copied before the second
+        // graph: 5.5 ms of device time for 2.6 ms of kernels)
+        orb_status st = out.staged ? queue_tree(ctx, out) : ORB_OK;
         if (st != ORB_OK) return st;
+        while (cudaStreamQuery(ctx->stream) == cudaErrorNotReady) {
+            cudaGetLastError();
+            if (!touch_some()) break;
+        }
         ORB_CUDA(cudaStreamSynchronize(ctx->stream));
-        if (ctx->h_sub_flag[0] == 1u) return ORB_OK;
+        if (ctx->h_sub_flag[0] == 1u) {
+            while (touch_some()) {
+            }
+            return out.staged ? ORB_OK : queue_tree(ctx, out);
+        }
         if (ctx->use_graphs) collect_graph_profile(ctx);  // the graph's kernel events
         const size_t at = (size_t)*sub_from;
         const uint32_t largest = ctx->h_sub_flag[1];

@@ -88,3 +88,24 @@ def test_odd_leaf_counts_are_not_refused(fresh, oracle, n, d):
     p = fresh.profile()
     assert "plan" not in p  # launched by a second graph alone
     assert p.get("subtree", {"launches": 0})["launches"] <= 1
+
+
+def test_a_refused_tree_is_copied_once(fresh):
+    """A tree of more than 1 MiB whose subtree level is refused: its cells are copied to the host when
+    the tree is done, not before as well (with 10 of 20 levels built, the copy was half of the
+    build's time)."""
+    torch = pytest.importorskip("torch")
+    n, d = 1 << 22, 1_407_823
+    src = [torch.from_numpy(a).cuda() for a in sites(n, 400, 5)]
+
+    def ms(most):
+        fresh.set_tuning(subtree_levels=most)
+        times = []
+        for _ in range(6):
+            dev = [s.clone() for s in src]
+            torch.cuda.synchronize()
+            times.append(fresh.build(*dev, d, levels=9, perm=None, device_pointers=True).info["device_ms"])
+        return min(times[2:])
+
+    refused, without = ms(6), ms(0)
+    assert refused < without + 0.4
