@@ -215,7 +215,16 @@ void touch_pages(void *ptr, size_t bytes, bool meanwhile) {
     const uintptr_t e = (reinterpret_cast<uintptr_t>(ptr) + bytes + page - 1) / page * page;
     constexpr int kPopulateWrite = 23;  // MADV_POPULATE_WRITE (Linux 5.14)
     const int saved = errno;
-    if (madvise(reinterpret_cast<void *>(a), e - a, kPopulateWrite) != 0) errno = saved;
+    // (looked at first: a store of 2^22 particles into resident pages 424 -> 403 us, 390 without either)
+    unsigned char in[4096];
+    bool resident = true;
+    for (uintptr_t q = a; resident && q < e; q += sizeof in * page) {
+        const size_t k = std::min<size_t>(sizeof in, (e - q) / page);
+        resident = mincore(reinterpret_cast<void *>(q), k * page, in) == 0;
+        for (size_t i = 0; resident && i < k; ++i) resident = in[i] & 1;
+    }
+    if (!resident) madvise(reinterpret_cast<void *>(a), e - a, kPopulateWrite);
+    errno = saved;
 }
 }  // namespace orb
 
