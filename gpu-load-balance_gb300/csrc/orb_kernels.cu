@@ -3874,10 +3874,17 @@ __global__ void __launch_bounds__(kThreads, 4) k_whist(const __grid_constant__ L
     const uint32_t tid = threadIdx.x;
     const uint32_t piece = (uint32_t)kTile / pieces;  // keys of a piece; `pieces` of them a tile
     unsigned long long bytes = 0;
+    // A run of consecutive tiles a CTA, so that a cell's bins go to global memory once a run; where
+    // most cells have one tile but not all, tiles apart: the few larger cells' tiles, next to each
+    // other in the plan and with up to hundreds of times as many keys, go to as many CTAs. (Half of
+    // 6.4 million particles on one point, 2^14 leaves: passes two and three of the last level 767 and
+    // 1197 us in runs, 82 and 122 apart. Levels of one-tile cells alone are 2% faster in runs.)
+    const uint64_t total = (v.tot->tiles >> 32) * pieces;
+    const bool apart = pieces == 1 && total != (uint64_t)v.C && 2 * total <= 3 * (uint64_t)v.C;
+    const uint32_t t_step = apart ? gridDim.x : 1u;
     if (tid == 0) {
-        const uint64_t total = (v.tot->tiles >> 32) * pieces;
-        sm.run[0] = (uint32_t)(total * blockIdx.x / gridDim.x);
-        sm.run[1] = (uint32_t)(total * (blockIdx.x + 1) / gridDim.x);
+        sm.run[0] = apart ? blockIdx.x : (uint32_t)(total * blockIdx.x / gridDim.x);
+        sm.run[1] = apart ? (uint32_t)total : (uint32_t)(total * (blockIdx.x + 1) / gridDim.x);
     }
     __syncthreads();
     const uint32_t t_end = sm.run[1];
@@ -4051,7 +4058,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_whist(const __grid_constant__ L
         flushed = false;
     };
     int skip_c = -1;  // an inactive cell whose tiles are being passed over
-    for (uint32_t t = sm.run[0]; t < t_end; ++t) {
+    for (uint32_t t = sm.run[0]; t < t_end; t += t_step) {
         const int c = (int)v.htile_cell[t / pieces];
         if (c == skip_c) continue;
         if (c != cur) {
