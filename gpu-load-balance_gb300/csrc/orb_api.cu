@@ -66,6 +66,8 @@ struct DevBuf {
 
 }  // namespace
 
+constexpr uint32_t kWindowsBySize = 0xffffffffu;  // orb_ctx::e2e_windows: as many as pay (windows_for)
+
 struct orb_ctx {
     int device = 0;
     int num_sms = 0;
@@ -160,7 +162,7 @@ struct orb_ctx {
     std::vector<Graph *> ran;  // graphs replayed since their profiles were last read
     static constexpr size_t kMaxGraphs = 256;
     // window reports of the subtree kernel (builds from host memory): pinned and mapped
-    uint32_t e2e_windows = 16;  // ORB_E2E_WINDOWS (0: the particles are copied back after the build)
+    uint32_t e2e_windows = kWindowsBySize;  // ORB_E2E_WINDOWS (0: the particles are copied back after the build)
     HostWindows *h_win = nullptr, *d_win = nullptr;
     DevBuf<uint32_t> win_cnt;
 };
@@ -1039,6 +1041,17 @@ orb_status orb_build_weighted(orb_ctx *ctx, float *x, float *y, float *z, uint32
     return st;
 }
 
+// Windows in which a build from host memory copies its particles back while its last levels are
+// built: each of at least 2^23 particles, at most 16, none of its own for less than two. A copy costs
+// the host 10 us an array from ordinary memory, 3 from page-locked: with 16 windows a build of 2^19
+// particles took 928 us instead of 517 (523 and 439 page-locked), one of 2^22 1780 instead of 1378
+// (1190, 1095); at 2^24 0, 2 and 16 windows take 4385, 4245 and 4563 us (3812, 3639, 3640), at 2^27
+// 30.6, 29.4 and 28.6 ms (27.8, 26.5, 25.4).
+static uint32_t windows_for(uint64_t n) {
+    const uint64_t m = n >> 23;
+    return m < 2 ? 0u : (uint32_t)std::min<uint64_t>(m, 16);
+}
+
 static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint32_t *w,
                                bool weighted, uint64_t n, uint32_t d, uint32_t levels,
                                const float lower[3], const float upper[3], orb_cell_t *heap,
@@ -1173,12 +1186,13 @@ static orb_status build_single(orb_ctx *ctx, float *x, float *y, float *z, uint3
     // window reports (builds from host memory that plan subtrees): the subtree kernel reports
     // each window of consecutive root cells once all of them are final, and the host copies
     // that window back while the kernel builds the next ones
-    const bool windows = !dev && n && !weighted && sub_from >= 0 && ctx->e2e_windows > 0;
+    const uint32_t want_windows = ctx->e2e_windows == kWindowsBySize ? windows_for(n) : ctx->e2e_windows;
+    const bool windows = !dev && n && !weighted && sub_from >= 0 && want_windows > 0;
     uint32_t nwin = 0;
     if (windows) {
         ORB_CUDA(ctx->win_cnt.ensure(kMaxWindows));
         const uint32_t cs = (uint32_t)lv[sub_from].C;
-        const uint32_t m = std::min<uint32_t>(ctx->e2e_windows, cs);
+        const uint32_t m = std::min<uint32_t>(want_windows, cs);
         v.hwin = ctx->d_win;
         v.win_cnt = ctx->win_cnt.p;
         v.win_cells = (cs + m - 1) / m;
