@@ -4109,6 +4109,77 @@ __global__ void __launch_bounds__(kThreads, 4) k_whist(const __grid_constant__ L
     if (tid == 0 && bytes) add_bytes(v, kKWHist, bytes);
 }
 
+// Weighted cells of at most 256 keys by a warp each, the whole loop, on levels of such cells on
+// average (then k_whist finds the larger ones, if any). A CTA a cell with a barrier a step took 17 us
+// a cell of many equal keys: 340783 particles on 1000 points into 2^16 leaves, the last level's 32768
+// cells 1046 us; 121 here and 50 for k_whist to pass them over. (As an instance of k_whist with a warp
+// a cell 357, and the other instances' registers suffered: 0.6% of 16 million particles.)
+constexpr int kWWarpKeys = 256;
+__global__ void __launch_bounds__(kThreads, kTileBlocksPerSm) k_wbisect_tile(const __grid_constant__ Level v) {
+    pdl_enter();
+    if (level_failed(v)) return;
+    const uint32_t lane = threadIdx.x & 31;
+    const int nwarps = (int)(gridDim.x * (blockDim.x >> 5));
+    for (int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); c < v.C; c += nwarps) {
+        if (v.state[c] != kActive) continue;
+        const int slot = level_slot(v, c);
+        const uint2 rg = v.ranges[slot];
+        const uint32_t n = rg.y - rg.x;
+        if (n > (uint32_t)kWWarpKeys) continue;
+        orb_cell_t &cell = v.heap[slot];
+        const float *keys = axis_keys(v, eff_axis(cell.cutAxis));
+        constexpr int kPer = kWWarpKeys / 32;
+        float k[kPer], L = cell.cutMarginLeft, R = cell.cutMarginRight;
+        uint32_t x[kPer];
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const uint32_t p = (uint32_t)j * 32u + lane;
+            k[j] = p < n ? __ldg(keys + rg.x + p) : __int_as_float(0x7fc00000);  // NaN: never below
+            x[j] = p < n ? __ldg(v.wt + rg.x + p) : 0u;
+        }
+        auto below = [&](float cut, bool all) -> unsigned long long {
+            uint32_t lo = 0, hi = 0;
+#pragma unroll
+            for (int j = 0; j < kPer; ++j) {
+                const uint32_t y = all || k[j] < cut ? x[j] : 0u;
+                lo += y & 0xffffu;
+                hi += y >> 16;
+            }
+            return (unsigned long long)__reduce_add_sync(0xffffffffu, lo) +
+                   ((unsigned long long)__reduce_add_sync(0xffffffffu, hi) << 16);
+        };
+        const WeightTest test(below(0.f, true), n, cell.nLeafCells);
+        uint32_t it = 0;
+        uint8_t st = kActive;
+        while (st == kActive) {
+            if (it >= (uint32_t)kMaxIterations) {
+                st = kCapped;
+                break;
+            }
+            const float cut = mid_cut(L, R);
+            ++it;
+            const int dir = test.dir(below(cut, false));
+            if (dir == 0)
+                st = kFound;
+            else if (dir > 0)
+                R = cut;
+            else
+                L = cut;
+        }
+        __syncwarp();
+        if (lane == 0) {
+            cell.cutMarginLeft = L;
+            cell.cutMarginRight = R;
+            cell.foundCut = st == kFound ? 1 : 0;
+            v.iters[c] = (uint8_t)it;
+            v.state[c] = st;
+            atomicMax(&v.counters->max_iters, it);
+            if (st == kCapped) atomicAdd(&v.counters->unfound, 1u);
+            add_bytes(v, kKBisectTile, 8ull * n);
+        }
+    }
+}
+
 // ------------------------------------------------------------------------------------
 // Service count-left: one plain pass at getCut() per cell, found cells skipped.
 // ------------------------------------------------------------------------------------
@@ -4393,7 +4464,7 @@ void launch_level_kernel(Kernel k, const Level &v, int grid, int arg, cudaStream
             else
                 launch_kernel(p, arg ? k_hist<kHFirstDense, kThreads> : k_hist<kHRest, kThreads>, dim3(grid), T, 0, st, v);
             break;
-        case kKBisectTile: launch_kernel(p, k_bisect_tile, dim3(grid), T, 0, st, v); break;
+        case kKBisectTile: launch_kernel(p, v.wt ? k_wbisect_tile : k_bisect_tile, dim3(grid), T, 0, st, v); break;
         case kKSubtreeCheck: launch_kernel(p, k_subtree_check, dim3(1), dim3(1024), 0, st, v, arg); break;
         case kKSubtree: launch_kernel(p, k_subtree, dim3(grid), dim3(kSubThreads), kSubBytes, st, v); break;
         case kKBisectCta:

@@ -44,3 +44,13 @@ def test_many_small_cells_beside_a_large_one_are_not_slow(engine):
 
         fine, coarse = ms(1 << 14), ms(1 << 9)
         assert fine < 2.6 * coarse, (fine, coarse)
+
+
+@pytest.mark.parametrize("n,d", [(256, 2), (257, 2), (512 * 256, 512), (512 * 256 + 900, 512), (60_000, 1 << 13), (60_000, 1 << 16)])
+def test_cells_a_warp_holds_match_oracle(ctx, oracle, n, d):
+    """Cells of at most 256 keys (every warp holds all of them) and of a few more, many equal keys,
+    weights whose 16-bit halves fill."""
+    for share, points, wmax in ((0.0, 1, 50), (0.8, 500, 1 << 32), (1.0, 37, 65_537)):
+        x, y, z = lump(n, share, points, n)
+        w = np.random.default_rng(n).integers(0, wmax, n, dtype=np.uint64).astype(np.uint32)
+        check(ctx, oracle, x, y, z, w, d)
