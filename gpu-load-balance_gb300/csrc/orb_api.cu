@@ -688,6 +688,7 @@ orb_status run_levels(orb_ctx *ctx, Level v, const std::vector<LevelDesc> &lv, u
             const int pieces = v.C <= ctx->num_sms ? 4 : 1;
             const uint64_t tiles = (n / kTile + (uint64_t)v.C) * pieces;
             v.last_pass = kWPasses - 1;
+            v.few_tiles = (max_n >> li) <= 1024;
             if ((max_n >> li) <= 256)  // cells of a warp's keys
                 run_kernel(ctx, kKBisectTile, v, std::min(v.C, ctx->num_sms * (int)ctx->tune.tile_blocks_per_sm));
             for (int pass = 0; pass < kWPasses; ++pass) {

@@ -152,6 +152,7 @@ struct Level {
     uint32_t small_next;
     uint32_t small;         // ... on this level (k_plan, k_init)
     int wide;               // 1: the box reaches 2^127, where midpoints overflow
+    int few_tiles;          // weighted, 1: cells of at most 1024 keys on average
     uint32_t hist_threads;  // threads of a count pass's CTA (kThreads, 512 or 1024)
     uint32_t plan_bins;     // cells with count tiles get a list and, with several tiles, bins (1);
                             // bins for all (2); neither (0)

@@ -3698,7 +3698,7 @@ struct WeightSmem {
     unsigned long long red[kThreads / 32];
     uint32_t sum[2][2][kThreads / 32];  // direct sums by parity of the step: halves, a warp each
     WeightCell cell;
-    uint32_t run[2];
+    uint32_t run[2], next;
 };
 
 // Replay of up to K iterations on the finished bins of cell c (in shared memory, or added up
@@ -3863,7 +3863,52 @@ __device__ __noinline__ void weighted_direct(const Level &v, int c, WeightSmem &
     __syncthreads();
 }
 
-template <bool kWide>
+// A later pass's round that leaves a warp many keys in the bracket, mostly equal ones (see
+// bracket_tile): bits `in` of its lanes' keys at p0, p0 + kThreads, ...; 32 at a time, the first
+// one's bin found once and its equals' weights added together. (A tile of equal keys took 85 us,
+// two additions to the same words a key; half of 6.4 million particles on one point, 2^14 leaves,
+// whose large cell's tiles are a few CTAs' runs among small cells: 7.1 -> 4.6 ms.)
+__device__ __noinline__ void tied_weights(const uint32_t *wt, uint32_t p0, uint32_t in, WeightSmem &sm) {
+    const uint32_t lane = threadIdx.x & 31u, top = (1u << sm.cell.K) - 1u;
+    const float *keys = sm.cell.keys;
+    float tie = __int_as_float(0x7fc00000);
+    uint32_t bin = 0;
+    auto bin_of = [&](float k) -> uint32_t {
+        uint32_t b;
+        return guess_bin(sm.cell.gs, k, &b) ? b : near_bin(k, sm.cell.gs, sm.edge, top);
+    };
+#pragma unroll 1
+    for (uint32_t any = __reduce_or_sync(0xffffffffu, in); any; any &= any - 1u) {
+        const uint32_t u = (uint32_t)__ffs(any) - 1u, p = p0 + u * kThreads;
+        const bool mine = (in >> u) & 1u;
+        const uint32_t first = (uint32_t)__ffs(__ballot_sync(0xffffffffu, mine)) - 1u;
+        const float k = mine ? __ldg(keys + p) : 0.0f;
+        const uint32_t y = mine ? __ldg(wt + p) : 0u;
+        const float t = __shfl_sync(0xffffffffu, k, (int)first);
+        if (t != tie) bin = bin_of(t);
+        tie = t;
+        const bool same = mine && k == t;
+        const uint32_t lo = __reduce_add_sync(0xffffffffu, same ? y & 0xffffu : 0u);
+        const uint32_t hi = __reduce_add_sync(0xffffffffu, same ? y >> 16 : 0u);
+        if (lane == first) {
+            atomicAdd(&sm.half[0][bin], lo);
+            if (hi) atomicAdd(&sm.half[1][bin], hi);
+        } else if (mine && !same && y) {
+            const uint32_t b = bin_of(k);
+            atomicAdd(&sm.half[0][b], y & 0xffffu);
+            if (y >> 16) atomicAdd(&sm.half[1][b], y >> 16);
+        }
+    }
+}
+
+// A run of consecutive tiles a CTA, so that a cell's bins go to global memory once a run and a cell of
+// several tiles ends in its CTA's first pass (apart, 2^26 particles into 2^16 leaves took 2% longer).
+// kFew: levels of cells of at most 1024 keys on average. If some have several tiles all the same,
+// these, next to each other in the plan and with many times the keys, would be a few CTAs' runs: the
+// tiles are dealt apart, and those of cells that are done passed over a CTA's width at a time. (Half
+// of 6.4 million particles on one point: 2^19 leaves 52.1 ms in runs, 12.9 apart, 2^14 4.6 and 3.8. An
+// instance of its own: the choice at run time was 2 to 3% of 2^24 particles into 2^11 to 2^14 leaves.)
+template <bool kWide, bool kFew>
 __global__ void __launch_bounds__(kThreads, 4) k_whist(const __grid_constant__ Level v, uint32_t pieces) {
     pdl_enter();
     __shared__ WeightSmem sm;
@@ -3874,14 +3919,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_whist(const __grid_constant__ L
     const uint32_t tid = threadIdx.x;
     const uint32_t piece = (uint32_t)kTile / pieces;  // keys of a piece; `pieces` of them a tile
     unsigned long long bytes = 0;
-    // A run of consecutive tiles a CTA, so that a cell's bins go to global memory once a run; where
-    // most cells have one tile but not all, tiles apart: the few larger cells' tiles, next to each
-    // other in the plan and with up to hundreds of times as many keys, go to as many CTAs. (Half of
-    // 6.4 million particles on one point, 2^14 leaves: passes two and three of the last level 767 and
-    // 1197 us in runs, 82 and 122 apart. Levels of one-tile cells alone are 2% faster in runs.)
     const uint64_t total = (v.tot->tiles >> 32) * pieces;
-    const bool apart = pieces == 1 && total != (uint64_t)v.C && 2 * total <= 3 * (uint64_t)v.C;
-    const uint32_t t_step = apart ? gridDim.x : 1u;
+    const bool apart = kFew && total != (uint64_t)v.C * pieces;
     if (tid == 0) {
         sm.run[0] = apart ? blockIdx.x : (uint32_t)(total * blockIdx.x / gridDim.x);
         sm.run[1] = apart ? (uint32_t)total : (uint32_t)(total * (blockIdx.x + 1) / gridDim.x);
@@ -3933,6 +3972,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_whist(const __grid_constant__ L
                 uint32_t in = 0;
 #pragma unroll
                 for (int u = 0; u < kLoads; ++u) in |= (uint32_t)(k[u] >= L && k[u] < R) << u;
+                if (p0 - tid + kThreads * kLoads <= e1 &&  // (a whole round: every lane is here)
+                    __reduce_add_sync(0xffffffffu, (uint32_t)__popc(in)) > kTies) {
+                    tied_weights(v.wt, p0, in, sm);
+                    continue;
+                }
                 for (; in; in &= in - 1u) {
                     const uint32_t p = p0 + ((uint32_t)__ffs(in) - 1u) * kThreads, y = __ldg(v.wt + p);
                     if (y) add(__ldg(keys + p), y);
@@ -4058,13 +4102,24 @@ __global__ void __launch_bounds__(kThreads, 4) k_whist(const __grid_constant__ L
         flushed = false;
     };
     int skip_c = -1;  // an inactive cell whose tiles are being passed over
+    const uint32_t t_step = apart ? gridDim.x : 1u;
     for (uint32_t t = sm.run[0]; t < t_end; t += t_step) {
         const int c = (int)v.htile_cell[t / pieces];
         if (c == skip_c) continue;
         if (c != cur) {
             // a cell with a tile still to come is not resolved in this pass: its state stands
             if (v.state[c] != kActive) {
-                skip_c = c;
+                if (!kFew) {
+                    skip_c = c;
+                } else {  // on to this CTA's next tile of an active cell
+                    if (tid == 0) sm.next = t + kThreads * t_step;
+                    __syncthreads();
+                    const uint32_t u = t + (tid + 1u) * t_step;
+                    if (u < t_end && v.state[v.htile_cell[u / pieces]] == kActive) atomicMin(&sm.next, u);
+                    __syncthreads();
+                    t = sm.next - t_step;
+                    __syncthreads();
+                }
                 continue;
             }
             if (cur >= 0) end_cell();
@@ -4491,7 +4546,12 @@ void launch_level_kernel(Kernel k, const Level &v, int grid, int arg, cudaStream
             else
                 launch_kernel(p, k_part_finish<false>, dim3(per_cell_warps), T, 0, st, v, arg);
             break;
-        case kKWHist: launch_kernel(p, v.wide ? k_whist<true> : k_whist<false>, dim3(grid), T, 0, st, v, (uint32_t)arg); break;
+        case kKWHist: {
+            auto *k = v.few_tiles ? (v.wide ? k_whist<true, true> : k_whist<false, true>)
+                                   : (v.wide ? k_whist<true, false> : k_whist<false, false>);
+            launch_kernel(p, k, dim3(grid), T, 0, st, v, (uint32_t)arg);
+            break;
+        }
         case kKCountLeft: launch_kernel(p, k_count_left, dim3(grid), T, 0, st, v); break;
         case kKSample:
             launch_kernel(p, k_sample_bin, dim3(kSampleMax / kSamplePerCta, (unsigned)min(v.C, 65535)),

@@ -1,6 +1,5 @@
-"""Weighted levels where most cells have one tile and a few have many (particles on a few points):
-their tiles are dealt to the CTAs apart from each other. Bit for bit against the oracle, and not
-slower by the number of small cells."""
+"""Weighted levels where most cells have one tile and a few have many (particles on a few points).
+Bit for bit against the oracle, and not slower by the number of small cells."""
 import numpy as np
 import pytest
 
@@ -19,7 +18,7 @@ def lump(n, share, points, seed):
 
 
 @pytest.mark.parametrize("share,points", [(0.5, 1), (0.9, 1), (0.3, 7), (1.0, 3)])
-@pytest.mark.parametrize("n,d", [(300_001, 1 << 9), (1 << 20, 1 << 12), (700_001, 3000)])
+@pytest.mark.parametrize("n,d", [(300_001, 1 << 9), (1 << 20, 1 << 12), (700_001, 3000), (300_001, 1 << 13), (200_000, 1 << 16)])
 def test_few_large_cells_match_oracle(ctx, oracle, n, d, share, points):
     x, y, z = lump(n, share, points, n + points)
     w = np.random.default_rng(n).integers(0, 1 << 18, n, dtype=np.uint64).astype(np.uint32)
